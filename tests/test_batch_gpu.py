@@ -47,3 +47,28 @@ def test_batch_tune_keeps_results(ecl, orc):
         assert np.array_equal(b.result(i, ecl.BATCH_CC), orc.cc(g))
         inm, tot = b.result(i, ecl.BATCH_MST)
         assert tot == orc.mst(g)[1]
+
+
+@pytest.mark.parametrize("sizes", [
+    [1, 2, 1, 2049, 1, 2048, 5000, 1, 1],  # pieces of 0, 1, 4094, 4096 and 9998 entries, cut inside and at a tile's end
+    [1, 1],  # no entries at all
+    [3] * 1500,  # many graphs in one tile
+    [40000, 2, 3],
+])
+def test_batch_mst_weights_at_tile_edges(ecl, orc, sizes):
+    b = ecl.Batch()
+    rng = np.random.default_rng(len(sizes))
+    for n in sizes:  # a path: every edge is in the forest
+        u = np.arange(n - 1)
+        ends = np.sort(np.concatenate([u * n + u + 1, (u + 1) * n + u]))
+        w = rng.integers(0, 1 << 30, size=max(n - 1, 1))
+        row, col = ends // n, ends % n
+        nindex = np.searchsorted(row, np.arange(n + 1)).astype(np.int32)
+        b.add(ecl.Graph(nindex, col.astype(np.int32), w[np.minimum(row, col)].astype(np.int32), symmetric=True))
+    b.build(ecl.BATCH_MST)
+    for _ in range(2):
+        b.run()
+        for i in range(0, b.graphs, max(1, b.graphs // 50)):
+            inm, tot = b.result(i, ecl.BATCH_MST)
+            einm, etot = orc.mst(b.graph(i))
+            assert tot == etot and np.array_equal(inm, einm), i
