@@ -25,7 +25,8 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* b, Status* status) {
     int ok = 1;
     const unsigned g = ld_acquire(&b->gen);
     __threadfence();
-    if (aref<unsigned>(b->count).fetch_add(1u, cuda::memory_order_acq_rel) == gridDim.x - 1) {
+    if (gridDim.x == 1) {  // the block barriers around this are the whole barrier
+    } else if (aref<unsigned>(b->count).fetch_add(1u, cuda::memory_order_acq_rel) == gridDim.x - 1) {
       st(&b->count, 0u);
       st_release(&b->gen, g + 1);
     } else {

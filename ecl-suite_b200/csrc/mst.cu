@@ -20,24 +20,15 @@
 //    reserved in the global list with one atomic per ~kStage entries;
 //    the heavy pass drops entries whose endpoints are already joined (the
 //    forest is flattened by pointer jumping first, so a root is one load);
-//  * mst_boruvka: ALL Boruvka rounds in one cooperative persistent launch
-//    (2 bounded grid barriers per round): phase A re-roots each edge, drops
-//    intra-component edges and atomicMin's its key into both roots; phase B
-//    joins every edge that is the minimum of one of its roots and flags it.
-//    Round 0 takes the scan's list as it stands (its entries already join
-//    two roots): it publishes the keys and joins along it without re-rooting
-//    or copying 10.6 M entries (heavy pass at R-MAT-22: 0.79 -> 0.74 ms).
-//    Per warp, every root is found, reset, loaded and min-published once
-//    (__match_any_sync groups), and per block every root of a large
-//    component once: a shared-memory table of roots takes the key minimums,
-//    serves phase B's key reads and ends phase A's finds without a load of
-//    the root's word.  Middle rounds give a few hundred large components most
-//    of the edges, and per-warp accesses to their words queue at their L2
-//    slices (R-MAT-22 light pass: 1.17 -> 0.96 ms).
-//    minv is double-buffered so its reset (a streaming pass over the
-//    vertices) rides along with phase A instead of costing a third barrier; per-round sizes live in a counter array, so
-//    no counter is ever reset concurrently with its use.
-#include <cooperative_groups.h>
+//  * mst_boruvka: ALL Boruvka rounds in one cooperative persistent launch, three
+//    phases a round with a bounded grid barrier after each: relabel the
+//    edges and lower both roots' keys, hook every root along its smallest
+//    edge, flatten the new trees.  Hooking writes one parent per root and
+//    flattening keeps every tree one level deep, so finding an edge's roots
+//    is one load each and no phase reads what it writes: the loads are plain
+//    ones that L1 serves.  Per-round sizes live in a counter array, so no
+//    counter is ever reset concurrently with its use.
+#include <algorithm>
 
 #include "csr_bins.cuh"
 #include "grid_sync.cuh"
@@ -58,16 +49,17 @@ constexpr int kSamples = 1024;
 
 struct MSTCtl {
   GridBarrier bar;
-  int wlcount[2][kMaxRounds + 2];  // [pass][round] sizes
+  int wlcount[2][kMaxRounds + 2];    // [pass][round] sizes of the edge list
+  int rootcount[2][kMaxRounds + 2];  // [pass][round] roots that may still have edges
   int nchunks;
   int threshold;
   int filter;
   int pad;
   u64 total;
   // %globaltimer when each pass started and after each of its barriers
-  // (phase A of round r ends at [2r + 1], phase B at [2r + 2]): a per-round
-  // time profile that costs one store per barrier.
-  u64 stamp[2][2 * kMaxRounds + 2];
+  // (phases A, B and C of round r end at [3r + 1], [3r + 2] and [3r + 3]): a
+  // per-round time profile that costs one store per barrier.
+  u64 stamp[2][3 * kMaxRounds + 2];
 };
 
 __device__ __forceinline__ u64 mst_now() {
@@ -76,42 +68,17 @@ __device__ __forceinline__ u64 mst_now() {
   return t;
 }
 
-__device__ __forceinline__ int mst_find(int v, int* parent) {
-  int cur = ld(&parent[v]);
-  if (cur == v) return v;
-  int prev = v, next;
-  while (cur != (next = ld(&parent[cur]))) {
-    st(&parent[prev], next);
-    prev = cur;
-    cur = next;
-  }
-  return cur;
-}
-
-__device__ __forceinline__ void mst_join(int a, int b, int* parent) {
-  while (true) {
-    a = mst_find(a, parent);
-    b = mst_find(b, parent);
-    if (a == b) return;
-    if (a < b) {
-      const int t = a;
-      a = b;
-      b = t;
-    }
-    if (cas(&parent[a], a, b) == a) return;
-  }
-}
-
 // parent[v] = root(v) between the passes, so the heavy scan reads each
 // entry's root with one load.  Pointer jumping: each thread rewrites only its
-// own parent[v] (parents point at smaller ids), stepping to the parent of its
-// current target, which its own thread is shortening at the same time.
+// own parent[v], stepping to the parent of its current target, which its own
+// thread is shortening at the same time (a vertex is a root iff it is its own
+// parent; hooks may point either way in the ids).
 __global__ void __launch_bounds__(kTPB) mst_flatten(int n, int* __restrict__ parent) {
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     int p = ld(&parent[v]);
     if (p == v) continue;
     int pp;
-    while ((pp = ld(&parent[p])) < p) {
+    while ((pp = ld(&parent[p])) != p) {
       st(&parent[v], pp);
       p = pp;
     }
@@ -123,7 +90,6 @@ __global__ void mst_init(int n, int* __restrict__ parent, u64* __restrict__ minv
     // race-free: thread-owned init, no reader in this launch
     parent[v] = v;
     minv[v] = ~0ull;
-    minv[n + v] = ~0ull;
   }
 }
 
@@ -408,37 +374,28 @@ __global__ void __launch_bounds__(kTPB) mst_chunks(int n, int m, const int* __re
   mst_overflow(overflow, status);
 }
 
-// Lowers mcur[root] to the smallest (weight << 32 | j) key among the lanes
-// of the warp that hold `root` and keep their edge: one atomic per root per
-// warp.  Late rounds give one giant component most of the edges, and an
-// atomic (or load) per edge on its root would queue at one L2 slice.  All
-// lanes call.
-// One-entry memo of a per-thread lookup (key -> value); key -1 = empty.
-struct MstMemo {
-  int key = -1;
-  u64 val = 0;
-};
+// A block's table of component roots (open addressing, kRootProbes probes)
+// with the smallest key the block has for each.  Once a few hundred large
+// components hold most of the edges, every thread of the grid publishes to
+// the same few hundred key words, and a first touch of such a word by all of
+// them queues at its L2 slice.  The table lowers a root's key in shared
+// memory and publishes it with one atomic per block and round; a root whose
+// probes meet only other roots goes to global memory directly, and so do all
+// roots of a block whose first step finds few roots twice (most components
+// still small: a table entry would then serve one edge).
+constexpr int kBorTPB = 1024;    // one block a SM: 148 tables to publish, and 148 arrivals a barrier
+constexpr int kBorBatch = 4;     // entries a thread keeps in flight
+constexpr int kRootSlots = 2048;
+constexpr int kRootProbes = 2;
+constexpr size_t kBorSmem =
+    sizeof(int4) * (kBorTPB / 32) * kStage + kRootSlots * (sizeof(u64) + sizeof(int)) + (kBorTPB / 32) * kStage * sizeof(int);
 
 template <typename T>
 using bref = cuda::atomic_ref<T, cuda::thread_scope_block>;
 
-// A block's table of component roots (open addressing, kRootProbes probes)
-// with the smallest key the block has for each.  Once a few hundred large
-// components hold most of the edges (R-MAT-22's light pass has ~250 in its
-// fourth round), every warp of the grid publishes to and reads the same few
-// hundred key words, and their L2 slices serialise the traffic: sending every
-// atomic there instead of loading first makes the pass 35 % slower.  The
-// table lowers a root's key in shared memory, publishes it with one atomic
-// per block, and serves phase B's reads of it from shared memory.  A root
-// whose probes meet only other roots goes to global memory directly.
-constexpr int kRootSlots = 1024;
-constexpr int kRootProbes = 4;
-
 struct RootTable {
   int* root;  // kRootSlots entries, -1 = empty
   u64* key;
-
-  __device__ static int first_slot(int r) { return (int)(((unsigned)r * 2654435761u) >> 22); }
 
   // All threads of the block call, between block barriers.
   __device__ void reset() {
@@ -447,154 +404,129 @@ struct RootTable {
       key[i] = ~0ull;
     }
   }
-  // Slot of r, claimed if r is absent and a probed slot is free; -1 if not.
-  __device__ int claim(int r) {
-    int h = first_slot(r);
+  // Lowers r's key in the table; false when r has no slot (the caller then
+  // publishes it).  *seen: r had a slot already.
+  __device__ bool lower(int r, u64 k, bool* seen) {
+    int h = (int)(((unsigned)r * 2654435761u) >> 21);
+    static_assert(kRootSlots == 1 << (32 - 21), "the slot is the hash's top bits");
     for (int p = 0; p < kRootProbes; p++, h = (h + 1) & (kRootSlots - 1)) {
       int c = bref<int>(root[h]).load(cuda::memory_order_relaxed);
-      if (c == -1 && bref<int>(root[h]).compare_exchange_strong(c, r, cuda::memory_order_relaxed)) return h;
-      if (c == r) return h;
-    }
-    return -1;
-  }
-  // Whether r has a slot, while claims may run (phase A).
-  __device__ bool has(int r) const {
-    int h = first_slot(r);
-    for (int p = 0; p < kRootProbes; p++, h = (h + 1) & (kRootSlots - 1)) {
-      const int c = bref<int>(root[h]).load(cuda::memory_order_relaxed);
-      if (c == r) return true;
-      if (c == -1) return false;
+      const bool mine = c == -1 && bref<int>(root[h]).compare_exchange_strong(c, r, cuda::memory_order_relaxed);
+      if (mine || c == r) {
+        *seen = !mine;
+        if (bref<u64>(key[h]).load(cuda::memory_order_relaxed) > k)
+          bref<u64>(key[h]).fetch_min(k, cuda::memory_order_relaxed);
+        return true;
+      }
     }
     return false;
   }
-  // Slot of r, or -1 (read-only phase: no claims run).
-  __device__ int find(int r) const {
-    int h = first_slot(r);
-    for (int p = 0; p < kRootProbes; p++, h = (h + 1) & (kRootSlots - 1)) {
-      const int c = root[h];  // race-free: no claim runs while find() does
-      if (c == r) return h;
-      if (c == -1) return -1;
-    }
-    return -1;
-  }
 };
 
-// Root of v during phase A.  Only roots are ever published, and no join runs
-// in phase A, so a vertex in the block's table is a root of this round: the
-// walk stops there without loading that root's word, which every find in a
-// large component would otherwise end on.
-__device__ __forceinline__ int mst_find_a(int v, int* parent, const RootTable& tab) {
-  if (tab.has(v)) return v;
-  int cur = ld(&parent[v]);
-  if (cur == v || tab.has(cur)) return cur;
-  int prev = v, next;
-  while (cur != (next = ld(&parent[cur]))) {
-    st(&parent[prev], next);
-    prev = cur;
-    cur = next;
-    if (tab.has(cur)) break;
-  }
-  return cur;
-}
-
-// ... and the calling thread remembers the last root it published to with
-// the smallest key it has seen there (a key word only decreases), so a giant
-// root met again in the next iterations costs no load.  Roots that get a
-// slot in the block's table are lowered there instead.
-__device__ __forceinline__ void mst_publish(u64* mcur, int root, bool keep, int w, int j, int lane, MstMemo& memo,
-                                            RootTable& tab) {
-  const unsigned g = __match_any_sync(kFull, keep ? root : -1);
-  const unsigned wmin = __reduce_min_sync(g, keep ? (unsigned)w : 0xffffffffu);
-  const unsigned jmin = __reduce_min_sync(g, (keep && (unsigned)w == wmin) ? (unsigned)j : 0xffffffffu);
-  if (keep && lane == __ffs(g) - 1) {
-    const u64 key = ((u64)wmin << 32) | jmin;
-    const int h = tab.claim(root);
-    if (h >= 0) {
-      bref<u64>(tab.key[h]).fetch_min(key, cuda::memory_order_relaxed);
-      return;
-    }
-    if (memo.key == root && memo.val <= key) return;
-    const u64 cur = ld(&mcur[root]);
-    if (cur > key) fetch_min(&mcur[root], key);
-    memo.key = root;
-    memo.val = cur < key ? cur : key;
-  }
-}
-
 // All Boruvka rounds of one pass.  wlA holds the pass's initial worklist
-// (size wlcount[pass][0]); rounds alternate wlA/wlB.
-__global__ void __launch_bounds__(kTPB) mst_boruvka(int n, int pass, int4* __restrict__ wlA, int4* __restrict__ wlB,
-                                                    int cap, int* __restrict__ parent, u64* __restrict__ minv,
-                                                    unsigned char* __restrict__ in_mst, MSTCtl* __restrict__ ctl,
-                                                    Status* __restrict__ status) {
-  const int tid = blockIdx.x * kTPB + threadIdx.x;
-  const int nthreads = gridDim.x * kTPB;
-  const int lane = threadIdx.x & 31;
+// (size wlcount[pass][0]), whose entries join two distinct roots; later rounds
+// alternate wlA / wlB.  A round has three phases, a grid barrier after each:
+//   A  relabels each entry's ends with one load each (the roots are flat),
+//      drops the entries inside one component, and lowers minv[root] of both
+//      ends to the entry's key.  Round 0 takes the list as it stands.
+//   B  hooks: the one entry that holds minv[a] sets parent[a] = b.  Keys are
+//      unique, so each root is written by one entry, and the only cycles are
+//      two roots that chose the same entry; the smaller of the two stays a root.
+//   C  flattens: every root that took part jumps to its component's new root
+//      and has its key word cleared; the new roots are listed for the next
+//      round (round 0 looks at all vertices instead of a list).
+// Only phase B writes what phase A reads and the other way round, so the loads
+// of parent[] in A and of minv[] in B are plain loads that the SM's L1 serves:
+// with a union-find walked by relaxed atomic loads, every entry of a middle
+// round ended its walk on the words of a few large components, and those L2
+// slices were the bound.  Bound now by the random loads and atomics of phase A
+// on the first two lists, and by three barriers a round on the short ones.
+// Measured, light + heavy pass: R-MAT-22 1.52 -> 0.78 ms, G(150 k, 600 k)
+// 0.89 -> 0.31 ms (its heavy pass 0.78 -> 0.22), 701 x 1031 grid 0.64 -> 0.34.
+__global__ void __launch_bounds__(kBorTPB, 1) mst_boruvka(int n, int pass, int4* __restrict__ wlA, int4* __restrict__ wlB,
+                                                          int cap, int* __restrict__ parent, u64* __restrict__ minv,
+                                                          int* __restrict__ rootsA, int* __restrict__ rootsB,
+                                                          unsigned char* __restrict__ in_mst, MSTCtl* __restrict__ ctl,
+                                                          Status* __restrict__ status) {
+  extern __shared__ __align__(16) unsigned char s_bor[];
+  __shared__ int s_seen;
+  const int tid = blockIdx.x * kBorTPB + threadIdx.x;
+  const int nthreads = gridDim.x * kBorTPB;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int* cnt = ctl->wlcount[pass];
-  __shared__ int4 stage_buf[kTPB / 32][kStage];
-  Stage stg{stage_buf[threadIdx.x >> 5]};
-  __shared__ int s_root[kRootSlots];
-  __shared__ u64 s_key[kRootSlots];
+  int* rcnt = ctl->rootcount[pass];
+  int4* stage_buf = reinterpret_cast<int4*>(s_bor);
+  u64* s_key = reinterpret_cast<u64*>(stage_buf + (kBorTPB / 32) * kStage);
+  int* s_root = reinterpret_cast<int*>(s_key + kRootSlots);
+  int* root_buf = s_root + kRootSlots;
+  Stage stg{stage_buf + wid * kStage};
+  WarpStage<int, kStage> rstg{root_buf + wid * kStage};
   RootTable tab{s_root, s_key};
   bool overflow = false;
   u64 local = 0;
   int r = 0;
   if (tid == 0) ctl->stamp[pass][0] = mst_now();
   for (; r < kMaxRounds; r++) {
-    // Round 0's list comes from a scan: its entries already join two
-    // distinct roots, so round 0 only publishes their keys and joins along
-    // the same list (no re-rooting, no copy); round r >= 1 re-roots the list
-    // round r - 1 left (wlA for r = 1) into the other buffer.
     int4* in = (r == 0 || (r & 1)) ? wlA : wlB;
     int4* out = r == 0 ? wlA : ((r & 1) ? wlB : wlA);
-    u64* mcur = minv + (size_t)(r & 1) * n;
-    u64* mprev = minv + (size_t)((r + 1) & 1) * n;
     // a scan that overflowed (reported as BAD_GRAPH) counted more entries
     // than the list holds
     const int sz = min(ld(&cnt[r]), cap);
-    // phase A: re-root, drop intra-component edges, publish keys.  The trip
-    // count is uniform across the grid so every warp step is converged for
-    // the warp-aggregated append.
-    // clear the keys round r-1 published: a streaming pass over all
-    // vertices (a reset per edge would store to the giant component's word
-    // from every warp)
-    if (r > 0)
-      for (int v = tid; v < n; v += nthreads) st(&mprev[v], ~0ull);
-    tab.reset();  // the last phase B's reads ended at its grid barrier
+    if (sz == 0) break;  // the same for every thread: no phase writes cnt[r] any more
+    // ---- A
+    tab.reset();
+    if (threadIdx.x == 0) s_seen = 0;
     __syncthreads();
-    const int iters = (sz + nthreads - 1) / nthreads;
-    // per-thread memos: roots cannot change during phase A (joins happen in
-    // phase B), so a remembered find is exact
-    MstMemo fx, fy, px, py;
-    // each step's entry is loaded one step ahead (the stream's latency then
-    // overlaps the previous step's finds and publishes)
-    int4 nx = tid < sz ? __ldcs(&in[tid]) : make_int4(-1, -1, 0, 0);
-    for (int it = 0; it < iters; it++) {
-      const int i = tid + it * nthreads;
-      const bool valid = i < sz;
-      const int4 e = nx;
-      const long long i1 = (long long)i + nthreads;
-      nx = i1 < sz ? __ldcs(&in[i1]) : make_int4(-1, -1, 0, 0);
-      // each lane finds its own entry's roots (a per-lane memo, and the
-      // block's table ends a find at a known root without a load): grouping
-      // equal endpoints per warp first measured slower
-      int ra = e.x, rb = e.y;  // round 0: the scan's entries hold roots
-      if (r > 0 && valid) {
-        if (fx.key != e.x) {
-          fx.key = e.x;
-          fx.val = (u64)mst_find_a(e.x, parent, tab);
+    bool use_tab = true;
+    const int step = nthreads * kBorBatch;
+    const int steps = (sz - 1) / step + 1;  // uniform over the grid: whole warps append together
+    for (int s = 0; s < steps; s++) {
+      // a warp's step takes kBorBatch slices of 32 consecutive entries
+      const long long i0 = (long long)s * step + (long long)(tid - lane) * kBorBatch + lane;
+      int4 e[kBorBatch];
+#pragma unroll
+      for (int k = 0; k < kBorBatch; k++) e[k] = i0 + 32 * k < sz ? __ldcs(&in[i0 + 32 * k]) : make_int4(-1, -1, 0, 0);
+      if (r > 0) {
+        int a[kBorBatch], b[kBorBatch];
+#pragma unroll
+        for (int k = 0; k < kBorBatch; k++) {
+          a[k] = e[k].x >= 0 ? parent[e[k].x] : -1;  // race-free: parent[] is not written in phase A
+          b[k] = e[k].x >= 0 ? parent[e[k].y] : -1;  // race-free: as above
         }
-        ra = (int)fx.val;
-        if (fy.key != e.y) {
-          fy.key = e.y;
-          fy.val = (u64)mst_find_a(e.y, parent, tab);
+#pragma unroll
+        for (int k = 0; k < kBorBatch; k++) {
+          e[k].x = a[k] != b[k] ? a[k] : -1;
+          e[k].y = b[k];
+          stg.push(e[k].x >= 0, e[k], out, &cnt[r + 1], cap, overflow);
         }
-        rb = (int)fy.val;
       }
-      const bool keep = valid && ra != rb;
-      if (r > 0) stg.push(keep, make_int4(ra, rb, e.z, e.w), out, &cnt[r + 1], cap, overflow);
-      mst_publish(mcur, ra, keep, e.z, e.w, lane, px, tab);
-      mst_publish(mcur, rb, keep, e.z, e.w, lane, py, tab);
+      int seen = 0;
+      unsigned direct = 0;
+#pragma unroll
+      for (int k = 0; k < 2 * kBorBatch; k++) {
+        const int4& x = e[k >> 1];
+        if (x.x < 0) continue;
+        bool had = false;
+        const u64 key = ((u64)(unsigned)x.z << 32) | (unsigned)x.w;
+        if (!use_tab || !tab.lower((k & 1) ? x.y : x.x, key, &had)) direct |= 1u << k;
+        seen += had;
+      }
+      u64 cur[2 * kBorBatch];
+#pragma unroll
+      for (int k = 0; k < 2 * kBorBatch; k++)
+        cur[k] = (direct >> k) & 1u ? ld(&minv[(k & 1) ? e[k >> 1].y : e[k >> 1].x]) : 0ull;
+#pragma unroll
+      for (int k = 0; k < 2 * kBorBatch; k++) {
+        const int4& x = e[k >> 1];
+        const u64 key = ((u64)(unsigned)x.z << 32) | (unsigned)x.w;
+        if (cur[k] > key) fetch_min(&minv[(k & 1) ? x.y : x.x], key);
+      }
+      if (s == 0 && steps > 1) {
+        seen = __reduce_add_sync(kFull, seen);
+        if (lane == 0) atomicAdd(&s_seen, seen);  // shared memory
+        __syncthreads();
+        use_tab = s_seen >= kBorTPB * kBorBatch / 2;  // a quarter of the ends or more had a slot
+      }
     }
     if (r > 0)
       stg.flush(out, &cnt[r + 1], cap, overflow);
@@ -602,74 +534,70 @@ __global__ void __launch_bounds__(kTPB) mst_boruvka(int n, int pass, int4* __res
       st(&cnt[1], sz);  // round 1 reads round 0's list, whole
     // publish the block's table: one load (and at most one atomic) per root
     __syncthreads();
-    for (int i = threadIdx.x; i < kRootSlots; i += kTPB) {
+    for (int i = threadIdx.x; i < kRootSlots; i += kBorTPB) {
       const int rt = s_root[i];  // race-free: claims ended at the barrier above
-      if (rt >= 0 && ld(&mcur[rt]) > s_key[i]) fetch_min(&mcur[rt], s_key[i]);
+      if (rt >= 0 && ld(&minv[rt]) > s_key[i]) fetch_min(&minv[rt], s_key[i]);
     }
     if (!grid_sync(&ctl->bar, status)) return;
-    if (tid == 0) ctl->stamp[pass][2 * r + 1] = mst_now();
+    if (tid == 0) ctl->stamp[pass][3 * r + 1] = mst_now();
     const int nsz = ld(&cnt[r + 1]);
     if (nsz == 0) break;
-    // phase B: join along every edge that is the minimum of one of its roots
-    // (each root's key is loaded once per warp, and key words do not change
-    // during phase B, so a per-thread memo of the last one is exact; the
-    // roots in the block's table once per block)
-    for (int i = threadIdx.x; i < kRootSlots; i += kTPB) {
-      const int rt = s_root[i];  // race-free: no claim runs after phase A
-      if (rt >= 0) s_key[i] = ld(&mcur[rt]);  // race-free: slot i is this thread's until the barrier below
-    }
-    __syncthreads();
-    MstMemo kxm, kym;
-    int4 nxb = tid < nsz ? __ldcs(&out[tid]) : make_int4(-1, -1, 0, 0);  // one step ahead, as in phase A
-    for (int i0 = tid - lane; i0 < nsz; i0 += nthreads) {
-      const int i = i0 + lane;
-      const bool valid = i < nsz;
-      const int4 e = nxb;
-      const long long i1 = (long long)i + nthreads;
-      nxb = i1 < nsz ? __ldcs(&out[i1]) : make_int4(-1, -1, 0, 0);
-      const unsigned gx = __match_any_sync(kFull, e.x), gy = __match_any_sync(kFull, e.y);
-      const int lx = __ffs(gx) - 1, ly = __ffs(gy) - 1;
-      u64 kx = 0, ky = 0;
-      if (valid && lane == lx) {
-        const int h = tab.find(e.x);
-        if (h >= 0) {
-          kx = s_key[h];  // race-free: read-only until the next round's reset
-        } else {
-          if (kxm.key != e.x) {
-            kxm.key = e.x;
-            kxm.val = ld(&mcur[e.x]);
-          }
-          kx = kxm.val;
-        }
+    // ---- B
+    for (long long i0 = tid; i0 < nsz; i0 += step) {
+      int4 e[kBorBatch];
+#pragma unroll
+      for (int k = 0; k < kBorBatch; k++) {
+        const long long i = i0 + (long long)k * nthreads;
+        e[k] = i < nsz ? __ldcs(&out[i]) : make_int4(-1, -1, 0, 0);
       }
-      if (valid && lane == ly) {
-        const int h = tab.find(e.y);
-        if (h >= 0) {
-          ky = s_key[h];  // race-free: as above
-        } else {
-          if (kym.key != e.y) {
-            kym.key = e.y;
-            kym.val = ld(&mcur[e.y]);
-          }
-          ky = kym.val;
-        }
+      u64 ka[kBorBatch], kb[kBorBatch];
+#pragma unroll
+      for (int k = 0; k < kBorBatch; k++) {
+        ka[k] = e[k].x >= 0 ? minv[e[k].x] : 0ull;  // race-free: minv[] is not written in phase B
+        kb[k] = e[k].x >= 0 ? minv[e[k].y] : 0ull;  // race-free: as above
       }
-      kx = __shfl_sync(kFull, kx, lx);
-      ky = __shfl_sync(kFull, ky, ly);
-      const u64 key = ((u64)(unsigned)e.z << 32) | (unsigned)e.w;
-      if (valid && (key == kx || key == ky)) {
-        mst_join(e.x, e.y, parent);
-        in_mst[e.w] = 1;  // race-free: each entry j is joined at most once, and never read here
-        local += (u64)(unsigned)e.z;
+#pragma unroll
+      for (int k = 0; k < kBorBatch; k++) {
+        const u64 key = ((u64)(unsigned)e[k].z << 32) | (unsigned)e[k].w;
+        const bool ha = e[k].x >= 0 && ka[k] == key, hb = e[k].x >= 0 && kb[k] == key;
+        if (!ha && !hb) continue;
+        if (ha && !(hb && e[k].x < e[k].y)) st(&parent[e[k].x], e[k].y);
+        if (hb && !(ha && e[k].y < e[k].x)) st(&parent[e[k].y], e[k].x);
+        in_mst[e[k].w] = 1;  // race-free: one entry j stands once in the list, and the flags are never read here
+        local += (u64)(unsigned)e[k].z;
       }
     }
     if (!grid_sync(&ctl->bar, status)) return;
-    if (tid == 0) ctl->stamp[pass][2 * r + 2] = mst_now();
+    if (tid == 0) ctl->stamp[pass][3 * r + 2] = mst_now();
+    // ---- C
+    const int* rin = (r & 1) ? rootsA : rootsB;
+    int* rout = (r & 1) ? rootsB : rootsA;
+    const int nr = r == 0 ? n : ld(&rcnt[r]);
+    for (long long i0 = tid - lane; i0 < nr; i0 += nthreads) {  // whole warps: they append together
+      const long long i = i0 + lane;
+      int v = -1;
+      if (i < nr) v = r == 0 ? (int)i : rin[i];
+      bool root = false;
+      if (v >= 0 && ld(&minv[v]) != ~0ull) {  // took part in this round
+        st(&minv[v], ~0ull);
+        int p = ld(&parent[v]);
+        root = p == v;
+        int pp;
+        while (!root && (pp = ld(&parent[p])) != p) {
+          st(&parent[v], pp);
+          p = pp;
+        }
+      }
+      rstg.push(root, v, rout, &rcnt[r + 1], n, overflow);
+    }
+    rstg.flush(rout, &rcnt[r + 1], n, overflow);
+    if (!grid_sync(&ctl->bar, status)) return;
+    if (tid == 0) ctl->stamp[pass][3 * r + 3] = mst_now();
   }
   if (r == kMaxRounds) raise(status, ECL_ERR_NO_CONVERGENCE, pass);
-  // per-block sum of the joined weights
+  // per-warp sum of the joined weights
   for (int o = 16; o > 0; o >>= 1) local += __shfl_down_sync(kFull, local, o);
-  if ((threadIdx.x & 31) == 0 && local) fetch_add(&ctl->total, local);
+  if (lane == 0 && local) fetch_add(&ctl->total, local);
   if (threadIdx.x == 0) fetch_max(&status->rounds, r + 1);
 }
 
@@ -677,6 +605,8 @@ struct MSTBufs {
   MSTCtl* ctl;
   int* parent;
   u64* minv;
+  int* rootsA;
+  int* rootsB;
   int2* chunks;
   int chunk_cap;
   int4* wlA;
@@ -687,7 +617,9 @@ struct MSTBufs {
 void mst_layout(Carve& c, int n, int m, bool symmetric, MSTBufs* b) {
   b->ctl = c.take<MSTCtl>(1);
   b->parent = c.take<int>((size_t)n);
-  b->minv = c.take<u64>((size_t)2 * n);
+  b->minv = c.take<u64>((size_t)n);
+  b->rootsA = c.take<int>((size_t)n);
+  b->rootsB = c.take<int>((size_t)n);
   b->chunks = c.take<int2>(row_chunk_capacity(m, kMinChunk));
   b->chunk_cap = (int)row_chunk_capacity(m, kMinChunk);
   // v<n entries: at most m/2 in a symmetric, self-loop-free graph, else m.
@@ -711,10 +643,11 @@ ecl_status mst_enqueue(const GraphDev& g, unsigned char* in_mst, char* ws, Statu
   Carve c{ws};
   MSTBufs b;
   mst_layout(c, g.n, g.m, sym, &b);
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mst_boruvka, kTPB, 0) != cudaSuccess || occ < 1)
-    return ECL_ERR_CUDA;
-  const int coop_grid = dev.sms * occ;
+  // One block of 1024 threads per SM, fewer for a graph that gives each less
+  // than 8 k vertices or entries: a barrier of few blocks is cheaper than the
+  // work it would spread (R-MAT with 1000 vertices and 12 k entries).
+  const int coop_grid = std::max(1, std::min(dev.sms, std::max(g.n, g.m) / 8192));
+  ECL_CUDA_TRY(cudaFuncSetAttribute(mst_boruvka, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBorSmem));
   const int grid = dev.grid_blocks(kTPB, g.n, g.m);
   const Bins bins = bins_of(dev, kMstBins);
   // 16-byte row loads need 16-byte-aligned arrays (entries j = 0 mod 4 then are)
@@ -742,8 +675,8 @@ ecl_status mst_enqueue(const GraphDev& g, unsigned char* in_mst, char* ws, Statu
                    b.ctl, b.chunks, b.chunk_cap, bins.chunk, vec, status);
       }
       mark();
-      ECL_CUDA_TRY(launch_cooperative(mst_boruvka, coop_grid, kTPB, stream, g.n, pass, b.wlA, b.wlB, b.cap, b.parent,
-                                      b.minv, in_mst, b.ctl, status));
+      ECL_CUDA_TRY(launch_cooperative_smem(mst_boruvka, coop_grid, kBorTPB, kBorSmem, stream, g.n, pass, b.wlA,
+                                           b.wlB, b.cap, b.parent, b.minv, b.rootsA, b.rootsB, in_mst, b.ctl, status));
       mark();
       // The heavy pass (pass 1) runs unconditionally: with no filter it finds
       // no entry above the INT_MAX threshold and ends after one round.

@@ -68,11 +68,12 @@ cudaError_t launch_cluster(void (*kernel)(KArgs...), int ctas, int block, size_t
 // the cooperative launch attribute, which stream capture turns into a
 // cooperative CUDA-graph kernel node.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_cooperative(void (*kernel)(KArgs...), int grid, int block, cudaStream_t stream, Args... args) {
+cudaError_t launch_cooperative_smem(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t stream,
+                                    Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -82,6 +83,11 @@ cudaError_t launch_cooperative(void (*kernel)(KArgs...), int grid, int block, cu
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
   count_launch();
   return e;
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_cooperative(void (*kernel)(KArgs...), int grid, int block, cudaStream_t stream, Args... args) {
+  return launch_cooperative_smem(kernel, grid, block, 0, stream, args...);
 }
 
 constexpr int kGridBlocksPerSm = 64;
