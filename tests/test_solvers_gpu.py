@@ -216,6 +216,29 @@ def test_apsp_reference_padded_layout(ecl, orc):
     assert np.all(out[100:, :] == ecl.APSP_INF) and np.all(out[:, 100:] == ecl.APSP_INF)
 
 
+# one tile and its edges, two tiles, the last size with one CTA per SM and the
+# first with two (tiles of 64: 20 blocks; tiles of 128: 26), the last size with
+# tiles of 64 and the first with tiles of 128
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 128, 130, 1280, 1281, 2687, 2688, 2689, 3328, 3329])
+def test_apsp_at_tile_edges(ecl, orc, n):
+    import torch
+
+    g = ecl.gen_er(n, min(0.5, 6.0 / n), seed=n, weight_seed=n + 1)
+    if g.edges == 0:
+        g.eweight = np.zeros(0, np.int32)
+    rows = np.unique(np.linspace(0, n - 1, 24).astype(np.int32))
+    exp = orc.apsp_rows(g, rows)
+    dg = g.to_device()
+    if dg.eweight is None or g.edges == 0:
+        dg.eweight = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = ecl.apsp(dg)
+    assert np.array_equal(got[torch.from_numpy(rows).long().cuda()].cpu().numpy(), exp)
+    # rows that start off the 16-byte boundaries: never computed in place
+    flat = torch.full((n * n + 1,), -7, dtype=torch.int32, device="cuda")
+    ecl.apsp(dg, out=flat[1:], ld=n)
+    assert int(flat[0]) == -7 and torch.equal(flat[1:].view(n, n), got)
+
+
 # ---------------------------------------------------------- malformed input and wait limits
 
 
