@@ -14,7 +14,7 @@
 //    list entry with one 8-byte key load and compact every row's
 //    higher-priority entries to the front of the row's slot in nl2[];
 //    hc[v] = their number.
-//  * radix_sort_pairs then ranks the vertices that have entries by priority
+//  * radix_order then ranks the vertices that have entries by priority
 //    (an LSD sort of their keys), which is a topological order of the
 //    colouring dependencies.
 //  * gc_pull is ONE cooperative persistent launch.  Ranks are dealt to the
@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "csr_bins.cuh"
+#include "grid_sync.cuh"
 #include "radix_sort.cuh"
 #include "solvers.cuh"
 
@@ -56,7 +57,10 @@ struct GCCtl {
   int nchunks;
   int nbig;        // rows longer than kWarpRow: a prefix of the priority order
   int nkeys;       // vertices with at least one entry: the ones sorted and pulled
-  int pad2[29];
+  int maxdeg;      // largest degree: how many digits of it the sort looks at
+  int sort_failed;  // the sort gave up: the order is not whole, and nothing is indexed by it
+  int pad2[27];
+  GridBarrier sort_bar;
 };
 
 // Priority hash of vertex x: the reference hashes the vertex id; in a union
@@ -218,12 +222,12 @@ __global__ void __launch_bounds__(kTPB) gc_keys(int n, const int* __restrict__ n
                                                 GCCtl* __restrict__ ctl) {
   // rows longer than kWarpRow are counted per block and added once per block;
   // the appends reserve their room with one atomic per block and step
-  __shared__ int s_big;
+  __shared__ int s_big, s_deg;
   __shared__ int s_woff[kTPB / 32];
   __shared__ int s_base;
-  if (threadIdx.x == 0) s_big = 0;
+  if (threadIdx.x == 0) s_big = s_deg = 0;
   __syncthreads();
-  int nb = 0;
+  int nb = 0, dmax = 0;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int bbase = blockIdx.x * kTPB; bbase < n; bbase += gridDim.x * kTPB) {  // block-uniform trip count
     const int i = bbase + threadIdx.x;
@@ -236,6 +240,7 @@ __global__ void __launch_bounds__(kTPB) gc_keys(int n, const int* __restrict__ n
       key = ~(((unsigned long long)deg << 32) | gc_h(vhash, v));
       keys[i] = key;
       big = deg > (unsigned)kWarpRow;
+      dmax = max(dmax, (int)min(deg, 0x7fffffffu));
       linked = deg > 0;
       if (!linked) color[v] = 0;  // race-free: the output, thread-owned; nothing reads it in this launch
     }
@@ -260,9 +265,16 @@ __global__ void __launch_bounds__(kTPB) gc_keys(int n, const int* __restrict__ n
     }
     __syncthreads();  // s_woff and s_base are rewritten next step
   }
-  if ((threadIdx.x & 31) == 0 && nb) atomicAdd(&s_big, nb);
+  dmax = __reduce_max_sync(kFull, dmax);
+  if (lane == 0) {
+    if (nb) atomicAdd(&s_big, nb);
+    atomicMax(&s_deg, dmax);
+  }
   __syncthreads();
-  if (threadIdx.x == 0 && s_big) fetch_add(&ctl->nbig, s_big);
+  if (threadIdx.x == 0) {
+    if (s_big) fetch_add(&ctl->nbig, s_big);
+    if (s_deg > ld(&ctl->maxdeg)) fetch_max(&ctl->maxdeg, s_deg);
+  }
 }
 
 __device__ __forceinline__ unsigned long long gc_now() {
@@ -502,7 +514,10 @@ static_assert(gc_core_segbuf(kCoreMax) >= 256 && gc_core_smem(kCoreMax) <= kCore
               "core shared memory over the per-block limit");
 
 // Core size of this solve: the long rows (a prefix of the order), at most cap.
-__device__ __forceinline__ int gc_core_size(const GCCtl* ctl, int cap) { return min(ld(&ctl->nbig), cap); }
+// None when the sort failed.
+__device__ __forceinline__ int gc_core_size(const GCCtl* ctl, int cap) {
+  return ld(&ctl->sort_failed) ? 0 : min(ld(&ctl->nbig), cap);
+}
 
 // rank[order[r]] = r over the core.
 __global__ void __launch_bounds__(kTPB) gc_core_rank(const int* __restrict__ order, int* __restrict__ rank,
@@ -902,6 +917,7 @@ __global__ void __launch_bounds__(kTPB) gc_pull(int n, const int* __restrict__ n
   const int lane = threadIdx.x & 31;
   unsigned* bits = s_bits[threadIdx.x >> 5];
   int* pend = s_pend[threadIdx.x >> 5];
+  if (ld(&ctl->sort_failed)) return;
   const int nbig = ld(&ctl->nbig);
   const int gwarp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -945,6 +961,7 @@ struct GCBufs {
   unsigned long long* keys1;
   int* vals0;
   int* vals1;
+  int* order;
   unsigned* sort_temp;
   unsigned* vhash;
   int2* chunks;
@@ -959,7 +976,8 @@ void gc_layout(Carve& c, int n, int m, GCBufs* b) {
   b->keys1 = c.take<unsigned long long>((size_t)n);
   b->vals0 = c.take<int>((size_t)n);
   b->vals1 = c.take<int>((size_t)n);
-  b->sort_temp = c.take<unsigned>(radix_temp_words((size_t)n));
+  b->order = c.take<int>((size_t)n);
+  b->sort_temp = c.take<unsigned>(kRadixTempWords);
   b->vhash = c.take<unsigned>((size_t)n);
   b->chunks = c.take<int2>(row_chunk_capacity(m, kMinChunk));
   b->rowinfo = c.take<int4>((size_t)std::min(n, kCoreMax));
@@ -995,9 +1013,6 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
   const int grid = dev.grid_blocks(kTPB, g.n, g.m);
   const RowChunks rc{b.chunks, &b.ctl->nchunks, (int)row_chunk_capacity(g.m, kMinChunk)};
   const Bins bins = bins_of(dev, Bins{kBinLane, kBinChunk});
-  // key bits that vary: 32 hash bits + enough bits for any degree <= m
-  int degbits = 1;
-  while (degbits < 31 && ((long long)1 << degbits) <= (long long)g.m) degbits++;
 
   if (cudaMemsetAsync(b.ctl, 0, sizeof(GCCtl), stream) != cudaSuccess) return ECL_ERR_CUDA;
   if (cudaMemsetAsync(color, 0xff, sizeof(int) * (size_t)g.n, stream) != cudaSuccess) return ECL_ERR_CUDA;
@@ -1015,9 +1030,10 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
   mark();
   // the nkeys appended pairs, sorted from (keys1, vals1); the per-vertex keys
   // in keys0 are dead once gc_init has run
-  const bool in0 = radix_sort_pairs(b.keys1, b.vals1, b.keys0, b.vals0, g.n, 0, 32 + degbits, b.sort_temp, stream,
-                                    &b.ctl->nkeys);
-  const int* order = in0 ? b.vals0 : b.vals1;
+  const ecl_status sorted = radix_order(b.keys1, b.vals1, b.keys0, b.vals0, b.order, g.n, &b.ctl->nkeys, &b.ctl->maxdeg,
+                                  b.sort_temp, &b.ctl->sort_bar, &b.ctl->sort_failed, dev, stream, status);
+  if (sorted != ECL_OK) return sorted;
+  const int* order = b.order;
   mark();
   // the hub core (the sort keys are dead now: their buffer holds the ranks)
   const int cap = std::min(std::min(dev.gc_core_ranks > 0 ? dev.gc_core_ranks : kCoreDefault, kCoreMax), g.n);

@@ -1,12 +1,10 @@
-// Stable LSD radix sort of (uint64 key, int32 value) pairs, 8-bit digits.
+// Stable LSD radix sort of (uint64 key, int32 value) pairs, 8-bit digits, in
+// ONE cooperative launch: the order of the values by key is all it returns.
 //
-// One pass = four launches: per-tile digit histograms, a per-digit-row scan
-// of the digit-major histogram table, a scan of the 256 row totals, and a
-// stable scatter.  The scatter
-// ranks keys inside a tile warp by warp (warp w of a tile takes the w-th
-// slice of it): __match_any_sync groups the lanes holding the same digit, a
-// shared-memory table gives every warp its base per digit, so equal digits
-// keep their input order and the sort is stable.
+// Keys are ~((d << 32) | h) with 32 varying bits h and a count d whose largest
+// value is known on the device only: the passes are the four over h and those
+// that the largest d needs (one below 256), so the pass count is decided
+// inside the launch and costs the host nothing.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -14,26 +12,25 @@
 #include <cstddef>
 #include <cstdint>
 
+#include "grid_sync.cuh"
+#include "runtime.cuh"
+
 namespace ecl {
 
-struct RadixSortTemp {
-  unsigned* counts;  // 256 * tiles
-  size_t tiles;
-};
+// Keys a block places per step (1024 threads x 8 keys).
+constexpr int kRadixTile = 8192;
+constexpr int kRadixMaxBlocks = 256;  // blocks the count table holds
+constexpr size_t kRadixTempWords = (size_t)256 * kRadixMaxBlocks;
 
-// Elements per tile (block of 256 threads x 16 items).
-constexpr int kRadixTile = 4096;
-
-inline size_t radix_tiles(size_t n) { return (n + kRadixTile - 1) / kRadixTile; }
-inline size_t radix_temp_words(size_t n) { return 256 * radix_tiles(n) + 256; }
-
-// Sorts keys[0..n) ascending by bits [begin_bit, end_bit) together with vals.
-// Ping-pongs between (k0, v0) and (k1, v1); returns true when the result is
-// in (k1, v1).  Launches are counted and stream-ordered on `stream`.  With
-// n_dev, the element count is read on the device when the sort runs (at most
-// n, which sizes the launches and the temp buffer), so a count produced by an
-// earlier kernel needs no host round trip.
-bool radix_sort_pairs(unsigned long long* k0, int* v0, unsigned long long* k1, int* v1, int n, int begin_bit,
-                      int end_bit, unsigned* temp, cudaStream_t stream, const int* n_dev = nullptr);
+// order[0 .. *n_dev) = the values of the pairs (k0, v0)[0 .. *n_dev) by
+// ascending key, equal keys in their input order.  *n_dev <= n (which sizes
+// the launch), *max_high = the largest d; (k1, v1) is scratch of n pairs, k0
+// and v0 are overwritten, `temp` holds kRadixTempWords and `bar` is zeroed.
+// The order is whole (every value once) whatever status->code says; only when
+// a grid barrier times out it is not: ECL_ERR_NO_CONVERGENCE is raised in
+// `status`, *failed (zeroed before) becomes 1, and readers must check it.
+ecl_status radix_order(unsigned long long* k0, int* v0, unsigned long long* k1, int* v1, int* order, int n,
+                       const int* n_dev, const int* max_high, unsigned* temp, dev::GridBarrier* bar, int* failed,
+                       const DeviceInfo& dev, cudaStream_t stream, dev::Status* status);
 
 }  // namespace ecl

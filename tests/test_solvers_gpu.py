@@ -173,6 +173,20 @@ def test_scc_matches_tarjan(ecl, orc):
         assert np.array_equal(got, orc.scc(g)), name
 
 
+def sort_cases(ecl):
+    for n in (2, 33, 4096, 8191, 8193, 12289, 40000):  # one block; shares of a part of a tile
+        yield f"er{n}", ecl.gen_er(n, min(1.0, 5.0 / n), seed=n, symmetrise=True)
+    yield "grid1440k", ecl.gen_grid(1200, 1200, 0.05, seed=1)  # shares of more than one tile
+    # largest degrees of one, two and three digits
+    for leaves in (255, 256, 65535, 65536):
+        yield f"star{leaves}", undirected(leaves + 1, [(leaves, i) for i in range(leaves)])
+
+
+def test_gc_order_at_sort_edges(ecl, orc):
+    for name, g in sort_cases(ecl):
+        assert np.array_equal(ecl.gc(g), orc.gc(g)), name
+
+
 # ------------------------------------------------------------------------ APSP
 
 
