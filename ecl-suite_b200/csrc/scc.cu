@@ -35,6 +35,7 @@
 //    list without a separate pass;
 //  * the final labels are written by the same launch (label = in-max).
 #include "csr_bins.cuh"
+#include "flat_scan.cuh"
 #include "grid_sync.cuh"
 #include "solvers.cuh"
 
@@ -51,7 +52,8 @@ constexpr int kStamps = 256;
 
 struct SCCCtl {
   GridBarrier bar;
-  int pad[64];
+  unsigned long long asym;  // scc_symmetry's sum: 0 iff every entry has its reverse
+  int pad[62];
   // %globaltimer at the start and after each grid barrier (the first
   // kStamps - 1): a time profile of sweeps, compactions and retirements that
   // costs one store per barrier
@@ -85,6 +87,98 @@ __device__ __forceinline__ bool io_raise(unsigned long long* p, unsigned long lo
   if ((kIn ? io_in(old) : io_out(old)) >= val) return false;
   fetch_max(reinterpret_cast<int*>(p) + (kIn ? 1 : 0), val);  // little-endian: high half at +1
   return true;
+}
+
+// ---- symmetric graphs ----
+//
+// In a graph whose entries all have their reverses the strongly connected
+// components are the connected ones: CC labels them with their smallest ids,
+// and two passes over the vertices turn those into the largest.  Otherwise
+// every sweep over all edges moves the largest id a few hops on (ten sweeps
+// for a 701 x 1031 grid, 97 for a union of many grids).
+// The caller's ECL_GRAPH_SYMMETRIC flag says when this is worth looking for,
+// but SCC has never relied on it, so it is checked: the sum over all entries
+// (v, u) of +h(v, u) where v < u and -h(u, v) where v > u, modulo 2^64 with a
+// 64-bit hash h of the pair, is 0 for every symmetric entry list; a list that
+// is not symmetric makes it 0 once in 2^64.  Any other sum, and the general
+// path below runs and overwrites the labels.
+
+// Mixing function of splitmix64 (Steele, Lea and Flood, OOPSLA 2014).
+__device__ __forceinline__ unsigned long long scc_mix(unsigned long long x) {
+  x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ull;
+  x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
+  return x ^ (x >> 31);
+}
+
+__global__ void __launch_bounds__(kTPB) scc_rows(int n, int m, const int* __restrict__ nindex,
+                                                 int* __restrict__ tilerow, Status* __restrict__ status) {
+  flat_rows_range(n, m, nindex, tilerow, (blockIdx.x * kTPB + threadIdx.x) & ~31, gridDim.x * kTPB, status);
+}
+
+// Bound by the one read of the entries: the hash is about 20 instructions each.
+__global__ void __launch_bounds__(kTPB) scc_symmetry(FlatCsr g, bool vec, SCCCtl* __restrict__ ctl,
+                                                     Status* __restrict__ status) {
+  __shared__ __align__(16) int s_mark[kTPB / 32][kFlatTile];
+  __shared__ unsigned long long s_sum[kTPB / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int stop = min(g.m, __ldg(&g.nindex[g.n]));
+  const int tiles = flat_tiles(g.m);
+  unsigned long long sum = 0;
+  for (int t = blockIdx.x * (kTPB / 32) + wid; t < tiles; t += gridDim.x * (kTPB / 32))
+    flat_tile(g, stop, vec, t, s_mark[wid], [&](int, const int (&row)[kFlatLane], const int (&u)[kFlatLane]) {
+#pragma unroll
+      for (int k = 0; k < kFlatLane; k++) {
+        if (row[k] < 0 || u[k] == row[k]) continue;
+        if ((unsigned)u[k] >= (unsigned)g.n) {
+          raise(status, ECL_ERR_BAD_GRAPH, u[k]);
+          continue;
+        }
+        const unsigned lo = min(row[k], u[k]), hi = max(row[k], u[k]);
+        const unsigned long long h = scc_mix(((unsigned long long)hi << 32 | lo) + 0x9e3779b97f4a7c15ull);
+        sum += row[k] < u[k] ? h : 0ull - h;
+      }
+    });
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(kFull, sum, o);
+  if (lane == 0) s_sum[wid] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kTPB / 32; w++) sum += s_sum[w];
+    if (sum) fetch_add(&ctl->asym, sum);
+  }
+}
+
+// Smallest -> largest id, first pass: top[r] (zeroed before) = the largest id
+// above r of the component that CC labelled r.  Warps go through the vertices
+// from the last to the first, so the first id a lane meets of a component is
+// the largest it will meet, and of a warp's lanes in the highest lane's
+// component only that lane counts: the giant component's word then takes one
+// access per warp of the launch, not one per vertex.
+__global__ void __launch_bounds__(kTPB) scc_top(int n, const int* __restrict__ comp, int* __restrict__ top,
+                                                const SCCCtl* __restrict__ ctl) {
+  if (ld(&ctl->asym) != 0) return;
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5, nwarps = (gridDim.x * kTPB) >> 5;
+  const int groups = (n - 1) / 32 + 1;
+  int seen = -1;  // component that this lane or, for it, its warp's highest lane dealt with last
+  for (int q = groups - 1 - warp; q >= 0; q -= nwarps) {
+    const int v = 32 * q + lane;
+    const int r = v < n ? __ldg(&comp[v]) : -1;
+    const unsigned in = __ballot_sync(kFull, r >= 0);
+    const int top_lane = 31 - __clz(in);
+    const int high = __shfl_sync(kFull, r, top_lane);
+    const bool covered = r == high && lane != top_lane;
+    if (r >= 0 && r != v && r != seen && !covered && ld(&top[r]) < v) fetch_max(&top[r], v);
+    if (r >= 0) seen = r;
+  }
+}
+
+__global__ void __launch_bounds__(kTPB) scc_relabel(int n, int* __restrict__ comp, const int* __restrict__ top,
+                                                    const SCCCtl* __restrict__ ctl) {
+  if (ld(&ctl->asym) != 0) return;
+  for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
+    const int r = comp[v];
+    comp[v] = max(r, __ldg(&top[r]));
+  }
 }
 
 // A vertex is live (can be in a non-trivial SCC) iff it has an in-entry and an
@@ -124,7 +218,8 @@ __device__ __forceinline__ void scc_mark_batch(const bool (&valid)[kScanBatch], 
 __global__ void __launch_bounds__(kTPB) scc_mark(int n, int m, const int* __restrict__ nindex,
                                                  const int* __restrict__ nlist, int* __restrict__ flags,
                                                  int2* __restrict__ wl, RowChunks rc, Bins bins, bool vec,
-                                                 Status* __restrict__ status) {
+                                                 const SCCCtl* __restrict__ solved, Status* __restrict__ status) {
+  if (solved && ld(&solved->asym) == 0) return;  // a symmetric graph: its labels are written
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -168,7 +263,9 @@ __global__ void __launch_bounds__(kTPB) scc_mark(int n, int m, const int* __rest
 __global__ void __launch_bounds__(kTPB) scc_mark_chunks(int n, int m, const int* __restrict__ nindex,
                                                         const int* __restrict__ nlist, int* __restrict__ flags,
                                                         int2* __restrict__ wl, RowChunks rc, int chunk, bool vec,
+                                                        const SCCCtl* __restrict__ solved,
                                                         Status* __restrict__ status) {
+  if (solved && ld(&solved->asym) == 0) return;
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -200,8 +297,9 @@ template <int kSweepBatch>
 __global__ void __launch_bounds__(kTPB, SweepOcc<kSweepBatch>::blocks) scc_solve(int n, int m0, int2* __restrict__ wlA, int2* __restrict__ wlB,
                                                   const int* __restrict__ flags, unsigned long long* __restrict__ io,
                                                   int* __restrict__ label, SCCCtl* __restrict__ ctl,
-                                                  int max_rounds,
+                                                  int max_rounds, bool checked,
                                                   Status* __restrict__ status) {
+  if (checked && ld(&ctl->asym) == 0) return;  // as scc_mark
   const int lane = threadIdx.x & 31;
   const int tid = blockIdx.x * kTPB + threadIdx.x;
   const int nthreads = gridDim.x * kTPB;
@@ -377,6 +475,8 @@ struct SCCBufs {
   unsigned long long* io;
   int2* wlA;
   int2* wlB;
+  int* tilerow;
+  char* cc_ws;
   int max_rounds;
 };
 
@@ -389,6 +489,8 @@ void scc_layout(Carve& c, int n, int m, SCCBufs* b) {
   b->io = c.take<unsigned long long>((size_t)n);
   b->wlA = c.take<int2>((size_t)(m > 0 ? m : 1));
   b->wlB = c.take<int2>((size_t)(m > 0 ? m : 1));
+  b->tilerow = c.take<int>((size_t)flat_tiles(m) + 1);
+  b->cc_ws = c.take<char>(cc_workspace_bytes(n, m));
 }
 
 }  // namespace
@@ -410,13 +512,16 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
   SCCBufs b;
   scc_layout(c, g.n, g.m, &b);
   const int batch = dev.scc_sweep_batch > 0 ? dev.scc_sweep_batch : kSweepBatchDefault;
-  void (*solve)(int, int, int2*, int2*, const int*, unsigned long long*, int*, SCCCtl*, int, Status*) =
+  void (*solve)(int, int, int2*, int2*, const int*, unsigned long long*, int*, SCCCtl*, int, bool, Status*) =
       batch == 1 ? scc_solve<1> : (batch == 4 ? scc_solve<4> : scc_solve<2>);
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, solve, kTPB, 0) != cudaSuccess || occ < 1)
     return ECL_ERR_CUDA;
   const int coop_grid = dev.sms * occ;
   const int grid = dev.grid_blocks(kTPB, g.n, g.m);
+  // a graph flagged symmetric may be solved as connected components (not when
+  // the caller limits the rounds: that limit is the general path's)
+  const bool check = (g.flags & ECL_GRAPH_SYMMETRIC) != 0 && max_rounds <= 0;
   if (max_rounds <= 0 || max_rounds > b.max_rounds) max_rounds = b.max_rounds;
 
   if (cudaMemsetAsync(b.ctl, 0, sizeof(SCCCtl), stream) != cudaSuccess) return ECL_ERR_CUDA;
@@ -427,12 +532,26 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
   // with them than with 256 (R-MAT-22: 0.65 vs 0.72 ms)
   const Bins bins = bins_of(dev, Bins{kBinLane, kMinChunk});
   const bool vec = (reinterpret_cast<uintptr_t>(g.nlist) & 15) == 0 && dev.row_vec;  // 16-byte row loads
-  ECL_LAUNCH(scc_mark, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, status);
+  if (check) {
+    ECL_CUDA_TRY(cudaMemsetAsync(b.tilerow, 0xff, sizeof(int) * ((size_t)flat_tiles(g.m) + 1), stream));
+    ECL_LAUNCH(scc_rows, dev.grid_blocks(kTPB, g.n, 0), kTPB, 0, stream, g.n, g.m, g.nindex, b.tilerow, status);
+    if (g.m > 0)
+      ECL_LAUNCH(scc_symmetry, dev.grid_blocks(kTPB, 0, g.m), kTPB, 0, stream,
+                 FlatCsr{g.n, g.m, g.nindex, g.nlist, b.tilerow}, (reinterpret_cast<uintptr_t>(g.nlist) & 15) == 0, b.ctl,
+                 status);
+    const ecl_status st = cc_enqueue(g, label, b.cc_ws, status, dev, stream);
+    if (st != ECL_OK) return st;
+    // (the general path's flags stay zero when the graph is not symmetric)
+    ECL_LAUNCH(scc_top, dev.sms * 4, kTPB, 0, stream, g.n, label, b.flags, b.ctl);
+    ECL_LAUNCH(scc_relabel, dev.grid_blocks(kTPB, g.n, 0), kTPB, 0, stream, g.n, label, b.flags, b.ctl);
+  }
+  const SCCCtl* solved = check ? b.ctl : nullptr;
+  ECL_LAUNCH(scc_mark, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, solved, status);
   ECL_LAUNCH(scc_mark_chunks, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins.chunk, vec,
-             status);
+             solved, status);
   mark();
   ECL_CUDA_TRY(launch_cooperative(solve, coop_grid, kTPB, stream, g.n, g.m, b.wlA, b.wlB, b.flags, b.io, label, b.ctl,
-                                  max_rounds, status));
+                                  max_rounds, check, status));
   mark();
   return ECL_OK;
 }

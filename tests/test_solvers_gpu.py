@@ -173,6 +173,42 @@ def test_scc_matches_tarjan(ecl, orc):
         assert np.array_equal(got, orc.scc(g)), name
 
 
+def flagged_cases(ecl):
+    """Graphs flagged symmetric: truly so, and falsely (SCC then must not rely on it)."""
+    yield "grid", ecl.gen_grid(70, 90, 0.3, seed=2)
+    yield "rmat13", ecl.gen_rmat(13, 8, seed=4)
+    yield "one_entry", ecl.Graph(np.array([0, 1, 1], np.int32), np.array([1], np.int32), None, True)
+    yield "no_entries", ecl.Graph(np.zeros(6, np.int32), np.zeros(0, np.int32), None, True)
+    d = ecl.gen_rmat(12, 8, seed=6, symmetrise=False)
+    yield "directed", ecl.Graph(d.nindex, d.nlist, None, True)
+    s = ecl.gen_rmat(11, 8, seed=5)
+    drop = s.edges // 2  # one direction of one edge is missing
+    row = int(np.searchsorted(s.nindex, drop, side="right")) - 1
+    ni = s.nindex.copy()
+    ni[row + 1:] -= 1
+    yield "one_missing", ecl.Graph(ni, np.delete(s.nlist, drop), None, True)
+    cyc = [(i, (i + 1) % 300) for i in range(300)]
+    yield "cycle", from_edges(700, cyc + [(i, i) for i in range(0, 700, 7)], symmetric=True)
+    # 256-entry tiles: rows that start and end on their edges, long runs of empty rows, a row of many tiles
+    yield "long_run", from_edges(9000, [(0, 8999), (8999, 0)] + [(8999, i) for i in range(4000, 4800)] +
+                                 [(i, 8999) for i in range(4000, 4800)], symmetric=True)
+    yield "hub", undirected(20000, [(19999, i) for i in range(19000)])
+    yield "exact", undirected(512, [(i, (i + 128) % 512) for i in range(256)] + [(i, (i + 64) % 512) for i in range(256)])
+
+
+def test_scc_of_graphs_flagged_symmetric(ecl, orc):
+    for name, g in flagged_cases(ecl):
+        exp = orc.scc(g)
+        assert np.array_equal(ecl.scc(g), exp), name
+        dg = g.to_device()
+        assert np.array_equal(ecl.scc(dg).cpu().numpy(), exp), name
+        if g.edges:  # entries off the 16-byte boundaries
+            import torch
+
+            dg.nlist = torch.cat((dg.nlist[:1], dg.nlist))[1:]
+            assert np.array_equal(ecl.scc(dg).cpu().numpy(), exp), name
+
+
 def sort_cases(ecl):
     for n in (2, 33, 4096, 8191, 8193, 12289, 40000):  # one block; shares of a part of a tile
         yield f"er{n}", ecl.gen_er(n, min(1.0, 5.0 / n), seed=n, symmetrise=True)
