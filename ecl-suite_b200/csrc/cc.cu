@@ -9,10 +9,10 @@
 // so any union-find with the same hooking rule reproduces it bit for bit.
 //
 // B200 design (graphs flagged ECL_GRAPH_SYMMETRIC take the sampling path
-// further down: link the first two entries of every list, find the giant
-// component, then skip every list inside it):
+// further down: link two entries of every list, find the giant component,
+// then skip every list inside it):
 //  * cc_init   - parent[v] = first smaller neighbour among the first
-//                kInitScan entries (one free hook per vertex).
+//                kInitScan entries, twice over (one free hook per vertex).
 //  * cc_hook   - one pass over the vertices, 32 per warp.  Lists of <= 16
 //                entries are walked by their own lane; lists of up to
 //                2048 entries are walked by the whole warp (ballot loop,
@@ -26,6 +26,7 @@
 // All parent accesses are device-scope relaxed atomics; links use CAS.
 #include "solvers.cuh"
 
+#include <algorithm>
 #include <mutex>
 
 namespace ecl {
@@ -38,6 +39,7 @@ constexpr int kTPB = 256;
 // 2048 entries (a launch knob may change both).
 constexpr Bins kCCBins{16, 2048};
 constexpr int kInitScan = 8;   // entries cc_init looks at for a first smaller neighbour
+constexpr int kInitHops = 2;   // hops of cc_init (R-MAT-22, whole solve: 1 hop 0.244 ms, 2 0.227, 4 0.217; G(3 M, 12 M): 0.354, 0.369, 0.396)
 
 // Row [beg, end) of v, or empty when the row is malformed (cc_init reports it).
 __device__ __forceinline__ void cc_row(const int* nindex, int v, int m, int& beg, int& end) {
@@ -115,11 +117,25 @@ __device__ __forceinline__ void cc_union(int u, int v, int* parent) {
   }
 }
 
+// First smaller neighbour of v among the first kInitScan entries of its list
+// (v itself: none).  Only those are looked at: the hook is an optional head
+// start (the labels do not depend on it), and scanning a whole hub row from
+// one thread would serialise a 163k-entry R-MAT hub.
+__device__ __forceinline__ int cc_first_smaller(int v, int beg, int end, const int* nlist) {
+  const int stop = min(end, beg + kInitScan);
+  for (int i = beg; i < stop; i++) {
+    const int u = __ldg(&nlist[i]);
+    if (u < v && u >= 0) return u;
+  }
+  return v;
+}
+
+// parent[v] = the vertex kInitHops first-smaller-neighbour hops from v.  The
+// hops go through the CSR, which nothing writes, so L1 serves the rows of the
+// hubs that most vertices of a power-law graph hop to; the same steps through
+// parent[] afterwards queue at the hubs' words.
 // Also checks the CSR rows once: a malformed row (end < beg, or outside
 // [0, m]) raises ECL_ERR_BAD_GRAPH and is treated as empty by every kernel.
-// kHook = false: every vertex starts as its own root (the symmetric path,
-// whose sampling rounds do the first links).
-template <bool kHook>
 __global__ void __launch_bounds__(kTPB) cc_init(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, int* __restrict__ parent,
                                                 Status* __restrict__ status) {
@@ -129,17 +145,12 @@ __global__ void __launch_bounds__(kTPB) cc_init(int n, int m, const int* __restr
       raise(status, ECL_ERR_BAD_GRAPH, v);
       beg = end = 0;
     }
-    // Only the first few entries are looked at: the hook is an optional head
-    // start (the labels do not depend on it), and scanning a whole hub row
-    // from one thread would serialise a 163k-entry R-MAT hub.
-    int p = v;
-    const int stop = kHook ? min(end, beg + kInitScan) : beg;
-    for (int i = beg; i < stop; i++) {
-      const int u = __ldg(&nlist[i]);
-      if (u < v && u >= 0) {
-        p = u;
-        break;
-      }
+    int p = cc_first_smaller(v, beg, end, nlist);
+    for (int h = 1; h < kInitHops && p != v; h++) {
+      cc_row(nindex, p, m, beg, end);
+      const int q = cc_first_smaller(p, beg, end, nlist);
+      if (q == p) break;
+      p = q;
     }
     parent[v] = p;  // race-free: thread-owned init, no reader in this launch
   }
@@ -247,16 +258,47 @@ __global__ void __launch_bounds__(kTPB) cc_chunks(int n, const int* __restrict__
 // dependent loads per thread instead of D (a mesh builds chains as long as a
 // grid column).  parent[v] has no other writer during the launch, so the
 // array ends fully flat.
-__global__ void __launch_bounds__(kTPB) cc_flatten(int n, int* __restrict__ parent) {
-  for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
-    int p = ld(&parent[v]);
-    if (p == v) continue;
-    int pp;
-    while ((pp = ld(&parent[p])) < p) {
-      st(&parent[v], pp);
-      p = pp;
+//
+// A root stays one for the whole launch, so a thread does not look again at
+// the root that it met last: with a giant component every vertex would
+// otherwise end on the same word, and its L2 slice would be the bound.  Hence
+// a grid that gives each thread several vertices of a large graph
+// (flatten_blocks), kFlattenBatch of them in flight.
+constexpr int kFlattenBatch = 4;
+
+// kMark: also ing[v] = whether v's root is the sampled giant component's.
+template <bool kMark>
+__global__ void __launch_bounds__(kTPB) cc_flatten(int n, int* __restrict__ parent, const CCCounters* __restrict__ ctr,
+                                                   unsigned char* __restrict__ ing) {
+  const int stride = gridDim.x * kTPB;
+  const int giant = kMark ? ctr->giant : -1;
+  int known = -1;  // a root of this launch
+  for (long long v0 = blockIdx.x * kTPB + threadIdx.x; v0 < n; v0 += (long long)stride * kFlattenBatch) {
+    int p[kFlattenBatch];
+#pragma unroll
+    for (int k = 0; k < kFlattenBatch; k++) {
+      const long long v = v0 + (long long)k * stride;
+      p[k] = v < n ? ld(&parent[v]) : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < kFlattenBatch; k++) {
+      if (p[k] < 0) continue;
+      const int v = (int)(v0 + (long long)k * stride);
+      int q = p[k], pp;
+      if (q != v) {
+        while (q != known && (pp = ld(&parent[q])) < q) {
+          st(&parent[v], pp);
+          q = pp;
+        }
+        known = q;
+      }
+      if (kMark) ing[v] = q == giant;
     }
   }
+}
+
+int flatten_blocks(const DeviceInfo& dev, int n) {
+  return std::min(dev.grid_blocks(kTPB, n, 0), dev.sms * 8);
 }
 
 // ---- symmetric graphs: sampling + giant-component skip ----------------------
@@ -267,76 +309,81 @@ __global__ void __launch_bounds__(kTPB) cc_flatten(int n, int* __restrict__ pare
 // computation via subgraph sampling", IPDPS 2018).  Links still hook the
 // larger root under the smaller one, so the labels stay the minimum ids.
 
-constexpr int kSample = 2;  // list entries linked per vertex before the skip
-
-// Sampling round r: links v with the r-th entry of its list.  The rounds run
-// as separate launches with a full compression in between, so every find of
-// the next round starts one step from its root -- on a mesh, linking both
-// samples at once builds chains as long as a grid column.
+// Sampling: cc_init hooks every vertex to its first smaller neighbour -- one
+// store, no atomics -- and after a full compression cc_sample links one more
+// entry of every list: the first where the list starts with a larger id (that
+// vertex was left a root, most likely), the second of the others.  A full
+// compression comes between any two steps, so every find starts one step from
+// its root: on a mesh, linking both samples at once builds chains as long as a
+// grid column.
+//
+// The links run in two launches, an eighth of the vertices first.  While the
+// giant component forms, every link climbs through the same few words, and
+// their L2 slices serialise it; once an eighth of the links is made and
+// flattened, the others mostly find their two ends in one tree after two loads
+// of words of their own (an eighth is enough for the giant component to form:
+// with a 32nd, G(3 M, 12 M) takes 1.27 ms).  Measured, whole solve, both
+// entries linked by all vertices at once -> this, with cc_flatten's known
+// roots: G(3 M, 12 M) 1.68 -> 0.37 ms, G(150 k, 600 k) 0.19 -> 0.09, R-MAT-22
+// 0.29 -> 0.22, 1024 x 1024 grid 0.122 -> 0.120.
+template <int kPart>  // 0: one vertex in kFirstOf, 1: the others, 2: all
 __global__ void __launch_bounds__(kTPB) cc_sample(int n, int m, const int* __restrict__ nindex,
-                                                  const int* __restrict__ nlist, int* __restrict__ parent, int r,
+                                                  const int* __restrict__ nlist, int* __restrict__ parent,
                                                   Status* __restrict__ status) {
-  for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
+  constexpr int kFirstOf = 8;
+  const int count = kPart == 0 ? (n - 1) / kFirstOf + 1 : n;
+  for (int i = blockIdx.x * kTPB + threadIdx.x; i < count; i += gridDim.x * kTPB) {
+    const int v = kPart == 0 ? i * kFirstOf : i;
+    if (kPart == 1 && v % kFirstOf == 0) continue;
     int beg, end;
     cc_row(nindex, v, m, beg, end);
-    if (beg + r >= end) continue;
-    const int u = __ldg(&nlist[beg + r]);
+    if (beg >= end) continue;
+    int u = __ldg(&nlist[beg]);
+    if (u < v && beg + 1 < end) u = __ldg(&nlist[beg + 1]);
     if (u == v || !cc_valid(u, n, status)) continue;
     cc_union(v, u, parent);
   }
 }
 
-// One block: the most frequent root among 1024 sampled vertices.
+// From this many vertices on the sample is split: below, the two more launches
+// cost more than the contention they avoid.
+constexpr int kSplitSample = 1 << 13;
+
+// One block: the most frequent root among 1024 sampled vertices, counted in a
+// hash table in shared memory (a sort of the samples took 9 us, this 3).  The
+// links are done when it runs, so the roots it walks to are the final ones.
+constexpr int kGiantSlots = 2048;
+
 __global__ void __launch_bounds__(1024) cc_giant(int n, const int* __restrict__ parent, CCCounters* __restrict__ ctr) {
-  __shared__ int s[1024];
+  __shared__ int s_root[kGiantSlots], s_count[kGiantSlots];
+  __shared__ unsigned long long s_best[32];
   const int t = threadIdx.x;
-  s[t] = ld(&parent[ecl_hash((unsigned)t * 2654435761u + 97u) % (unsigned)n]);
+  for (int i = t; i < kGiantSlots; i += 1024) s_root[i] = -1, s_count[i] = 0;
   __syncthreads();
-  for (int k = 2; k <= 1024; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      const int p = t ^ j;
-      if (p > t) {
-        const int a = s[t], b = s[p];
-        if ((a > b) == ((t & k) == 0)) {
-          s[t] = b;
-          s[p] = a;
-        }
-      }
-      __syncthreads();
+  int r = (int)(ecl_hash((unsigned)t * 2654435761u + 97u) % (unsigned)n), p;
+  while ((p = ld(&parent[r])) != r) r = p;
+  const unsigned same = __match_any_sync(kFull, r);
+  if ((t & 31) == __ffs(same) - 1) {
+    // at most 1024 roots in 2048 slots: the probe ends
+    int h = (int)(((unsigned)r * 2654435761u) >> 21);
+    for (;; h = (h + 1) & (kGiantSlots - 1)) {
+      const int c = atomicCAS(&s_root[h], -1, r);
+      if (c == -1 || c == r) break;
     }
+    atomicAdd(&s_count[h], __popc(same));
   }
-  // Longest run of equal roots, ties to the smallest root: every run start
-  // finds its end by binary search, then a block-wide max over
-  // (length, ~root) keys (a serial scan by one thread cost ~15 us).
-  unsigned long long key = 0;
-  if (t == 0 || s[t] != s[t - 1]) {
-    int lo = t + 1, hi = 1024;  // first index past the run
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (s[mid] == s[t])
-        lo = mid + 1;
-      else
-        hi = mid;
-    }
-    key = ((unsigned long long)(lo - t) << 32) | (0xffffffffu - (unsigned)s[t]);
-  }
+  __syncthreads();
+  unsigned long long key = 0;  // largest count, ties to the smallest root
+  for (int i = t; i < kGiantSlots; i += 1024)
+    if (s_root[i] >= 0) key = max(key, ((unsigned long long)s_count[i] << 32) | (0xffffffffu - (unsigned)s_root[i]));
   for (int o = 16; o > 0; o >>= 1) key = max(key, __shfl_xor_sync(kFull, key, o));
-  __shared__ unsigned long long wbest[32];
-  if ((t & 31) == 0) wbest[t >> 5] = key;
+  if ((t & 31) == 0) s_best[t >> 5] = key;
   __syncthreads();
   if (t < 32) {
-    key = wbest[t];
+    key = s_best[t];
     for (int o = 16; o > 0; o >>= 1) key = max(key, __shfl_xor_sync(kFull, key, o));
     if (t == 0) ctr->giant = (int)(0xffffffffu - (unsigned)key);
   }
-}
-
-// Frozen membership of the sampled giant component (parent is flattened).
-__global__ void __launch_bounds__(kTPB) cc_mark_giant(int n, const int* __restrict__ parent,
-                                                      const CCCounters* __restrict__ ctr,
-                                                      unsigned char* __restrict__ ing) {
-  const int gr = ctr->giant;
-  for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) ing[v] = parent[v] == gr;  // race-free: parent is not written in this launch
 }
 
 // Remaining entries of vertices outside the giant component.  An entry is
@@ -357,10 +404,7 @@ __global__ void __launch_bounds__(kTPB) cc_rest(int n, int m, const int* __restr
   for (int base = warp * 32; base < n; base += nwarps * 32) {
     const int v = base + lane;
     int beg = 0, end = 0;
-    if (v < n && !__ldg(&ing[v])) {
-      cc_row(nindex, v, m, beg, end);
-      beg = min(end, beg + kSample);  // the first entries were linked by cc_sample
-    }
+    if (v < n && !__ldg(&ing[v])) cc_row(nindex, v, m, beg, end);
     const int deg = end - beg;
     if (deg > bins.chunk) {
       cc_push_chunks(v, beg, deg, bins.chunk, chunks, chunk_cap, ctr, status);
@@ -453,13 +497,18 @@ ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, 
   const int cap = chunk_capacity(g.m, kMinChunk);  // cc_layout sized the records for the smallest chunk
   ECL_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(CCCounters), stream));
   if (g.flags & ECL_GRAPH_SYMMETRIC) {
-    ECL_LAUNCH(cc_init<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
-    for (int r = 0; r < kSample; r++) {
-      ECL_LAUNCH(cc_sample, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, r, status);
-      ECL_LAUNCH(cc_flatten, grid, kTPB, 0, stream, g.n, parent);
+    ECL_LAUNCH(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
+    ECL_LAUNCH(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
+    if (g.n >= kSplitSample) {
+      ECL_LAUNCH(cc_sample<0>, dev.grid_blocks(kTPB, g.n / 8, 0), kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent,
+                 status);
+      ECL_LAUNCH(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
+      ECL_LAUNCH(cc_sample<1>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
+    } else {
+      ECL_LAUNCH(cc_sample<2>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
     }
     ECL_LAUNCH(cc_giant, 1, 1024, 0, stream, g.n, parent, ctr);
-    ECL_LAUNCH(cc_mark_giant, grid, kTPB, 0, stream, g.n, parent, ctr, ing);
+    ECL_LAUNCH(cc_flatten<true>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, ctr, ing);
     mark();
     ECL_LAUNCH(cc_rest, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ing, chunks, cap, bins, ctr,
                status);
@@ -467,17 +516,17 @@ ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, 
     ECL_LAUNCH(cc_rest_chunks, grid, kTPB, 0, stream, g.n, g.nindex, g.nlist, parent, ing, chunks, cap, bins.chunk,
                ctr, status);
     mark();
-    ECL_LAUNCH(cc_flatten, grid, kTPB, 0, stream, g.n, parent);
+    ECL_LAUNCH(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
     mark();
     return ECL_OK;
   }
-  ECL_LAUNCH(cc_init<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
+  ECL_LAUNCH(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
   mark();
   ECL_LAUNCH(cc_hook, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, chunks, cap, bins, ctr, status);
   mark();
   ECL_LAUNCH(cc_chunks, grid, kTPB, 0, stream, g.n, g.nindex, g.nlist, parent, chunks, cap, bins.chunk, ctr, status);
   mark();
-  ECL_LAUNCH(cc_flatten, grid, kTPB, 0, stream, g.n, parent);
+  ECL_LAUNCH(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
   mark();
   return ECL_OK;
 }
@@ -610,12 +659,12 @@ extern "C" ecl_status ecl_cc_noalloc(int32_t nodes, int32_t edges, const int32_t
   // the counters (adjacent, at the front of the array) before every solve.
   ECL_CUDA_TRY(cudaMemsetAsync(base, 0, kStatusBytes + sizeof(CCCounters), stream));
   const int grid = dev.grid_blocks(kTPB, nodes, edges);
-  ECL_LAUNCH(cc_init<true>, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, status);
+  ECL_LAUNCH(cc_init, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, status);
   ECL_LAUNCH(cc_hook, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, chunks,
              chunk_capacity(edges, kCCBins.chunk), kCCBins, ctr, status);
   ECL_LAUNCH(cc_chunks, grid, kTPB, 0, stream, nodes, nindex, nlist, label, chunks,
              chunk_capacity(edges, kCCBins.chunk), kCCBins.chunk, ctr, status);
-  ECL_LAUNCH(cc_flatten, grid, kTPB, 0, stream, nodes, label);
+  ECL_LAUNCH(cc_flatten<false>, flatten_blocks(dev, nodes), kTPB, 0, stream, nodes, label, nullptr, nullptr);
   Status hs{};
   ECL_CUDA_TRY(cudaMemcpyAsync(&hs, status, sizeof(hs), cudaMemcpyDeviceToHost, stream));
   ECL_CUDA_TRY(cudaStreamSynchronize(stream));

@@ -56,3 +56,15 @@ def test_cc_validate_rejects_bad_graph(ecl):
     with pytest.raises(ecl.EclError) as e:
         ecl.cc(g, validate=True)
     assert e.value.status == ecl.ERR_BAD_GRAPH
+
+
+@pytest.mark.parametrize("n", [8191, 8192, 8193, 65536 + 7])  # around the size from which the sample is split
+@pytest.mark.parametrize("degree", [1.5, 3.0, 8.0])  # many small components, a forming giant, one giant
+def test_cc_sampling_edges(ecl, orc, n, degree):
+    g = ecl.gen_er(n, degree / n, seed=n + int(degree * 10), symmetrise=True)
+    exp = orc.cc(g)
+    assert np.array_equal(ecl.cc(g), exp)
+    rng = np.random.default_rng(n)  # lists in any order: the first entries are no longer the smallest
+    order = np.argsort(np.repeat(np.arange(n), np.diff(g.nindex)) + rng.random(g.edges))
+    shuffled = ecl.Graph(g.nindex, g.nlist[order], None, symmetric=True)
+    assert np.array_equal(ecl.cc(shuffled), exp)
