@@ -468,49 +468,50 @@ __device__ int gc_short_row(int beg, int h, const int* nl2, const int* color, St
 // inverse of the order over the core) and record each core rank's row
 // (start, length, vertex).
 //
-// The cluster's SMs stream all core rows (16.6 M entries for the first 32k
-// ranks of R-MAT-22), and a warp that fetched each row with its own loads paid a
-// dependent L2 round trip per 128 entries.  Instead every warp stages its
-// rows through two shared-memory buffers with bulk asynchronous copies
-// (cp.async.bulk, completion counted on an mbarrier): while it colours one
-// segment of a row, the next segment -- of this row or of its next row -- is
-// already on its way, and the scan itself reads shared memory only.  Colours
-// are 16-bit words (0xffff = not yet coloured; a core colour is at most the
-// row's length, below 2^15).
+// The cluster's SMs stream all core rows (5.4 M entries for the first 8192
+// ranks of R-MAT-22, 660 a row), so the instructions and shared-memory cycles
+// per entry bound the core as much as the chain does.  Rows hold 16-bit ranks,
+// packed and 16-byte aligned by gc_core_translate, and arrive through two
+// shared-memory buffers per warp with bulk asynchronous copies (cp.async.bulk,
+// completion counted on an mbarrier): while a warp colours one segment of a
+// row, the next segment -- of this row or of its next row -- is already on its
+// way.  A lane reads eight ranks with one 16-byte load, looks each colour up
+// (16-bit words, 0xffff = not yet coloured; a core colour is at most the row's
+// length, below 2^15), sets a byte of the warp's mark array for it without any
+// test -- undecided and far colours go to a byte that nobody reads -- and keeps
+// the undecided entries in a 32-bit mask.  A byte store needs no atomic: lanes
+// that mark the same colour store the same value.
 constexpr int kCoreThreads = 1024;
 constexpr int kCoreWarps = kCoreThreads / 32;
-// Default CTAs of the core's cluster.  R-MAT-22, core + pull: 1 CTA with 4096
-// ranks 3.15 ms; 2 CTAs with 8192 ranks 2.86 ms; 4 CTAs 2.92 ms (a hop
-// between CTAs, through distributed shared memory, costs more than one inside
-// a CTA, so more CTAs than two buy nothing).
+// Default CTAs of the core's cluster.  A hop between CTAs, through distributed
+// shared memory, costs more than one inside a CTA.  R-MAT-22, core time by
+// CTAs (8192 ranks): 1: 1.59 ms, 2: 1.43, 4: 1.73; core + pull by ranks (2
+// CTAs): 4096: 2.90 ms, 8192: 2.54, 16384: 2.67, 32768: 3.23.
 constexpr int kCoreCtas = 2;
-constexpr int kCoreBatch = 4;           // entries per lane whose loads are in flight together
 constexpr int kCoreDefault = 8192;      // default core size (ranks): the measured best at R-MAT-22 with 2 CTAs
 constexpr int kCoreMax = 36864;         // shared memory bound
-constexpr int kSegSlack = 8;            // a buffer holds a segment plus its 16-byte alignment slack
-constexpr int kCorePend = 1024;         // per-warp list of undecided entries (16-bit ranks)
-constexpr int kSegBufMax = 384;  // longer segments measured slower (one copy's latency per row is exposed)
+constexpr int kSegMax = 1024;           // entries per segment: a bit each of a lane's 32-bit mask
 constexpr unsigned kUncoloured = 0xffffu;
+constexpr int kWin = 1016;              // colours of a mark window; the bytes up to kMarkBytes take what is outside
+constexpr int kMarkBytes = 1024;
 constexpr size_t kCoreSmemLimit = 227 * 1024;
 
-// Dynamic shared memory of the core CTA: colours (16-bit, per rank), then per
-// warp two mbarriers, two staging buffers of `segbuf` entries, a 2048-colour
-// bitmap and a list of up to kCorePend undecided entries (16-bit ranks).  The
-// buffers take what the colours leave, up to kSegBufMax entries.
+// Dynamic shared memory of a core CTA: colours (16-bit, per rank), then per
+// warp two mbarriers, two staging buffers of `seg` entries and the mark bytes.
+// The buffers take what the colours leave, up to kSegMax entries.
 __host__ __device__ constexpr size_t gc_core_colour_bytes(int cap) { return ((size_t)cap * 2 + 15) & ~size_t(15); }
-__host__ __device__ constexpr size_t gc_core_warp_bytes(int segbuf) {
-  return 2 * sizeof(unsigned long long) + (size_t)segbuf * 2 * sizeof(int) + kMexWords * sizeof(unsigned) +
-         kCorePend * sizeof(unsigned short);
+__host__ __device__ constexpr size_t gc_core_warp_bytes(int seg) {
+  return 2 * sizeof(unsigned long long) + (size_t)seg * 2 * sizeof(unsigned short) + kMarkBytes;
 }
-__host__ __device__ constexpr int gc_core_segbuf(int cap) {
+__host__ __device__ constexpr int gc_core_seg(int cap) {
   const size_t fixed = gc_core_colour_bytes(cap) + kCoreWarps * gc_core_warp_bytes(0);
-  const size_t per = (kCoreSmemLimit - fixed) / kCoreWarps / (2 * sizeof(int));
-  return (int)((per < (size_t)kSegBufMax ? per : (size_t)kSegBufMax) & ~size_t(7));
+  const size_t per = (kCoreSmemLimit - fixed) / kCoreWarps / (2 * sizeof(unsigned short));
+  return (int)((per < (size_t)kSegMax ? per : (size_t)kSegMax) & ~size_t(7));
 }
 __host__ __device__ constexpr size_t gc_core_smem(int cap) {
-  return gc_core_colour_bytes(cap) + kCoreWarps * gc_core_warp_bytes(gc_core_segbuf(cap));
+  return gc_core_colour_bytes(cap) + kCoreWarps * gc_core_warp_bytes(gc_core_seg(cap));
 }
-static_assert(gc_core_segbuf(kCoreMax) >= 256 && gc_core_smem(kCoreMax) <= kCoreSmemLimit,
+static_assert(gc_core_seg(kCoreMax) >= 256 && gc_core_smem(kCoreMax) <= kCoreSmemLimit,
               "core shared memory over the per-block limit");
 
 // Core size of this solve: the long rows (a prefix of the order), at most cap.
@@ -527,10 +528,14 @@ __global__ void __launch_bounds__(kTPB) gc_core_rank(const int* __restrict__ ord
 }
 
 // Rewrites the higher-priority entries of every core row from vertex ids to
-// ranks, one warp per row, and records the row: rowinfo[r] = (first entry,
+// 16-bit ranks, one warp per row, packed from the first 16-byte boundary of the
+// row's slot on, and records the row: rowinfo[r] = (start in 16-byte units,
 // length, vertex).  Such an entry outranks its row, so its rank is below the
-// row's and inside the core.
-__global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict__ nindex, int* __restrict__ nl2,
+// row's and inside the core.  In place: a step's 32 entries are read before
+// any rank of them is written, and the ranks written up to step i end below
+// the first entry of step i + 1.  A core row has more than kWarpRow entries,
+// so its 4-byte slot holds the packed ranks and the copies' rounding.
+__global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict__ nindex, int* nl2,
                                                           const int* __restrict__ hc, const int* __restrict__ order,
                                                           const int* __restrict__ rank, int4* __restrict__ rowinfo,
                                                           const GCCtl* __restrict__ ctl, int cap) {
@@ -541,8 +546,17 @@ __global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict_
   for (int r = warp; r < core; r += nwarps) {
     const int v = __ldg(&order[r]);
     const int b = __ldg(&nindex[v]), h = __ldg(&hc[v]);
-    for (int i = b + lane; i < b + h; i += 32) nl2[i] = __ldg(&rank[nl2[i]]);
-    if (lane == 0) rowinfo[r] = make_int4(b, h, v, 0);
+    const int first = (int)(((long long)b + 3) >> 2);  // 16-byte units
+    unsigned short* out = reinterpret_cast<unsigned short*>(nl2) + (size_t)first * 8;
+    for (int i0 = 0; i0 < h; i0 += 32) {
+      const int i = i0 + lane;
+      unsigned short q = 0;
+      if (i < h) q = (unsigned short)__ldg(&rank[nl2[(size_t)b + i]]);
+      __syncwarp();
+      if (i < h) out[i] = q;
+      __syncwarp();
+    }
+    if (lane == 0) rowinfo[r] = make_int4(first, h, v, 0);
   }
 }
 
@@ -622,112 +636,65 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
   }
 }
 
-// Colour of core rank q once it is published; -1 when the wait gives up (2 s
-// without the colour, or another error raised).
-__device__ __forceinline__ int gc_core_wait(const unsigned short* col_s, int q, Status* status) {
-  unsigned c = col_ld(&col_s[q]);
-  if (c != kUncoloured) return (int)c;
-  const unsigned long long t0 = gc_now();
-  for (unsigned spins = 1;; spins++) {
-    c = col_ld(&col_s[q]);
-    if (c != kUncoloured) return (int)c;
-    if ((spins & 1023u) == 0 && (gc_now() - t0 > kStallNs || ld(&status->code) != 0)) {
-      raise(status, ECL_ERR_NO_CONVERGENCE, q);
-      return -1;
+// The smallest colour of the window at `off` that the warp's marks leave free,
+// or -1; clears the marks.  All lanes call, behind a __syncwarp.
+__device__ __forceinline__ int gc_core_mex(unsigned char* marks, int off) {
+  const int lane = threadIdx.x & 31;
+  int c = -1;
+  for (int i = 0; i < kMarkBytes / 128; i++) {
+    const unsigned w = reinterpret_cast<const unsigned*>(marks)[32 * i + lane];
+    unsigned z = (w - 0x01010101u) & ~w & 0x80808080u;  // lowest set bit: the lowest zero byte
+    if (128 * i + 4 * lane >= kWin) z = 0;              // kWin is a multiple of 4
+    const unsigned f = __ballot_sync(kFull, z != 0);
+    if (f) {
+      const int who = __ffs(f) - 1;
+      c = off + 128 * i + 4 * who + ((__ffs(__shfl_sync(kFull, z, who)) - 1) >> 3);
+      break;
     }
-    // no nap: the core is bound by its chain, and every nap length tried
-    // (32 to 512 ns) measured slower than spinning on shared memory
   }
+  __syncwarp();
+  uint4* m4 = reinterpret_cast<uint4*>(marks) + 2 * lane;
+  m4[0] = m4[1] = make_uint4(0u, 0u, 0u, 0u);
+  __syncwarp();
+  return c;
 }
 
-// Colour of core rank r whose entries (ranks) are nl2[wb, we), for colours
-// from `off0` on, read straight from global memory: the fallback for a row
-// whose first 2048 colours are all taken by its neighbours.  -1 on a stall.
-__device__ int gc_core_row_global(int r, int wb, int we, int off0, const int* nl2, const unsigned short* col_s,
-                                  unsigned* bits, unsigned short* pend, Status* status) {
+// Colour of a core row of `h` ranks at `row` whose first kWin colours are all
+// taken by its neighbours; every neighbour is coloured by now.
+__device__ int gc_core_far(const unsigned short* row, int h, const unsigned short* col_s, unsigned char* marks) {
   const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1;
-  for (int off = off0;; off += 32 * kMexWords) {
-    bits[lane] = 0;
-    bits[lane + 32] = 0;
-    __syncwarp();
-    for (int i0 = wb; i0 < we; i0 += 32 * kCoreBatch) {
-      int np = 0;
-      int q[kCoreBatch];
-#pragma unroll
-      for (int k = 0; k < kCoreBatch; k++) {
-        const int i = i0 + 32 * k + lane;
-        q[k] = i < we ? __ldg(&nl2[i]) : -1;
-        if (i < we && (unsigned)q[k] >= (unsigned)r) {
-          raise(status, ECL_ERR_BAD_GRAPH, r);
-          q[k] = -1;
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < kCoreBatch; k++) {
-        const unsigned c = q[k] >= 0 ? col_ld(&col_s[q[k]]) : 0u;
-        const bool undecided = q[k] >= 0 && c == kUncoloured;
-        if (q[k] >= 0 && !undecided) gc_mark(bits, (int)c, off);
-        const unsigned ub = __ballot_sync(kFull, undecided);
-        if (undecided) pend[np + __popc(ub & lt)] = (unsigned short)q[k];
-        np += __popc(ub);
-      }
-      __syncwarp();
-      bool stalled = false;
-      for (int j = lane; j < np; j += 32) {
-        const int c = gc_core_wait(col_s, pend[j], status);
-        if (c < 0) {
-          stalled = true;
-          break;
-        }
-        gc_mark(bits, c, off);
-      }
-      if (__any_sync(kFull, stalled)) return -1;
+  for (int off = kWin;; off += kWin) {
+    for (int i = lane; i < h; i += 32) {
+      const int d = (int)col_ld(&col_s[__ldg(&row[i])]) - off;
+      if (d >= 0 && d < kWin) marks[d] = 1;
     }
     __syncwarp();
-    const unsigned w0 = bits[lane], w1 = bits[lane + 32];
-    const unsigned f0 = __ballot_sync(kFull, w0 != ~0u), f1 = __ballot_sync(kFull, w1 != ~0u);
-    int c = -1;
-    if (f0) {
-      const int wi = __ffs(f0) - 1;
-      c = off + wi * 32 + __ffs(~__shfl_sync(kFull, w0, wi)) - 1;
-    } else if (f1) {
-      const int wi = __ffs(f1) - 1;
-      c = off + (wi + 32) * 32 + __ffs(~__shfl_sync(kFull, w1, wi)) - 1;
-    }
-    __syncwarp();
+    const int c = gc_core_mex(marks, off);
     if (c >= 0) return c;
   }
 }
 
 // Per-warp staging of row segments: two buffers, each with its mbarrier and
-// the parity of its next phase.  A segment is (first entry in nl2, length <=
-// segbuf - 8); the copy starts at the 16-byte boundary at or below the first entry
-// and ends at the one at or above its end (nl2 holds 4 spare entries past m,
-// so the rounding never leaves the array).
+// the parity of its next phase.  A segment starts at a 16-byte unit of the
+// packed rows and has at most the buffer's entries; the copy is rounded up to
+// 16 bytes (the row's slot has room).
 struct CoreStage {
-  int* buf[2];
+  unsigned short* buf[2];
   unsigned long long* bar[2];
   unsigned parity[2] = {0u, 0u};
   int first[2] = {-1, -1};  // segment in each buffer (-1: none in flight)
-  int len[2] = {0, 0};
 
-  __device__ __forceinline__ void issue(int b, const int* nl2, int f, int l) {
-    first[b] = f;
-    len[b] = l;
-    if ((threadIdx.x & 31) == 0) {
-      const int a = f & ~3, e = (f + l + 3) & ~3;
-      bulk_load(buf[b], nl2 + a, 4u * (unsigned)(e - a), bar[b]);
-    }
+  __device__ __forceinline__ void issue(int b, const int* nl2, int unit, int len) {
+    first[b] = unit;
+    if ((threadIdx.x & 31) == 0)
+      bulk_load(buf[b], reinterpret_cast<const char*>(nl2) + (size_t)unit * 16, (2u * (unsigned)len + 15u) & ~15u, bar[b]);
   }
-  // Waits for buffer b's copy; the segment's entries then start at
-  // buf[b] + offset(b).  False when the wait ran out.
+  // Waits for buffer b's copy.  False when the wait ran out.
   __device__ __forceinline__ bool wait(int b) {
     const bool ok = mbar_wait(bar[b], parity[b]);
     if (ok) parity[b] ^= 1u;  // a copy that did not land stays listed for drain()
     return ok;
   }
-  __device__ __forceinline__ int offset(int b) const { return first[b] & 3; }
   // Bounded wait for every copy still in flight (before leaving on an error).
   __device__ __forceinline__ void drain() {
     for (int b = 0; b < 2; b++)
@@ -738,37 +705,38 @@ struct CoreStage {
   }
 };
 
-// One CTA colours the core: rank r goes to warp r mod 32, each warp takes its
-// ranks in increasing order (the warp holding the lowest uncoloured rank can
-// always finish it), and every colour is published to shared memory for the
-// core and to color[] for gc_pull.  A warp's rows are a stream of segments;
+// The cluster colours the core: rank r goes to warp r mod (32 ctas), each warp
+// takes its ranks in increasing order (the warp holding the lowest uncoloured
+// rank can always finish it), and every colour is published to the core's
+// copies and to color[] for gc_pull.  A warp's rows are a stream of segments;
 // while one segment is scanned from shared memory the next is being copied.
+// CAUTION for the look-ups: a malformed graph (reported by gc_init) may leave
+// any 16-bit value in a row; 2 * 0xffff bytes is inside this CTA's shared
+// memory for every core size, and a wait on what is read there ends on the
+// status word.
 __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* __restrict__ nl2, const int4* __restrict__ rowinfo,
                                                            int* __restrict__ color, const GCCtl* __restrict__ ctl,
                                                            int cap, Status* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char s_core[];
   const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1;
   const int core = gc_core_size(ctl, cap);
-  // The core runs on a cluster of `ctas` CTAs (1 without a cluster launch):
   // rank r belongs to warp r mod (32 ctas) of the cluster, so each CTA takes
   // every ctas-th block of 32 consecutive ranks (dealing longer runs of
-  // consecutive ranks to one CTA measured slower; single ranks, no faster).
+  // consecutive ranks to one CTA measured slower; single ranks, no faster)
   const int ctas = (int)cluster_ctas();
   const int warp = (int)cluster_rank() * kCoreWarps + (threadIdx.x >> 5);
   const int cwarps = ctas * kCoreWarps;
   unsigned short* col_s = reinterpret_cast<unsigned short*>(s_core);
-  const int segbuf = gc_core_segbuf(cap);
-  const int kSeg = segbuf - kSegSlack;  // row entries staged at a time
-  unsigned char* wbase = s_core + gc_core_colour_bytes(cap) + (size_t)(threadIdx.x >> 5) * gc_core_warp_bytes(segbuf);
+  const int seg = gc_core_seg(cap);  // row entries staged at a time
+  unsigned char* wbase = s_core + gc_core_colour_bytes(cap) + (size_t)(threadIdx.x >> 5) * gc_core_warp_bytes(seg);
   CoreStage stg;
   stg.bar[0] = reinterpret_cast<unsigned long long*>(wbase);
   stg.bar[1] = stg.bar[0] + 1;
-  stg.buf[0] = reinterpret_cast<int*>(wbase + 2 * sizeof(unsigned long long));
-  stg.buf[1] = stg.buf[0] + segbuf;
-  unsigned* bits = reinterpret_cast<unsigned*>(stg.buf[1] + segbuf);
-  unsigned short* pend = reinterpret_cast<unsigned short*>(bits + kMexWords);
+  stg.buf[0] = reinterpret_cast<unsigned short*>(wbase + 2 * sizeof(unsigned long long));
+  stg.buf[1] = stg.buf[0] + seg;
+  unsigned char* marks = reinterpret_cast<unsigned char*>(stg.buf[1] + seg);
   for (int r = threadIdx.x; r < core; r += kCoreThreads) col_st(&col_s[r], kUncoloured);
+  reinterpret_cast<uint4*>(marks)[2 * lane] = reinterpret_cast<uint4*>(marks)[2 * lane + 1] = make_uint4(0u, 0u, 0u, 0u);
   if (lane == 0) {
     mbar_init(stg.bar[0]);
     mbar_init(stg.bar[1]);
@@ -791,35 +759,32 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* __restrict
     return make_int4(__shfl_sync(kFull, rec.x, src), __shfl_sync(kFull, rec.y, src), __shfl_sync(kFull, rec.z, src),
                      0);
   };
+  // looks entry e of the staged segment up; true when it is undecided
+  auto look = [&](unsigned q) -> bool {
+    const unsigned c = col_ld(&col_s[q]);
+    marks[min(c, (unsigned)kWin)] = 1;
+    return c == kUncoloured;
+  };
   const int nrows = core > warp ? (core - warp + cwarps - 1) / cwarps : 0;
   int b = 0;  // buffer holding (or about to hold) the segment to scan next
   for (int j = 0; j < nrows; j++) {
     const int r = warp + cwarps * j;
     const int4 row = row_of(j);
-    const int wb = row.x, h = row.y, v = row.z;
-    bits[lane] = 0;
-    bits[lane + 32] = 0;
-    __syncwarp();
-    int np = 0;
+    const int unit = row.x, h = row.y, v = row.z;
     bool stalled = false;
-    for (int off = 0; off < h && !stalled; off += kSeg) {
-      const int f = wb + off, l = min(kSeg, h - off);
-      if (stg.first[b] >= 0 && stg.first[b] != f) {  // a prefetch of another segment: cannot happen
-        raise(status, ECL_ERR_CUDA, r);
-        stalled = true;
-        break;
-      }
+    for (int off = 0; off < h && !stalled; off += seg) {
+      const int f = unit + off / 8, l = min(seg, h - off);
       if (stg.first[b] != f) stg.issue(b, nl2, f, l);  // not prefetched
       // prefetch what comes next: this row's next segment, or the first one
       // of the warp's next row with entries (rows without any are skipped)
       __syncwarp();  // buffer b ^ 1 was scanned by every lane
-      if (off + kSeg < h) {
-        stg.issue(b ^ 1, nl2, f + kSeg, min(kSeg, h - off - kSeg));
+      if (off + seg < h) {
+        stg.issue(b ^ 1, nl2, f + seg / 8, min(seg, h - off - seg));
       } else {
         for (int jn = j + 1; jn < nrows; jn++) {
           const int4 nx = row_of(jn);
           if (nx.y > 0) {
-            stg.issue(b ^ 1, nl2, nx.x, min(kSeg, nx.y));
+            stg.issue(b ^ 1, nl2, nx.x, min(seg, nx.y));
             break;
           }
         }
@@ -829,74 +794,57 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* __restrict
         stalled = true;
         break;
       }
-      const int* seg = stg.buf[b] + stg.offset(b);
       stg.first[b] = -1;
-      // scan the staged entries: colours already published go into the
-      // bitmap, the others into the pending list
-      for (int i0 = 0; i0 < l; i0 += 32 * kCoreBatch) {
-        int q[kCoreBatch];
-        unsigned c[kCoreBatch];
+      const unsigned short* sg = stg.buf[b];
+      // eight entries a lane and step; bit 8 s + k of `wait`: entry k of the
+      // lane's step s is undecided
+      unsigned wait = 0;
+      const uint4* sv = reinterpret_cast<const uint4*>(sg);
+      for (int s = 0; 256 * s < l; s++) {
+        const int e = 256 * s + 8 * lane;
+        unsigned undecided = 0;
+        if (e + 8 <= l) {
+          const uint4 x = sv[32 * s + lane];
+          const unsigned w[4] = {x.x, x.y, x.z, x.w};
+          unsigned c[8];
 #pragma unroll
-        for (int k = 0; k < kCoreBatch; k++) {
-          const int i = i0 + 32 * k + lane;
-          q[k] = i < l ? seg[i] : -1;
-          if (i < l && (unsigned)q[k] >= (unsigned)r) {
-            raise(status, ECL_ERR_BAD_GRAPH, r);
-            q[k] = -1;
+          for (int k = 0; k < 8; k++) c[k] = col_ld(&col_s[(k & 1) ? w[k >> 1] >> 16 : w[k >> 1] & 0xffffu]);
+#pragma unroll
+          for (int k = 0; k < 8; k++) {
+            marks[min(c[k], (unsigned)kWin)] = 1;
+            undecided |= c[k] == kUncoloured ? 1u << k : 0u;
+          }
+        } else {
+          for (int k = 0; e + k < l; k++) undecided |= look(sg[e + k]) ? 1u << k : 0u;
+        }
+        wait |= undecided << (8 * s);
+      }
+      // Wait for the undecided ones: a lane polls its lowest.
+      unsigned spins = 0;
+      unsigned long long t0 = 0;
+      while (wait) {
+        const int k = __ffs(wait) - 1;
+        if (!look(sg[256 * (k >> 3) + 8 * lane + (k & 7)])) {
+          wait &= wait - 1;
+        } else if ((++spins & 1023u) == 0) {  // no nap: every nap length tried was slower than spinning
+          if (t0 == 0) t0 = gc_now();
+          if (gc_now() - t0 > kStallNs || ld(&status->code) != 0) {
+            raise(status, ECL_ERR_NO_CONVERGENCE, r);
+            stalled = true;
+            break;
           }
         }
-#pragma unroll
-        for (int k = 0; k < kCoreBatch; k++) c[k] = q[k] >= 0 ? col_ld(&col_s[q[k]]) : 0u;
-#pragma unroll
-        for (int k = 0; k < kCoreBatch; k++) {
-          const bool undecided = q[k] >= 0 && c[k] == kUncoloured;
-          if (q[k] >= 0 && !undecided) gc_mark(bits, (int)c[k], 0);
-          const unsigned ub = __ballot_sync(kFull, undecided);
-          if (undecided) pend[np + __popc(ub & lt)] = (unsigned short)q[k];
-          np += __popc(ub);
-        }
       }
+      stalled = __any_sync(kFull, stalled);
       b ^= 1;
-      // resolve the pending entries once the list could not take another
-      // segment, and at the end of the row
-      if (np + kSeg > kCorePend || off + kSeg >= h) {  // before the list could overflow, and at the row's end
-        __syncwarp();
-        for (int jj = lane; jj < np && !stalled; jj += 32) {
-          const int cc = gc_core_wait(col_s, pend[jj], status);
-          if (cc < 0)
-            stalled = true;
-          else
-            gc_mark(bits, cc, 0);
-        }
-        stalled = __any_sync(kFull, stalled);
-        np = 0;
-        __syncwarp();
-      }
     }
     if (stalled) {
       stg.drain();
       break;
     }
-    // the smallest colour of the first window the bitmap leaves free
     __syncwarp();
-    const unsigned w0 = bits[lane], w1 = bits[lane + 32];
-    const unsigned f0 = __ballot_sync(kFull, w0 != ~0u), f1 = __ballot_sync(kFull, w1 != ~0u);
-    int c = -1;
-    if (f0) {
-      const int wi = __ffs(f0) - 1;
-      c = wi * 32 + __ffs(~__shfl_sync(kFull, w0, wi)) - 1;
-    } else if (f1) {
-      const int wi = __ffs(f1) - 1;
-      c = (wi + 32) * 32 + __ffs(~__shfl_sync(kFull, w1, wi)) - 1;
-    }
-    __syncwarp();
-    if (c < 0) {  // all 2048 first colours taken: scan the row again for the next windows
-      c = gc_core_row_global(r, wb, wb + h, 32 * kMexWords, nl2, col_s, bits, pend, status);
-      if (c < 0) {
-        stg.drain();
-        break;
-      }
-    }
+    int c = gc_core_mex(marks, 0);
+    if (c < 0) c = gc_core_far(reinterpret_cast<const unsigned short*>(nl2) + (size_t)unit * 8, h, col_s, marks);
     if (lane == 0) {
       col_publish(&col_s[r], (unsigned)c, ctas);
       st(&color[v], c);
