@@ -10,14 +10,12 @@
 //
 // B200 design:
 //  * mst_threshold: one block samples 1024 weights on the device and picks
-//    the quantile that leaves ~0.75 n light CSR entries (no host round
-//    trip).  Fewer light edges than the reference's 3n: on R-MAT-22 the light
-//    Boruvka pass then runs on ~1.6 M instead of ~6.4 M edges, and the
-//    flattened heavy pass absorbs the rest (factor 3 -> 0.75: MST 6.5 -> 5.0 ms);
-//  * mst_scan: builds a worklist of int4 {a, b, weight, j} from the CSR,
-//    lane-level for lists <= 32 entries, warp-level up to 256, chunk
-//    records beyond; appends are staged per warp in shared memory and
-//    reserved in the global list with one atomic per ~kStage entries;
+//    the quantile that leaves ~0.75 n (2 n in a sparse graph) light CSR
+//    entries, with no host round trip;
+//  * mst_scan: builds a worklist of int4 {a, b, weight, j} from the CSR in
+//    tiles of 256 entries a warp, whatever rows they belong to; appends are
+//    staged per warp in shared memory and reserved in the global list with one
+//    atomic per ~kStage entries;
 //    the heavy pass drops entries whose endpoints are already joined (the
 //    forest is flattened by pointer jumping first, so a root is one load);
 //  * mst_boruvka: ALL Boruvka rounds in one cooperative persistent launch, three
@@ -31,6 +29,7 @@
 #include <algorithm>
 
 #include "csr_bins.cuh"
+#include "flat_scan.cuh"
 #include "grid_sync.cuh"
 #include "solvers.cuh"
 
@@ -41,20 +40,23 @@ using namespace dev;
 typedef unsigned long long u64;
 
 constexpr int kTPB = 256;
-// Default degree bins: rows of <= 32 entries per lane, chunk records of 256
-// entries (R-MAT's heavy low-id rows share warp groups: keep warp rows short).
-constexpr Bins kMstBins{32, 256};
 constexpr int kMaxRounds = 64;
+// Light entries aimed at, in multiples of n: 0.75 from this average degree on,
+// 2 below.  Rounds whose list does not shrink cost most; in a sparse random
+// graph the light edges have to join most vertices (about n of them) before
+// the heavy pass drops the bulk of its entries in the scan, while a dense
+// power-law graph's hubs do that with few.  Measured, 0.75 / 1.5 / 2.5: G(3 M,
+// 12 M) 2.06 / 1.12 / 1.09 ms, G(150 k, 600 k) 0.314 / 0.302 / 0.299, R-MAT-22
+// (degree 30) 1.67 / 1.69 / 1.78.
+constexpr int kDenseDegree = 16;
 constexpr int kSamples = 1024;
 
 struct MSTCtl {
   GridBarrier bar;
   int wlcount[2][kMaxRounds + 2];    // [pass][round] sizes of the edge list
   int rootcount[2][kMaxRounds + 2];  // [pass][round] roots that may still have edges
-  int nchunks;
   int threshold;
   int filter;
-  int pad;
   u64 total;
   // %globaltimer when each pass started and after each of its barriers
   // (phases A, B and C of round r end at [3r + 1], [3r + 2] and [3r + 3]): a
@@ -85,12 +87,17 @@ __global__ void __launch_bounds__(kTPB) mst_flatten(int n, int* __restrict__ par
   }
 }
 
-__global__ void mst_init(int n, int* __restrict__ parent, u64* __restrict__ minv) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+// Also finds the rows of the scans' tiles (and so checks the CSR rows once: a
+// malformed row raises ECL_ERR_BAD_GRAPH).
+__global__ void __launch_bounds__(kTPB) mst_init(int n, int m, const int* __restrict__ nindex, int* __restrict__ parent,
+                                                 u64* __restrict__ minv, int* __restrict__ tilerow,
+                                                 Status* __restrict__ status) {
+  for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     // race-free: thread-owned init, no reader in this launch
     parent[v] = v;
     minv[v] = ~0ull;
   }
+  if (m > 0) flat_rows_range(n, m, nindex, tilerow, (blockIdx.x * kTPB + threadIdx.x) & ~31, gridDim.x * kTPB, status);
 }
 
 // Threshold = the k-th smallest of kSamples sampled weights, k chosen so the
@@ -131,11 +138,6 @@ __global__ void __launch_bounds__(kSamples) mst_threshold(int n, int m, const in
   }
 }
 
-template <bool kLight>
-__device__ __forceinline__ bool mst_keep(int w, int thr) {
-  return kLight ? (w <= thr) : (w > thr);
-}
-
 // Slots per warp in the shared-memory staging of worklist appends.
 constexpr int kStage = 128;
 // Worklists are 16 B per edge (100 MB each for R-MAT-22's light edges):
@@ -143,233 +145,80 @@ constexpr int kStage = 128;
 // arrays, which Boruvka reads at random, stay in L2.
 typedef WarpStage<int4, kStage, true> Stage;
 
-// Entries per lane whose loads are issued together in the scans.
-constexpr int kScanBatch = 4;
-
-// Emits the worklist entries for kScanBatch CSR entries of vertex v per lane
-// (rv = v's root in the heavy pass): entry k of this lane is j0 + k * stride,
-// present when `active` and below jend.  All index loads, then the weight
-// loads of the v < u entries, then (heavy pass) their roots are in flight
-// together before any is used; every lane pushes kScanBatch times.
-template <bool kLight>
-__device__ __forceinline__ void mst_emit_batch(int j0, int stride, int jend, bool active, int v, int rv, int n,
-                                               const int* nlist, const int* eweight, int thr, const int* parent,
-                                               Stage& stg, int4* wl, int* cnt, int cap, bool& overflow,
-                                               Status* status) {
-  int u[kScanBatch], w[kScanBatch], ru[kScanBatch];
-#pragma unroll
-  for (int k = 0; k < kScanBatch; k++) {
-    const int j = j0 + k * stride;
-    u[k] = (active && j < jend) ? __ldg(&nlist[j]) : -1;
-  }
-  if (kLight) {
-#pragma unroll
-    for (int k = 0; k < kScanBatch; k++) {
-      const int j = j0 + k * stride;
-      w[k] = ((unsigned)u[k] < (unsigned)n && u[k] > v) ? __ldg(&eweight[j]) : 0;
-      ru[k] = -1;
-    }
-  } else {
-    // Heavy pass: the root first (flat after mst_flatten), the weight only
-    // for entries between two components.  The light pass joined the ends of
-    // every light entry (and checked every weight), so those are all heavy,
-    // and the ~80 % of entries inside one component cost no weight load.
-#pragma unroll
-    for (int k = 0; k < kScanBatch; k++)
-      ru[k] = ((unsigned)u[k] < (unsigned)n && u[k] > v) ? ld(&parent[u[k]]) : -1;
-#pragma unroll
-    for (int k = 0; k < kScanBatch; k++) {
-      const int j = j0 + k * stride;
-      w[k] = (ru[k] >= 0 && ru[k] != rv) ? __ldg(&eweight[j]) : 0;
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < kScanBatch; k++) {
-    const int j = j0 + k * stride;
-    bool keep = false;
-    int4 e = make_int4(0, 0, 0, 0);
-    if (active && j < jend) {
-      if ((unsigned)u[k] >= (unsigned)n) {
-        raise(status, ECL_ERR_BAD_GRAPH, u[k]);
-      } else if (u[k] > v) {
-        if (w[k] < 0) {
-          raise(status, ECL_ERR_BAD_GRAPH, j);
-        } else if (kLight) {
-          if (mst_keep<true>(w[k], thr)) {
-            keep = true;
-            e = make_int4(v, u[k], w[k], j);
-          }
-        } else if (ru[k] != rv) {
-          keep = true;
-          e = make_int4(rv, ru[k], w[k], j);
-        }
-      }
-    }
-    stg.push(keep, e, wl, cnt, cap, overflow);
-  }
-}
-
-// Emits the worklist entries of one warp-walked row segment [jb, je) of v.
-// With `vec` (nlist and eweight 16-byte aligned) the segment is walked in
-// 16-byte-aligned quads of entries, one quad a lane (128 entries a warp
-// step): one 16-byte load of nlist and, when any of the quad's entries is a
-// v < u entry, one of eweight.  The quads at the segment's ends are masked to
-// it, and a quad reaching past the arrays' m entries is read entry by entry.
-// Without `vec` the scalar mst_emit_batch walks it.  All lanes call.
-template <bool kLight>
-__device__ __forceinline__ void mst_emit_row(int jb, int je, int m, bool vec, int v, int rv, int n, const int* nlist,
-                                             const int* eweight, int thr, const int* parent, Stage& stg, int4* wl,
-                                             int* cnt, int cap, bool& overflow, Status* status) {
-  const int lane = threadIdx.x & 31;
-  if (!vec) {
-    for (int i0 = jb; i0 < je; i0 += 32 * kScanBatch)
-      mst_emit_batch<kLight>(i0 + lane, 32, je, true, v, rv, n, nlist, eweight, thr, parent, stg, wl, cnt, cap,
-                             overflow, status);
-    return;
-  }
-  for (int i0 = jb & ~3; i0 < je; i0 += 4 * 32) {
-    const int q = i0 + 4 * lane;  // this lane's quad [q, q + 4)
-    const bool whole = q + 4 <= m && q < je;
-    bool valid[4];
-    int u[4], w[4] = {0, 0, 0, 0}, ru[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) valid[k] = q + k >= jb && q + k < je;
-    if (whole) {
-      const int4 x = __ldg(reinterpret_cast<const int4*>(nlist + q));
-      u[0] = x.x, u[1] = x.y, u[2] = x.z, u[3] = x.w;
-    } else {
-#pragma unroll
-      for (int k = 0; k < 4; k++) u[k] = valid[k] ? __ldg(&nlist[q + k]) : -1;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (!valid[k]) u[k] = -1;
-    if (u[0] > v || u[1] > v || u[2] > v || u[3] > v) {
-      if (whole) {
-        const int4 y = __ldg(reinterpret_cast<const int4*>(eweight + q));
-        w[0] = y.x, w[1] = y.y, w[2] = y.z, w[3] = y.w;
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; k++) w[k] = u[k] > v ? __ldg(&eweight[q + k]) : 0;
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      ru[k] = (!kLight && (unsigned)u[k] < (unsigned)n && u[k] > v && mst_keep<false>(w[k], thr))
-                  ? ld(&parent[u[k]])  // flat after mst_flatten
-                  : -1;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int j = q + k;
-      bool keep = false;
-      int4 e = make_int4(0, 0, 0, 0);
-      if (valid[k]) {
-        if ((unsigned)u[k] >= (unsigned)n) {
-          raise(status, ECL_ERR_BAD_GRAPH, u[k]);
-        } else if (u[k] > v) {
-          if (w[k] < 0) {
-            raise(status, ECL_ERR_BAD_GRAPH, j);
-          } else if (mst_keep<kLight>(w[k], thr)) {
-            if (kLight) {
-              keep = true;
-              e = make_int4(v, u[k], w[k], j);
-            } else {
-              keep = ru[k] != rv;
-              e = make_int4(rv, ru[k], w[k], j);
-            }
-          }
-        }
-      }
-      stg.push(keep, e, wl, cnt, cap, overflow);
-    }
-  }
-}
-
 // More v<n entries than the worklist holds: an asymmetric graph flagged
 // symmetric.
 __device__ __forceinline__ void mst_overflow(bool overflow, Status* status) {
   if (__any_sync(kFull, overflow) && (threadIdx.x & 31) == 0) raise(status, ECL_ERR_BAD_GRAPH, -2);
 }
 
+// The worklist entries of a pass, from one pass over the CSR in tiles of 256
+// entries a warp (flat_scan.cuh): the v < u entries of light weight, as they
+// are; or, for the heavy pass, those whose ends lie in different components,
+// as their roots.  The heavy pass loads an entry's root first and its weight
+// only for entries between two components: the light pass joined the ends of
+// every light entry (and checked every weight), so those are all heavy, and
+// the ~80 % of entries inside one component cost no weight load.  parent[] is
+// flat and not written in this launch, so its loads are read-only ones that L1
+// serves.  Bound by the stream of nlist and weights (light) and by the 4-byte
+// root gathers, one for half the entries (heavy), and in both by about 400 to 650 warp
+// instructions a tile.  Measured at R-MAT-22, rows per lane / warp / chunk
+// record in two launches -> this: light 0.55 -> 0.32 ms, heavy (with the
+// flattening) 0.86 -> 0.55; 1000 vertices, 12 k entries: 36 -> 9 us and 50 -> 13.
 template <bool kLight>
-__global__ void __launch_bounds__(kTPB) mst_scan(int n, int m, const int* __restrict__ nindex,
-                                                 const int* __restrict__ nlist, const int* __restrict__ eweight,
-                                                 int* __restrict__ parent, int4* __restrict__ wl, int cap,
-                                                 MSTCtl* __restrict__ ctl, int2* __restrict__ chunks, Bins bins,
-                                                 bool vec, Status* __restrict__ status) {
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * kTPB) >> 5;
+__global__ void __launch_bounds__(kTPB) mst_scan(FlatCsr g, bool vec, const int* __restrict__ eweight,
+                                                 const int* __restrict__ parent, int4* __restrict__ wl, int cap,
+                                                 MSTCtl* __restrict__ ctl, Status* __restrict__ status) {
+  __shared__ int4 stage_buf[kTPB / 32][kStage];
+  __shared__ __align__(16) int s_mark[kTPB / 32][kFlatTile];
+  const int wid = threadIdx.x >> 5;
   const int thr = ctl->threshold;
   int* cnt = &ctl->wlcount[kLight ? 0 : 1][0];
-  __shared__ int4 stage_buf[kTPB / 32][kStage];
-  Stage stg{stage_buf[threadIdx.x >> 5]};
+  Stage stg{stage_buf[wid]};
   bool overflow = false;
-  for (int base = warp * 32; base < n; base += nwarps * 32) {
-    const int v = base + lane;
-    int beg = 0, end = 0;
-    if (v < n) {
-      beg = __ldg(&nindex[v]);
-      end = __ldg(&nindex[v + 1]);
-      if (beg < 0 || end < beg || end > m) {
-        raise(status, ECL_ERR_BAD_GRAPH, v);
-        beg = end = 0;
+  const int stop = min(g.m, __ldg(&g.nindex[g.n]));
+  const int tiles = flat_tiles(g.m);
+  for (int t = blockIdx.x * (kTPB / 32) + wid; t < tiles; t += gridDim.x * (kTPB / 32))
+    flat_tile(g, stop, vec, t, s_mark[wid], [&](int e0, const int (&row)[kFlatLane], const int (&u)[kFlatLane]) {
+      unsigned want = 0;  // bit k: entry k may be kept
+#pragma unroll
+      for (int k = 0; k < kFlatLane; k++) {
+        if ((unsigned)u[k] >= (unsigned)g.n)
+          raise(status, ECL_ERR_BAD_GRAPH, u[k]);
+        else if (row[k] >= 0 && u[k] > row[k])
+          want |= 1u << k;
       }
-    }
-    const int deg = end - beg;
-    const bool lanelvl = deg > 0 && deg <= bins.lane;
-    int rv = v;
-    if (!kLight && deg > 0 && v < n) rv = ld(&parent[v]);
-    if (kLight)  // chunk records are built once, in the light pass
-      push_chunks_warp(RowChunks{chunks, &ctl->nchunks, (int)row_chunk_capacity(m, kMinChunk)}, bins.chunk,
-                       deg > bins.chunk, v, beg, end, status);
-    // lane level: all lanes step through offset k together
-    const int kmax = __reduce_max_sync(kFull, lanelvl ? deg : 0);
-    for (int k0 = 0; k0 < kmax; k0 += kScanBatch)
-      mst_emit_batch<kLight>(beg + k0, 1, end, lanelvl, v, rv, n, nlist, eweight, thr, parent, stg, wl, cnt, cap,
-                             overflow, status);
-    // warp level
-    unsigned todo = __ballot_sync(kFull, deg > bins.lane && deg <= bins.chunk);
-    while (todo) {
-      const int who = __ffs(todo) - 1;
-      todo &= todo - 1;
-      const int wv = __shfl_sync(kFull, v, who);
-      const int wrv = __shfl_sync(kFull, rv, who);
-      const int wbeg = __shfl_sync(kFull, beg, who);
-      const int wend = __shfl_sync(kFull, end, who);
-      mst_emit_row<kLight>(wbeg, wend, m, vec, wv, wrv, n, nlist, eweight, thr, parent, stg, wl, cnt, cap, overflow,
-                           status);
-    }
-  }
-  stg.flush(wl, cnt, cap, overflow);
-  mst_overflow(overflow, status);
-  // chunk records (hubs): the light pass sees them only after all warps
-  // passed the vertex loop, so they are handled by mst_chunks.
-}
-
-template <bool kLight>
-__global__ void __launch_bounds__(kTPB) mst_chunks(int n, int m, const int* __restrict__ nindex,
-                                                   const int* __restrict__ nlist,
-                                                   const int* __restrict__ eweight, int* __restrict__ parent,
-                                                   int4* __restrict__ wl, int cap, MSTCtl* __restrict__ ctl,
-                                                   const int2* __restrict__ chunks, int chunk_cap, int chunk,
-                                                   bool vec, Status* __restrict__ status) {
-  const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * kTPB) >> 5;
-  const int thr = ctl->threshold;
-  int* cnt = &ctl->wlcount[kLight ? 0 : 1][0];
-  const int total = min((unsigned)ctl->nchunks, (unsigned)chunk_cap);
-  __shared__ int4 stage_buf[kTPB / 32][kStage];
-  Stage stg{stage_buf[threadIdx.x >> 5]};
-  bool overflow = false;
-  for (int c = warp; c < total; c += nwarps) {
-    const int2 rec = chunks[c];
-    const int v = rec.x;
-    const int end = min(rec.y + chunk, __ldg(&nindex[v + 1]));
-    const int rv = kLight ? v : ld(&parent[v]);
-    mst_emit_row<kLight>(rec.y, end, m, vec, v, rv, n, nlist, eweight, thr, parent, stg, wl, cnt, cap, overflow, status);
-  }
+      int a[kFlatLane], b[kFlatLane], w[kFlatLane];
+      if (!kLight) {
+#pragma unroll
+        for (int k = 0; k < kFlatLane; k++) b[k] = (want >> k) & 1u ? __ldg(&parent[u[k]]) : -1;  // race-free: not written in this launch
+#pragma unroll
+        for (int k = 0; k < kFlatLane; k++) {
+          a[k] = -1;
+          if (!((want >> k) & 1u)) continue;
+          a[k] = k > 0 && row[k] == row[k - 1] && a[k - 1] >= 0 ? a[k - 1] : __ldg(&parent[row[k]]);  // race-free: as above
+          if (a[k] == b[k]) want &= ~(1u << k);
+        }
+      }
+      if (kLight && vec && want && e0 <= g.m - kFlatLane) {
+        const int4 x = __ldcs(reinterpret_cast<const int4*>(eweight + e0));
+        const int4 y = __ldcs(reinterpret_cast<const int4*>(eweight + e0 + 4));
+        w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w, w[4] = y.x, w[5] = y.y, w[6] = y.z, w[7] = y.w;
+      } else {
+#pragma unroll
+        for (int k = 0; k < kFlatLane; k++) w[k] = (want >> k) & 1u ? __ldcs(&eweight[e0 + k]) : 0;
+      }
+#pragma unroll
+      for (int k = 0; k < kFlatLane; k++) {
+        bool keep = (want >> k) & 1u;
+        if (keep && w[k] < 0) {
+          raise(status, ECL_ERR_BAD_GRAPH, e0 + k);
+          keep = false;
+        }
+        if (kLight) keep = keep && w[k] <= thr;
+        if (__any_sync(kFull, keep))
+          stg.push(keep, make_int4(kLight ? row[k] : a[k], kLight ? u[k] : b[k], w[k], e0 + k), wl, cnt, cap, overflow);
+      }
+    });
   stg.flush(wl, cnt, cap, overflow);
   mst_overflow(overflow, status);
 }
@@ -607,8 +456,7 @@ struct MSTBufs {
   u64* minv;
   int* rootsA;
   int* rootsB;
-  int2* chunks;
-  int chunk_cap;
+  int* tilerow;
   int4* wlA;
   int4* wlB;
   int cap;
@@ -620,8 +468,7 @@ void mst_layout(Carve& c, int n, int m, bool symmetric, MSTBufs* b) {
   b->minv = c.take<u64>((size_t)n);
   b->rootsA = c.take<int>((size_t)n);
   b->rootsB = c.take<int>((size_t)n);
-  b->chunks = c.take<int2>(row_chunk_capacity(m, kMinChunk));
-  b->chunk_cap = (int)row_chunk_capacity(m, kMinChunk);
+  b->tilerow = c.take<int>((size_t)flat_tiles(m) + 1);
   // v<n entries: at most m/2 in a symmetric, self-loop-free graph, else m.
   b->cap = symmetric ? m / 2 + 1 : (m > 0 ? m : 1);
   b->wlA = c.take<int4>((size_t)b->cap);
@@ -649,30 +496,25 @@ ecl_status mst_enqueue(const GraphDev& g, unsigned char* in_mst, char* ws, Statu
   const int coop_grid = std::max(1, std::min(dev.sms, std::max(g.n, g.m) / 8192));
   ECL_CUDA_TRY(cudaFuncSetAttribute(mst_boruvka, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBorSmem));
   const int grid = dev.grid_blocks(kTPB, g.n, g.m);
-  const Bins bins = bins_of(dev, kMstBins);
-  // 16-byte row loads need 16-byte-aligned arrays (entries j = 0 mod 4 then are)
-  const bool vec =
-      ((reinterpret_cast<uintptr_t>(g.nlist) | reinterpret_cast<uintptr_t>(g.eweight)) & 15) == 0 && dev.row_vec;
+  // 16-byte loads need 16-byte-aligned arrays (a lane's entries start at a multiple of 8)
+  const bool vec = ((reinterpret_cast<uintptr_t>(g.nlist) | reinterpret_cast<uintptr_t>(g.eweight)) & 15) == 0;
+  const int scan_grid = dev.grid_blocks(kTPB, 0, g.m);  // a thread per lane's share of a tile
+  const FlatCsr fc{g.n, g.m, g.nindex, g.nlist, b.tilerow};
   if (total_dev) *total_dev = &b.ctl->total;
   ECL_CUDA_TRY(cudaMemsetAsync(b.ctl, 0, sizeof(MSTCtl), stream));
   if (g.m > 0) ECL_CUDA_TRY(cudaMemsetAsync(in_mst, 0, (size_t)g.m, stream));
-  ECL_LAUNCH(mst_init, grid, kTPB, 0, stream, g.n, b.parent, b.minv);
+  ECL_CUDA_TRY(cudaMemsetAsync(b.tilerow, 0xff, sizeof(int) * ((size_t)flat_tiles(g.m) + 1), stream));
+  ECL_LAUNCH(mst_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, b.parent, b.minv, b.tilerow, status);
   if (g.m > 0) {
-    const float light = dev.mst_light_factor > 0.f ? dev.mst_light_factor : 0.75f;
+    const float light = dev.mst_light_factor > 0.f ? dev.mst_light_factor : (g.m / g.n >= kDenseDegree ? 0.75f : 2.f);
     ECL_LAUNCH(mst_threshold, 1, kSamples, 0, stream, g.n, g.m, g.eweight, b.ctl, light);
     mark();
     for (int pass = 0; pass < 2; pass++) {
       if (pass == 0) {
-        ECL_LAUNCH(mst_scan<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, g.eweight, b.parent, b.wlA,
-                   b.cap, b.ctl, b.chunks, bins, vec, status);
-        ECL_LAUNCH(mst_chunks<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, g.eweight, b.parent, b.wlA, b.cap,
-                   b.ctl, b.chunks, b.chunk_cap, bins.chunk, vec, status);
+        ECL_LAUNCH(mst_scan<true>, scan_grid, kTPB, 0, stream, fc, vec, g.eweight, b.parent, b.wlA, b.cap, b.ctl, status);
       } else {
         ECL_LAUNCH(mst_flatten, grid, kTPB, 0, stream, g.n, b.parent);
-        ECL_LAUNCH(mst_scan<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, g.eweight, b.parent, b.wlA,
-                   b.cap, b.ctl, b.chunks, bins, vec, status);
-        ECL_LAUNCH(mst_chunks<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, g.eweight, b.parent, b.wlA, b.cap,
-                   b.ctl, b.chunks, b.chunk_cap, bins.chunk, vec, status);
+        ECL_LAUNCH(mst_scan<false>, scan_grid, kTPB, 0, stream, fc, vec, g.eweight, b.parent, b.wlA, b.cap, b.ctl, status);
       }
       mark();
       ECL_CUDA_TRY(launch_cooperative_smem(mst_boruvka, coop_grid, kBorTPB, kBorSmem, stream, g.n, pass, b.wlA,

@@ -173,6 +173,37 @@ def test_scc_matches_tarjan(ecl, orc):
         assert np.array_equal(got, orc.scc(g)), name
 
 
+def flat_cases():
+    """Rows against the 256-entry tiles of the entry-balanced scans, and average
+    degrees on both sides of the MST light-edge rule."""
+    yield "ring", undirected(128, [(i, (i + 1) % 128) for i in range(128)])  # rows end exactly on a tile's end
+    yield "ring129", undirected(129, [(i, (i + 1) % 129) for i in range(129)])
+    yield "hub", undirected(5000, [(4999, i) for i in range(4600)] + [(0, i) for i in range(1, 700)])  # rows of many tiles
+    yield "empty_run", undirected(9000, [(0, 8999), (1, 8999), (8998, 8999)])  # over 2048 empty rows in one tile
+    yield "two", undirected(2, [(0, 1)])
+    yield "clique48", undirected(48, [(i, j) for i in range(48) for j in range(i)])
+    yield "clique600", undirected(600, [(i, j) for i in range(600) for j in range(i)])
+
+
+def test_mst_at_scan_tile_edges(ecl, orc):
+    import torch
+
+    for name, g in flat_cases():
+        rng = np.random.default_rng(g.edges)
+        for weight_max in (2, 1000):  # ties everywhere, and few
+            row = np.repeat(np.arange(g.nodes), np.diff(g.nindex))
+            w = rng.integers(1, weight_max, size=(g.nodes, 1 + g.nodes % 97)).astype(np.int32)
+            lo, hi = np.minimum(row, g.nlist), np.maximum(row, g.nlist)
+            g.eweight = w[lo, hi % w.shape[1]].astype(np.int32)
+            flags, total = orc.mst(g)
+            dg = g.to_device()
+            got, t = ecl.mst(dg)
+            assert t == total and np.array_equal(got.cpu().numpy(), flags), (name, weight_max)
+            dg.nlist = torch.cat((dg.nlist[:1], dg.nlist))[1:]  # entries off the 16-byte boundaries
+            got, t = ecl.mst(dg)
+            assert t == total and np.array_equal(got.cpu().numpy(), flags), (name, weight_max)
+
+
 def flagged_cases(ecl):
     """Graphs flagged symmetric: truly so, and falsely (SCC then must not rely on it)."""
     yield "grid", ecl.gen_grid(70, 90, 0.3, seed=2)
