@@ -19,7 +19,7 @@ namespace ecl {
 namespace dev {
 
 struct GridBarrier {
-  unsigned count;  // arrivals since the launch (zeroed before it)
+  unsigned count;  // arrivals (zeroed before the first launch; all launches that share it have one grid size)
   unsigned pad[63];
 };
 

@@ -10,7 +10,10 @@
 // is the largest vertex id of v's SCC -- schedule independent.
 //
 // B200 design:
-//  * graphs flagged symmetric are first tried as connected components (below);
+//  * graphs flagged symmetric are first tried as connected components, and in
+//    a large graph the component of the vertex with the most entries is found
+//    by a forward and a backward search (both below); what follows is for the
+//    edges that are left;
 //  * scc_mark trims first: a vertex with no in-entry or no out-entry
 //    (self-loops ignored) is its own SCC and contributes no edge.  The same
 //    pass writes the int2 edge list in CSR positions -- slot i holds
@@ -35,6 +38,9 @@
 //    which raised nothing, so it read final words -- leaves the next round's
 //    list without a separate pass;
 //  * the final labels are written by the same launch (label = in-max).
+#include <algorithm>
+#include <type_traits>
+
 #include "csr_bins.cuh"
 #include "flat_scan.cuh"
 #include "grid_sync.cuh"
@@ -50,11 +56,23 @@ constexpr int kMaxSweeps = 1 << 16;
 constexpr int kScanBatch = 4;  // list entries per lane whose loads are issued together
 
 constexpr int kStamps = 256;
+constexpr int kGiantLevels = 40;
+constexpr int kGiantRounds = 40;
 
 struct SCCCtl {
-  GridBarrier bar;
+  GridBarrier bar;        // scc_solve's
+  GridBarrier giant_bar;  // scc_giant's (another grid: a barrier counts in multiples of one)
   unsigned long long asym;  // scc_symmetry's sum: 0 iff every entry has its reverse
-  int pad[62];
+  // scc_giant
+  unsigned long long pivot;  // (out-degree << 32) | ~id of the vertex with the most entries
+  int giant_ok;              // 1: the pivot's component is found
+  int giant_label;           // its largest id
+  int rest;                  // edges scc_mark<true> kept for scc_solve
+  int level_new[kGiantLevels];     // per forward level: vertices it added to the queue
+  int level_chunks[kGiantLevels];  // ... and chunk records of its long rows
+  int left[kGiantRounds + 1];  // per backward round: vertices not known to reach the pivot
+  int moved[kGiantRounds];     // per backward round: some vertex was found to reach it
+  int pad[64];
   // %globaltimer at the start and after each grid barrier (the first
   // kStamps - 1): a time profile of sweeps, compactions and retirements that
   // costs one store per barrier
@@ -185,6 +203,284 @@ __global__ void __launch_bounds__(kTPB) scc_relabel(int n, int* __restrict__ com
   }
 }
 
+// ---- the giant component ----
+//
+// Most directed graphs that are not meshes have one component with most of the
+// edges.  Before any propagation scc_giant finds the component of the vertex
+// with the most out-entries: the vertices it reaches (forward search over a
+// queue, every edge looked at once), and of those the ones that reach it (each
+// looks for one out-neighbour known to, and stops at the first: two or three
+// entries a vertex).  What is left for the propagation sweeps -- each of them
+// two random words for every edge -- is the few edges between other vertices
+// on the same side of the search.  The forward search gives up on graphs whose
+// distances are long (kGiantLevels levels, or few vertices reached by level
+// kGiantPatience); the sweeps then run on all edges as before.
+// Bound by the latency of the two widest levels' look-ups (a third of the time
+// each at R-MAT-22).  Measured, whole solve, sweeps over all edges -> this:
+// directed R-MAT-22 (65 M edges) 2.47 -> 0.83 ms, 500 k vertices (5.7 M) 0.58
+// -> 0.33, G(3 M, 12 M) 2.14 -> 1.45; a 701 x 1031 grid without cycles, where
+// it gives up, 17.3 -> 17.4.
+constexpr int kGTPB = 512;
+constexpr int kGiantPatience = 16;
+constexpr int kGiantEntries = 1 << 20;  // from this many entries on: R-MAT with 0.45 M entries 229 -> 227 us, 1.05 M 266 -> 250,
+                                        // 1.8 M 363 -> 261; G(150 k, 600 k) 329 -> 444, G(400 k, 1.6 M) 546 -> 532
+constexpr int kGiantLong = 256;   // longer rows are cut into chunk records of this many entries
+
+struct Giant {
+  unsigned* fwd;  // bit per vertex: reached from the pivot
+  unsigned* bwd;  // bit per vertex: reaches the pivot (complete inside fwd)
+  __device__ __forceinline__ bool has(const unsigned* bits, int v) const { return (__ldg(&bits[v >> 5]) >> (v & 31)) & 1u; }
+  // After scc_giant's launch.
+  __device__ __forceinline__ bool in(int v) const { return has(fwd, v) && has(bwd, v); }
+};
+
+// Visits the entries of 32 rows, one per lane ([beg, beg + deg)), spread evenly
+// over the warp: f(owner, j, valid) for entry j of lane `owner`'s row, four
+// steps of 32 consecutive entries per call round.  All lanes call f together.
+template <class F>
+__device__ __forceinline__ void warp_rows(int beg, int deg, F&& f) {
+  const int lane = threadIdx.x & 31;
+  int incl = deg;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(kFull, incl, o);
+    if (lane >= o) incl += x;
+  }
+  const int excl = incl - deg, total = __shfl_sync(kFull, incl, 31);
+  for (int base = 0; base < total; base += 128) {
+    int owner[4], j[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int e = base + 32 * k + lane;
+      int lo = 0;  // the last lane whose row starts at or before e
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (__shfl_sync(kFull, excl, lo + o) <= e) lo += o;
+      owner[k] = lo;
+      j[k] = __shfl_sync(kFull, beg, lo) + e - __shfl_sync(kFull, excl, lo);
+      if (e >= total) j[k] = -1;
+    }
+    f(owner, j);
+  }
+}
+
+// bits |= next, next = 0, for all words; the caller's barriers are around it.
+__device__ __forceinline__ void merge_bits(unsigned* bits, unsigned* next, int words, int tid, int nthreads) {
+  for (int i = tid; i < words; i += nthreads) {
+    const unsigned x = ld(&next[i]);
+    if (x == 0) continue;
+    bits[i] |= x;  // race-free: word i is this thread's between the barriers
+    st(&next[i], 0u);
+  }
+}
+
+// The bits that a level (round) finds go to `next`, and fwd (bwd) is not
+// written before its end: looking a vertex up first there is a plain load that
+// L1 serves.  The hubs that most edges lead to are found in the first levels;
+// looked up by relaxed loads, the few words that hold their bits were the
+// bound (R-MAT-22: 1.18 ms for the whole search against 0.6).
+__global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* __restrict__ nindex,
+                                                      const int* __restrict__ nlist, unsigned* fwd, unsigned* bwd,
+                                                      unsigned* next, int* queue, int* candA, int* candB, int2* chunks,
+                                                      int chunk_cap, SCCCtl* __restrict__ ctl, bool checked,
+                                                      Status* __restrict__ status) {
+  if (checked && ld(&ctl->asym) == 0) return;  // as scc_mark
+  __shared__ int s_stage[kGTPB / 32][128];
+  __shared__ int s_moved;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int tid = blockIdx.x * kGTPB + threadIdx.x, nthreads = gridDim.x * kGTPB;
+  const int warp = tid >> 5, nwarps = nthreads >> 5;
+  const int words = (n + 31) / 32;
+  WarpStage<int, 128> stg{s_stage[wid]};
+  bool overflow = false;
+  // row of v; a malformed one (reported by scc_mark) is empty
+  auto row_of = [&](int v, int& beg, int& deg) {
+    beg = __ldg(&nindex[v]);
+    const int end = __ldg(&nindex[v + 1]);
+    deg = end - beg;
+    if (beg < 0 || end < beg || end > m) beg = deg = 0;
+  };
+  // the pivot
+  unsigned long long key = 0;
+  for (int v = tid; v < n; v += nthreads) {
+    int beg, deg;
+    row_of(v, beg, deg);
+    key = max(key, ((unsigned long long)deg << 32) | (0xffffffffu - (unsigned)v));
+  }
+  for (int o = 16; o > 0; o >>= 1) key = max(key, __shfl_xor_sync(kFull, key, o));
+  if (lane == 0 && key > ld(&ctl->pivot)) fetch_max(&ctl->pivot, key);
+  if (!grid_sync(&ctl->giant_bar, status)) return;
+  key = ld(&ctl->pivot);
+  if ((key >> 32) == 0) return;  // no entries at all
+  const int pivot = (int)(0xffffffffu - (unsigned)key);
+  if (tid == 0) {
+    fetch_or(&fwd[pivot >> 5], 1u << (pivot & 31));
+    fetch_or(&bwd[pivot >> 5], 1u << (pivot & 31));
+    queue[0] = pivot;
+  }
+  if (!grid_sync(&ctl->giant_bar, status)) return;
+  int qs = 0, qe = 1, level = 0;
+  // chunk records of the frontier's long rows
+  auto cut_long_rows = [&]() {
+    const RowChunks rc{chunks, &ctl->level_chunks[level], chunk_cap};
+    for (int i0 = qs + warp * 32; i0 < qe; i0 += nwarps * 32) {
+      const int i = i0 + lane;
+      const int v = i < qe ? queue[i] : 0;  // written before the last grid barrier
+      int beg = 0, deg = 0;
+      if (i < qe) row_of(v, beg, deg);
+      push_chunks_warp(rc, kGiantLong, deg > kGiantLong, v, beg, beg + deg, status);
+    }
+  };
+  // the entries j[k] of the rows of v[k]: newly reached vertices join the queue
+  // behind its present end (counted per level: a block may still be reading the
+  // last level's count when another one is adding to the next), and an entry
+  // that is the pivot says that v[k] reaches it
+  auto reach = [&](auto count, const int* v, const int* j) {
+    constexpr int K = decltype(count)::value;
+    int w[K];
+    unsigned have[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) w[k] = j[k] >= 0 ? __ldg(&nlist[j[k]]) : -1;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      if (j[k] >= 0 && (unsigned)w[k] >= (unsigned)n) {
+        raise(status, ECL_ERR_BAD_GRAPH, w[k]);
+        w[k] = -1;
+      }
+      have[k] = w[k] >= 0 ? fwd[w[k] >> 5] : ~0u;  // race-free: not written during a level
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (!((have[k] >> (w[k] & 31)) & 1u)) have[k] = ld(&next[w[k] >> 5]);
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const unsigned bit = 1u << (w[k] & 31);
+      const bool found = !(have[k] & bit) && !(fetch_or(&next[w[k] >> 5], bit) & bit);
+      if (w[k] == pivot) fetch_or(&bwd[v[k] >> 5], 1u << (v[k] & 31));
+      if (__any_sync(kFull, found)) stg.push(found, w[k], queue + qe, &ctl->level_new[level], n - qe, overflow);
+    }
+  };
+  cut_long_rows();
+  if (!grid_sync(&ctl->giant_bar, status)) return;
+  for (; qs < qe; level++) {
+    if (level + 1 == kGiantLevels || (level == kGiantPatience && qe < n / 64)) return;  // long distances: not this way
+    const int nch = chunk_total(RowChunks{chunks, &ctl->level_chunks[level], chunk_cap});
+    for (int c = warp; c < nch; c += nwarps) {
+      const int2 r = chunks[c];
+      const int end = min(r.y + kGiantLong, __ldg(&nindex[r.x + 1]));
+      constexpr int K = kGiantLong / 32;
+      int vv[K], j[K];
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        vv[k] = r.x;
+        j[k] = r.y + 32 * k + lane < end ? r.y + 32 * k + lane : -1;
+      }
+      reach(std::integral_constant<int, K>{}, vv, j);
+    }
+    // a warp takes up to 32 rows at a time, fewer while there are not enough
+    // for all warps (the hubs stand side by side in the queue)
+    const int per = min(32, (qe - qs - 1) / nwarps + 1);
+    for (int i0 = qs + warp * per; i0 < qe; i0 += nwarps * per) {
+      const int i = lane < per ? i0 + lane : qe;
+      const int v = i < qe ? queue[i] : 0;  // written before the last grid barrier
+      int beg = 0, deg = 0;
+      if (i < qe) row_of(v, beg, deg);
+      if (deg > kGiantLong) deg = 0;  // in chunk records
+      warp_rows(beg, deg, [&](const int (&owner)[4], const int (&j)[4]) {
+        int vv[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) vv[k] = __shfl_sync(kFull, v, owner[k]);
+        reach(std::integral_constant<int, 4>{}, vv, j);
+      });
+    }
+    stg.flush(queue + qe, &ctl->level_new[level], n - qe, overflow);
+    if (!grid_sync(&ctl->giant_bar, status)) return;
+    merge_bits(fwd, next, words, tid, nthreads);
+    qs = qe;
+    qe += ld(&ctl->level_new[level]);
+    level++;
+    cut_long_rows();
+    level--;
+    if (!grid_sync(&ctl->giant_bar, status)) return;
+  }
+  // backward, inside the vertices reached
+  int cnt = qe;
+  for (int round = 0;; round++) {
+    if (round == kGiantRounds) return;
+    const int* in = round == 0 ? queue : ((round & 1) ? candA : candB);
+    int* out = (round & 1) ? candB : candA;
+    bool moved = false;
+    if (threadIdx.x == 0) s_moved = 0;
+    __syncthreads();
+    auto reaches = [&](int w) {
+      return (unsigned)w < (unsigned)n && ((bwd[w >> 5] >> (w & 31)) & 1u);  // race-free: not written during a round
+    };
+    auto reaches_now = [&](int w) {  // found in this round
+      return (unsigned)w < (unsigned)n && ((ld(&next[w >> 5]) >> (w & 31)) & 1u);
+    };
+    const int per = min(32, (cnt - 1) / nwarps + 1);
+    for (int i0 = warp * per; i0 < cnt; i0 += nwarps * per) {
+      const int i = lane < per ? i0 + lane : cnt;
+      const int v = i < cnt ? in[i] : 0;  // written before the last grid barrier
+      int beg = 0, deg = 0;
+      if (i < cnt && !reaches(v)) row_of(v, beg, deg);
+      bool found = false;
+      for (int k0 = 0; k0 < min(deg, 32) && !found; k0 += 4) {
+        int w[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) w[k] = k0 + k < deg ? __ldg(&nlist[beg + k0 + k]) : -1;
+#pragma unroll
+        for (int k = 0; k < 4; k++) found |= reaches(w[k]);
+        if (!found) {
+#pragma unroll
+          for (int k = 0; k < 4; k++) found |= reaches_now(w[k]);
+        }
+      }
+      unsigned todo = __ballot_sync(kFull, !found && deg > 32);
+      while (todo) {  // the rest of the long rows, by the whole warp
+        const int who = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int wbeg = __shfl_sync(kFull, beg, who), wdeg = __shfl_sync(kFull, deg, who);
+        bool hit = false;
+        for (int k0 = 32; k0 < wdeg && !hit; k0 += 128) {
+          bool mine = false;
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            const int e = k0 + 32 * k + lane;
+            const int w = e < wdeg ? __ldg(&nlist[wbeg + e]) : -1;
+            mine = mine || reaches(w) || reaches_now(w);
+          }
+          hit = __any_sync(kFull, mine);
+        }
+        if (lane == who) found = hit;
+      }
+      if (found) {
+        fetch_or(&next[v >> 5], 1u << (v & 31));
+        moved = true;
+      }
+      stg.push(deg > 0 && !found, v, out, &ctl->left[round + 1], n, overflow);
+    }
+    stg.flush(out, &ctl->left[round + 1], n, overflow);
+    if (moved) s_moved = 1;  // every writer stores the same value
+    __syncthreads();
+    if (threadIdx.x == 0 && s_moved) st(&ctl->moved[round], 1);
+    if (!grid_sync(&ctl->giant_bar, status)) return;
+    if (!ld(&ctl->moved[round])) break;
+    cnt = ld(&ctl->left[round + 1]);
+    merge_bits(bwd, next, words, tid, nthreads);
+    if (!grid_sync(&ctl->giant_bar, status)) return;
+  }
+  // its largest id
+  int top = -1;
+  for (int i = tid; i < words; i += nthreads) {
+    const unsigned x = ld(&fwd[i]) & ld(&bwd[i]);
+    if (x) top = max(top, 32 * i + 31 - __clz(x));
+  }
+  top = __reduce_max_sync(kFull, top);
+  if (lane == 0 && top > ld(&ctl->giant_label)) fetch_max(&ctl->giant_label, top);
+  if (tid == 0) st(&ctl->giant_ok, 1);
+}
+
 // A vertex is live (can be in a non-trivial SCC) iff it has an in-entry and an
 // out-entry other than self-loops.  Both facts share one flag word per vertex
 // (kHasIn | kHasOut), so the liveness test is one load; scc_mark ORs kHasIn
@@ -199,38 +495,65 @@ constexpr int kHasIn = 1, kHasOut = 2;
 // OR'ed only where kHasIn is still clear: R-MAT sends a large share of all
 // entries to a few hub ids, whose words would otherwise take an atomic from
 // every one of them.
+// kRest (after scc_giant): only edges between two vertices outside the giant
+// component and on the same side of its forward search count, and they are
+// appended to the list (`keep`) instead of standing at their CSR positions.
+template <bool kRest, class Keep>
 __device__ __forceinline__ void scc_mark_batch(const bool (&valid)[kScanBatch], int v, const int (&w)[kScanBatch],
-                                               const int (&j)[kScanBatch], int n, int* flags, int2* wl, bool& out,
-                                               Status* status) {
+                                               const int (&j)[kScanBatch], int n, int* flags, int2* wl, const Giant& gi,
+                                               Keep&& keep, bool& out, Status* status) {
   int f[kScanBatch];
 #pragma unroll
   for (int k = 0; k < kScanBatch; k++)
     f[k] = (valid[k] && (unsigned)w[k] < (unsigned)n && w[k] != v) ? ld(&flags[w[k]]) : kHasIn;
+  if constexpr (kRest) {
 #pragma unroll
-  for (int k = 0; k < kScanBatch; k++) {
-    if (!valid[k]) continue;
-    const bool edge = (unsigned)w[k] < (unsigned)n && w[k] != v;
-    if ((unsigned)w[k] >= (unsigned)n) raise(status, ECL_ERR_BAD_GRAPH, w[k]);
-    if (edge) {
-      if (!(f[k] & kHasIn)) fetch_or(&flags[w[k]], kHasIn);
-      out = true;
+    for (int k = 0; k < kScanBatch; k++) {
+      bool edge = valid[k] && (unsigned)w[k] < (unsigned)n && w[k] != v;
+      if (valid[k] && (unsigned)w[k] >= (unsigned)n) raise(status, ECL_ERR_BAD_GRAPH, w[k]);
+      edge = edge && !gi.in(w[k]) && gi.has(gi.fwd, w[k]) == gi.has(gi.fwd, v);
+      if (edge) {
+        if (!(f[k] & kHasIn)) fetch_or(&flags[w[k]], kHasIn);
+        out = true;
+      }
+      keep(edge, make_int2(v, w[k]));
     }
-    __stcs(&wl[j[k]], edge ? make_int2(v, w[k]) : make_int2(-1, -1));
+  } else {
+#pragma unroll
+    for (int k = 0; k < kScanBatch; k++) {
+      if (!valid[k]) continue;
+      const bool edge = (unsigned)w[k] < (unsigned)n && w[k] != v;
+      if ((unsigned)w[k] >= (unsigned)n) raise(status, ECL_ERR_BAD_GRAPH, w[k]);
+      if (edge) {
+        if (!(f[k] & kHasIn)) fetch_or(&flags[w[k]], kHasIn);
+        out = true;
+      }
+      __stcs(&wl[j[k]], edge ? make_int2(v, w[k]) : make_int2(-1, -1));
+    }
   }
 }
 
+template <bool kRest>
 __global__ void __launch_bounds__(kTPB) scc_mark(int n, int m, const int* __restrict__ nindex,
                                                  const int* __restrict__ nlist, int* __restrict__ flags,
                                                  int2* __restrict__ wl, RowChunks rc, Bins bins, bool vec,
-                                                 const SCCCtl* __restrict__ solved, Status* __restrict__ status) {
-  if (solved && ld(&solved->asym) == 0) return;  // a symmetric graph: its labels are written
+                                                 Giant gi, SCCCtl* __restrict__ ctl, bool checked, Status* __restrict__ status) {
+  // nothing to do for a symmetric graph (its labels are written), and one of
+  // the two forms runs, by whether the giant component was found
+  if ((checked && ld(&ctl->asym) == 0) || (ld(&ctl->giant_ok) != 0) != kRest) return;
+  __shared__ int2 s_stage[kTPB / 32][kRest ? 128 : 1];
+  WarpStage<int2, 128, true> stg{s_stage[threadIdx.x >> 5]};
+  bool overflow = false;
+  auto keep = [&](bool edge, int2 e) {
+    if (__any_sync(kFull, edge)) stg.push(edge, e, wl, &ctl->rest, m, overflow);
+  };
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
   for (int base = warp * 32; base < n; base += nwarps * 32) {
     const int v = base + lane;
     int beg = 0, end = 0;
-    if (v < n) csr_row(nindex, v, m, beg, end, status);
+    if (v < n && !(kRest && gi.in(v))) csr_row(nindex, v, m, beg, end, status);
     const int deg = end - beg;
     push_chunks_warp(rc, bins.chunk, deg > bins.chunk, v, beg, end, status);
     bool out = false;
@@ -245,7 +568,7 @@ __global__ void __launch_bounds__(kTPB) scc_mark(int n, int m, const int* __rest
         j[k] = beg + k0 + k;
         w[k] = valid[k] ? __ldg(&nlist[j[k]]) : 0;
       }
-      scc_mark_batch(valid, v, w, j, n, flags, wl, out, status);
+      scc_mark_batch<kRest>(valid, v, w, j, n, flags, wl, gi, keep, out, status);
     }
     unsigned todo = __ballot_sync(kFull, deg > bins.lane && deg <= bins.chunk);
     while (todo) {
@@ -256,20 +579,28 @@ __global__ void __launch_bounds__(kTPB) scc_mark(int n, int m, const int* __rest
       const int wend = __shfl_sync(kFull, end, who);
       bool wout = false;
       warp_row(wbeg, wend, m, vec, nlist, [&](const int (&j)[4], const int (&w)[4], const bool (&valid)[4]) {
-        scc_mark_batch(valid, wv, w, j, n, flags, wl, wout, status);
+        scc_mark_batch<kRest>(valid, wv, w, j, n, flags, wl, gi, keep, wout, status);
       });
       if (__any_sync(kFull, wout) && lane == who) out = true;
     }
     if (v < n && deg <= bins.chunk && out) fetch_or(&flags[v], kHasOut);  // long rows: scc_mark_chunks
   }
+  if (kRest) stg.flush(wl, &ctl->rest, m, overflow);
 }
 
+template <bool kRest>
 __global__ void __launch_bounds__(kTPB) scc_mark_chunks(int n, int m, const int* __restrict__ nindex,
                                                         const int* __restrict__ nlist, int* __restrict__ flags,
                                                         int2* __restrict__ wl, RowChunks rc, int chunk, bool vec,
-                                                        const SCCCtl* __restrict__ solved,
+                                                        Giant gi, SCCCtl* __restrict__ ctl, bool checked,
                                                         Status* __restrict__ status) {
-  if (solved && ld(&solved->asym) == 0) return;
+  if ((checked && ld(&ctl->asym) == 0) || (ld(&ctl->giant_ok) != 0) != kRest) return;
+  __shared__ int2 s_stage[kTPB / 32][kRest ? 128 : 1];
+  WarpStage<int2, 128, true> stg{s_stage[threadIdx.x >> 5]};
+  bool overflow = false;
+  auto keep = [&](bool edge, int2 e) {
+    if (__any_sync(kFull, edge)) stg.push(edge, e, wl, &ctl->rest, m, overflow);
+  };
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -279,10 +610,11 @@ __global__ void __launch_bounds__(kTPB) scc_mark_chunks(int n, int m, const int*
     const int end = min(r.y + chunk, __ldg(&nindex[r.x + 1]));
     bool out = false;
     warp_row(r.y, end, m, vec, nlist, [&](const int (&j)[4], const int (&w)[4], const bool (&valid)[4]) {
-      scc_mark_batch(valid, r.x, w, j, n, flags, wl, out, status);
+      scc_mark_batch<kRest>(valid, r.x, w, j, n, flags, wl, gi, keep, out, status);
     });
     if (__any_sync(kFull, out) && lane == 0) fetch_or(&flags[r.x], kHasOut);
   }
+  if (kRest) stg.flush(wl, &ctl->rest, m, overflow);
 }
 
 // Word of a trimmed vertex: it is its own SCC, and sweeps skip its edges.
@@ -296,11 +628,12 @@ struct SweepOcc {
 };
 
 // Round 0 sweeps the CSR-position edge list of `m0` slots (dead slots have
-// x < 0); later rounds sweep the compacted survivors.
+// x < 0) or, after scc_giant, the list of the edges outside its component;
+// later rounds sweep the compacted survivors.
 template <int kSweepBatch>
 __global__ void __launch_bounds__(kTPB, SweepOcc<kSweepBatch>::blocks) scc_solve(int n, int m0, int2* __restrict__ wlA, int2* __restrict__ wlB,
                                                   const int* __restrict__ flags, unsigned long long* __restrict__ io,
-                                                  int* __restrict__ label, SCCCtl* __restrict__ ctl,
+                                                  int* __restrict__ label, Giant gi, SCCCtl* __restrict__ ctl,
                                                   int max_rounds, bool checked,
                                                   Status* __restrict__ status) {
   if (checked && ld(&ctl->asym) == 0) return;  // as scc_mark
@@ -314,6 +647,8 @@ __global__ void __launch_bounds__(kTPB, SweepOcc<kSweepBatch>::blocks) scc_solve
     io[v] = __ldg(&flags[v]) == (kHasIn | kHasOut) ? io_pack(v, v) : kDead;  // race-free: owned, barrier next
   if (!grid_sync(&ctl->bar, status)) return;
   if (tid == 0 && ++nstamp < kStamps) ctl->stamp[nstamp] = scc_now();
+  const bool giant = ld(&ctl->giant_ok) != 0;
+  if (giant) m0 = min(ld(&ctl->rest), m0);
   int size = m0;
   int sweep = 0;
   int round = 0;
@@ -451,7 +786,7 @@ __global__ void __launch_bounds__(kTPB, SweepOcc<kSweepBatch>::blocks) scc_solve
     for (int v = tid; v < n; v += nthreads) {
       const unsigned long long A = ld(&io[v]);
       if (A == kDead) {
-        label[v] = v;  // race-free: the output, thread-owned and never read here
+        label[v] = giant && gi.in(v) ? ld(&ctl->giant_label) : v;  // race-free: the output, thread-owned and never read here
       } else if (io_in(A) == io_out(A)) {
         label[v] = io_in(A);  // race-free: as above
       } else {
@@ -480,6 +815,10 @@ struct SCCBufs {
   int2* wlA;
   int2* wlB;
   int* tilerow;
+  unsigned* bits;  // Giant's two bit arrays and scc_giant's next
+  int* queue;
+  int* candA;
+  int* candB;
   char* cc_ws;
   int max_rounds;
 };
@@ -494,6 +833,10 @@ void scc_layout(Carve& c, int n, int m, SCCBufs* b) {
   b->wlA = c.take<int2>((size_t)(m > 0 ? m : 1));
   b->wlB = c.take<int2>((size_t)(m > 0 ? m : 1));
   b->tilerow = c.take<int>((size_t)flat_tiles(m) + 1);
+  b->bits = c.take<unsigned>(3 * (((size_t)n + 31) / 32));
+  b->queue = c.take<int>((size_t)n);
+  b->candA = c.take<int>((size_t)n);
+  b->candB = c.take<int>((size_t)n);
   b->cc_ws = c.take<char>(cc_workspace_bytes(n, m));
 }
 
@@ -516,7 +859,8 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
   SCCBufs b;
   scc_layout(c, g.n, g.m, &b);
   const int batch = dev.scc_sweep_batch > 0 ? dev.scc_sweep_batch : kSweepBatchDefault;
-  void (*solve)(int, int, int2*, int2*, const int*, unsigned long long*, int*, SCCCtl*, int, bool, Status*) =
+  void (*solve)(int, int, int2*, int2*, const int*, unsigned long long*, int*, Giant, SCCCtl*, int, bool,
+                Status*) =
       batch == 1 ? scc_solve<1> : (batch == 4 ? scc_solve<4> : scc_solve<2>);
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, solve, kTPB, 0) != cudaSuccess || occ < 1)
@@ -526,6 +870,7 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
   // a graph flagged symmetric may be solved as connected components (not when
   // the caller limits the rounds: that limit is the general path's)
   const bool check = (g.flags & ECL_GRAPH_SYMMETRIC) != 0 && max_rounds <= 0;
+  const bool giant = max_rounds <= 0 && g.m >= kGiantEntries;  // (the same limit)
   if (max_rounds <= 0 || max_rounds > b.max_rounds) max_rounds = b.max_rounds;
 
   if (cudaMemsetAsync(b.ctl, 0, sizeof(SCCCtl), stream) != cudaSuccess) return ECL_ERR_CUDA;
@@ -549,13 +894,31 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
     ECL_LAUNCH(scc_top, dev.sms * 4, kTPB, 0, stream, g.n, label, b.flags, b.ctl);
     ECL_LAUNCH(scc_relabel, dev.grid_blocks(kTPB, g.n, 0), kTPB, 0, stream, g.n, label, b.flags, b.ctl);
   }
-  const SCCCtl* solved = check ? b.ctl : nullptr;
-  ECL_LAUNCH(scc_mark, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, solved, status);
-  ECL_LAUNCH(scc_mark_chunks, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins.chunk, vec,
-             solved, status);
+  const size_t words = ((size_t)g.n + 31) / 32;
+  const Giant gi{b.bits, b.bits + words};
+  if (giant) {
+    int gocc = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&gocc, scc_giant, kGTPB, 0) != cudaSuccess || gocc < 1)
+      return ECL_ERR_CUDA;
+    ECL_CUDA_TRY(cudaMemsetAsync(b.bits, 0, sizeof(unsigned) * 3 * words, stream));
+    const int blocks = std::max(1, std::min(dev.sms * gocc, (int)(std::max((long long)g.n, (long long)g.m / 4) / kGTPB)));
+    ECL_CUDA_TRY(launch_cooperative(scc_giant, blocks, kGTPB, stream, g.n, g.m, g.nindex, g.nlist, gi.fwd, gi.bwd,
+                                    b.bits + 2 * words, b.queue, b.candA, b.candB, b.chunks, (int)row_chunk_capacity(g.m, kMinChunk), b.ctl,
+                                    check, status));
+  }
+  ECL_LAUNCH(scc_mark<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, gi,
+             b.ctl, check, status);
+  ECL_LAUNCH(scc_mark_chunks<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins.chunk,
+             vec, gi, b.ctl, check, status);
+  if (giant) {
+    ECL_LAUNCH(scc_mark<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, gi,
+               b.ctl, check, status);
+    ECL_LAUNCH(scc_mark_chunks<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins.chunk,
+               vec, gi, b.ctl, check, status);
+  }
   mark();
-  ECL_CUDA_TRY(launch_cooperative(solve, coop_grid, kTPB, stream, g.n, g.m, b.wlA, b.wlB, b.flags, b.io, label, b.ctl,
-                                  max_rounds, check, status));
+  ECL_CUDA_TRY(launch_cooperative(solve, coop_grid, kTPB, stream, g.n, g.m, b.wlA, b.wlB, b.flags, b.io, label, gi,
+                                  b.ctl, max_rounds, check, status));
   mark();
   return ECL_OK;
 }

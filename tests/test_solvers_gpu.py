@@ -173,6 +173,38 @@ def test_scc_matches_tarjan(ecl, orc):
         assert np.array_equal(got, orc.scc(g)), name
 
 
+def giant_cases(ecl):
+    """Directed graphs against the giant-component step: found, given up, with
+    long rows, and with what is left for the propagation sweeps."""
+    for d in (0.5, 1.2, 2.0, 6.0):
+        yield f"er{d}", ecl.gen_er(6000, d / 6000, seed=int(d * 10))
+    yield "rmat13", ecl.gen_rmat(13, 8, seed=3, symmetrise=False)
+    yield "self_loops", from_edges(64, [(i, i) for i in range(64)] + [(5, 6), (6, 5)])
+    yield "star_out", from_edges(3000, [(0, i) for i in range(1, 3000)])  # a pivot nobody reaches
+    cyc = lambda a, b: [(i, i + 1 if i + 1 < b else a) for i in range(a, b)]  # noqa: E731
+    yield "cycle39", from_edges(39, cyc(0, 39))  # the last length that the level limit allows, and more
+    yield "cycle40", from_edges(40, cyc(0, 40))
+    yield "cycle41", from_edges(41, cyc(0, 41))
+    yield "cycle5000", from_edges(5000, cyc(0, 5000))
+    # the pivot's component, one upstream, one downstream, one apart
+    e = cyc(0, 20) + cyc(20, 35) + cyc(35, 50) + cyc(50, 64)
+    yield "bowtie", from_edges(70, sorted(e + [(0, j) for j in range(2, 20)] + [(25, 3), (7, 40), (20, 45), (66, 50), (63, 67)]))
+    rng = np.random.default_rng(1)  # rows just below, at and above the chunk record length
+    hubs = [(h, int(x)) for h, k in ((0, 1023), (1, 1024), (2, 1025), (3, 5000)) for x in rng.permutation(9000)[:k]]
+    yield "hubs", from_edges(9000, sorted(hubs + [(int(a), int(b)) for a, b in rng.integers(0, 9000, (12000, 2))]))
+
+
+def test_scc_giant_component(ecl, orc):
+    for name, g in giant_cases(ecl):
+        exp = orc.scc(g)
+        assert np.array_equal(ecl.scc(g.to_device()).cpu().numpy(), exp), name
+        # every entry many times over: the same components, and entries enough
+        # (2^20) for the giant-component step
+        r = (1 << 20) // g.edges + 1
+        big = ecl.Graph(g.nindex * r, np.repeat(g.nlist, r), None)
+        assert np.array_equal(ecl.scc(big.to_device()).cpu().numpy(), exp), name
+
+
 def flat_cases():
     """Rows against the 256-entry tiles of the entry-balanced scans, and average
     degrees on both sides of the MST light-edge rule."""
