@@ -13,12 +13,17 @@
 //    device-scope relaxed atomic on the word;
 //  * mis_init computes the priority bytes with the reference's fp32 formula
 //    using explicit round-to-nearest intrinsics (no contraction);
-//  * mis_run is ONE persistent cooperative launch (all blocks co-resident):
-//    each warp sweeps its vertex groups until all are decided.  Lists of <= 32 entries are scanned by their own
-//    lane with an early exit at the first blocker; longer lists are scanned
-//    32 entries per step by the whole warp (two ballots per step); a joining
-//    vertex claims itself with one CAS, then clears its neighbours' bytes
-//    (fetch_and), so blocked neighbours see OUT without rescanning;
+//  * mis_run is ONE persistent cooperative launch (all blocks co-resident).
+//    A first sweep scans every vertex's list up to the first blocker (an
+//    undecided neighbour that outranks it); vertices that have to wait become
+//    items {vertex, blocker's place in the list, blocker, list end} in a list of
+//    their warp's own, and later sweeps look at two status words per item --
+//    the vertex's and its blocker's -- until one is decided, then scan on from
+//    the blocker.  No entry is scanned twice: one that was passed is out, or
+//    outranked and cannot join before the vertex is decided.  Lists of <= 16
+//    entries are scanned by their own lane; longer ones, from the second sweep
+//    on, 128 entries per step by the whole warp; a joining vertex claims itself with one CAS, then clears
+//    its neighbours' bytes (fetch_and);
 //  * a self-loop (the reference spins forever on one: v never outranks
 //    itself) raises ECL_ERR_BAD_GRAPH when it is met; a sweep cap turns any
 //    other non-converging input into ECL_ERR_NO_CONVERGENCE.
@@ -32,7 +37,10 @@ namespace {
 using namespace dev;
 
 constexpr int kTPB = 256;
-constexpr int kLaneMax = 32;  // default: lists of up to 32 entries per lane (a launch knob)
+// Lists of up to this many entries are scanned by their own lane, in the first
+// sweep; longer ones wait for the second (a launch knob).  R-MAT-22, mis_run,
+// 32 / 16 / 8: 350 / 297 / 352 us; G(3 M, 24 M): 279 / 287 / 488.
+constexpr int kLaneMax = 16;
 constexpr int kBatch = 4;  // list entries per lane whose loads are issued together
 constexpr unsigned kIn = 0xfe;
 
@@ -138,123 +146,159 @@ __device__ __forceinline__ void mis_clear_list(unsigned* st4, const int* nlist, 
   }
 }
 
+// Scans entries [pos, end) of v (byte b) by its own lane; stops at the first
+// verdict other than kJoin and leaves pos and *blocker there.
+__device__ __forceinline__ int mis_scan_lane(int v, unsigned b, int& pos, int end, int n, const int* nlist,
+                                             unsigned* st4, int* blocker, Status* status) {
+  for (; pos < end; pos += kBatch) {
+    int u[kBatch];
+    unsigned w[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; k++) u[k] = pos + k < end ? __ldg(&nlist[pos + k]) : -1;
+#pragma unroll
+    for (int k = 0; k < kBatch; k++) w[k] = (unsigned)u[k] < (unsigned)n ? ld(&st4[u[k] >> 2]) : 0u;
+#pragma unroll
+    for (int k = 0; k < kBatch; k++) {
+      if (pos + k >= end) break;
+      if ((unsigned)u[k] >= (unsigned)n || u[k] == v) {  // out of range, or a self-loop
+        raise(status, ECL_ERR_BAD_GRAPH, u[k]);
+        continue;
+      }
+      const int r = mis_verdict(byte_of(w[k], u[k]), b, u[k], v);
+      if (r != kJoin) {
+        pos += k;
+        *blocker = u[k];
+        return r;
+      }
+    }
+  }
+  return kJoin;
+}
+
+// The same by the whole warp, 128 entries a step; the arguments are
+// warp-uniform and all lanes call.  An IN neighbour of the step decides before
+// an undecided one does.
+__device__ __forceinline__ int mis_scan_warp(int v, unsigned b, int& pos, int end, int n, const int* nlist,
+                                             unsigned* st4, int* blocker, Status* status) {
+  const int lane = threadIdx.x & 31;
+  for (; pos < end; pos += 32 * kBatch) {
+    int u[kBatch];
+    unsigned w[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; k++) {
+      const int i = pos + 32 * k + lane;
+      u[k] = i < end ? __ldg(&nlist[i]) : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < kBatch; k++) w[k] = (unsigned)u[k] < (unsigned)n ? ld(&st4[u[k] >> 2]) : 0u;
+    bool out = false;
+    int who = -1;  // a blocker among this lane's entries
+#pragma unroll
+    for (int k = 0; k < kBatch; k++) {
+      if (pos + 32 * k + lane >= end) continue;
+      if ((unsigned)u[k] >= (unsigned)n || u[k] == v) {
+        raise(status, ECL_ERR_BAD_GRAPH, u[k]);
+        continue;
+      }
+      const int r = mis_verdict(byte_of(w[k], u[k]), b, u[k], v);
+      out |= r == kOut;
+      if (r == kWait) who = u[k];
+    }
+    if (__any_sync(kFull, out)) return kOut;
+    const unsigned wait = __ballot_sync(kFull, who >= 0);
+    if (wait) {  // pos stays: the step is looked at again once this blocker is decided
+      *blocker = __shfl_sync(kFull, who, __ffs(wait) - 1);
+      return kWait;
+    }
+  }
+  return kJoin;
+}
+
+// A warp's g-th group is the vertices 32 (g nwarps + warp) ..+31, and its g-th
+// 32 items lie at the same places, so the warps' lists share one array of n
+// (rounded up) items and need no counters.  Bound by the latency of the chains
+// of decisions: DRAM and L2 are far from busy.  Measured, groups of 32 vertices
+// swept and scanned from the start until decided -> items: R-MAT-22 525 -> 297
+// us, 500 k vertices 169 -> 80, 1000 vertices (fewer blocks) 40 -> 16; with the
+// long lists scanned in the first sweep as well, R-MAT-22 525.
 __global__ void __launch_bounds__(kTPB) mis_run(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, unsigned* __restrict__ st4,
-                                                Status* __restrict__ status, int max_sweeps, int lane_max) {
+                                                int4* __restrict__ items, Status* __restrict__ status, int max_sweeps,
+                                                int lane_max) {
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
-  int sweep = 0;
-  // Bit g: this warp's g-th vertex group is fully decided and is skipped
-  // without a load (groups beyond the 64th are re-read every sweep).  Late
-  // sweeps then cost only the groups that still wait, not one L2 round trip
-  // per group owned.
-  unsigned long long done = 0;
-  for (;; sweep++) {
-    bool missing = false;
-    int gi = 0;
-    for (int base = warp * 32; base < n; base += nwarps * 32, gi++) {
-      if (gi < 64 && ((done >> gi) & 1ull)) continue;
-      const int v = base + lane;
-      unsigned b = 0;
-      if (v < n) b = byte_of(ld(&st4[v >> 2]), v);
-      const bool und = (b & 1u) != 0;
-      if (!__any_sync(kFull, und)) {
-        if (gi < 64) done |= 1ull << gi;
-        continue;
-      }
-      int beg = 0, end = 0;
-      if (und) {
-        beg = __ldg(&nindex[v]);
-        end = __ldg(&nindex[v + 1]);
-        if (beg < 0 || end < beg || end > m) beg = end = 0;  // reported by mis_init
-      }
-      const bool big = und && (end - beg) > lane_max;
-      int verdict = kWait;
-      if (und && !big) {
-        verdict = kJoin;
-        // kBatch entries at a time: their index loads, then their status
-        // loads, are all in flight before the first verdict is needed
-        for (int i0 = beg; i0 < end && verdict == kJoin; i0 += kBatch) {
-          int u[kBatch];
-          unsigned w[kBatch];
-#pragma unroll
-          for (int k = 0; k < kBatch; k++) u[k] = i0 + k < end ? __ldg(&nlist[i0 + k]) : -1;
-#pragma unroll
-          for (int k = 0; k < kBatch; k++) w[k] = (unsigned)u[k] < (unsigned)n ? ld(&st4[u[k] >> 2]) : 0u;
-#pragma unroll
-          for (int k = 0; k < kBatch; k++) {
-            if (i0 + k >= end || verdict != kJoin) continue;
-            if ((unsigned)u[k] >= (unsigned)n || u[k] == v) {  // out of range, or a self-loop
-              raise(status, ECL_ERR_BAD_GRAPH, u[k]);
-              continue;
-            }
-            const int r = mis_verdict(byte_of(w[k], u[k]), b, u[k], v);
-            if (r != kJoin) verdict = r;
-          }
-        }
-        if (verdict == kJoin) {
-          if (mis_claim(st4, v, b)) mis_clear_list(st4, nlist, beg, end, 1, n);
-        } else if (verdict == kOut) {
-          mis_set_out(st4, v);
-        }
-      }
-      // Long lists: the whole warp scans one list, 32 entries per step.
-      unsigned todo = __ballot_sync(kFull, big);
-      while (todo) {
-        const int who = __ffs(todo) - 1;
-        todo &= todo - 1;
-        const int wv = __shfl_sync(kFull, v, who);
-        const int wbeg = __shfl_sync(kFull, beg, who);
-        const int wend = __shfl_sync(kFull, end, who);
-        const unsigned wb = __shfl_sync(kFull, b, who);
-        int wverdict = kJoin;
-        for (int i0 = wbeg; i0 < wend; i0 += 32 * kBatch) {
-          int u[kBatch];
-          unsigned w[kBatch];
-#pragma unroll
-          for (int k = 0; k < kBatch; k++) {
-            const int i = i0 + 32 * k + lane;
-            u[k] = i < wend ? __ldg(&nlist[i]) : -1;
-          }
-#pragma unroll
-          for (int k = 0; k < kBatch; k++) w[k] = (unsigned)u[k] < (unsigned)n ? ld(&st4[u[k] >> 2]) : 0u;
-          bool out = false, wait = false;
-#pragma unroll
-          for (int k = 0; k < kBatch; k++) {
-            if (i0 + 32 * k + lane >= wend) continue;
-            if ((unsigned)u[k] < (unsigned)n && u[k] != wv) {
-              const int r = mis_verdict(byte_of(w[k], u[k]), wb, u[k], wv);
-              out |= r == kOut;
-              wait |= r == kWait;
-            } else {
-              raise(status, ECL_ERR_BAD_GRAPH, u[k]);
-            }
-          }
-          if (__any_sync(kFull, out)) {
-            wverdict = kOut;
-            break;
-          }
-          if (__any_sync(kFull, wait)) {
-            wverdict = kWait;
-            break;
-          }
-        }
-        if (wverdict == kJoin) {
-          bool claimed = false;
-          if (lane == 0) claimed = mis_claim(st4, wv, wb);
-          if (__shfl_sync(kFull, claimed, 0)) mis_clear_list(st4, nlist, wbeg + lane, wend, 32, n);
-        } else if (wverdict == kOut && lane == 0) {
-          mis_set_out(st4, wv);
-        }
-        if (lane == who) verdict = wverdict;
-      }
-      if (und && verdict == kWait) missing = true;
+  int kept = 0;  // items of this warp's list
+  auto slot = [&](int k) -> long long { return ((long long)(k >> 5) * nwarps + warp) * 32 + (k & 31); };
+  // Scans on for the lanes with `go` (entries [pos, end) of v), carries the
+  // verdicts out and keeps the waiting ones.  All lanes call.
+  auto advance = [&](bool go, bool wait, int v, unsigned b, int pos, int end, int blocker) {
+    int verdict = kWait;
+    const bool big = go && end - pos > lane_max;
+    if (go && !big) {
+      verdict = mis_scan_lane(v, b, pos, end, n, nlist, st4, &blocker, status);
     }
-    if (!__any_sync(kFull, missing)) break;
+    unsigned todo = __ballot_sync(kFull, big);
+    while (todo) {
+      const int who = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int wv = __shfl_sync(kFull, v, who), wend = __shfl_sync(kFull, end, who);
+      const unsigned wb = __shfl_sync(kFull, b, who);
+      int wpos = __shfl_sync(kFull, pos, who), wblock = -1;
+      const int r = mis_scan_warp(wv, wb, wpos, wend, n, nlist, st4, &wblock, status);
+      if (lane == who) verdict = r, pos = wpos, blocker = wblock;
+    }
+    if (go && verdict == kOut) mis_set_out(st4, v);
+    // joins: the claim first, then the neighbours
+    bool joined = go && verdict == kJoin && mis_claim(st4, v, b);
+    const int beg = joined ? __ldg(&nindex[v]) : 0;
+    if (joined && end - beg <= lane_max) mis_clear_list(st4, nlist, beg, end, 1, n);
+    unsigned clear = __ballot_sync(kFull, joined && end - beg > lane_max);
+    while (clear) {
+      const int who = __ffs(clear) - 1;
+      clear &= clear - 1;
+      mis_clear_list(st4, nlist, __shfl_sync(kFull, beg, who) + lane, __shfl_sync(kFull, end, who), 32, n);
+    }
+    const bool keep = wait || (go && verdict == kWait);
+    const unsigned bal = __ballot_sync(kFull, keep);
+    if (keep) items[slot(kept + __popc(bal & ((1u << lane) - 1)))] = make_int4(v, pos, blocker, end);
+    kept += __popc(bal);
+  };
+  for (int base = warp * 32; base < n; base += nwarps * 32) {
+    const int v = base + lane;
+    unsigned b = 0;
+    if (v < n) b = byte_of(ld(&st4[v >> 2]), v);
+    const bool und = (b & 1u) != 0;
+    if (!__any_sync(kFull, und)) continue;
+    int beg = 0, end = 0;
+    if (und) {
+      beg = __ldg(&nindex[v]);
+      end = __ldg(&nindex[v + 1]);
+      if (beg < 0 || end < beg || end > m) beg = end = 0;  // reported by mis_init
+    }
+    // long lists first wait for a sweep: their vertices rank low (the priority
+    // falls with the degree), and most are out before they are looked at
+    const bool big = end - beg > lane_max;
+    advance(und && !big, und && big, v, b, beg, end, -1);
+  }
+  int sweep = 0;
+  for (; kept > 0; sweep++) {
     if (sweep >= max_sweeps) {
       if (lane == 0) raise(status, ECL_ERR_NO_CONVERGENCE, warp);
       break;
+    }
+    const int count = kept;
+    kept = 0;
+    __syncwarp();
+    for (int c = 0; c < count; c += 32) {
+      const int4 it = c + lane < count ? items[slot(c + lane)] : make_int4(-1, 0, 0, 0);  // race-free: the warp's own
+      __syncwarp();
+      const unsigned sv = it.x >= 0 ? ld(&st4[it.x >> 2]) : 0u;
+      const unsigned su = it.x >= 0 && it.z >= 0 ? ld(&st4[it.z >> 2]) : 0u;
+      const unsigned b = it.x >= 0 ? byte_of(sv, it.x) : 0u;  // even: a neighbour joined, the vertex is out
+      const unsigned bu = byte_of(su, it.z & 3);  // 0: out, or no blocker yet
+      const bool und = (b & 1u) != 0, wait = und && (bu & 1u) != 0;
+      advance(und && !wait, wait, it.x, b, it.y, it.w, it.z);
     }
   }
   if (lane == 0) fetch_max(&status->rounds, sweep + 1);
@@ -267,7 +311,10 @@ __global__ void __launch_bounds__(kTPB) mis_emit(int n, const unsigned* __restri
   }
 }
 
-void mis_layout(Carve& c, int n, unsigned** st4) { *st4 = c.take<unsigned>((size_t)(n + 3) / 4); }
+void mis_layout(Carve& c, int n, unsigned** st4, int4** items) {
+  *st4 = c.take<unsigned>((size_t)(n + 3) / 4);
+  *items = c.take<int4>(((size_t)n + 31) / 32 * 32);
+}
 
 }  // namespace
 
@@ -275,7 +322,8 @@ size_t mis_workspace_bytes(int n, int m) {
   (void)m;
   Carve c;
   unsigned* st4;
-  mis_layout(c, n, &st4);
+  int4* items;
+  mis_layout(c, n, &st4, &items);
   return c.bytes();
 }
 
@@ -287,7 +335,8 @@ ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, Status* 
                        cudaStream_t stream, int max_sweeps, const UnionInfo* uni, Marker mark) {
   Carve c{ws};
   unsigned* st4;
-  mis_layout(c, g.n, &st4);
+  int4* items;
+  mis_layout(c, g.n, &st4, &items);
   const int nwords = (g.n + 3) / 4;
   const int grid = dev.grid_blocks(kTPB, g.n, g.m);
   const int* vbase = uni ? uni->vbase : nullptr;
@@ -301,8 +350,9 @@ ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, Status* 
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mis_run, kTPB, 0) != cudaSuccess || occ < 1)
     return ECL_ERR_CUDA;
-  ECL_CUDA_TRY(launch_cooperative(mis_run, dev.sms * std::min(occ, dev.max_threads_per_sm / kTPB), kTPB, stream, g.n,
-                                  g.m, g.nindex, g.nlist, st4, status, max_sweeps,
+  const int full = dev.sms * std::min(occ, dev.max_threads_per_sm / kTPB);
+  ECL_CUDA_TRY(launch_cooperative(mis_run, std::min(full, (g.n - 1) / kTPB + 1), kTPB, stream, g.n,
+                                  g.m, g.nindex, g.nlist, st4, items, status, max_sweeps,
                                   bins_of(dev, Bins{kLaneMax, kBinChunk}).lane));
   mark();
   ECL_LAUNCH(mis_emit, grid, kTPB, 0, stream, g.n, st4, out);

@@ -830,14 +830,17 @@ void scc_layout(Carve& c, int n, int m, SCCBufs* b) {
   b->nchunks = c.take<int>(64);
   b->chunks = c.take<int2>(row_chunk_capacity(m, kMinChunk));
   b->io = c.take<unsigned long long>((size_t)n);
-  b->wlA = c.take<int2>((size_t)(m > 0 ? m : 1));
-  b->wlB = c.take<int2>((size_t)(m > 0 ? m : 1));
-  b->tilerow = c.take<int>((size_t)flat_tiles(m) + 1);
+  // The search's lists lie where the second edge list comes later, and the
+  // union-find's scratch where the first one does.
   b->bits = c.take<unsigned>(3 * (((size_t)n + 31) / 32));
-  b->queue = c.take<int>((size_t)n);
-  b->candA = c.take<int>((size_t)n);
-  b->candB = c.take<int>((size_t)n);
-  b->cc_ws = c.take<char>(cc_workspace_bytes(n, m));
+  b->tilerow = c.take<int>((size_t)flat_tiles(m) + 1);
+  const size_t list = sizeof(int2) * (size_t)(m > 0 ? m : 1), ids = sizeof(int) * (size_t)n;
+  b->cc_ws = c.take<char>(std::max(list, cc_workspace_bytes(n, m)));
+  b->wlA = reinterpret_cast<int2*>(b->cc_ws);
+  b->queue = reinterpret_cast<int*>(c.take<char>(std::max(list, 3 * ids)));
+  b->wlB = reinterpret_cast<int2*>(b->queue);
+  b->candA = b->queue + n;
+  b->candB = b->candA + n;
 }
 
 }  // namespace

@@ -236,6 +236,17 @@ def test_mst_at_scan_tile_edges(ecl, orc):
             assert t == total and np.array_equal(got.cpu().numpy(), flags), (name, weight_max)
 
 
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 255, 257, 8191])  # partial groups and warps without any
+def test_mis_item_lists(ecl, orc, n):
+    graphs = [ecl.gen_er(n, min(1.0, d / n), seed=n + d, symmetrise=True) for d in (1, 6, 16, 17)]
+    graphs.append(undirected(n, [(i, i + 1) for i in range(n - 1)]))  # long chains of decisions
+    if n > 40:  # lists of 16 and 17 entries, and a hub past one 128-entry step
+        graphs.append(undirected(n, [(0, i) for i in range(1, min(n, 300))] +
+                                 [(1 + i, 20 + j) for i in range(8) for j in range(15 + i % 3)]))
+    for k, g in enumerate(graphs):
+        assert np.array_equal(ecl.mis(g), orc.mis(g)), k
+
+
 def flagged_cases(ecl):
     """Graphs flagged symmetric: truly so, and falsely (SCC then must not rely on it)."""
     yield "grid", ecl.gen_grid(70, 90, 0.3, seed=2)
