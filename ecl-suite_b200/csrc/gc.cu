@@ -323,10 +323,13 @@ __device__ __forceinline__ void gc_mark(unsigned* bits, int c, int off) {
 // from its colour -- a lane no longer walks the rest of its share of the row
 // after each wait.  The pass stops while the list still has room for a whole
 // step of 32 entries; the listed ones are resolved and the pass resumes where
-// it stopped, so every entry is read once by the pass.  Returns -1 on a
-// stall.  All lanes call.
-__device__ int gc_long_row(int wb, int we, const int* nl2, const int* color, unsigned* bits, int* pend, int pend_cap,
-                           unsigned nap_cap, Status* status) {
+// it stopped, so every entry is read once by the pass.  `ahead` holds the
+// row's first 32 * kAhead entries (entry 32 k + lane), loaded while the row
+// before was being coloured.  Returns -1 on a stall.  All lanes call.
+constexpr int kAhead = 4;
+
+__device__ int gc_long_row(int wb, int we, const int (&ahead)[kAhead], const int* nl2, const int* color, unsigned* bits,
+                           int* pend, int pend_cap, unsigned nap_cap, Status* status) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1;
   for (int off = 0;; off += 32 * kMexWords) {
@@ -337,6 +340,20 @@ __device__ int gc_long_row(int wb, int we, const int* nl2, const int* color, uns
     while (cursor < we) {
       int np = 0;
       int i0 = cursor;
+      if (off == 0 && i0 == wb) {
+        int c[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) c[k] = wb + 32 * k + lane < we ? ld(&color[ahead[k]]) : 0;
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) {
+          const bool in = wb + 32 * k + lane < we, undecided = in && c[k] < 0;
+          if (in && !undecided) gc_mark(bits, c[k], off);
+          const unsigned ub = __ballot_sync(kFull, undecided);
+          if (undecided) pend[np + __popc(ub & lt)] = ahead[k];
+          np += __popc(ub);
+        }
+        i0 += 32 * kAhead;
+      }
       // kBatch entries per lane per step: all index loads, then all colour
       // loads, are issued before any result is used (one round trip per
       // 32 * kBatch entries instead of two per 32)
@@ -819,21 +836,31 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* __restrict
         }
         wait |= undecided << (8 * s);
       }
-      // Wait for the undecided ones: a lane polls its lowest.
+      // Wait for the undecided ones: a lane polls its lowest, on its own and in
+      // as few instructions as can be.  The polls of 32 warps share one
+      // shared-memory pipe, and all the loop does comes on top of every hop of
+      // the chain (R-MAT-22: 1.40 ms; two entries a lane at a time 1.48, four
+      // 1.94, naps of 16 to 100 ns 1.49 to 1.53; scanning the warp's next row
+      // first 1.99, which doubles the undecided entries of that row).
       unsigned spins = 0;
       unsigned long long t0 = 0;
       while (wait) {
         const int k = __ffs(wait) - 1;
-        if (!look(sg[256 * (k >> 3) + 8 * lane + (k & 7)])) {
-          wait &= wait - 1;
-        } else if ((++spins & 1023u) == 0) {  // no nap: every nap length tried was slower than spinning
-          if (t0 == 0) t0 = gc_now();
-          if (gc_now() - t0 > kStallNs || ld(&status->code) != 0) {
-            raise(status, ECL_ERR_NO_CONVERGENCE, r);
-            stalled = true;
-            break;
+        const unsigned short* p = &col_s[sg[256 * (k >> 3) + 8 * lane + (k & 7)]];
+        unsigned c;
+        while ((c = col_ld(p)) == kUncoloured) {
+          if ((++spins & 1023u) == 0) {
+            if (t0 == 0) t0 = gc_now();
+            if (gc_now() - t0 > kStallNs || ld(&status->code) != 0) {
+              raise(status, ECL_ERR_NO_CONVERGENCE, r);
+              stalled = true;
+              break;
+            }
           }
         }
+        if (stalled) break;
+        marks[min(c, (unsigned)kWin)] = 1;
+        wait &= wait - 1;
       }
       stalled = __any_sync(kFull, stalled);
       b ^= 1;
@@ -877,27 +904,60 @@ __global__ void __launch_bounds__(kTPB) gc_pull(int n, const int* __restrict__ n
   // Long rows, ONE per warp at a time: every long row in flight scans its
   // higher-priority list concurrently, so the dense hub core's rows all wait
   // at the same time instead of one after another.
+  // A row's vertex, its place and length, and its first entries are three
+  // dependent loads, the last one from DRAM; they are made two, one and one
+  // row ahead.  Bound by what is left: a round trip to L2 for the colours, and
+  // the chain.  Measured, pull, nothing loaded ahead -> this: R-MAT-22 1.12 ->
+  // 0.98 ms, G(3 M, 12 M) 0.246 -> 0.217.
   // ranks below the core size were coloured by gc_core
-  for (int r = gc_core_size(ctl, core_cap) + gwarp; r < nbig; r += nwarps) {
-    const int wv = __ldg(&order[r]);
-    const int wb = __ldg(&nindex[wv]);
-    const int c = gc_long_row(wb, wb + __ldg(&hc[wv]), nl2, color, bits, pend, kPend, long_nap, status);
+  const int r0 = gc_core_size(ctl, core_cap) + gwarp;
+  auto vertex = [&](int r) { return r < nbig ? __ldg(&order[r]) : -1; };
+  auto place = [&](int v, int& b, int& h) {
+    b = v >= 0 ? __ldg(&nindex[v]) : 0;
+    h = v >= 0 ? __ldg(&hc[v]) : 0;
+  };
+  int v = vertex(r0), v1 = vertex(min(r0, nbig) + nwarps);
+  int b, h;
+  place(v, b, h);
+  int ahead[kAhead];
+#pragma unroll
+  for (int k = 0; k < kAhead; k++) ahead[k] = 32 * k + lane < h ? __ldg(&nl2[b + 32 * k + lane]) : 0;
+  for (int r = r0; r < nbig; r += nwarps) {
+    const int v2 = r < nbig - 2 * nwarps ? __ldg(&order[r + 2 * nwarps]) : -1;
+    int b1, h1;
+    place(v1, b1, h1);
+    int next[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; k++) next[k] = 32 * k + lane < h1 ? __ldg(&nl2[b1 + 32 * k + lane]) : 0;
+    const int c = gc_long_row(b, b + h, ahead, nl2, color, bits, pend, kPend, long_nap, status);
     if (c < 0) return;
-    if (lane == 0) st(&color[wv], c);
+    if (lane == 0) st(&color[v], c);
     __syncwarp();
+    v = v1, v1 = v2, b = b1, h = h1;
+#pragma unroll
+    for (int k = 0; k < kAhead; k++) ahead[k] = next[k];
   }
   // Short rows: 32 consecutive ranks per warp step, every lane its own vertex
   // (the order holds the nkeys vertices with entries; the isolated ones were
-  // coloured by gc_keys).
+  // coloured by gc_keys).  The next step's vertices and places are loaded a
+  // step ahead, and the lines of its entries asked for.
   const int nk = min(ld(&ctl->nkeys), n);
+  const int first = nbig + gwarp * 32 + lane;
+  int sv = first < nk ? __ldg(&order[first]) : -1;
+  int sb, sh;
+  place(sv, sb, sh);
   for (int base = nbig + gwarp * 32; base < nk; base += nwarps * 32) {
-    const int r = base + lane;
-    if (r < nk) {
-      const int v = __ldg(&order[r]);
-      const int c = gc_short_row(__ldg(&nindex[v]), __ldg(&hc[v]), nl2, color, status);
-      if (c >= 0) st(&color[v], c);
+    const int rn = base + lane + nwarps * 32;
+    const int svn = rn < nk ? __ldg(&order[rn]) : -1;
+    int sbn, shn;
+    place(svn, sbn, shn);
+    if (shn > 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(nl2 + sbn));
+    if (sv >= 0) {
+      const int c = gc_short_row(sb, sh, nl2, color, status);
+      if (c >= 0) st(&color[sv], c);
     }
     if (__any_sync(kFull, ld(&status->code) != 0)) return;
+    sv = svn, sb = sbn, sh = shn;
   }
 }
 
