@@ -282,9 +282,8 @@ __device__ __forceinline__ void merge_bits(unsigned* bits, unsigned* next, int w
 __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* __restrict__ nindex,
                                                       const int* __restrict__ nlist, unsigned* fwd, unsigned* bwd,
                                                       unsigned* next, int* queue, int* candA, int* candB, int2* chunks,
-                                                      int chunk_cap, SCCCtl* __restrict__ ctl, bool checked,
+                                                      int chunk_cap, SCCCtl* __restrict__ ctl,
                                                       Status* __restrict__ status) {
-  if (checked && ld(&ctl->asym) == 0) return;  // as scc_mark
   __shared__ int s_stage[kGTPB / 32][128];
   __shared__ int s_moved;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -873,7 +872,10 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
   // a graph flagged symmetric may be solved as connected components (not when
   // the caller limits the rounds: that limit is the general path's)
   const bool check = (g.flags & ECL_GRAPH_SYMMETRIC) != 0 && max_rounds <= 0;
-  const bool giant = max_rounds <= 0 && g.m >= kGiantEntries;  // (the same limit)
+  // (the same limit; and a flagged graph that is what its flag says needs no
+  // propagation: the search and the second form of the mark passes would be
+  // three launches that leave at once, 8 us on a mesh of 0.7 M vertices)
+  const bool giant = max_rounds <= 0 && !check && g.m >= kGiantEntries;
   if (max_rounds <= 0 || max_rounds > b.max_rounds) max_rounds = b.max_rounds;
 
   if (cudaMemsetAsync(b.ctl, 0, sizeof(SCCCtl), stream) != cudaSuccess) return ECL_ERR_CUDA;
@@ -907,7 +909,7 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
     const int blocks = std::max(1, std::min(dev.sms * gocc, (int)(std::max((long long)g.n, (long long)g.m / 4) / kGTPB)));
     ECL_CUDA_TRY(launch_cooperative(scc_giant, blocks, kGTPB, stream, g.n, g.m, g.nindex, g.nlist, gi.fwd, gi.bwd,
                                     b.bits + 2 * words, b.queue, b.candA, b.candB, b.chunks, (int)row_chunk_capacity(g.m, kMinChunk), b.ctl,
-                                    check, status));
+                                    status));
   }
   ECL_LAUNCH(scc_mark<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, gi,
              b.ctl, check, status);
@@ -915,9 +917,9 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
              vec, gi, b.ctl, check, status);
   if (giant) {
     ECL_LAUNCH(scc_mark<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, gi,
-               b.ctl, check, status);
+               b.ctl, false, status);
     ECL_LAUNCH(scc_mark_chunks<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins.chunk,
-               vec, gi, b.ctl, check, status);
+               vec, gi, b.ctl, false, status);
   }
   mark();
   ECL_CUDA_TRY(launch_cooperative(solve, coop_grid, kTPB, stream, g.n, g.m, b.wlA, b.wlB, b.flags, b.io, label, gi,
