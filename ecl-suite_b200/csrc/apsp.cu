@@ -606,6 +606,7 @@ __global__ void __launch_bounds__(kThreads, Apsp<T>::kCtasPerSm) apsp_run(int* _
 }
 
 __global__ void apsp_fill(int* __restrict__ A, long ld, int N, int n) {
+  dep_wait();
   const long total4 = (long)N * N / 4;
   for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < total4; q += (long)gridDim.x * blockDim.x) {
     const long idx = q * 4;
@@ -620,6 +621,7 @@ __global__ void apsp_fill(int* __restrict__ A, long ld, int N, int n) {
 // duplicate wins exactly as in init2 (ECL-APSP-atomic.cu:74-83).
 __global__ void apsp_edges(int* __restrict__ A, long ld, int n, int m, const int* __restrict__ nindex,
                            const int* __restrict__ nlist, const int* __restrict__ eweight, Status* __restrict__ status) {
+  dep_wait();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int beg = __ldg(&nindex[i]), end = __ldg(&nindex[i + 1]);
     if (beg < 0 || end < beg || end > m) {
@@ -709,8 +711,8 @@ extern "C" ecl_status ecl_apsp(const ecl_graph_view* g, int32_t* dist, int64_t l
   const int grid = s.dev.sms * 4;
 
   s.start_timer();
-  ECL_LAUNCH(apsp_fill, grid, 256, 0, s.stream, W, (long)N, N, s.n);
-  if (s.m > 0) ECL_LAUNCH(apsp_edges, (s.n + 255) / 256, 256, 0, s.stream, W, (long)N, s.n, s.m, s.nindex, s.nlist, s.eweight, s.status);
+  ECL_LAUNCH_NEXT(apsp_fill, grid, 256, 0, s.stream, W, (long)N, N, s.n);
+  if (s.m > 0) ECL_LAUNCH_NEXT(apsp_edges, (s.n + 255) / 256, 256, 0, s.stream, W, (long)N, s.n, s.m, s.nindex, s.nlist, s.eweight, s.status);
   s.mark();
   st = apsp_tile(s.n) == 64 ? apsp_launch<64>(W, N, ctl, s.dev, s.stream, s.status)
                             : apsp_launch<128>(W, N, ctl, s.dev, s.stream, s.status);

@@ -67,6 +67,7 @@ __global__ void __launch_bounds__(256) batch_mst_totals(int ngraphs, int m, cons
                                                         const unsigned* __restrict__ in_mst4,
                                                         const int* __restrict__ eweight,
                                                         unsigned long long* __restrict__ totals) {
+  dep_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -167,7 +168,7 @@ ecl_status enqueue_run(ecl_batch* b) {
       st = mst_enqueue(g, s.mst, s.ws, stat(3), dev, b->stream, nullptr);
       if (st == ECL_OK) {
         ECL_CUDA_TRY(cudaMemsetAsync(s.totals, 0, sizeof(unsigned long long) * (size_t)s.count, b->stream));
-        ECL_LAUNCH(batch_mst_totals, dev.grid_blocks(256, 0, s.m), 256, 0, b->stream, s.count, s.m, s.ebase,
+        ECL_LAUNCH_NEXT(batch_mst_totals, dev.grid_blocks(256, 0, s.m), 256, 0, b->stream, s.count, s.m, s.ebase,
                    reinterpret_cast<const unsigned*>(s.mst), s.eweight, s.totals);
       }
     }

@@ -139,6 +139,7 @@ __device__ __forceinline__ int cc_first_smaller(int v, int beg, int end, const i
 __global__ void __launch_bounds__(kTPB) cc_init(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, int* __restrict__ parent,
                                                 Status* __restrict__ status) {
+  dep_wait();
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     int beg = __ldg(&nindex[v]), end = __ldg(&nindex[v + 1]);
     if (beg < 0 || end < beg || end > m) {
@@ -185,6 +186,7 @@ __global__ void __launch_bounds__(kTPB) cc_hook(int n, int m, const int* __restr
                                                 const int* __restrict__ nlist, int* __restrict__ parent,
                                                 int2* __restrict__ chunks, int chunk_cap, Bins bins,
                                                 CCCounters* __restrict__ ctr, Status* __restrict__ status) {
+  dep_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -231,6 +233,7 @@ __global__ void __launch_bounds__(kTPB) cc_chunks(int n, const int* __restrict__
                                                   const int* __restrict__ nlist, int* __restrict__ parent,
                                                   const int2* __restrict__ chunks, int chunk_cap, int chunk,
                                                   const CCCounters* __restrict__ ctr, Status* __restrict__ status) {
+  dep_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -270,6 +273,7 @@ constexpr int kFlattenBatch = 4;
 template <bool kMark>
 __global__ void __launch_bounds__(kTPB) cc_flatten(int n, int* __restrict__ parent, const CCCounters* __restrict__ ctr,
                                                    unsigned char* __restrict__ ing) {
+  dep_wait();
   const int stride = gridDim.x * kTPB;
   const int giant = kMark ? ctr->giant : -1;
   int known = -1;  // a root of this launch
@@ -330,6 +334,7 @@ template <int kPart>  // 0: one vertex in kFirstOf, 1: the others, 2: all
 __global__ void __launch_bounds__(kTPB) cc_sample(int n, int m, const int* __restrict__ nindex,
                                                   const int* __restrict__ nlist, int* __restrict__ parent,
                                                   Status* __restrict__ status) {
+  dep_wait();
   constexpr int kFirstOf = 8;
   const int count = kPart == 0 ? (n - 1) / kFirstOf + 1 : n;
   for (int i = blockIdx.x * kTPB + threadIdx.x; i < count; i += gridDim.x * kTPB) {
@@ -355,6 +360,7 @@ constexpr int kSplitSample = 1 << 13;
 constexpr int kGiantSlots = 2048;
 
 __global__ void __launch_bounds__(1024) cc_giant(int n, const int* __restrict__ parent, CCCounters* __restrict__ ctr) {
+  dep_wait();
   __shared__ int s_root[kGiantSlots], s_count[kGiantSlots];
   __shared__ unsigned long long s_best[32];
   const int t = threadIdx.x;
@@ -398,6 +404,7 @@ __global__ void __launch_bounds__(kTPB) cc_rest(int n, int m, const int* __restr
                                                 const unsigned char* __restrict__ ing, int2* __restrict__ chunks,
                                                 int chunk_cap, Bins bins, CCCounters* __restrict__ ctr,
                                                 Status* __restrict__ status) {
+  dep_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -444,6 +451,7 @@ __global__ void __launch_bounds__(kTPB) cc_rest_chunks(int n, const int* __restr
                                                        const unsigned char* __restrict__ ing,
                                                        const int2* __restrict__ chunks, int chunk_cap, int chunk,
                                                        const CCCounters* __restrict__ ctr, Status* __restrict__ status) {
+  dep_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -497,36 +505,36 @@ ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, 
   const int cap = chunk_capacity(g.m, kMinChunk);  // cc_layout sized the records for the smallest chunk
   ECL_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(CCCounters), stream));
   if (g.flags & ECL_GRAPH_SYMMETRIC) {
-    ECL_LAUNCH(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
-    ECL_LAUNCH(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
+    ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
+    ECL_LAUNCH_NEXT(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
     if (g.n >= kSplitSample) {
-      ECL_LAUNCH(cc_sample<0>, dev.grid_blocks(kTPB, g.n / 8, 0), kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent,
+      ECL_LAUNCH_NEXT(cc_sample<0>, dev.grid_blocks(kTPB, g.n / 8, 0), kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent,
                  status);
-      ECL_LAUNCH(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
-      ECL_LAUNCH(cc_sample<1>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
+      ECL_LAUNCH_NEXT(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
+      ECL_LAUNCH_NEXT(cc_sample<1>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
     } else {
-      ECL_LAUNCH(cc_sample<2>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
+      ECL_LAUNCH_NEXT(cc_sample<2>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
     }
-    ECL_LAUNCH(cc_giant, 1, 1024, 0, stream, g.n, parent, ctr);
-    ECL_LAUNCH(cc_flatten<true>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, ctr, ing);
+    ECL_LAUNCH_NEXT(cc_giant, 1, 1024, 0, stream, g.n, parent, ctr);
+    ECL_LAUNCH_NEXT(cc_flatten<true>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, ctr, ing);
     mark();
-    ECL_LAUNCH(cc_rest, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ing, chunks, cap, bins, ctr,
+    ECL_LAUNCH_NEXT(cc_rest, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ing, chunks, cap, bins, ctr,
                status);
     mark();
-    ECL_LAUNCH(cc_rest_chunks, grid, kTPB, 0, stream, g.n, g.nindex, g.nlist, parent, ing, chunks, cap, bins.chunk,
+    ECL_LAUNCH_NEXT(cc_rest_chunks, grid, kTPB, 0, stream, g.n, g.nindex, g.nlist, parent, ing, chunks, cap, bins.chunk,
                ctr, status);
     mark();
-    ECL_LAUNCH(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
+    ECL_LAUNCH_NEXT(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
     mark();
     return ECL_OK;
   }
-  ECL_LAUNCH(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
+  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
   mark();
-  ECL_LAUNCH(cc_hook, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, chunks, cap, bins, ctr, status);
+  ECL_LAUNCH_NEXT(cc_hook, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, chunks, cap, bins, ctr, status);
   mark();
-  ECL_LAUNCH(cc_chunks, grid, kTPB, 0, stream, g.n, g.nindex, g.nlist, parent, chunks, cap, bins.chunk, ctr, status);
+  ECL_LAUNCH_NEXT(cc_chunks, grid, kTPB, 0, stream, g.n, g.nindex, g.nlist, parent, chunks, cap, bins.chunk, ctr, status);
   mark();
-  ECL_LAUNCH(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
+  ECL_LAUNCH_NEXT(cc_flatten<false>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, nullptr, nullptr);
   mark();
   return ECL_OK;
 }
@@ -659,12 +667,12 @@ extern "C" ecl_status ecl_cc_noalloc(int32_t nodes, int32_t edges, const int32_t
   // the counters (adjacent, at the front of the array) before every solve.
   ECL_CUDA_TRY(cudaMemsetAsync(base, 0, kStatusBytes + sizeof(CCCounters), stream));
   const int grid = dev.grid_blocks(kTPB, nodes, edges);
-  ECL_LAUNCH(cc_init, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, status);
-  ECL_LAUNCH(cc_hook, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, chunks,
+  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, status);
+  ECL_LAUNCH_NEXT(cc_hook, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, chunks,
              chunk_capacity(edges, kCCBins.chunk), kCCBins, ctr, status);
-  ECL_LAUNCH(cc_chunks, grid, kTPB, 0, stream, nodes, nindex, nlist, label, chunks,
+  ECL_LAUNCH_NEXT(cc_chunks, grid, kTPB, 0, stream, nodes, nindex, nlist, label, chunks,
              chunk_capacity(edges, kCCBins.chunk), kCCBins.chunk, ctr, status);
-  ECL_LAUNCH(cc_flatten<false>, flatten_blocks(dev, nodes), kTPB, 0, stream, nodes, label, nullptr, nullptr);
+  ECL_LAUNCH_NEXT(cc_flatten<false>, flatten_blocks(dev, nodes), kTPB, 0, stream, nodes, label, nullptr, nullptr);
   Status hs{};
   ECL_CUDA_TRY(cudaMemcpyAsync(&hs, status, sizeof(hs), cudaMemcpyDeviceToHost, stream));
   ECL_CUDA_TRY(cudaStreamSynchronize(stream));

@@ -25,6 +25,10 @@ constexpr unsigned kFull = 0xffffffffu;
 template <typename T>
 using aref = cuda::atomic_ref<T, cuda::thread_scope_device>;
 
+// First statement of a kernel that is launched by launch_next(): returns when
+// the kernels before it in the stream have ended and their writes are visible.
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <typename T>
 __device__ __forceinline__ T ld(const T* p) {
   return aref<T>(*const_cast<T*>(p)).load(cuda::memory_order_relaxed);

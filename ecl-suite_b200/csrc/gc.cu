@@ -102,6 +102,7 @@ __device__ __forceinline__ void gc_class_batch(const int (&u)[kInitBatch], const
 // vhash[v] = hash of v's local id in a union of graphs.
 __global__ void __launch_bounds__(kTPB) gc_union_hash(int n, const int* __restrict__ vbase, int ngraphs,
                                                       unsigned* __restrict__ vhash) {
+  dep_wait();
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     int lo = 0, hi = ngraphs - 1;
     while (lo < hi) {
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(kTPB) gc_init(int n, int m, const int* __restr
                                                 int* __restrict__ hc, RowChunks rc, Bins bins, bool vec,
                                                 const unsigned long long* __restrict__ keys,
                                                 Status* __restrict__ status) {
+  dep_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -175,6 +177,7 @@ __global__ void __launch_bounds__(kTPB) gc_init_chunks(int n, int m, const int* 
                                                        int* __restrict__ hc, RowChunks rc, int chunk, bool vec,
                                                        const unsigned long long* __restrict__ keys,
                                                        Status* __restrict__ status) {
+  dep_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -220,6 +223,7 @@ __global__ void __launch_bounds__(kTPB) gc_keys(int n, const int* __restrict__ n
                                                 unsigned long long* __restrict__ skeys, int* __restrict__ svals,
                                                 const unsigned* __restrict__ vhash, int* __restrict__ color,
                                                 GCCtl* __restrict__ ctl) {
+  dep_wait();
   // rows longer than kWarpRow are counted per block and added once per block;
   // the appends reserve their room with one atomic per block and step
   __shared__ int s_big, s_deg;
@@ -540,6 +544,7 @@ __device__ __forceinline__ int gc_core_size(const GCCtl* ctl, int cap) {
 // rank[order[r]] = r over the core.
 __global__ void __launch_bounds__(kTPB) gc_core_rank(const int* __restrict__ order, int* __restrict__ rank,
                                                      const GCCtl* __restrict__ ctl, int cap) {
+  dep_wait();
   const int core = gc_core_size(ctl, cap);
   for (int r = blockIdx.x * kTPB + threadIdx.x; r < core; r += gridDim.x * kTPB) rank[__ldg(&order[r])] = r;
 }
@@ -556,6 +561,7 @@ __global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict_
                                                           const int* __restrict__ hc, const int* __restrict__ order,
                                                           const int* __restrict__ rank, int4* __restrict__ rowinfo,
                                                           const GCCtl* __restrict__ ctl, int cap) {
+  dep_wait();
   const int lane = threadIdx.x & 31;
   const int core = gc_core_size(ctl, cap);
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
@@ -734,6 +740,7 @@ struct CoreStage {
 __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* __restrict__ nl2, const int4* __restrict__ rowinfo,
                                                            int* __restrict__ color, const GCCtl* __restrict__ ctl,
                                                            int cap, Status* __restrict__ status) {
+  dep_wait();
   extern __shared__ __align__(16) unsigned char s_core[];
   const int lane = threadIdx.x & 31;
   const int core = gc_core_size(ctl, cap);
@@ -1026,14 +1033,14 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
   if (cudaMemsetAsync(color, 0xff, sizeof(int) * (size_t)g.n, stream) != cudaSuccess) return ECL_ERR_CUDA;
   const unsigned* vhash = nullptr;
   if (uni && uni->vbase) {
-    ECL_LAUNCH(gc_union_hash, grid, kTPB, 0, stream, g.n, uni->vbase, uni->ngraphs, b.vhash);
+    ECL_LAUNCH_NEXT(gc_union_hash, grid, kTPB, 0, stream, g.n, uni->vbase, uni->ngraphs, b.vhash);
     vhash = b.vhash;
   }
   // the priority keys first: gc_init compares neighbours by them
-  ECL_LAUNCH(gc_keys, grid, kTPB, 0, stream, g.n, g.nindex, b.keys0, b.keys1, b.vals1, vhash, color, b.ctl);
+  ECL_LAUNCH_NEXT(gc_keys, grid, kTPB, 0, stream, g.n, g.nindex, b.keys0, b.keys1, b.vals1, vhash, color, b.ctl);
   const bool vec = (reinterpret_cast<uintptr_t>(g.nlist) & 15) == 0 && dev.row_vec;  // 16-byte row loads
-  ECL_LAUNCH(gc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.nl2, b.hc, rc, bins, vec, b.keys0, status);
-  ECL_LAUNCH(gc_init_chunks, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.nl2, b.hc, rc, bins.chunk, vec, b.keys0,
+  ECL_LAUNCH_NEXT(gc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.nl2, b.hc, rc, bins, vec, b.keys0, status);
+  ECL_LAUNCH_NEXT(gc_init_chunks, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.nl2, b.hc, rc, bins.chunk, vec, b.keys0,
              status);
   mark();
   // the nkeys appended pairs, sorted from (keys1, vals1); the per-vertex keys
@@ -1046,8 +1053,8 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
   // the hub core (the sort keys are dead now: their buffer holds the ranks)
   const int cap = std::min(std::min(dev.gc_core_ranks > 0 ? dev.gc_core_ranks : kCoreDefault, kCoreMax), g.n);
   int* rank = reinterpret_cast<int*>(b.keys0);
-  ECL_LAUNCH(gc_core_rank, grid, kTPB, 0, stream, order, rank, b.ctl, cap);
-  ECL_LAUNCH(gc_core_translate, grid, kTPB, 0, stream, g.nindex, b.nl2, b.hc, order, rank, b.rowinfo, b.ctl, cap);
+  ECL_LAUNCH_NEXT(gc_core_rank, grid, kTPB, 0, stream, order, rank, b.ctl, cap);
+  ECL_LAUNCH_NEXT(gc_core_translate, grid, kTPB, 0, stream, g.nindex, b.nl2, b.hc, order, rank, b.rowinfo, b.ctl, cap);
   ECL_CUDA_TRY(cudaFuncSetAttribute(gc_core, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gc_core_smem(cap)));
   // the core's cluster: as many CTAs as asked for when such a cluster fits
   // the device, else one CTA
@@ -1075,7 +1082,7 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
     ECL_CUDA_TRY(launch_cluster(gc_core, ctas, kCoreThreads, gc_core_smem(cap), stream, b.nl2, b.rowinfo, color,
                                 b.ctl, cap, status));
   else
-    ECL_LAUNCH(gc_core, 1, kCoreThreads, gc_core_smem(cap), stream, b.nl2, b.rowinfo, color, b.ctl, cap, status);
+    ECL_LAUNCH_NEXT(gc_core, 1, kCoreThreads, gc_core_smem(cap), stream, b.nl2, b.rowinfo, color, b.ctl, cap, status);
   mark();
   // the long rows' polls back off to at most gc_poll_ns, 64 ns by default
   // (they carry the dependency chain; the short rows keep 512 ns)

@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(kTPB) mis_init(int n, int m, const int* __rest
                                                  unsigned* __restrict__ st4, int nwords, const int* __restrict__ vbase,
                                                  const float* __restrict__ avgs, int ngraphs,
                                                  Status* __restrict__ status) {
+  dep_wait();
   const float avg1 = __fdiv_rn(__int2float_rn(m), __int2float_rn(n));
   for (int w = blockIdx.x * kTPB + threadIdx.x; w < nwords; w += gridDim.x * kTPB) {
     unsigned word = 0;
@@ -306,6 +307,7 @@ __global__ void __launch_bounds__(kTPB) mis_run(int n, int m, const int* __restr
 
 __global__ void __launch_bounds__(kTPB) mis_emit(int n, const unsigned* __restrict__ st4,
                                                  unsigned char* __restrict__ out) {
+  dep_wait();
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     out[v] = (unsigned char)byte_of(st4[v >> 2], v);  // race-free: st4 is final (mis_run finished)
   }
@@ -342,7 +344,7 @@ ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, Status* 
   const int* vbase = uni ? uni->vbase : nullptr;
   const float* avgs = uni ? uni->avg : nullptr;
   const int ngraphs = uni ? uni->ngraphs : 0;
-  ECL_LAUNCH(mis_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, st4, nwords, vbase, avgs, ngraphs, status);
+  ECL_LAUNCH_NEXT(mis_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, st4, nwords, vbase, avgs, ngraphs, status);
   mark();
   // Warps of mis_run wait (by sweeping) for vertices owned by other warps,
   // so all its blocks must be resident together: a cooperative launch
@@ -355,7 +357,7 @@ ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, Status* 
                                   g.m, g.nindex, g.nlist, st4, items, status, max_sweeps,
                                   bins_of(dev, Bins{kLaneMax, kBinChunk}).lane));
   mark();
-  ECL_LAUNCH(mis_emit, grid, kTPB, 0, stream, g.n, st4, out);
+  ECL_LAUNCH_NEXT(mis_emit, grid, kTPB, 0, stream, g.n, st4, out);
   mark();
   return ECL_OK;
 }

@@ -76,6 +76,7 @@ __device__ __forceinline__ u64 mst_now() {
 // thread is shortening at the same time (a vertex is a root iff it is its own
 // parent; hooks may point either way in the ids).
 __global__ void __launch_bounds__(kTPB) mst_flatten(int n, int* __restrict__ parent) {
+  dep_wait();
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     int p = ld(&parent[v]);
     if (p == v) continue;
@@ -92,6 +93,7 @@ __global__ void __launch_bounds__(kTPB) mst_flatten(int n, int* __restrict__ par
 __global__ void __launch_bounds__(kTPB) mst_init(int n, int m, const int* __restrict__ nindex, int* __restrict__ parent,
                                                  u64* __restrict__ minv, int* __restrict__ tilerow,
                                                  Status* __restrict__ status) {
+  dep_wait();
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     // race-free: thread-owned init, no reader in this launch
     parent[v] = v;
@@ -107,6 +109,7 @@ __global__ void __launch_bounds__(kTPB) mst_init(int n, int m, const int* __rest
 // filtering when edges/nodes < 4.
 __global__ void __launch_bounds__(kSamples) mst_threshold(int n, int m, const int* __restrict__ eweight,
                                                          MSTCtl* __restrict__ ctl, float light_factor) {
+  dep_wait();
   __shared__ int s[kSamples];
   const int t = threadIdx.x;
   const bool filter = m > 0 && (m / n) >= 4;
@@ -168,6 +171,7 @@ template <bool kLight>
 __global__ void __launch_bounds__(kTPB) mst_scan(FlatCsr g, bool vec, const int* __restrict__ eweight,
                                                  const int* __restrict__ parent, int4* __restrict__ wl, int cap,
                                                  MSTCtl* __restrict__ ctl, Status* __restrict__ status) {
+  dep_wait();
   __shared__ int4 stage_buf[kTPB / 32][kStage];
   __shared__ __align__(16) int s_mark[kTPB / 32][kFlatTile];
   const int wid = threadIdx.x >> 5;
@@ -504,17 +508,17 @@ ecl_status mst_enqueue(const GraphDev& g, unsigned char* in_mst, char* ws, Statu
   ECL_CUDA_TRY(cudaMemsetAsync(b.ctl, 0, sizeof(MSTCtl), stream));
   if (g.m > 0) ECL_CUDA_TRY(cudaMemsetAsync(in_mst, 0, (size_t)g.m, stream));
   ECL_CUDA_TRY(cudaMemsetAsync(b.tilerow, 0xff, sizeof(int) * ((size_t)flat_tiles(g.m) + 1), stream));
-  ECL_LAUNCH(mst_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, b.parent, b.minv, b.tilerow, status);
+  ECL_LAUNCH_NEXT(mst_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, b.parent, b.minv, b.tilerow, status);
   if (g.m > 0) {
     const float light = dev.mst_light_factor > 0.f ? dev.mst_light_factor : (g.m / g.n >= kDenseDegree ? 0.75f : 2.f);
-    ECL_LAUNCH(mst_threshold, 1, kSamples, 0, stream, g.n, g.m, g.eweight, b.ctl, light);
+    ECL_LAUNCH_NEXT(mst_threshold, 1, kSamples, 0, stream, g.n, g.m, g.eweight, b.ctl, light);
     mark();
     for (int pass = 0; pass < 2; pass++) {
       if (pass == 0) {
-        ECL_LAUNCH(mst_scan<true>, scan_grid, kTPB, 0, stream, fc, vec, g.eweight, b.parent, b.wlA, b.cap, b.ctl, status);
+        ECL_LAUNCH_NEXT(mst_scan<true>, scan_grid, kTPB, 0, stream, fc, vec, g.eweight, b.parent, b.wlA, b.cap, b.ctl, status);
       } else {
-        ECL_LAUNCH(mst_flatten, grid, kTPB, 0, stream, g.n, b.parent);
-        ECL_LAUNCH(mst_scan<false>, scan_grid, kTPB, 0, stream, fc, vec, g.eweight, b.parent, b.wlA, b.cap, b.ctl, status);
+        ECL_LAUNCH_NEXT(mst_flatten, grid, kTPB, 0, stream, g.n, b.parent);
+        ECL_LAUNCH_NEXT(mst_scan<false>, scan_grid, kTPB, 0, stream, fc, vec, g.eweight, b.parent, b.wlA, b.cap, b.ctl, status);
       }
       mark();
       ECL_CUDA_TRY(launch_cooperative_smem(mst_boruvka, coop_grid, kBorTPB, kBorSmem, stream, g.n, pass, b.wlA,

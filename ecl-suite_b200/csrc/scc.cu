@@ -134,12 +134,14 @@ __device__ __forceinline__ unsigned long long scc_mix(unsigned long long x) {
 
 __global__ void __launch_bounds__(kTPB) scc_rows(int n, int m, const int* __restrict__ nindex,
                                                  int* __restrict__ tilerow, Status* __restrict__ status) {
+  dep_wait();
   flat_rows_range(n, m, nindex, tilerow, (blockIdx.x * kTPB + threadIdx.x) & ~31, gridDim.x * kTPB, status);
 }
 
 // Bound by the one read of the entries: the hash is about 20 instructions each.
 __global__ void __launch_bounds__(kTPB) scc_symmetry(FlatCsr g, bool vec, SCCCtl* __restrict__ ctl,
                                                      Status* __restrict__ status) {
+  dep_wait();
   __shared__ __align__(16) int s_mark[kTPB / 32][kFlatTile];
   __shared__ unsigned long long s_sum[kTPB / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -177,6 +179,7 @@ __global__ void __launch_bounds__(kTPB) scc_symmetry(FlatCsr g, bool vec, SCCCtl
 // access per warp of the launch, not one per vertex.
 __global__ void __launch_bounds__(kTPB) scc_top(int n, const int* __restrict__ comp, int* __restrict__ top,
                                                 const SCCCtl* __restrict__ ctl) {
+  dep_wait();
   if (ld(&ctl->asym) != 0) return;
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5, nwarps = (gridDim.x * kTPB) >> 5;
@@ -196,6 +199,7 @@ __global__ void __launch_bounds__(kTPB) scc_top(int n, const int* __restrict__ c
 
 __global__ void __launch_bounds__(kTPB) scc_relabel(int n, int* __restrict__ comp, const int* __restrict__ top,
                                                     const SCCCtl* __restrict__ ctl) {
+  dep_wait();
   if (ld(&ctl->asym) != 0) return;
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     const int r = comp[v];
@@ -537,6 +541,7 @@ __global__ void __launch_bounds__(kTPB) scc_mark(int n, int m, const int* __rest
                                                  const int* __restrict__ nlist, int* __restrict__ flags,
                                                  int2* __restrict__ wl, RowChunks rc, Bins bins, bool vec,
                                                  Giant gi, SCCCtl* __restrict__ ctl, bool checked, Status* __restrict__ status) {
+  dep_wait();
   // nothing to do for a symmetric graph (its labels are written), and one of
   // the two forms runs, by whether the giant component was found
   if ((checked && ld(&ctl->asym) == 0) || (ld(&ctl->giant_ok) != 0) != kRest) return;
@@ -593,6 +598,7 @@ __global__ void __launch_bounds__(kTPB) scc_mark_chunks(int n, int m, const int*
                                                         int2* __restrict__ wl, RowChunks rc, int chunk, bool vec,
                                                         Giant gi, SCCCtl* __restrict__ ctl, bool checked,
                                                         Status* __restrict__ status) {
+  dep_wait();
   if ((checked && ld(&ctl->asym) == 0) || (ld(&ctl->giant_ok) != 0) != kRest) return;
   __shared__ int2 s_stage[kTPB / 32][kRest ? 128 : 1];
   WarpStage<int2, 128, true> stg{s_stage[threadIdx.x >> 5]};
@@ -888,16 +894,16 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
   const bool vec = (reinterpret_cast<uintptr_t>(g.nlist) & 15) == 0 && dev.row_vec;  // 16-byte row loads
   if (check) {
     ECL_CUDA_TRY(cudaMemsetAsync(b.tilerow, 0xff, sizeof(int) * ((size_t)flat_tiles(g.m) + 1), stream));
-    ECL_LAUNCH(scc_rows, dev.grid_blocks(kTPB, g.n, 0), kTPB, 0, stream, g.n, g.m, g.nindex, b.tilerow, status);
+    ECL_LAUNCH_NEXT(scc_rows, dev.grid_blocks(kTPB, g.n, 0), kTPB, 0, stream, g.n, g.m, g.nindex, b.tilerow, status);
     if (g.m > 0)
-      ECL_LAUNCH(scc_symmetry, dev.grid_blocks(kTPB, 0, g.m), kTPB, 0, stream,
+      ECL_LAUNCH_NEXT(scc_symmetry, dev.grid_blocks(kTPB, 0, g.m), kTPB, 0, stream,
                  FlatCsr{g.n, g.m, g.nindex, g.nlist, b.tilerow}, (reinterpret_cast<uintptr_t>(g.nlist) & 15) == 0, b.ctl,
                  status);
     const ecl_status st = cc_enqueue(g, label, b.cc_ws, status, dev, stream);
     if (st != ECL_OK) return st;
     // (the general path's flags stay zero when the graph is not symmetric)
-    ECL_LAUNCH(scc_top, dev.sms * 4, kTPB, 0, stream, g.n, label, b.flags, b.ctl);
-    ECL_LAUNCH(scc_relabel, dev.grid_blocks(kTPB, g.n, 0), kTPB, 0, stream, g.n, label, b.flags, b.ctl);
+    ECL_LAUNCH_NEXT(scc_top, dev.sms * 4, kTPB, 0, stream, g.n, label, b.flags, b.ctl);
+    ECL_LAUNCH_NEXT(scc_relabel, dev.grid_blocks(kTPB, g.n, 0), kTPB, 0, stream, g.n, label, b.flags, b.ctl);
   }
   const size_t words = ((size_t)g.n + 31) / 32;
   const Giant gi{b.bits, b.bits + words};
@@ -911,14 +917,14 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
                                     b.bits + 2 * words, b.queue, b.candA, b.candB, b.chunks, (int)row_chunk_capacity(g.m, kMinChunk), b.ctl,
                                     status));
   }
-  ECL_LAUNCH(scc_mark<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, gi,
+  ECL_LAUNCH_NEXT(scc_mark<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, gi,
              b.ctl, check, status);
-  ECL_LAUNCH(scc_mark_chunks<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins.chunk,
+  ECL_LAUNCH_NEXT(scc_mark_chunks<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins.chunk,
              vec, gi, b.ctl, check, status);
   if (giant) {
-    ECL_LAUNCH(scc_mark<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, gi,
+    ECL_LAUNCH_NEXT(scc_mark<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, gi,
                b.ctl, false, status);
-    ECL_LAUNCH(scc_mark_chunks<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins.chunk,
+    ECL_LAUNCH_NEXT(scc_mark_chunks<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins.chunk,
                vec, gi, b.ctl, false, status);
   }
   mark();
