@@ -278,25 +278,55 @@ __global__ void __launch_bounds__(kTPB) cc_flatten(int n, int* __restrict__ pare
   const int giant = kMark ? ctr->giant : -1;
   int known = -1;  // a root of this launch
   for (long long v0 = blockIdx.x * kTPB + threadIdx.x; v0 < n; v0 += (long long)stride * kFlattenBatch) {
-    int p[kFlattenBatch];
+    int q[kFlattenBatch];
+    bool go[kFlattenBatch];
+    bool any = false;
 #pragma unroll
     for (int k = 0; k < kFlattenBatch; k++) {
       const long long v = v0 + (long long)k * stride;
-      p[k] = v < n ? ld(&parent[v]) : -1;
+      q[k] = v < n ? ld(&parent[v]) : -1;
     }
 #pragma unroll
     for (int k = 0; k < kFlattenBatch; k++) {
-      if (p[k] < 0) continue;
-      const int v = (int)(v0 + (long long)k * stride);
-      int q = p[k], pp;
-      if (q != v) {
-        while (q != known && (pp = ld(&parent[q])) < q) {
-          st(&parent[v], pp);
-          q = pp;
-        }
-        known = q;
+      go[k] = q[k] >= 0 && q[k] != (int)(v0 + (long long)k * stride) && q[k] != known;
+      any |= go[k];
+    }
+    while (any) {
+      int pp[kFlattenBatch];
+#pragma unroll
+      for (int k = 0; k < kFlattenBatch; k++) {
+        bool first = go[k];
+#pragma unroll
+        for (int j = 0; j < k; j++) first = first && !(go[j] && q[j] == q[k]);
+        if (first) pp[k] = ld(&parent[q[k]]);
       }
-      if (kMark) ing[v] = q == giant;
+#pragma unroll
+      for (int k = 1; k < kFlattenBatch; k++)
+#pragma unroll
+        for (int j = k - 1; j >= 0; j--)  // the smallest such j is one that loaded
+          if (go[k] && go[j] && q[j] == q[k]) pp[k] = pp[j];
+#pragma unroll
+      for (int k = 0; k < kFlattenBatch; k++) {
+        if (!go[k]) continue;
+        if (pp[k] < q[k]) {
+          st(&parent[(int)(v0 + (long long)k * stride)], pp[k]);
+          q[k] = pp[k];
+        } else {
+          known = q[k];
+          go[k] = false;
+        }
+      }
+      any = false;
+#pragma unroll
+      for (int k = 0; k < kFlattenBatch; k++) {
+        go[k] = go[k] && q[k] != known;
+        any |= go[k];
+      }
+    }
+    if (kMark) {
+#pragma unroll
+      for (int k = 0; k < kFlattenBatch; k++)
+        if (q[k] >= 0) ing[v0 + (long long)k * stride] = q[k] == giant;
     }
   }
 }

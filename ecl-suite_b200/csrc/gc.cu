@@ -1053,8 +1053,12 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
   // the hub core (the sort keys are dead now: their buffer holds the ranks)
   const int cap = std::min(std::min(dev.gc_core_ranks > 0 ? dev.gc_core_ranks : kCoreDefault, kCoreMax), g.n);
   int* rank = reinterpret_cast<int*>(b.keys0);
-  ECL_LAUNCH_NEXT(gc_core_rank, grid, kTPB, 0, stream, order, rank, b.ctl, cap);
-  ECL_LAUNCH_NEXT(gc_core_translate, grid, kTPB, 0, stream, g.nindex, b.nl2, b.hc, order, rank, b.rowinfo, b.ctl, cap);
+  // (no more blocks than a full core has rows for: every warp of the launch
+  // asks for the core's size, and thousands of them queue at its word; a mesh
+  // of 0.7 M vertices, no core at all: 11 + 12 us with one block per 256
+  // vertices)
+  ECL_LAUNCH_NEXT(gc_core_rank, std::min(grid, (cap - 1) / kTPB + 1), kTPB, 0, stream, order, rank, b.ctl, cap);
+  ECL_LAUNCH_NEXT(gc_core_translate, std::min(grid, (cap - 1) / (kTPB / 32) + 1), kTPB, 0, stream, g.nindex, b.nl2, b.hc, order, rank, b.rowinfo, b.ctl, cap);
   ECL_CUDA_TRY(cudaFuncSetAttribute(gc_core, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gc_core_smem(cap)));
   // the core's cluster: as many CTAs as asked for when such a cluster fits
   // the device, else one CTA

@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kTPB) scc_symmetry(FlatCsr g, bool vec, SCCCtl
 __global__ void __launch_bounds__(kTPB) scc_top(int n, const int* __restrict__ comp, int* __restrict__ top,
                                                 const SCCCtl* __restrict__ ctl) {
   dep_wait();
-  if (ld(&ctl->asym) != 0) return;
+  if (ctl->asym != 0) return;  // as scc_mark
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5, nwarps = (gridDim.x * kTPB) >> 5;
   const int groups = (n - 1) / 32 + 1;
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(kTPB) scc_top(int n, const int* __restrict__ c
 __global__ void __launch_bounds__(kTPB) scc_relabel(int n, int* __restrict__ comp, const int* __restrict__ top,
                                                     const SCCCtl* __restrict__ ctl) {
   dep_wait();
-  if (ld(&ctl->asym) != 0) return;
+  if (ctl->asym != 0) return;  // as scc_mark
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     const int r = comp[v];
     comp[v] = max(r, __ldg(&top[r]));
@@ -543,8 +543,11 @@ __global__ void __launch_bounds__(kTPB) scc_mark(int n, int m, const int* __rest
                                                  Giant gi, SCCCtl* __restrict__ ctl, bool checked, Status* __restrict__ status) {
   dep_wait();
   // nothing to do for a symmetric graph (its labels are written), and one of
-  // the two forms runs, by whether the giant component was found
-  if ((checked && ld(&ctl->asym) == 0) || (ld(&ctl->giant_ok) != 0) != kRest) return;
+  // the two forms runs, by whether the giant component was found.  Words that
+  // nothing writes in this launch: plain loads, which L1 serves (as relaxed
+  // loads every warp of the grid queues at one L2 word: 6.4 us for 2824 blocks
+  // with nothing to do)
+  if ((checked && ctl->asym == 0) || (ctl->giant_ok != 0) != kRest) return;
   __shared__ int2 s_stage[kTPB / 32][kRest ? 128 : 1];
   WarpStage<int2, 128, true> stg{s_stage[threadIdx.x >> 5]};
   bool overflow = false;
@@ -599,7 +602,7 @@ __global__ void __launch_bounds__(kTPB) scc_mark_chunks(int n, int m, const int*
                                                         Giant gi, SCCCtl* __restrict__ ctl, bool checked,
                                                         Status* __restrict__ status) {
   dep_wait();
-  if ((checked && ld(&ctl->asym) == 0) || (ld(&ctl->giant_ok) != 0) != kRest) return;
+  if ((checked && ctl->asym == 0) || (ctl->giant_ok != 0) != kRest) return;  // as scc_mark
   __shared__ int2 s_stage[kTPB / 32][kRest ? 128 : 1];
   WarpStage<int2, 128, true> stg{s_stage[threadIdx.x >> 5]};
   bool overflow = false;
