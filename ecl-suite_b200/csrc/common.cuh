@@ -75,6 +75,17 @@ __device__ __forceinline__ T fetch_and(T* p, T v) {
 // Read-only input loads (never written during a solve).
 __device__ __forceinline__ int ldg(const int* p) { return __ldg(p); }
 
+// Graph of union vertex v: the last g with vbase[g] <= v (binary search).
+__device__ __forceinline__ int union_graph_of(const int* vbase, int ngraphs, int v) {
+  int lo = 0, hi = ngraphs - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (__ldg(&vbase[mid]) <= v) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
 // Device status block, one per solve, in the workspace.  Kernels report
 // failures here instead of trapping; the host reads it after the solve.
 struct Status {

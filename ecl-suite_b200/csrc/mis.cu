@@ -55,17 +55,6 @@ __device__ __forceinline__ unsigned mis_priority(int v, int degree, float avg, f
   return (unsigned)((res + res) | 1) & 0xffu;
 }
 
-// Graph of union vertex v: the last g with vbase[g] <= v (binary search).
-__device__ __forceinline__ int union_graph_of(const int* vbase, int ngraphs, int v) {
-  int lo = 0, hi = ngraphs - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (__ldg(&vbase[mid]) <= v) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-
 // For a union of graphs (vbase != nullptr) every vertex uses ITS graph's
 // average degree and its local id, so each graph's bytes are exactly the ones
 // a solve of that graph alone computes.

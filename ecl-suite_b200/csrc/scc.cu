@@ -865,7 +865,7 @@ size_t scc_workspace_bytes(int n, int m) {
 namespace ecl {
 
 ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, const DeviceInfo& dev,
-                       cudaStream_t stream, int max_rounds, Marker mark) {
+                       cudaStream_t stream, int max_rounds, Marker mark, const UnionInfo* uni) {
   Carve c{ws};
   SCCBufs b;
   scc_layout(c, g.n, g.m, &b);
@@ -902,7 +902,7 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
       ECL_LAUNCH_NEXT(scc_symmetry, dev.grid_blocks(kTPB, 0, g.m), kTPB, 0, stream,
                  FlatCsr{g.n, g.m, g.nindex, g.nlist, b.tilerow}, (reinterpret_cast<uintptr_t>(g.nlist) & 15) == 0, b.ctl,
                  status);
-    const ecl_status st = cc_enqueue(g, label, b.cc_ws, status, dev, stream);
+    const ecl_status st = cc_enqueue(g, label, b.cc_ws, status, dev, stream, {}, uni);
     if (st != ECL_OK) return st;
     // (the general path's flags stay zero when the graph is not symmetric)
     ECL_LAUNCH_NEXT(scc_top, dev.sms * 4, kTPB, 0, stream, g.n, label, b.flags, b.ctl);

@@ -23,11 +23,13 @@ struct GraphDev {
 
 // A disjoint union of graphs (batched engine): graph g owns vertices
 // [vbase[g], vbase[g+1]); avg[g] = (float)edges_g / nodes_g, the value the
-// MIS priority of that graph uses.
+// MIS priority of that graph uses; giants[] is scratch of one word a graph
+// for CC.
 struct UnionInfo {
   int ngraphs = 0;
   const int* vbase = nullptr;
   const float* avg = nullptr;
+  int* giants = nullptr;
 };
 
 // Optional phase marks (Solve::mark) between kernel phases.
@@ -45,7 +47,7 @@ size_t mst_workspace_bytes(int n, int m);
 size_t scc_workspace_bytes(int n, int m);
 
 ecl_status cc_enqueue(const GraphDev& g, int* label, char* ws, dev::Status* status, const DeviceInfo& dev,
-                      cudaStream_t stream, Marker mark = {});
+                      cudaStream_t stream, Marker mark = {}, const UnionInfo* uni = nullptr);
 ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, dev::Status* status, const DeviceInfo& dev,
                        cudaStream_t stream, int max_sweeps, const UnionInfo* uni = nullptr, Marker mark = {});
 ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, dev::Status* status, const DeviceInfo& dev,
@@ -54,6 +56,6 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, dev::Status* stat
 ecl_status mst_enqueue(const GraphDev& g, unsigned char* in_mst, char* ws, dev::Status* status, const DeviceInfo& dev,
                        cudaStream_t stream, unsigned long long** total_dev, Marker mark = {});
 ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, dev::Status* status, const DeviceInfo& dev,
-                       cudaStream_t stream, int max_rounds, Marker mark = {});
+                       cudaStream_t stream, int max_rounds, Marker mark = {}, const UnionInfo* uni = nullptr);
 
 }  // namespace ecl

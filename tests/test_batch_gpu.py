@@ -72,3 +72,36 @@ def test_batch_mst_weights_at_tile_edges(ecl, orc, sizes):
             inm, tot = b.result(i, ecl.BATCH_MST)
             einm, etot = orc.mst(b.graph(i))
             assert tot == etot and np.array_equal(inm, einm), i
+
+
+@pytest.mark.parametrize("directed", [False, True])
+@pytest.mark.parametrize("count", [1, 2, 33])
+def test_batch_labels_with_a_large_tree_in_every_graph(ecl, orc, count, directed):
+    """CC and SCC labels are ids of the vertex's own graph, wherever its
+    largest component lies and whatever is left outside it."""
+    rng = np.random.default_rng(100 * count + directed)
+    b = ecl.Batch()
+    for k in range(count):
+        kind = k % 4
+        if kind == 0:  # two trees of the same size, a star of 300 and vertices without entries
+            n = 1800
+            edges = [(i, i + 1) for i in range(100, 700)] + [(i, i + 1) for i in range(800, 1400)]
+            edges += [(1400, i) for i in range(1401, 1701)]
+        elif kind == 1:
+            n, edges = 1, []
+        elif kind == 2:  # one tree, with the hub last
+            n = 9000
+            edges = [(n - 1, i) for i in range(0, n - 1, 2)] + [(i, i + 1) for i in range(0, n - 2, 2)]
+        else:  # about as many edges as vertices: one large and many small components
+            n = 3000
+            edges = [(int(u), int(v)) for u, v in rng.integers(0, n, (n // 2 + 300, 2)) if u != v]
+        g = undirected(n, edges)
+        g.symmetric = not directed  # unflagged, the union takes the general paths
+        b.add(g)
+    b.build(ecl.BATCH_CC | ecl.BATCH_SCC)
+    for _ in range(2):  # (the second a replay)
+        b.run()
+        for i in range(b.graphs):
+            g = b.graph(i)
+            assert np.array_equal(b.result(i, ecl.BATCH_CC), orc.cc(g)), i
+            assert np.array_equal(b.result(i, ecl.BATCH_SCC), orc.scc(g)), i
