@@ -215,6 +215,13 @@ ecl_status check_status(const ecl_batch* b) {
   return ECL_OK;
 }
 
+cudaError_t result_to_host(const ecl_batch* b, void* dst, const void* src, size_t bytes) {
+  Staging g;
+  cudaError_t e;
+  if (g.to_host(dst, src, bytes, b->stream, &e)) return e;
+  return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
+}
+
 }  // namespace
 }  // namespace ecl
 
@@ -564,16 +571,16 @@ ecl_status ecl_batch_result(const ecl_batch* b, int32_t i, uint32_t code, void* 
   switch (code) {
     case ECL_BATCH_CC:
     case ECL_BATCH_SCC:
-      ECL_CUDA_TRY(cudaMemcpy(host_out, (code == ECL_BATCH_CC ? s.cc : s.scc) + v0, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost));
+      ECL_CUDA_TRY(result_to_host(b, host_out, (code == ECL_BATCH_CC ? s.cc : s.scc) + v0, sizeof(int) * (size_t)n));
       return ECL_OK;
     case ECL_BATCH_MIS:
-      ECL_CUDA_TRY(cudaMemcpy(host_out, s.mis + v0, (size_t)n, cudaMemcpyDeviceToHost));
+      ECL_CUDA_TRY(result_to_host(b, host_out, s.mis + v0, (size_t)n));
       return ECL_OK;
     case ECL_BATCH_GC:
-      ECL_CUDA_TRY(cudaMemcpy(host_out, s.gc + v0, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost));
+      ECL_CUDA_TRY(result_to_host(b, host_out, s.gc + v0, sizeof(int) * (size_t)n));
       return ECL_OK;
     case ECL_BATCH_MST:
-      if (m) ECL_CUDA_TRY(cudaMemcpy(host_out, s.mst + e0, (size_t)m, cudaMemcpyDeviceToHost));
+      if (m) ECL_CUDA_TRY(result_to_host(b, host_out, s.mst + e0, (size_t)m));
       if (total_weight) *total_weight = s.h_totals()[k];
       return ECL_OK;
   }

@@ -128,9 +128,9 @@ ecl_status Solve::begin(const GraphNeeds& needs, size_t ws_bytes) {
     int* d_w = nullptr;
     if (needs.weights && g_->eweight) d_w = static_cast<int*>(temp(sizeof(int) * (size_t)(m > 0 ? m : 1)));
     if (alloc_failed) return ECL_ERR_OOM;
-    ECL_CUDA_TRY(cudaMemcpyAsync(d_idx, g_->nindex, sizeof(int) * ((size_t)n + 1), cudaMemcpyHostToDevice, stream));
-    if (m) ECL_CUDA_TRY(cudaMemcpyAsync(d_list, g_->nlist, sizeof(int) * (size_t)m, cudaMemcpyHostToDevice, stream));
-    if (d_w && m) ECL_CUDA_TRY(cudaMemcpyAsync(d_w, g_->eweight, sizeof(int) * (size_t)m, cudaMemcpyHostToDevice, stream));
+    ECL_CUDA_TRY(to_device(d_idx, g_->nindex, sizeof(int) * ((size_t)n + 1)));
+    if (m) ECL_CUDA_TRY(to_device(d_list, g_->nlist, sizeof(int) * (size_t)m));
+    if (d_w && m) ECL_CUDA_TRY(to_device(d_w, g_->eweight, sizeof(int) * (size_t)m));
     nindex = d_idx;
     nlist = d_list;
     eweight = d_w;
@@ -152,6 +152,18 @@ ecl_status Solve::begin(const GraphNeeds& needs, size_t ws_bytes) {
   ws += kStatusBytes;
   ECL_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(dev::Status), stream));
   return ECL_OK;
+}
+
+cudaError_t Solve::to_device(void* dst, const void* src, size_t bytes) {
+  cudaError_t e;
+  if (staging_.to_device(dst, src, bytes, stream, &e)) return e;
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream);
+}
+
+cudaError_t Solve::to_host(void* dst, const void* src, size_t bytes) {
+  cudaError_t e;
+  if (staging_.to_host(dst, src, bytes, stream, &e)) return e;
+  return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream);
 }
 
 void* Solve::temp(size_t bytes) {
@@ -199,7 +211,7 @@ ecl_status Solve::finish(ecl_status st) {
   dev::Status hs{};
   if (st == ECL_OK && status) {
     for (const Copy& c : outs_) {
-      if (c.bytes && cudaMemcpyAsync(c.host, c.dev, c.bytes, cudaMemcpyDeviceToHost, stream) != cudaSuccess) {
+      if (c.bytes && to_host(c.host, c.dev, c.bytes) != cudaSuccess) {
         set_last_error("cudaMemcpyAsync(D2H)", cudaGetLastError());
         st = ECL_ERR_CUDA;
       }
@@ -207,6 +219,7 @@ ecl_status Solve::finish(ecl_status st) {
     if (cudaMemcpyAsync(&hs, status, sizeof(hs), cudaMemcpyDeviceToHost, stream) != cudaSuccess) st = ECL_ERR_CUDA;
   }
   cudaError_t e = cudaStreamSynchronize(stream);
+  staging_.release();
   if (e != cudaSuccess && st == ECL_OK) {
     set_last_error("solve", e);
     st = ECL_ERR_CUDA;

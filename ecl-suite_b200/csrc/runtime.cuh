@@ -15,6 +15,7 @@
 #include "common.cuh"
 #include "csr_bins.cuh"
 #include "ecl_b200.h"
+#include "staging.cuh"
 
 namespace ecl {
 
@@ -234,6 +235,9 @@ class Solve {
     void* dev;
     size_t bytes;
   };
+  cudaError_t to_device(void* dst, const void* src, size_t bytes);
+  cudaError_t to_host(void* dst, const void* src, size_t bytes);
+  Staging staging_;
   std::vector<Copy> outs_;
   std::vector<void*> temps_;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;

@@ -465,3 +465,55 @@ def test_mst_on_arrays_that_are_not_16_byte_aligned(ecl, orc):
     inm, tot = ecl.mst(dg)
     einm, etot = orc.mst(g)
     assert tot == etot and np.array_equal(inm.cpu().numpy(), einm)
+
+
+@pytest.mark.parametrize("users", [1, 7])
+def test_host_graphs_through_page_locked_pieces(ecl, users):
+    """Pageable inputs and outputs around the smallest size that goes through
+    page-locked memory, one piece, one block and several of them; and by more
+    threads at once than there are blocks."""
+    import threading
+
+    import torch
+
+    rng = np.random.default_rng(11)
+    graphs = []
+    for n in (65535, 65536, 262144, 262145, 1048576, 1048577, 1350001):  # labels of 4 bytes
+        # a long path without a tenth of its links
+        link = rng.random(n - 1) < 0.9
+        deg = np.zeros(n, np.int64)
+        deg[:-1] += link
+        deg[1:] += link
+        nindex = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+        u = np.flatnonzero(link)
+        row, col = np.concatenate([u, u + 1]), np.concatenate([u + 1, u])
+        nlist = col[np.lexsort((col, row))].astype(np.int32)
+        w = rng.integers(1, 1 << 30, n).astype(np.int32)
+        src = np.repeat(np.arange(n), deg)
+        g = ecl.Graph(nindex, nlist, w[np.minimum(src, nlist)], True)
+        start = np.concatenate([[True], ~link])
+        want = np.maximum.accumulate(np.where(start, np.arange(n), 0))
+        graphs.append((g, want, int(w[u].astype(np.int64).sum())))
+    bad = []
+
+    def user(k):
+        s = torch.cuda.Stream()
+        for i in range(len(graphs)):
+            g, want, total = graphs[(i + k) % len(graphs)]
+            labels = np.full(g.nodes, -1, np.int32)
+            ecl.cc(g, out=labels, stream=s.cuda_stream)
+            inm, tot = ecl.mst(g, stream=s.cuda_stream)[:2]
+            src = np.repeat(np.arange(g.nodes), np.diff(g.nindex))
+            once = np.asarray(inm).astype(bool)
+            if not np.array_equal(labels, want) or tot != total or once.sum() != g.edges // 2:
+                bad.append((k, i))
+            a, b = np.minimum(src[once], g.nlist[once]), np.maximum(src[once], g.nlist[once])
+            if len(np.unique(a)) != len(a) or not np.array_equal(b, a + 1):
+                bad.append((k, i, "edges"))
+
+    threads = [threading.Thread(target=user, args=(k,)) for k in range(users)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
