@@ -171,6 +171,34 @@ struct WarpStage {
     if (count > kCap - 32) flush(out, counter, cap, overflow);
   }
 
+  // As kMany pushes, the k-th of item(k) where bit k of `mask` is set: one
+  // prefix sum over the lanes instead of a ballot for each.
+  template <int kMany, class F>
+  __device__ __forceinline__ void push_some(unsigned mask, F&& item, T* out, int* counter, long long cap, bool& overflow) {
+    const int lane = threadIdx.x & 31;
+    const int mine = __popc(mask);
+    int at = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(kFull, at, o);
+      if (lane >= o) at += x;
+    }
+    const int total = __shfl_sync(kFull, at, 31);
+    if (total == 0) return;
+    if (total > kCap) {
+#pragma unroll
+      for (int k = 0; k < kMany; k++) push((mask >> k) & 1u, item(k), out, counter, cap, overflow);
+      return;
+    }
+    if (count + total > kCap) flush(out, counter, cap, overflow);
+    at += count - mine;
+#pragma unroll
+    for (int k = 0; k < kMany; k++)
+      if ((mask >> k) & 1u) buf[at++] = item(k);
+    count += total;
+    if (count > kCap - 32) flush(out, counter, cap, overflow);
+  }
+
   __device__ __forceinline__ void flush(T* out, int* counter, long long cap, bool& overflow) {
     const int lane = threadIdx.x & 31;
     __syncwarp();

@@ -56,7 +56,6 @@ struct MSTCtl {
   int wlcount[2][kMaxRounds + 2];    // [pass][round] sizes of the edge list
   int rootcount[2][kMaxRounds + 2];  // [pass][round] roots that may still have edges
   int threshold;
-  int filter;
   u64 total;
   // %globaltimer when each pass started and after each of its barriers
   // (phases A, B and C of round r end at [3r + 1], [3r + 2] and [3r + 3]): a
@@ -88,37 +87,19 @@ __global__ void __launch_bounds__(kTPB) mst_flatten(int n, int* __restrict__ par
   }
 }
 
-// Also finds the rows of the scans' tiles (and so checks the CSR rows once: a
-// malformed row raises ECL_ERR_BAD_GRAPH).
-__global__ void __launch_bounds__(kTPB) mst_init(int n, int m, const int* __restrict__ nindex, int* __restrict__ parent,
-                                                 u64* __restrict__ minv, int* __restrict__ tilerow,
-                                                 Status* __restrict__ status) {
-  dep_wait();
-  for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
-    // race-free: thread-owned init, no reader in this launch
-    parent[v] = v;
-    minv[v] = ~0ull;
-  }
-  if (m > 0) flat_rows_range(n, m, nindex, tilerow, (blockIdx.x * kTPB + threadIdx.x) & ~31, gridDim.x * kTPB, status);
-}
-
 // Threshold = the k-th smallest of kSamples sampled weights, k chosen so the
 // light pass keeps about light_factor * n of the m entries (the reference
 // aims at 3n, ECL-MST_10-atomic.cu:450-459; the batched engine's autotuner
-// may pick another factor -- the forest does not depend on it).  No
-// filtering when edges/nodes < 4.
-__global__ void __launch_bounds__(kSamples) mst_threshold(int n, int m, const int* __restrict__ eweight,
-                                                         MSTCtl* __restrict__ ctl, float light_factor) {
-  dep_wait();
+// may pick another factor -- the forest does not depend on it).
+__device__ void mst_threshold(int n, int m, const int* eweight, MSTCtl* ctl, float light_factor) {
   __shared__ int s[kSamples];
-  const int t = threadIdx.x;
-  const bool filter = m > 0 && (m / n) >= 4;
-  s[t] = filter ? __ldg(&eweight[ecl_hash((unsigned)t * 2654435761u + 12345u) % (unsigned)m]) : 0;
+  for (int t = threadIdx.x; t < kSamples; t += kTPB)
+    s[t] = __ldg(&eweight[ecl_hash((unsigned)t * 2654435761u + 12345u) % (unsigned)m]);
   __syncthreads();
   for (int k = 2; k <= kSamples; k <<= 1) {
     for (int j = k >> 1; j > 0; j >>= 1) {
-      const int p = t ^ j;
-      if (p > t) {
+      for (int i = threadIdx.x; i < kSamples / 2; i += kTPB) {
+        const int t = 2 * i - (i & (j - 1)), p = t + j;  // the i-th pair j apart
         const int a = s[t], b = s[p];
         const bool up = (t & k) == 0;
         if ((a > b) == up) {
@@ -129,16 +110,32 @@ __global__ void __launch_bounds__(kSamples) mst_threshold(int n, int m, const in
       __syncthreads();
     }
   }
-  if (t == 0) {
-    ctl->filter = filter ? 1 : 0;
-    if (filter) {
-      const double frac = (double)light_factor * (double)n / (double)m;
-      const int k = min(kSamples - 1, (int)(frac * kSamples));
-      ctl->threshold = s[k];
-    } else {
-      ctl->threshold = 0x7fffffff;
-    }
+  if (threadIdx.x == 0) {
+    const double frac = (double)light_factor * (double)n / (double)m;
+    ctl->threshold = s[min(kSamples - 1, (int)(frac * kSamples))];
   }
+}
+
+// Also finds the rows of the scans' tiles (and so checks the CSR rows once: a
+// malformed row raises ECL_ERR_BAD_GRAPH).  With a light pass to come, the
+// first block finds its threshold meanwhile (in a launch of its own this took
+// 7 to 10 us).
+__global__ void __launch_bounds__(kTPB) mst_init(int n, int m, const int* __restrict__ nindex, int* __restrict__ parent,
+                                                 u64* __restrict__ minv, int* __restrict__ tilerow,
+                                                 const int* __restrict__ eweight, MSTCtl* __restrict__ ctl,
+                                                 float light_factor, bool filter, Status* __restrict__ status) {
+  dep_wait();
+  if (filter && blockIdx.x == 0) {
+    mst_threshold(n, m, eweight, ctl, light_factor);
+    return;
+  }
+  const int first = ((int)blockIdx.x - filter) * kTPB + threadIdx.x, stride = ((int)gridDim.x - filter) * kTPB;
+  for (int v = first; v < n; v += stride) {
+    // race-free: thread-owned init, no reader in this launch
+    parent[v] = v;
+    minv[v] = ~0ull;
+  }
+  if (m > 0) flat_rows_range(n, m, nindex, tilerow, first & ~31, stride, status);
 }
 
 // Slots per warp in the shared-memory staging of worklist appends.
@@ -162,20 +159,25 @@ __device__ __forceinline__ void mst_overflow(bool overflow, Status* status) {
 // every light entry (and checked every weight), so those are all heavy, and
 // the ~80 % of entries inside one component cost no weight load.  parent[] is
 // flat and not written in this launch, so its loads are read-only ones that L1
-// serves.  Bound by the stream of nlist and weights (light) and by the 4-byte
-// root gathers, one for half the entries (heavy), and in both by about 400 to 650 warp
-// instructions a tile.  Measured at R-MAT-22, rows per lane / warp / chunk
-// record in two launches -> this: light 0.55 -> 0.32 ms, heavy (with the
-// flattening) 0.86 -> 0.55; 1000 vertices, 12 k entries: 36 -> 9 us and 50 -> 13.
+// serves.  Bound by instructions (about 450 a tile in the light scan, 650 in
+// the heavy one) at the half of the warps that 48 and 64 registers leave: the
+// entries and weights alone would take 0.13 ms at R-MAT-22 (128 M entries).
+// The light scan takes 0.29 ms with five blocks an SM and 0.31 with four, the
+// heavy one 0.54 with four and 0.55 with five (spilled registers).  One bit a
+// vertex for "in the largest tree", looked up before the roots, did not make
+// it faster (0.53 -> 0.53): the gathers are not the bound.  Before the flat
+// tiles, rows per lane / warp / chunk record in two launches: light 0.55 ms,
+// heavy (with the flattening) 0.86; 1000 vertices, 12 k entries: 36 us and 50,
+// now 9 and 13.
 template <bool kLight>
-__global__ void __launch_bounds__(kTPB) mst_scan(FlatCsr g, bool vec, const int* __restrict__ eweight,
-                                                 const int* __restrict__ parent, int4* __restrict__ wl, int cap,
+__global__ void __launch_bounds__(kTPB, kLight ? 5 : 4) mst_scan(FlatCsr g, bool vec, const int* __restrict__ eweight,
+                                                 const int* __restrict__ parent, int4* __restrict__ wl, int cap, bool filter,
                                                  MSTCtl* __restrict__ ctl, Status* __restrict__ status) {
   dep_wait();
   __shared__ int4 stage_buf[kTPB / 32][kStage];
   __shared__ __align__(16) int s_mark[kTPB / 32][kFlatTile];
   const int wid = threadIdx.x >> 5;
-  const int thr = ctl->threshold;
+  const int thr = filter ? ctl->threshold : 0x7fffffff;
   int* cnt = &ctl->wlcount[kLight ? 0 : 1][0];
   Stage stg{stage_buf[wid]};
   bool overflow = false;
@@ -219,9 +221,11 @@ __global__ void __launch_bounds__(kTPB) mst_scan(FlatCsr g, bool vec, const int*
           keep = false;
         }
         if (kLight) keep = keep && w[k] <= thr;
-        if (__any_sync(kFull, keep))
-          stg.push(keep, make_int4(kLight ? row[k] : a[k], kLight ? u[k] : b[k], w[k], e0 + k), wl, cnt, cap, overflow);
+        if (!keep) want &= ~(1u << k);
       }
+      stg.template push_some<kFlatLane>(
+          want, [&](int k) { return make_int4(kLight ? row[k] : a[k], kLight ? u[k] : b[k], w[k], e0 + k); }, wl, cnt, cap,
+          overflow);
     });
   stg.flush(wl, cnt, cap, overflow);
   mst_overflow(overflow, status);
@@ -508,24 +512,32 @@ ecl_status mst_enqueue(const GraphDev& g, unsigned char* in_mst, char* ws, Statu
   ECL_CUDA_TRY(cudaMemsetAsync(b.ctl, 0, sizeof(MSTCtl), stream));
   if (g.m > 0) ECL_CUDA_TRY(cudaMemsetAsync(in_mst, 0, (size_t)g.m, stream));
   ECL_CUDA_TRY(cudaMemsetAsync(b.tilerow, 0xff, sizeof(int) * ((size_t)flat_tiles(g.m) + 1), stream));
-  ECL_LAUNCH_NEXT(mst_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, b.parent, b.minv, b.tilerow, status);
+  // No light pass below 4 entries a vertex: all weights pass the first scan,
+  // and the second would find nothing.
+  const bool filter = g.m / g.n >= 4;
+  const float light = dev.mst_light_factor > 0.f ? dev.mst_light_factor : (g.m / g.n >= kDenseDegree ? 0.75f : 2.f);
+  ECL_LAUNCH_NEXT(mst_init, grid + filter, kTPB, 0, stream, g.n, g.m, g.nindex, b.parent, b.minv, b.tilerow, g.eweight,
+                  b.ctl, light, filter, status);
   if (g.m > 0) {
-    const float light = dev.mst_light_factor > 0.f ? dev.mst_light_factor : (g.m / g.n >= kDenseDegree ? 0.75f : 2.f);
-    ECL_LAUNCH_NEXT(mst_threshold, 1, kSamples, 0, stream, g.n, g.m, g.eweight, b.ctl, light);
     mark();
     for (int pass = 0; pass < 2; pass++) {
+      if (pass == 1 && !filter) {
+        mark();
+        mark();
+        break;
+      }
       if (pass == 0) {
-        ECL_LAUNCH_NEXT(mst_scan<true>, scan_grid, kTPB, 0, stream, fc, vec, g.eweight, b.parent, b.wlA, b.cap, b.ctl, status);
+        ECL_LAUNCH_NEXT(mst_scan<true>, scan_grid, kTPB, 0, stream, fc, vec, g.eweight, b.parent, b.wlA, b.cap, filter,
+                        b.ctl, status);
       } else {
         ECL_LAUNCH_NEXT(mst_flatten, grid, kTPB, 0, stream, g.n, b.parent);
-        ECL_LAUNCH_NEXT(mst_scan<false>, scan_grid, kTPB, 0, stream, fc, vec, g.eweight, b.parent, b.wlA, b.cap, b.ctl, status);
+        ECL_LAUNCH_NEXT(mst_scan<false>, scan_grid, kTPB, 0, stream, fc, vec, g.eweight, b.parent, b.wlA, b.cap, filter,
+                        b.ctl, status);
       }
       mark();
       ECL_CUDA_TRY(launch_cooperative_smem(mst_boruvka, coop_grid, kBorTPB, kBorSmem, stream, g.n, pass, b.wlA,
                                            b.wlB, b.cap, b.parent, b.minv, b.rootsA, b.rootsB, in_mst, b.ctl, status));
       mark();
-      // The heavy pass (pass 1) runs unconditionally: with no filter it finds
-      // no entry above the INT_MAX threshold and ends after one round.
     }
   }
   return ECL_OK;
