@@ -280,6 +280,108 @@ struct RootTable {
   }
 };
 
+// Phase B for one entry: the root whose smallest key it is hooks to the other;
+// of two that both chose it the smaller id stays a root.
+__device__ __forceinline__ void mst_hook(const int4& e, u64 ka, u64 kb, int* parent, unsigned char* in_mst, u64& local) {
+  const u64 key = ((u64)(unsigned)e.z << 32) | (unsigned)e.w;
+  const bool ha = ka == key, hb = kb == key;
+  if (!ha && !hb) return;
+  if (ha && !(hb && e.x < e.y)) st(&parent[e.x], e.y);
+  if (hb && !(ha && e.y < e.x)) st(&parent[e.y], e.x);
+  in_mst[e.w] = 1;  // race-free: one entry j stands once in the list, and the flags are never read here
+  local += (u64)(unsigned)e.z;
+}
+
+// The remaining rounds of a list of at most kSolo entries, by the first block
+// alone: the same three phases with block barriers between them, the entries
+// relabelled in place and the key words cleared by the entries that lowered
+// them.  A short round is all latency, and the block's own rounds have no grid
+// barriers, no list to write and no roots to list: 5 us each against 14 for the
+// general form on one block.  Measured, the light pass's rounds, general form /
+// kSolo = 512 / 2048 / 8192: R-MAT with 1 k vertices 64 / 24 / 25 / 24 us, with
+// 2 k 57 / 57 / 49 / 47, G(5 k, 15 k) 98 / 98 / 85 / 134, G(20 k, 80 k) 124 /
+// 123 / 124 / 154: one block is too narrow for longer lists.  All threads of
+// the block call.
+constexpr int kSolo = 2048;
+
+__device__ __forceinline__ int mst_root(int v, const int* parent) {
+  int p;
+  while ((p = ld(&parent[v])) != v) v = p;
+  return v;
+}
+
+__device__ __noinline__ void mst_solo(int4* list, int sz, int& r, int* parent, u64* minv, unsigned char* in_mst,
+                                      RootTable tab, u64& local) {
+  bool lowered = false;
+  for (; r < kMaxRounds; r++) {
+    tab.reset();
+    bool live = false;
+    for (int i0 = threadIdx.x; i0 < sz; i0 += kBorTPB * kBorBatch) {
+      int2 e[kBorBatch];
+      int a[kBorBatch], b[kBorBatch];
+#pragma unroll
+      for (int k = 0; k < kBorBatch; k++) {
+        const int i = i0 + k * kBorTPB;
+        e[k] = i < sz ? *reinterpret_cast<const int2*>(&list[i]) : make_int2(-1, -1);
+      }
+#pragma unroll
+      for (int k = 0; k < kBorBatch; k++) {
+        if (e[k].x < 0) continue;
+        if (lowered) {
+          st(&minv[e[k].x], ~0ull);
+          st(&minv[e[k].y], ~0ull);
+        }
+        a[k] = ld(&parent[e[k].x]);
+        b[k] = ld(&parent[e[k].y]);
+      }
+#pragma unroll
+      for (int k = 0; k < kBorBatch; k++) {
+        if (e[k].x < 0) continue;
+        if (a[k] != e[k].x) a[k] = mst_root(a[k], parent);
+        if (b[k] != e[k].y) b[k] = mst_root(b[k], parent);
+        if (a[k] == b[k]) a[k] = -1;
+        live |= a[k] >= 0;
+        *reinterpret_cast<int2*>(&list[i0 + k * kBorTPB]) = make_int2(a[k], b[k]);
+      }
+    }
+    if (!__syncthreads_or(live)) break;
+    for (int i = threadIdx.x; i < sz; i += kBorTPB) {
+      const int4 e = list[i];
+      if (e.x < 0) continue;
+      const u64 key = ((u64)(unsigned)e.z << 32) | (unsigned)e.w;
+      bool had;
+      if (!tab.lower(e.x, key, &had)) fetch_min(&minv[e.x], key);
+      if (!tab.lower(e.y, key, &had)) fetch_min(&minv[e.y], key);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < kRootSlots; i += kBorTPB) {
+      const int rt = tab.root[i];  // race-free: claims ended at the barrier above
+      if (rt >= 0) fetch_min(&minv[rt], tab.key[i]);
+    }
+    __syncthreads();
+    for (int i0 = threadIdx.x; i0 < sz; i0 += kBorTPB * kBorBatch) {
+      int4 e[kBorBatch];
+      u64 ka[kBorBatch], kb[kBorBatch];
+#pragma unroll
+      for (int k = 0; k < kBorBatch; k++) {
+        const int i = i0 + k * kBorTPB;
+        e[k] = i < sz ? list[i] : make_int4(-1, -1, 0, 0);
+      }
+#pragma unroll
+      for (int k = 0; k < kBorBatch; k++) {
+        if (e[k].x < 0) continue;
+        ka[k] = ld(&minv[e[k].x]);
+        kb[k] = ld(&minv[e[k].y]);
+      }
+#pragma unroll
+      for (int k = 0; k < kBorBatch; k++)
+        if (e[k].x >= 0) mst_hook(e[k], ka[k], kb[k], parent, in_mst, local);
+    }
+    lowered = true;
+    __syncthreads();
+  }
+}
+
 // All Boruvka rounds of one pass.  wlA holds the pass's initial worklist
 // (size wlcount[pass][0]), whose entries join two distinct roots; later rounds
 // alternate wlA / wlB.  A round has three phases, a grid barrier after each:
@@ -330,6 +432,10 @@ __global__ void __launch_bounds__(kBorTPB, 1) mst_boruvka(int n, int pass, int4*
     // than the list holds
     const int sz = min(ld(&cnt[r]), cap);
     if (sz == 0) break;  // the same for every thread: no phase writes cnt[r] any more
+    if (sz <= kSolo) {
+      if (blockIdx.x == 0) mst_solo(in, sz, r, parent, minv, in_mst, tab, local);
+      break;
+    }
     // ---- A
     tab.reset();
     if (threadIdx.x == 0) s_seen = 0;
@@ -415,13 +521,7 @@ __global__ void __launch_bounds__(kBorTPB, 1) mst_boruvka(int n, int pass, int4*
       }
 #pragma unroll
       for (int k = 0; k < kBorBatch; k++) {
-        const u64 key = ((u64)(unsigned)e[k].z << 32) | (unsigned)e[k].w;
-        const bool ha = e[k].x >= 0 && ka[k] == key, hb = e[k].x >= 0 && kb[k] == key;
-        if (!ha && !hb) continue;
-        if (ha && !(hb && e[k].x < e[k].y)) st(&parent[e[k].x], e[k].y);
-        if (hb && !(ha && e[k].y < e[k].x)) st(&parent[e[k].y], e[k].x);
-        in_mst[e[k].w] = 1;  // race-free: one entry j stands once in the list, and the flags are never read here
-        local += (u64)(unsigned)e[k].z;
+        if (e[k].x >= 0) mst_hook(e[k], ka[k], kb[k], parent, in_mst, local);
       }
     }
     if (!grid_sync(&ctl->bar, status)) return;

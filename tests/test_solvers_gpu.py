@@ -517,3 +517,24 @@ def test_host_graphs_through_page_locked_pieces(ecl, users):
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("edges", [1, 31, 1024, 1025, 2047, 2048, 2049, 40000])
+def test_mst_lists_that_one_block_finishes(ecl, orc, edges):
+    """Lists of at most 2048 entries are finished by one block: from the first
+    round, from a later one, with many components and with one hub; equal
+    weights are told apart by the entry."""
+    rng = np.random.default_rng(edges)
+    n = edges + 1
+    chain = [(i, i + 1) for i in range(edges)]
+    star = [(0, i) for i in range(1, n)]
+    k = max(2, edges // 3)  # about three edges a vertex
+    dense = sorted({(int(min(u, v)), int(max(u, v))) for u, v in rng.integers(0, k, (edges, 2)) if u != v}) or [(0, 1)]
+    pairs = [(2 * i, 2 * i + 1) for i in range(edges // 2)] or [(0, 1)]  # nothing left after a round
+    for size, e in ((n, chain), (n, star), (k, dense), (n + 1, pairs)):
+        for top in (2, 1 << 30):
+            w = rng.integers(1, top, len(e)).tolist()
+            g = undirected(size, e, w)
+            want, total = orc.mst(g)
+            inm, tot = ecl.mst(g)
+            assert tot == total and np.array_equal(inm, want)
