@@ -114,17 +114,23 @@ __global__ void __launch_bounds__(kTPB) gc_union_hash(int n, const int* __restri
   }
 }
 
+constexpr int kSmallGroup = 4;
+
+// A warp takes `group` (a power of two, at most 32) vertices at a time: 32 on
+// graphs that give every warp of the device some, fewer below, because a
+// group's rows of more than bins.lane entries run one after another, and the
+// first groups of a power-law graph have little else.
 __global__ void __launch_bounds__(kTPB) gc_init(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, int* __restrict__ nl2,
-                                                int* __restrict__ hc, RowChunks rc, Bins bins, bool vec,
+                                                int* __restrict__ hc, RowChunks rc, Bins bins, int group, bool vec,
                                                 const unsigned long long* __restrict__ keys,
                                                 Status* __restrict__ status) {
   dep_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
-  for (int base = warp * 32; base < n; base += nwarps * 32) {
-    const int v = base + lane;
+  for (long long base = (long long)warp * group; base < n; base += (long long)nwarps * group) {
+    const int v = lane < group ? (int)min(base + lane, (long long)n) : n;
     int beg = 0, end = 0;
     if (v < n) csr_row(nindex, v, m, beg, end, status);
     const int dv = end - beg;
@@ -1039,7 +1045,12 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
   // the priority keys first: gc_init compares neighbours by them
   ECL_LAUNCH_NEXT(gc_keys, grid, kTPB, 0, stream, g.n, g.nindex, b.keys0, b.keys1, b.vals1, vhash, color, b.ctl);
   const bool vec = (reinterpret_cast<uintptr_t>(g.nlist) & 15) == 0 && dev.row_vec;  // 16-byte row loads
-  ECL_LAUNCH_NEXT(gc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.nl2, b.hc, rc, bins, vec, b.keys0, status);
+  const int warps = dev.sms * (dev.max_threads_per_sm / 32);
+  int group = 32;
+  while (group > kSmallGroup && g.n / group < warps) group /= 2;
+  const int init_grid = group == 32 ? grid : (g.n - 1) / (group * (kTPB / 32)) + 1;
+  ECL_LAUNCH_NEXT(gc_init, init_grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.nl2, b.hc, rc, bins, group, vec,
+                  b.keys0, status);
   ECL_LAUNCH_NEXT(gc_init_chunks, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.nl2, b.hc, rc, bins.chunk, vec, b.keys0,
              status);
   mark();
