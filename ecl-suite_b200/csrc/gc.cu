@@ -1057,7 +1057,7 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
   // the nkeys appended pairs, sorted from (keys1, vals1); the per-vertex keys
   // in keys0 are dead once gc_init has run
   const ecl_status sorted = radix_order(b.keys1, b.vals1, b.keys0, b.vals0, b.order, g.n, &b.ctl->nkeys, &b.ctl->maxdeg,
-                                  b.sort_temp, &b.ctl->sort_bar, &b.ctl->sort_failed, dev, stream, status);
+                                  b.sort_temp, vhash == nullptr, &b.ctl->sort_bar, &b.ctl->sort_failed, dev, stream, status);
   if (sorted != ECL_OK) return sorted;
   const int* order = b.order;
   mark();

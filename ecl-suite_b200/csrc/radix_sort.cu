@@ -29,6 +29,15 @@ __device__ __forceinline__ unsigned same_digit(int d, bool in) {
   return m;
 }
 
+// With h spread evenly and (nearly) without repeats, the passes need not look at
+// all of it: the lowest two digits (one, of more than kSkipTwo keys) are left
+// out, and at the end each key finds its place in its run of keys equal so far,
+// of kSkipTwo / 65536 at most on average.  A pass costs 12 us and more, the end
+// 5.  Measured, all digits / one left out / two: 20 k keys 73 / - / 54 us, 723 k
+// 96 / 87 / 77, 2 M of four degrees 227 / 203 / 215, R-MAT-22 (2.4 M keys) 336 /
+// 305 / 266: beyond a million keys that can share one degree the runs get long.
+constexpr int kSkipTwo = 1 << 20;
+
 // Every block sorts its own contiguous share of the keys.  A pass: rank the
 // share (a warp its 256 keys of a tile, 32 at a time), publish its digit
 // counts, grid barrier, base of each digit = the smaller digits' totals + the
@@ -37,12 +46,12 @@ __device__ __forceinline__ unsigned same_digit(int d, bool in) {
 // latency for small n (two barriers and three dependent memory rounds a pass),
 // by the ranking and the scattered 12-byte writes for large (ranking by ballots
 // instead of __match_any_sync: R-MAT-22 0.39 -> 0.35 ms).  Measured, whole
-// sort, four launches a pass -> this: 1000 keys 136 -> 32 us, 150 k 197 -> 69,
-// 723 k 224 -> 98, R-MAT-22 (2.4 M keys, seven passes) 382 -> 342.
+// sort, four launches a pass -> this, all digits: 1000 keys 136 -> 32 us, 150 k
+// 197 -> 69, 723 k 224 -> 98, R-MAT-22 (2.4 M keys, seven passes) 382 -> 342.
 __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, int* v0, unsigned long long* k1, int* v1,
                                                        int* __restrict__ order, int n_max,
                                                        const int* __restrict__ n_dev, const int* __restrict__ max_high,
-                                                       unsigned* __restrict__ counts, GridBarrier* bar, int* failed,
+                                                       unsigned* __restrict__ counts, bool spread, GridBarrier* bar, int* failed,
                                                        Status* __restrict__ status) {
   __shared__ unsigned s_base[kDigits];               // where the next tile's keys of each digit go
   __shared__ unsigned short s_warp[kWarps][kDigits];  // per-warp digit counts of a tile, then their prefix sums
@@ -54,8 +63,11 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
   const int blocks = gridDim.x;
   const int n = max(0, min(ld(n_dev), n_max));
   const int high = ld(max_high);
+  // digits of h that the passes leave to the end (see kSkipTwo)
+  const int skip = !spread ? 0 : (n <= kSkipTwo ? 2 : 1);
   int passes = 5;
   while (passes < 8 && (high >> (8 * (passes - 4))) != 0) passes++;
+  passes -= skip;
   const int share = ((n + blocks - 1) / blocks + 31) & ~31;
   const int beg = (int)min((long long)n, (long long)share * blockIdx.x), end = (int)min((long long)n, (long long)beg + share);
   const bool one = share <= kRadixTile;  // uniform over the grid
@@ -63,11 +75,12 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
   int v[kItems];
   unsigned rank[kItems];
   for (int p = 0; p < passes; p++) {
-    const int shift = 8 * p;
+    const int shift = 8 * (p + skip);
+    const bool last = p == passes - 1;
     const unsigned long long* kin = (p & 1) ? k1 : k0;
     const int* vin = (p & 1) ? v1 : v0;
     unsigned long long* kout = (p & 1) ? k0 : k1;
-    int* vout = p == passes - 1 ? order : ((p & 1) ? v0 : v1);
+    int* vout = last && skip == 0 ? order : ((p & 1) ? v0 : v1);
     // Loads the tile at t0, ranks each key among its warp's keys of the same
     // digit, and leaves in s_warp[w][d] the tile's keys of digit d in earlier
     // warps; returns the tile's keys of digit `dig`.  All threads call.
@@ -173,30 +186,49 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
         if (i0 + 32 * j >= end) continue;
         const int d = digit_of(k[j], shift);
         const unsigned pos = s_base[d] + s_warp[warp][d] + rank[j];
-        if (p < passes - 1) kout[pos] = k[j];
+        if (!last || skip > 0) kout[pos] = k[j];
         vout[pos] = v[j];
       }
       __syncthreads();
       if (!one && quarter == 0) s_base[dig] += tile;
       __syncthreads();
     }
-    if (p < passes - 1 && !grid_sync<true>(bar, status)) {
+    if ((!last || skip > 0) && !grid_sync<true>(bar, status)) {
       if (threadIdx.x == 0) st(failed, 1);
       return;
     }
+  }
+  if (skip == 0) return;
+  // runs of keys equal in the sorted digits: each key to its place among them
+  const unsigned long long* kin = (passes & 1) ? k1 : k0;
+  const int* vin = (passes & 1) ? v1 : v0;
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += blocks * kThreads) {
+    const unsigned long long key = kin[i];  // written before the last grid barrier
+    int pos = i;
+    for (int j = i - 1; j >= 0; j--) {
+      const unsigned long long x = kin[j];
+      if ((x ^ key) >> (8 * skip)) break;
+      pos -= x > key;
+    }
+    for (int j = i + 1; j < n; j++) {
+      const unsigned long long x = kin[j];
+      if ((x ^ key) >> (8 * skip)) break;
+      pos += x < key;
+    }
+    order[pos] = vin[i];
   }
 }
 
 }  // namespace
 
 ecl_status radix_order(unsigned long long* k0, int* v0, unsigned long long* k1, int* v1, int* order, int n,
-                       const int* n_dev, const int* max_high, unsigned* temp, GridBarrier* bar, int* failed,
+                       const int* n_dev, const int* max_high, unsigned* temp, bool spread, GridBarrier* bar, int* failed,
                        const DeviceInfo& dev, cudaStream_t stream, Status* status) {
   // A block per half tile: latency bounds a small sort, so blocks are worth
   // their barrier arrivals; a single block needs no barrier at all.
   const int blocks = std::max(1, std::min({dev.sms, kRadixMaxBlocks, n / (kRadixTile / 2)}));
   ECL_CUDA_TRY(launch_cooperative(rs_sort, blocks, kThreads, stream, k0, v0, k1, v1, order, n, n_dev, max_high, temp,
-                                  bar, failed, status));
+                                  spread, bar, failed, status));
   return ECL_OK;
 }
 

@@ -538,3 +538,14 @@ def test_mst_lists_that_one_block_finishes(ecl, orc, edges):
             want, total = orc.mst(g)
             inm, tot = ecl.mst(g)
             assert tot == total and np.array_equal(inm, want)
+
+
+@pytest.mark.parametrize("n", [1025, 65537, (1 << 20) - 1, (1 << 20) + 1025])
+def test_gc_order_of_equal_degrees(ecl, orc, n):
+    """One degree for all vertices: the sort's left-out digits decide between
+    most neighbours, on both sides of its rule, and its runs meet block and
+    tile ends."""
+    ring = np.stack(((np.arange(n) - 1) % n, (np.arange(n) + 1) % n), 1)
+    ring.sort(axis=1)
+    g = ecl.Graph((2 * np.arange(n + 1)).astype(np.int32), ring.ravel().astype(np.int32), None, True)
+    assert np.array_equal(ecl.gc(g), orc.gc(g))
