@@ -150,8 +150,9 @@ __device__ __forceinline__ int cc_first_smaller(int v, int beg, int end, const i
 // [0, m]) raises ECL_ERR_BAD_GRAPH and is treated as empty by every kernel.
 __global__ void __launch_bounds__(kTPB) cc_init(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, int* __restrict__ parent,
-                                                Status* __restrict__ status) {
+                                                CCCounters* __restrict__ ctr, Status* __restrict__ status) {
   dep_wait();
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctr->nchunks = 0;  // race-free: first used by later launches
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     int beg = __ldg(&nindex[v]), end = __ldg(&nindex[v + 1]);
     if (beg < 0 || end < beg || end > m) {
@@ -559,9 +560,8 @@ ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, 
   const int grid = dev.grid_blocks(kTPB, g.n, g.m);
   const Bins bins = bins_of(dev, kCCBins);
   const int cap = chunk_capacity(g.m, kMinChunk);  // cc_layout sized the records for the smallest chunk
-  ECL_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(CCCounters), stream));
   if (g.flags & ECL_GRAPH_SYMMETRIC) {
-    ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
+    ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, status);
     ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, Giants{}, nullptr);
     if (g.n >= kSplitSample) {
       ECL_LAUNCH_NEXT(cc_sample<0>, dev.grid_blocks(kTPB, g.n / 8, 0), kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent,
@@ -590,7 +590,7 @@ ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, 
     mark();
     return ECL_OK;
   }
-  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
+  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, status);
   mark();
   ECL_LAUNCH_NEXT(cc_hook, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, chunks, cap, bins, ctr, status);
   mark();
@@ -729,7 +729,7 @@ extern "C" ecl_status ecl_cc_noalloc(int32_t nodes, int32_t edges, const int32_t
   // the counters (adjacent, at the front of the array) before every solve.
   ECL_CUDA_TRY(cudaMemsetAsync(base, 0, kStatusBytes + sizeof(CCCounters), stream));
   const int grid = dev.grid_blocks(kTPB, nodes, edges);
-  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, status);
+  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, ctr, status);
   ECL_LAUNCH_NEXT(cc_hook, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, chunks,
              chunk_capacity(edges, kCCBins.chunk), kCCBins, ctr, status);
   ECL_LAUNCH_NEXT(cc_chunks, grid, kTPB, 0, stream, nodes, nindex, nlist, label, chunks,

@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "csr_bins.cuh"
+#include "fill.cuh"
 #include "grid_sync.cuh"
 #include "radix_sort.cuh"
 #include "solvers.cuh"
@@ -1035,8 +1036,7 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
   const RowChunks rc{b.chunks, &b.ctl->nchunks, (int)row_chunk_capacity(g.m, kMinChunk)};
   const Bins bins = bins_of(dev, Bins{kBinLane, kBinChunk});
 
-  if (cudaMemsetAsync(b.ctl, 0, sizeof(GCCtl), stream) != cudaSuccess) return ECL_ERR_CUDA;
-  if (cudaMemsetAsync(color, 0xff, sizeof(int) * (size_t)g.n, stream) != cudaSuccess) return ECL_ERR_CUDA;
+  fill_ranges({{b.ctl, sizeof(GCCtl), 0}, {color, sizeof(int) * (size_t)g.n, 0xff}}, dev, stream);
   const unsigned* vhash = nullptr;
   if (uni && uni->vbase) {
     ECL_LAUNCH_NEXT(gc_union_hash, grid, kTPB, 0, stream, g.n, uni->vbase, uni->ngraphs, b.vhash);

@@ -29,6 +29,7 @@
 #include <algorithm>
 
 #include "csr_bins.cuh"
+#include "fill.cuh"
 #include "flat_scan.cuh"
 #include "grid_sync.cuh"
 #include "solvers.cuh"
@@ -609,9 +610,10 @@ ecl_status mst_enqueue(const GraphDev& g, unsigned char* in_mst, char* ws, Statu
   const int scan_grid = dev.grid_blocks(kTPB, 0, g.m);  // a thread per lane's share of a tile
   const FlatCsr fc{g.n, g.m, g.nindex, g.nlist, b.tilerow};
   if (total_dev) *total_dev = &b.ctl->total;
-  ECL_CUDA_TRY(cudaMemsetAsync(b.ctl, 0, sizeof(MSTCtl), stream));
-  if (g.m > 0) ECL_CUDA_TRY(cudaMemsetAsync(in_mst, 0, (size_t)g.m, stream));
-  ECL_CUDA_TRY(cudaMemsetAsync(b.tilerow, 0xff, sizeof(int) * ((size_t)flat_tiles(g.m) + 1), stream));
+  fill_ranges({{b.ctl, sizeof(MSTCtl), 0},
+               {in_mst, (size_t)g.m, 0},
+               {b.tilerow, sizeof(int) * ((size_t)flat_tiles(g.m) + 1), 0xff}},
+              dev, stream);
   // No light pass below 4 entries a vertex: all weights pass the first scan,
   // and the second would find nothing.
   const bool filter = g.m / g.n >= 4;
