@@ -12,7 +12,7 @@
 // further down: link two entries of every list, find the giant component,
 // then skip every list inside it):
 //  * cc_init   - parent[v] = first smaller neighbour among the first
-//                kInitScan entries, twice over (one free hook per vertex).
+//                kInitScan entries, kInitHops times over (free hooks).
 //  * cc_hook   - one pass over the vertices, 32 per warp.  Lists of <= 16
 //                entries are walked by their own lane; lists of up to
 //                2048 entries are walked by the whole warp (ballot loop,
@@ -279,7 +279,9 @@ __global__ void __launch_bounds__(kTPB) cc_chunks(int n, const int* __restrict__
 // the root that it met last: with a giant component every vertex would
 // otherwise end on the same word, and its L2 slice would be the bound.  Hence
 // a grid that gives each thread several vertices of a large graph
-// (flatten_blocks), kFlattenBatch of them in flight.
+// (flatten_blocks), kFlattenBatch of them in flight; chains that have met share
+// the load.  The batch's chains walked one after another took 31 us on a
+// 1024 x 1024 grid (512 deep), side by side 23.
 constexpr int kFlattenBatch = 4;
 
 // kMark, kMarkUnion: also ing[v] = whether v's root is the sampled giant

@@ -9,9 +9,10 @@
 // gives the same forest.
 //
 // B200 design:
-//  * mst_threshold: one block samples 1024 weights on the device and picks
+//  * mst_threshold: one block of mst_init samples 1024 weights and picks
 //    the quantile that leaves ~0.75 n (2 n in a sparse graph) light CSR
-//    entries, with no host round trip;
+//    entries, with no host round trip; below 4 entries a vertex there is one
+//    pass over all entries instead of a light and a heavy one;
 //  * mst_scan: builds a worklist of int4 {a, b, weight, j} from the CSR in
 //    tiles of 256 entries a warp, whatever rows they belong to; appends are
 //    staged per warp in shared memory and reserved in the global list with one
@@ -25,7 +26,8 @@
 //    flattening keeps every tree one level deep, so finding an edge's roots
 //    is one load each and no phase reads what it writes: the loads are plain
 //    ones that L1 serves.  Per-round sizes live in a counter array, so no
-//    counter is ever reset concurrently with its use.
+//    counter is ever reset concurrently with its use.  The last, short rounds
+//    are run by one block.
 #include <algorithm>
 
 #include "csr_bins.cuh"

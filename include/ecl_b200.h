@@ -88,14 +88,16 @@ typedef struct ecl_opts {
  * (ECL-MST_10-atomic.cu:197,450-459). */
 typedef struct ecl_tune {
   int32_t blocks_per_sm;  /* blocks of 256 threads per SM in the grid-stride kernels' grids, 1..128; 0 = 64 */
-  float mst_light_factor; /* MST light-edge target, in multiples of n; 0 = 0.75 */
+  float mst_light_factor; /* MST light-edge target, in multiples of n; 0 = 0.75 from 16 entries a vertex
+                             on, else 2 */
   int32_t gc_core_ranks;  /* GC: leading ranks coloured in shared memory (the core), 0..36864; 0 = 8192 */
-  int32_t row_lane_max;   /* CSR scans: rows of at most this many entries go to one lane, 0..32; 0 = per code */
-  int32_t row_chunk;      /* CSR scans: rows longer than this are cut into chunks of this many entries;
+  int32_t row_lane_max;   /* row scans (not MST's, which go by entries): rows of at most this many entries go
+                             to one lane, 0..32; 0 = per code */
+  int32_t row_chunk;      /* row scans (CC, GC, SCC): longer rows are cut into chunks of this many entries;
                              0 = per code, else a power of two in 128..8192 */
   int32_t scc_sweep_batch; /* SCC: edges per lane whose loads a sweep keeps in flight: 1, 2 or 4; 0 = 1 */
   int32_t gc_poll_ns;      /* GC: longest sleep between polls of a long row's dependency, 0..4096 ns; 0 = 64 */
-  int32_t row_vec;         /* CSR scans: 1 = warp rows read in 16-byte quads where aligned; 0 = 4-byte loads
+  int32_t row_vec;         /* row scans (GC, SCC): 1 = warp rows read in 16-byte quads where aligned; 0 = 4-byte loads
                               (measured faster: the quads scatter the per-entry writes that follow) */
   int32_t gc_pull_blocks;  /* GC pull: blocks of 256 threads per SM, 1..4; 0 = 2 */
   int32_t gc_core_ctas;    /* GC core: CTAs of the cluster that colours it, 1..8; 0 = 2 */
