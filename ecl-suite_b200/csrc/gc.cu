@@ -224,7 +224,11 @@ __global__ void __launch_bounds__(kTPB) gc_init_chunks(int n, int m, const int* 
 // one entry are also appended to (skeys, svals), the sort's input, counted in
 // ctl->nkeys.  An isolated vertex has no neighbour to wait for or to block:
 // its colour is 0, written here, and it is neither sorted nor pulled
-// (R-MAT-22 has 1.8 M of them among its 4.2 M vertices).
+// (R-MAT-22 has 1.8 M of them among its 4.2 M vertices).  Bound by the appends'
+// counter: with one vertex a thread and reservation the pass took 46 us at
+// R-MAT-22 (75 MB), with four 29.
+constexpr int kKeyBatch = 4;
+
 __global__ void __launch_bounds__(kTPB) gc_keys(int n, const int* __restrict__ nindex,
                                                 unsigned long long* __restrict__ keys,
                                                 unsigned long long* __restrict__ skeys, int* __restrict__ svals,
@@ -232,47 +236,60 @@ __global__ void __launch_bounds__(kTPB) gc_keys(int n, const int* __restrict__ n
                                                 GCCtl* __restrict__ ctl) {
   dep_wait();
   // rows longer than kWarpRow are counted per block and added once per block;
-  // the appends reserve their room with one atomic per block and step
+  // the appends reserve their room with one atomic per block and step of
+  // kKeyBatch vertices a thread, as all of them meet at one word
   __shared__ int s_big, s_deg;
-  __shared__ int s_woff[kTPB / 32];
+  __shared__ int s_woff[kKeyBatch * kTPB / 32];
   __shared__ int s_base;
   if (threadIdx.x == 0) s_big = s_deg = 0;
   __syncthreads();
   int nb = 0, dmax = 0;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int bbase = blockIdx.x * kTPB; bbase < n; bbase += gridDim.x * kTPB) {  // block-uniform trip count
-    const int i = bbase + threadIdx.x;
-    bool big = false, linked = false;
-    unsigned long long key = 0;
-    int v = 0;
-    if (i < n) {
-      v = n - 1 - i;
-      const unsigned deg = (unsigned)(__ldg(&nindex[v + 1]) - __ldg(&nindex[v]));
-      key = ~(((unsigned long long)deg << 32) | gc_h(vhash, v));
-      keys[i] = key;
-      big = deg > (unsigned)kWarpRow;
-      dmax = max(dmax, (int)min(deg, 0x7fffffffu));
-      linked = deg > 0;
-      if (!linked) color[v] = 0;  // race-free: the output, thread-owned; nothing reads it in this launch
+  constexpr int kStep = kKeyBatch * kTPB, kGroups = kKeyBatch * kTPB / 32;
+  static_assert(kGroups == 32, "one warp adds the groups up");
+  for (long long bbase = (long long)blockIdx.x * kStep; bbase < n; bbase += (long long)gridDim.x * kStep) {  // block-uniform
+    unsigned long long key[kKeyBatch];
+    unsigned deg[kKeyBatch], bal[kKeyBatch];
+#pragma unroll
+    for (int k = 0; k < kKeyBatch; k++) {
+      const long long i = bbase + k * kTPB + threadIdx.x;
+      const int v = n - 1 - (int)i;
+      deg[k] = i < n ? (unsigned)(__ldg(&nindex[v + 1]) - __ldg(&nindex[v])) : 0u;
     }
-    nb += __popc(__ballot_sync(kFull, big));
-    const unsigned bal = __ballot_sync(kFull, linked);
-    if (lane == 0) s_woff[wid] = __popc(bal);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int run = 0;
-      for (int w = 0; w < kTPB / 32; w++) {
-        const int c = s_woff[w];
-        s_woff[w] = run;
-        run += c;
+#pragma unroll
+    for (int k = 0; k < kKeyBatch; k++) {
+      const long long i = bbase + k * kTPB + threadIdx.x;
+      const int v = n - 1 - (int)i;
+      key[k] = 0;
+      if (i < n) {
+        key[k] = ~(((unsigned long long)deg[k] << 32) | gc_h(vhash, v));
+        keys[i] = key[k];
+        dmax = max(dmax, (int)min(deg[k], 0x7fffffffu));
+        if (deg[k] == 0) color[v] = 0;  // race-free: the output, thread-owned; nothing reads it in this launch
       }
-      s_base = run ? fetch_add(&ctl->nkeys, run) : 0;
+      nb += __popc(__ballot_sync(kFull, deg[k] > (unsigned)kWarpRow));
+      bal[k] = __ballot_sync(kFull, deg[k] > 0);
+      if (lane == 0) s_woff[k * (kTPB / 32) + wid] = __popc(bal[k]);
     }
     __syncthreads();
-    if (linked) {
-      const int at = s_base + s_woff[wid] + __popc(bal & ((1u << lane) - 1));
-      skeys[at] = key;
-      svals[at] = v;
+    if (wid == 0) {
+      const int c = s_woff[lane];
+      int incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += x;
+      }
+      s_woff[lane] = incl - c;
+      if (lane == 31) s_base = incl ? fetch_add(&ctl->nkeys, incl) : 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kKeyBatch; k++) {
+      if (deg[k] == 0) continue;
+      const int at = s_base + s_woff[k * (kTPB / 32) + wid] + __popc(bal[k] & ((1u << lane) - 1));
+      skeys[at] = key[k];
+      svals[at] = n - 1 - (int)(bbase + k * kTPB + threadIdx.x);
     }
     __syncthreads();  // s_woff and s_base are rewritten next step
   }
