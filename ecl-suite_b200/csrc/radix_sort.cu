@@ -32,8 +32,8 @@ __device__ __forceinline__ unsigned same_digit(int d, bool in) {
 // With h spread evenly and (nearly) without repeats, the passes need not look at
 // all of it: the lowest two digits (one, of more than kSkipTwo keys) are left
 // out, and at the end each key finds its place in its run of keys equal so far,
-// of kSkipTwo / 65536 at most on average.  A pass costs 12 us and more, the end
-// 5.  Measured, all digits / one left out / two: 20 k keys 73 / - / 54 us, 723 k
+// of kSkipTwo / 65536 at most on average.  A pass costs 7 us and more, the end
+// 5.  Measured (with a block per 4096 keys), all digits / one left out / two: 20 k keys 73 / - / 54 us, 723 k
 // 96 / 87 / 77, 2 M of four degrees 227 / 203 / 215, R-MAT-22 (2.4 M keys) 336 /
 // 305 / 266: beyond a million keys that can share one degree the runs get long.
 constexpr int kSkipTwo = 1 << 20;
@@ -48,6 +48,9 @@ constexpr int kSkipTwo = 1 << 20;
 // instead of __match_any_sync: R-MAT-22 0.39 -> 0.35 ms).  Measured, whole
 // sort, four launches a pass -> this, all digits: 1000 keys 136 -> 32 us, 150 k
 // 197 -> 69, 723 k 224 -> 98, R-MAT-22 (2.4 M keys, seven passes) 382 -> 342.
+// kShort: every share is at most a tile, and a warp takes only as many slices of
+// it as there are for all warps.
+template <bool kShort>
 __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, int* v0, unsigned long long* k1, int* v1,
                                                        int* __restrict__ order, int n_max,
                                                        const int* __restrict__ n_dev, const int* __restrict__ max_high,
@@ -71,6 +74,7 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
   const int share = ((n + blocks - 1) / blocks + 31) & ~31;
   const int beg = (int)min((long long)n, (long long)share * blockIdx.x), end = (int)min((long long)n, (long long)beg + share);
   const bool one = share <= kRadixTile;  // uniform over the grid
+  const int per = kShort ? (share + kThreads - 1) / kThreads : kItems;  // slices of 32 keys a warp takes of a tile
   unsigned long long k[kItems];
   int v[kItems];
   unsigned rank[kItems];
@@ -85,10 +89,10 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
     // digit, and leaves in s_warp[w][d] the tile's keys of digit d in earlier
     // warps; returns the tile's keys of digit `dig`.  All threads call.
     auto rank_tile = [&](int t0, bool values) -> unsigned {
-      const int i0 = t0 + warp * kItems * 32 + lane;
+      const int i0 = t0 + warp * per * 32 + lane;
 #pragma unroll
       for (int j = 0; j < kItems; j++) {
-        const int i = i0 + 32 * j;
+        const int i = j < per ? i0 + 32 * j : end;
         k[j] = i < end ? kin[i] : 0ull;  // written before the last grid barrier
         if (values) v[j] = i < end ? vin[i] : 0;
       }
@@ -96,7 +100,7 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
       __syncwarp();
 #pragma unroll
       for (int j = 0; j < kItems; j++) {
-        if (i0 - lane + 32 * j >= end) break;  // the same for the whole warp
+        if (j >= per || i0 - lane + 32 * j >= end) break;  // the same for the whole warp
         const bool in = i0 + 32 * j < end;
         const int d = digit_of(k[j], shift);
         const unsigned same = same_digit(d, in);
@@ -180,10 +184,10 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
     for (int t0 = beg; t0 < end; t0 += kRadixTile) {
       unsigned tile = 0;
       if (!one) tile = rank_tile(t0, true);
-      const int i0 = t0 + warp * kItems * 32 + lane;
+      const int i0 = t0 + warp * per * 32 + lane;
 #pragma unroll
       for (int j = 0; j < kItems; j++) {
-        if (i0 + 32 * j >= end) continue;
+        if (j >= per || i0 + 32 * j >= end) continue;
         const int d = digit_of(k[j], shift);
         const unsigned pos = s_base[d] + s_warp[warp][d] + rank[j];
         if (!last || skip > 0) kout[pos] = k[j];
@@ -224,10 +228,15 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
 ecl_status radix_order(unsigned long long* k0, int* v0, unsigned long long* k1, int* v1, int* order, int n,
                        const int* n_dev, const int* max_high, unsigned* temp, bool spread, GridBarrier* bar, int* failed,
                        const DeviceInfo& dev, cudaStream_t stream, Status* status) {
-  // A block per half tile: latency bounds a small sort, so blocks are worth
-  // their barrier arrivals; a single block needs no barrier at all.
-  const int blocks = std::max(1, std::min({dev.sms, kRadixMaxBlocks, n / (kRadixTile / 2)}));
-  ECL_CUDA_TRY(launch_cooperative(rs_sort, blocks, kThreads, stream, k0, v0, k1, v1, order, n, n_dev, max_high, temp,
+  // A block per kShare keys: ranking a share is a serial chain of its slices, so
+  // blocks are worth their barrier arrivals; a single block needs no barrier at
+  // all.  Whole sort with a block per 4096 keys -> this: 5 k keys 36 -> 34 us,
+  // 20 k 52 -> 34, 100 k 51 -> 39; the slices spread over the warps, one block of
+  // 1000 keys 28 -> 22.
+  constexpr int kShare = 1024;
+  const int blocks = std::max(1, std::min({dev.sms, kRadixMaxBlocks, n / kShare}));
+  auto kernel = (long long)n <= (long long)blocks * (kRadixTile - 32) ? rs_sort<true> : rs_sort<false>;
+  ECL_CUDA_TRY(launch_cooperative(kernel, blocks, kThreads, stream, k0, v0, k1, v1, order, n, n_dev, max_high, temp,
                                   spread, bar, failed, status));
   return ECL_OK;
 }
