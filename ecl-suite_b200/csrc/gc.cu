@@ -60,7 +60,8 @@ struct GCCtl {
   int nkeys;       // vertices with at least one entry: the ones sorted and pulled
   int maxdeg;      // largest degree: how many digits of it the sort looks at
   int sort_failed;  // the sort gave up: the order is not whole, and nothing is indexed by it
-  int pad2[27];
+  int bad_rows;  // some row is malformed, so rows may overlap
+  int pad2[26];
   GridBarrier sort_bar;
 };
 
@@ -229,7 +230,7 @@ __global__ void __launch_bounds__(kTPB) gc_init_chunks(int n, int m, const int* 
 // R-MAT-22 (75 MB), with four 29.
 constexpr int kKeyBatch = 4;
 
-__global__ void __launch_bounds__(kTPB) gc_keys(int n, const int* __restrict__ nindex,
+__global__ void __launch_bounds__(kTPB) gc_keys(int n, int m, const int* __restrict__ nindex,
                                                 unsigned long long* __restrict__ keys,
                                                 unsigned long long* __restrict__ skeys, int* __restrict__ svals,
                                                 const unsigned* __restrict__ vhash, int* __restrict__ color,
@@ -254,7 +255,12 @@ __global__ void __launch_bounds__(kTPB) gc_keys(int n, const int* __restrict__ n
     for (int k = 0; k < kKeyBatch; k++) {
       const long long i = bbase + k * kTPB + threadIdx.x;
       const int v = n - 1 - (int)i;
-      deg[k] = i < n ? (unsigned)(__ldg(&nindex[v + 1]) - __ldg(&nindex[v])) : 0u;
+      deg[k] = 0u;
+      if (i < n) {
+        const int beg = __ldg(&nindex[v]), end = __ldg(&nindex[v + 1]);
+        deg[k] = (unsigned)(end - beg);
+        if (beg < 0 || end < beg || end > m) st(&ctl->bad_rows, 1);  // (gc_init reports it)
+      }
     }
 #pragma unroll
     for (int k = 0; k < kKeyBatch; k++) {
@@ -560,9 +566,11 @@ static_assert(gc_core_seg(kCoreMax) >= 256 && gc_core_smem(kCoreMax) <= kCoreSme
               "core shared memory over the per-block limit");
 
 // Core size of this solve: the long rows (a prefix of the order), at most cap.
-// None when the sort failed.
+// None when the sort failed, and none when rows may overlap: the core's rows
+// are packed in place, and another row in the same slot would take two of
+// their 16-bit ranks for a vertex.
 __device__ __forceinline__ int gc_core_size(const GCCtl* ctl, int cap) {
-  return ld(&ctl->sort_failed) ? 0 : min(ld(&ctl->nbig), cap);
+  return ld(&ctl->sort_failed) || ld(&ctl->bad_rows) ? 0 : min(ld(&ctl->nbig), cap);
 }
 
 // rank[order[r]] = r over the core.
@@ -584,7 +592,8 @@ __global__ void __launch_bounds__(kTPB) gc_core_rank(const int* __restrict__ ord
 __global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict__ nindex, int* nl2,
                                                           const int* __restrict__ hc, const int* __restrict__ order,
                                                           const int* __restrict__ rank, int4* __restrict__ rowinfo,
-                                                          const GCCtl* __restrict__ ctl, int cap) {
+                                                          const GCCtl* __restrict__ ctl, int cap,
+                                                          Status* __restrict__ status) {
   dep_wait();
   const int lane = threadIdx.x & 31;
   const int core = gc_core_size(ctl, cap);
@@ -598,7 +607,13 @@ __global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict_
     for (int i0 = 0; i0 < h; i0 += 32) {
       const int i = i0 + lane;
       unsigned short q = 0;
-      if (i < h) q = (unsigned short)__ldg(&rank[nl2[(size_t)b + i]]);
+      if (i < h) {
+        const int x = __ldg(&rank[nl2[(size_t)b + i]]);
+        if ((unsigned)x < (unsigned)r)
+          q = (unsigned short)x;
+        else  // only where a union's entry leaves its graph for a vertex of the same key
+          raise(status, ECL_ERR_BAD_GRAPH, v);
+      }
       __syncwarp();
       if (i < h) out[i] = q;
       __syncwarp();
@@ -1060,7 +1075,7 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
     vhash = b.vhash;
   }
   // the priority keys first: gc_init compares neighbours by them
-  ECL_LAUNCH_NEXT(gc_keys, grid, kTPB, 0, stream, g.n, g.nindex, b.keys0, b.keys1, b.vals1, vhash, color, b.ctl);
+  ECL_LAUNCH_NEXT(gc_keys, grid, kTPB, 0, stream, g.n, g.m, g.nindex, b.keys0, b.keys1, b.vals1, vhash, color, b.ctl);
   const bool vec = (reinterpret_cast<uintptr_t>(g.nlist) & 15) == 0 && dev.row_vec;  // 16-byte row loads
   const int warps = dev.sms * (dev.max_threads_per_sm / 32);
   int group = 32;
@@ -1086,7 +1101,7 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
   // of 0.7 M vertices, no core at all: 11 + 12 us with one block per 256
   // vertices)
   ECL_LAUNCH_NEXT(gc_core_rank, std::min(grid, (cap - 1) / kTPB + 1), kTPB, 0, stream, order, rank, b.ctl, cap);
-  ECL_LAUNCH_NEXT(gc_core_translate, std::min(grid, (cap - 1) / (kTPB / 32) + 1), kTPB, 0, stream, g.nindex, b.nl2, b.hc, order, rank, b.rowinfo, b.ctl, cap);
+  ECL_LAUNCH_NEXT(gc_core_translate, std::min(grid, (cap - 1) / (kTPB / 32) + 1), kTPB, 0, stream, g.nindex, b.nl2, b.hc, order, rank, b.rowinfo, b.ctl, cap, status);
   ECL_CUDA_TRY(cudaFuncSetAttribute(gc_core, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gc_core_smem(cap)));
   // the core's cluster: as many CTAs as asked for when such a cluster fits
   // the device, else one CTA
