@@ -17,6 +17,34 @@ DeviceInfo g_dev_cache[64];
 ecl_tune g_tune{};  // process-wide knobs of the single-graph entry points (under g_dev_mu)
 }  // namespace
 
+unsigned long long context_id() {
+  // cuCtxGetCurrent and cuCtxGetId, reached through the runtime's driver entry
+  // points so the library needs no link against libcuda.
+  typedef int (*CtxGetCurrentFn)(void** ctx);
+  typedef int (*CtxGetIdFn)(void* ctx, unsigned long long* id);
+  struct Fns {
+    CtxGetCurrentFn current = nullptr;
+    CtxGetIdFn id = nullptr;
+    Fns() {
+      void *c = nullptr, *i = nullptr;
+      cudaDriverEntryPointQueryResult qc, qi;
+      if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &c, cudaEnableDefault, &qc) == cudaSuccess &&
+          cudaGetDriverEntryPoint("cuCtxGetId", &i, cudaEnableDefault, &qi) == cudaSuccess &&
+          qc == cudaDriverEntryPointSuccess && qi == cudaDriverEntryPointSuccess) {
+        current = reinterpret_cast<CtxGetCurrentFn>(c);
+        id = reinterpret_cast<CtxGetIdFn>(i);
+      } else {
+        cudaGetLastError();
+      }
+    }
+  };
+  static const Fns fns;
+  void* ctx = nullptr;
+  unsigned long long id = 0;
+  if (!fns.current || !fns.id || fns.current(&ctx) != 0 || !ctx || fns.id(ctx, &id) != 0) return 0;
+  return id;
+}
+
 bool tune_valid(const ecl_tune& t) {
   const bool chunk_ok = t.row_chunk == 0 || (t.row_chunk >= dev::kMinChunk && t.row_chunk <= dev::kMaxChunk &&
                                               (t.row_chunk & (t.row_chunk - 1)) == 0);

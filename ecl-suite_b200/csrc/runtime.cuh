@@ -155,6 +155,12 @@ struct DeviceInfo {
 // Properties of the current device (cached per device id), with the
 // process-wide knobs of ecl_set_tune applied.
 ecl_status current_device(DeviceInfo* info);
+// Id of the calling thread's current CUDA context, 0 when there is none yet.
+// cudaDeviceReset ends a device's context and the next runtime call makes a new
+// one, often at the same handle: only the id, which the driver gives out once
+// in a process, tells them apart.  What the library keeps between calls of
+// memory or events is kept with this id and not used under another.
+unsigned long long context_id();
 // Range check of a knob set, and its application to a DeviceInfo.
 bool tune_valid(const ecl_tune& t);
 void apply_tune(DeviceInfo* d, const ecl_tune& t);

@@ -15,13 +15,16 @@
 #include <cstring>
 #include <mutex>
 
+#include "runtime.cuh"
+
 namespace ecl {
 
 namespace {
 
 constexpr size_t kPiece = size_t(1) << 20;
-constexpr int kPieces = 4;  // per block
-constexpr int kMaxBlocks = 4;  // 16 MB of page-locked memory at most
+constexpr int kPieces = 4;       // per block
+constexpr int kMaxBlocks = 4;    // 16 MB of page-locked memory for a context at most ...
+constexpr int kMaxContexts = 8;  // ... and for this many of them (one for each device)
 constexpr size_t kStageMin = size_t(256) << 10;  // below, the plain copy is as fast
 constexpr int kCopyThreads = 4;
 
@@ -29,42 +32,80 @@ constexpr int kCopyThreads = 4;
 
 struct StageBlock {
   char* base = nullptr;
-  int device = -1;  // of the events
+  unsigned long long ctx = 0;  // context of the memory and the events (0: not made)
   cudaEvent_t done[kPieces] = {};
+  bool taken = false;
 };
 
 namespace {
 
 // Blocks are made when first wanted (4 ms each) and kept until the process
-// ends, kMaxBlocks in all: a copy that finds none free is made without.
+// ends, kMaxBlocks for a context: a copy that finds none is made without.  A
+// block belongs to the context it was made in.  When that context has ended
+// (cudaDeviceReset), the memory and the events ended with it: the block is made
+// anew, and nothing of the old one is touched, not even to free it.
 class Pool {
  public:
-  StageBlock* take() {
+  StageBlock* take(unsigned long long ctx) {
     std::lock_guard<std::mutex> lk(mu_);
-    if (nfree_ > 0) return free_[--nfree_];
-    if (made_ == kMaxBlocks) return nullptr;
-    void* p = nullptr;
-    if (cudaHostAlloc(&p, kPiece * kPieces, cudaHostAllocPortable) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
+    int made = 0;
+    for (StageBlock& b : blocks_) {
+      if (b.ctx != ctx) continue;
+      made++;
+      if (b.taken) continue;
+      b.taken = true;
+      return &b;
     }
-    StageBlock* b = &blocks_[made_++];
-    b->base = static_cast<char*>(p);
-    return b;
+    if (made == kMaxBlocks) return nullptr;
+    StageBlock* room = nullptr;
+    for (StageBlock& b : blocks_)
+      if (!room && !b.taken && (b.ctx == 0 || gone(b))) room = &b;
+    if (!room || !make(room, ctx)) return nullptr;
+    room->taken = true;
+    return room;
   }
   void give(StageBlock* b) {
     std::lock_guard<std::mutex> lk(mu_);
-    free_[nfree_++] = b;
+    b->taken = false;
   }
   ~Pool() {
-    for (int i = 0; i < nfree_; i++) cudaFreeHost(free_[i]->base);
+    const unsigned long long ctx = context_id();
+    for (StageBlock& b : blocks_)
+      if (ctx != 0 && b.ctx == ctx) cudaFreeHost(b.base);
   }
 
  private:
+  // Another context's block is taken to be gone when its memory is no longer
+  // page-locked; a live one stays for its own context.
+  static bool gone(const StageBlock& b) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, b.base) == cudaSuccess) return at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return false;
+  }
+  static bool make(StageBlock* b, unsigned long long ctx) {
+    *b = StageBlock{};
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, kPiece * kPieces, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    for (cudaEvent_t& e : b->done)
+      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        for (cudaEvent_t made : b->done)
+          if (made) cudaEventDestroy(made);
+        cudaFreeHost(p);
+        *b = StageBlock{};
+        return false;
+      }
+    b->base = static_cast<char*>(p);
+    b->ctx = ctx;
+    return true;
+  }
+
   std::mutex mu_;
-  StageBlock blocks_[kMaxBlocks];
-  StageBlock* free_[kMaxBlocks] = {};
-  int nfree_ = 0, made_ = 0;
+  StageBlock blocks_[kMaxBlocks * kMaxContexts];
 };
 
 Pool g_pool;
@@ -90,28 +131,12 @@ bool Staging::ready(const void* host, size_t bytes) {
     return false;
   }
   if (at.type != cudaMemoryTypeUnregistered) return false;
-  int device = -1;
-  if (cudaGetDevice(&device) != cudaSuccess) return false;
-  if (block_ && block_->device != device) return false;  // (its events are another device's)
-  if (block_) return true;
-  block_ = g_pool.take();
-  if (!block_) return false;
+  const unsigned long long ctx = context_id();
+  if (ctx == 0) return false;
+  if (block_) return block_->ctx == ctx;
+  block_ = g_pool.take(ctx);
   used_ = 0;
-  if (block_->device != device) {
-    for (cudaEvent_t& e : block_->done) {
-      if (e) cudaEventDestroy(e);
-      e = nullptr;
-    }
-    block_->device = -1;
-    for (cudaEvent_t& e : block_->done)
-      if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
-        cudaGetLastError();
-        release();
-        return false;
-      }
-    block_->device = device;
-  }
-  return true;
+  return block_ != nullptr;
 }
 
 bool Staging::to_device(void* dst, const void* src, size_t bytes, cudaStream_t stream, cudaError_t* err) {

@@ -1,0 +1,66 @@
+"""Copies of pageable host memory through the library's page-locked blocks:
+what the pool keeps between calls, and every way in which a copy goes without
+a block.  Each test runs in a process of its own, because the pool, the OpenMP
+settings and the CUDA context belong to the process."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+from conftest import ROOT
+
+pytestmark = pytest.mark.gpu
+
+# A path of n vertices without every tenth link: labels, forest and weight are
+# known without a solver.  The CSR and the outputs are above the size from
+# which a copy goes through a block (256 kB).
+PRELUDE = """
+import sys
+import numpy as np
+
+sys.path.insert(0, sys.argv[1])
+import ecl_b200 as ecl
+
+
+def graph(n):
+    link = np.arange(n - 1) % 10 != 9
+    u = np.flatnonzero(link)
+    row, col = np.concatenate([u, u + 1]), np.concatenate([u + 1, u])
+    order = np.lexsort((col, row))
+    row, col = row[order], col[order]
+    nindex = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=n))])
+    w = 1 + np.minimum(row, col) % 1000
+    g = ecl.Graph(nindex, col, w, True)
+    want = np.arange(n) // 10 * 10
+    return g, want, int((1 + u % 1000).sum())
+
+
+def check(g, want, total):
+    out = np.full(g.nodes, -1, np.int32)
+    ecl.cc(g, out=out)
+    assert np.array_equal(out, want)
+    flags, weight = ecl.mst(g)
+    assert weight == total and int(flags.sum()) == g.edges // 2
+    return 1
+"""
+
+
+def run(body, **env):
+    r = subprocess.run([sys.executable, "-c", PRELUDE + body, os.path.join(ROOT, "ecl-suite_b200")],
+                       env={**os.environ, **env}, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert r.stdout.split()[-1] == "done"
+
+
+def test_blocks_do_not_outlive_their_context():
+    """cudaDeviceReset ends the context and with it the blocks and their events:
+    the solves after it make new ones, more often than there are blocks."""
+    run("""
+g = graph(300000)
+for _ in range(6):
+    check(*g)
+    assert ecl.lib.cudaDeviceReset() == 0
+check(*g)
+print("done")
+""", OMP_NUM_THREADS="4")
