@@ -653,14 +653,10 @@ static_assert(kStatusBytes + sizeof(CCCounters) + 256 +
 
 static __device__ __align__(256) unsigned char g_cc_noalloc_scratch[kNoAllocBytes];
 
-// cuCtxGetCurrent, reached through the runtime's driver entry point so the
-// library needs no link against libcuda.
-typedef int (*CtxGetCurrentFn)(void** ctx);
-
 std::mutex g_noalloc_mu;
 struct NoAllocSlot {
-  void* ctx = nullptr;   // context the address belongs to
-  void* addr = nullptr;  // device address of g_cc_noalloc_scratch in it
+  unsigned long long ctx = 0;  // id of the context the address belongs to
+  void* addr = nullptr;        // device address of g_cc_noalloc_scratch in it
 };
 NoAllocSlot g_noalloc_slot[64];
 
@@ -671,32 +667,17 @@ NoAllocSlot g_noalloc_slot[64];
 // address is looked up again instead of reusing a dead one.
 ecl_status noalloc_scratch(int device, void** out) {
   if (device < 0 || device >= 64) return ECL_ERR_NO_DEVICE;
+  const unsigned long long ctx = context_id();
   std::lock_guard<std::mutex> lk(g_noalloc_mu);
-  static CtxGetCurrentFn ctx_get = nullptr;
-  if (!ctx_get) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &fn, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess || !fn) {
-      set_last_error_msg("ecl_cc_noalloc: cuCtxGetCurrent is not available");
-      return ECL_ERR_CUDA;
-    }
-    ctx_get = reinterpret_cast<CtxGetCurrentFn>(fn);
-  }
-  void* ctx = nullptr;
-  if (ctx_get(&ctx) != 0 || !ctx) {
-    set_last_error_msg("ecl_cc_noalloc: no current CUDA context");
-    return ECL_ERR_CUDA;
-  }
   NoAllocSlot& slot = g_noalloc_slot[device];
-  if (slot.ctx != ctx || !slot.addr) {
+  if (ctx == 0 || slot.ctx != ctx || !slot.addr) {  // (0: no context yet; the look-up makes it)
     void* p = nullptr;
     const cudaError_t e = cudaGetSymbolAddress(&p, g_cc_noalloc_scratch);
     if (e != cudaSuccess) {
       set_last_error("cudaGetSymbolAddress(g_cc_noalloc_scratch)", e);
       return ECL_ERR_CUDA;
     }
-    slot.ctx = ctx;
+    slot.ctx = context_id();
     slot.addr = p;
   }
   *out = slot.addr;

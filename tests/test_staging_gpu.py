@@ -64,3 +64,31 @@ for _ in range(6):
 check(*g)
 print("done")
 """, OMP_NUM_THREADS="4")
+
+
+def test_allocation_free_cc_after_its_context_was_replaced():
+    """ecl_cc_noalloc's scratch array has another address, or none yet, in the
+    context that follows a reset, whose handle may well be the old one."""
+    run("""
+import ctypes as C
+
+f = ecl.lib.ecl_cc_noalloc
+f.restype, f.argtypes = C.c_int, [C.c_int32, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
+rt = ecl.lib
+rt.cudaMalloc.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
+rt.cudaMemcpy.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
+g, want, _ = graph(20000)
+for k in range(3):
+    pad, d = C.c_void_p(), [C.c_void_p() for _ in range(3)]
+    assert rt.cudaMalloc(C.byref(pad), (k + 1) << 20) == 0  # another start for what the context loads
+    for p, a in zip(d, (g.nindex, g.nlist, want.astype(np.int32))):
+        assert rt.cudaMalloc(C.byref(p), a.nbytes) == 0
+        assert rt.cudaMemcpy(p, a.ctypes.data, a.nbytes, 1) == 0
+    for _ in range(2):
+        assert f(g.nodes, g.edges, d[0], d[1], d[2], None) == ecl.OK
+    out = np.empty(g.nodes, np.int32)
+    assert rt.cudaMemcpy(out.ctypes.data, d[2], out.nbytes, 2) == 0
+    assert np.array_equal(out, want)
+    assert rt.cudaDeviceReset() == 0
+print("done")
+""")
