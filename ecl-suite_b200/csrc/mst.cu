@@ -385,6 +385,20 @@ __device__ __noinline__ void mst_solo(int4* list, int sz, int& r, int* parent, u
   }
 }
 
+// Moves parent[v] (p as loaded) up v's tree by at most kJumps steps; true when
+// it is the root.  The tree is fixed; every parent on it moves up meanwhile.
+constexpr int kJumps = 32;
+
+__device__ __forceinline__ bool mst_jump(int v, int p, int* parent) {
+  for (int k = 0; k < kJumps; k++) {
+    const int pp = ld(&parent[p]);
+    if (pp == p) return true;
+    st(&parent[v], pp);
+    p = pp;
+  }
+  return false;
+}
+
 // All Boruvka rounds of one pass.  wlA holds the pass's initial worklist
 // (size wlcount[pass][0]), whose entries join two distinct roots; later rounds
 // alternate wlA / wlB.  A round has three phases, a grid barrier after each:
@@ -396,7 +410,11 @@ __device__ __noinline__ void mst_solo(int4* list, int sz, int& r, int* parent, u
 //      two roots that chose the same entry; the smaller of the two stays a root.
 //   C  flattens: every root that took part jumps to its component's new root
 //      and has its key word cleared; the new roots are listed for the next
-//      round (round 0 looks at all vertices instead of a list).
+//      round (round 0 looks at all vertices instead of a list).  A vertex goes
+//      up kJumps steps and then waits until its thread has been through all of
+//      its own: a tree can be as deep as the round has roots (a path whose
+//      weights fall along it), and a thread that climbs on alone meets parents
+//      that nobody has moved yet, one by one (1 M vertices: 464 ms; so, 0.17).
 // Only phase B writes what phase A reads and the other way round, so the loads
 // of parent[] in A and of minv[] in B are plain loads that the SM's L1 serves:
 // with a union-find walked by relaxed atomic loads, every entry of a middle
@@ -533,6 +551,7 @@ __global__ void __launch_bounds__(kBorTPB, 1) mst_boruvka(int n, int pass, int4*
     const int* rin = (r & 1) ? rootsA : rootsB;
     int* rout = (r & 1) ? rootsB : rootsA;
     const int nr = r == 0 ? n : ld(&rcnt[r]);
+    bool left = false;  // one of this thread's vertices has not reached its root
     for (long long i0 = tid - lane; i0 < nr; i0 += nthreads) {  // whole warps: they append together
       const long long i = i0 + lane;
       int v = -1;
@@ -540,17 +559,21 @@ __global__ void __launch_bounds__(kBorTPB, 1) mst_boruvka(int n, int pass, int4*
       bool root = false;
       if (v >= 0 && ld(&minv[v]) != ~0ull) {  // took part in this round
         st(&minv[v], ~0ull);
-        int p = ld(&parent[v]);
+        const int p = ld(&parent[v]);
         root = p == v;
-        int pp;
-        while (!root && (pp = ld(&parent[p])) != p) {
-          st(&parent[v], pp);
-          p = pp;
-        }
+        left |= !root && !mst_jump(v, p, parent);
       }
       rstg.push(root, v, rout, &rcnt[r + 1], n, overflow);
     }
     rstg.flush(rout, &rcnt[r + 1], n, overflow);
+    while (left) {
+      left = false;
+      for (long long i = tid; i < nr; i += nthreads) {
+        const int v = r == 0 ? (int)i : rin[i];
+        const int p = ld(&parent[v]);
+        left |= p != v && !mst_jump(v, p, parent);
+      }
+    }
     if (!grid_sync(&ctl->bar, status)) return;
     if (tid == 0) ctl->stamp[pass][3 * r + 3] = mst_now();
   }

@@ -540,6 +540,51 @@ def test_mst_lists_that_one_block_finishes(ecl, orc, edges):
             assert tot == total and np.array_equal(inm, want)
 
 
+def path_csr(ecl, n, w, cut=0):
+    """A path 0 - 1 - ... of n vertices with weights w[i] on (i, i + 1), without
+    every cut-th link."""
+    u = np.arange(n - 1)
+    u = u[u % cut != cut - 1] if cut else u
+    row, col = np.concatenate([u, u + 1]), np.concatenate([u + 1, u])
+    order = np.lexsort((col, row))
+    row, col = row[order], col[order]
+    nindex = np.concatenate([[0], np.cumsum(np.bincount(row, minlength=n))])
+    return ecl.Graph(nindex, col, np.asarray(w)[np.minimum(row, col)], True)
+
+
+def best_ms(ecl, dg, code, **kw):
+    """Device time of the fastest of five calls, in ms."""
+    best = 1e9
+    for _ in range(5):
+        o = ecl.Opts()
+        getattr(ecl, code)(dg, opts=o, **kw)
+        best = min(best, o.elapsed_ms)
+    return best
+
+
+@pytest.mark.parametrize("length", [31, 32, 33, 34, 35, 1024, 1025, 1026, 1100])  # around 32 steps, and 32 * 32
+@pytest.mark.parametrize("falling", [False, True])
+def test_mst_of_chains_as_deep_as_the_list(ecl, length, falling):
+    """Weights that fall or rise along a path hook all of it in one round into
+    one chain, towards the larger ids or the smaller."""
+    n = max(4000 // length, 2) * length
+    w = np.arange(n)[::-1] + 1 if falling else np.arange(n) + 1
+    g = path_csr(ecl, n, w, cut=length)
+    flags, total = ecl.mst(g)
+    row = np.repeat(np.arange(n), np.diff(g.nindex))
+    assert np.array_equal(flags.astype(bool), row < g.nlist)
+    assert total == int(g.eweight[row < g.nlist].astype(np.int64).sum())
+
+
+def test_mst_chain_of_half_a_million_is_climbed_by_all_threads(ecl):
+    """One chain much longer than the launch has threads costs about the same
+    whichever way it is numbered (climbed link by link: 160 ms and more)."""
+    n = 500000
+    rising, falling = (path_csr(ecl, n, w).to_device() for w in (np.arange(n) + 1, np.arange(n)[::-1] + 1))
+    assert best_ms(ecl, falling, "mst") < 10 * best_ms(ecl, rising, "mst") + 1.0
+    assert ecl.mst(falling)[1] == n * (n + 1) // 2 - 1
+
+
 @pytest.mark.parametrize("n", [1025, 65537, (1 << 20) - 1, (1 << 20) + 1025])
 def test_gc_order_of_equal_degrees(ecl, orc, n):
     """One degree for all vertices: the sort's left-out digits decide between
