@@ -303,15 +303,13 @@ __device__ __forceinline__ void mst_hook(const int4& e, u64 ka, u64 kb, int* par
 // general form on one block.  Measured, the light pass's rounds, general form /
 // kSolo = 512 / 2048 / 8192: R-MAT with 1 k vertices 64 / 24 / 25 / 24 us, with
 // 2 k 57 / 57 / 49 / 47, G(5 k, 15 k) 98 / 98 / 85 / 134, G(20 k, 80 k) 124 /
-// 123 / 124 / 154: one block is too narrow for longer lists.  All threads of
-// the block call.
+// 123 / 124 / 154: one block is too narrow for longer lists.  An entry's two
+// ends climbed one after another, link by link -> side by side, leaving what
+// they reach to the others: a path of 2 k vertices with random weights 63 -> 55
+// us, with equal ones, which all hook into one chain, 1284 -> 36.  All threads
+// of the block call.
 constexpr int kSolo = 2048;
-
-__device__ __forceinline__ int mst_root(int v, const int* parent) {
-  int p;
-  while ((p = ld(&parent[v])) != v) v = p;
-  return v;
-}
+constexpr int kSoloBatch = kSolo / kBorTPB;  // entries a thread keeps in flight: its share of the list
 
 __device__ __noinline__ void mst_solo(int4* list, int sz, int& r, int* parent, u64* minv, unsigned char* in_mst,
                                       RootTable tab, u64& local) {
@@ -319,16 +317,16 @@ __device__ __noinline__ void mst_solo(int4* list, int sz, int& r, int* parent, u
   for (; r < kMaxRounds; r++) {
     tab.reset();
     bool live = false;
-    for (int i0 = threadIdx.x; i0 < sz; i0 += kBorTPB * kBorBatch) {
-      int2 e[kBorBatch];
-      int a[kBorBatch], b[kBorBatch];
+    for (int i0 = threadIdx.x; i0 < sz; i0 += kBorTPB * kSoloBatch) {
+      int2 e[kSoloBatch];
+      int a[kSoloBatch], b[kSoloBatch];
 #pragma unroll
-      for (int k = 0; k < kBorBatch; k++) {
+      for (int k = 0; k < kSoloBatch; k++) {
         const int i = i0 + k * kBorTPB;
         e[k] = i < sz ? *reinterpret_cast<const int2*>(&list[i]) : make_int2(-1, -1);
       }
 #pragma unroll
-      for (int k = 0; k < kBorBatch; k++) {
+      for (int k = 0; k < kSoloBatch; k++) {
         if (e[k].x < 0) continue;
         if (lowered) {
           st(&minv[e[k].x], ~0ull);
@@ -337,11 +335,36 @@ __device__ __noinline__ void mst_solo(int4* list, int sz, int& r, int* parent, u
         a[k] = ld(&parent[e[k].x]);
         b[k] = ld(&parent[e[k].y]);
       }
+      // All ends go up side by side, and what they reach they leave in their
+      // parent words for the others: the entries can have hooked into one chain
+      // as long as the list (equal weights along a path), of which every end so
+      // leaves half at each step.
+      unsigned go = 0;  // bits 2 k, 2 k + 1: entry k's ends are below a[k], b[k]
 #pragma unroll
-      for (int k = 0; k < kBorBatch; k++) {
+      for (int k = 0; k < kSoloBatch; k++)
+        if (e[k].x >= 0) go |= (a[k] != e[k].x ? 1u << (2 * k) : 0u) | (b[k] != e[k].y ? 2u << (2 * k) : 0u);
+      while (go) {
+        int pa[kSoloBatch], pb[kSoloBatch];
+#pragma unroll
+        for (int k = 0; k < kSoloBatch; k++) {
+          if ((go >> (2 * k)) & 1u) pa[k] = ld(&parent[a[k]]);
+          if ((go >> (2 * k)) & 2u) pb[k] = ld(&parent[b[k]]);
+        }
+#pragma unroll
+        for (int k = 0; k < kSoloBatch; k++) {
+          if ((go >> (2 * k)) & 1u) {
+            if (pa[k] == a[k]) go &= ~(1u << (2 * k));
+            else st(&parent[e[k].x], a[k] = pa[k]);
+          }
+          if ((go >> (2 * k)) & 2u) {
+            if (pb[k] == b[k]) go &= ~(2u << (2 * k));
+            else st(&parent[e[k].y], b[k] = pb[k]);
+          }
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kSoloBatch; k++) {
         if (e[k].x < 0) continue;
-        if (a[k] != e[k].x) a[k] = mst_root(a[k], parent);
-        if (b[k] != e[k].y) b[k] = mst_root(b[k], parent);
         if (a[k] == b[k]) a[k] = -1;
         live |= a[k] >= 0;
         *reinterpret_cast<int2*>(&list[i0 + k * kBorTPB]) = make_int2(a[k], b[k]);
@@ -362,22 +385,22 @@ __device__ __noinline__ void mst_solo(int4* list, int sz, int& r, int* parent, u
       if (rt >= 0) fetch_min(&minv[rt], tab.key[i]);
     }
     __syncthreads();
-    for (int i0 = threadIdx.x; i0 < sz; i0 += kBorTPB * kBorBatch) {
-      int4 e[kBorBatch];
-      u64 ka[kBorBatch], kb[kBorBatch];
+    for (int i0 = threadIdx.x; i0 < sz; i0 += kBorTPB * kSoloBatch) {
+      int4 e[kSoloBatch];
+      u64 ka[kSoloBatch], kb[kSoloBatch];
 #pragma unroll
-      for (int k = 0; k < kBorBatch; k++) {
+      for (int k = 0; k < kSoloBatch; k++) {
         const int i = i0 + k * kBorTPB;
         e[k] = i < sz ? list[i] : make_int4(-1, -1, 0, 0);
       }
 #pragma unroll
-      for (int k = 0; k < kBorBatch; k++) {
+      for (int k = 0; k < kSoloBatch; k++) {
         if (e[k].x < 0) continue;
         ka[k] = ld(&minv[e[k].x]);
         kb[k] = ld(&minv[e[k].y]);
       }
 #pragma unroll
-      for (int k = 0; k < kBorBatch; k++)
+      for (int k = 0; k < kSoloBatch; k++)
         if (e[k].x >= 0) mst_hook(e[k], ka[k], kb[k], parent, in_mst, local);
     }
     lowered = true;

@@ -585,6 +585,20 @@ def test_mst_chain_of_half_a_million_is_climbed_by_all_threads(ecl):
     assert ecl.mst(falling)[1] == n * (n + 1) // 2 - 1
 
 
+@pytest.mark.parametrize("kind", ["equal", "rising", "falling"])
+def test_mst_chain_of_a_short_list_is_climbed_in_steps_that_double(ecl, orc, kind):
+    """One block's list hooked into one chain costs no more than the rounds of
+    random weights do (climbed link by link: twenty times as much)."""
+    n = 2049
+    rng = np.random.default_rng(3)
+    w = dict(equal=np.full(n, 7), rising=np.arange(n) + 1, falling=np.arange(n)[::-1] + 1)[kind]
+    g, plain = path_csr(ecl, n, w), path_csr(ecl, n, rng.permutation(n) + 1)
+    want, total = orc.mst(g)
+    flags, weight = ecl.mst(g)
+    assert weight == total and np.array_equal(flags, want)
+    assert best_ms(ecl, g.to_device(), "mst") < 3 * best_ms(ecl, plain.to_device(), "mst")
+
+
 @pytest.mark.parametrize("n", [1025, 65537, (1 << 20) - 1, (1 << 20) + 1025])
 def test_gc_order_of_equal_degrees(ecl, orc, n):
     """One degree for all vertices: the sort's left-out digits decide between
