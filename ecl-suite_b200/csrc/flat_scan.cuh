@@ -64,7 +64,7 @@ __device__ __forceinline__ void flat_rows_range(int n, int m, const int* nindex,
 
 // One tile: f(e0, row, u) with e0 the lane's first entry and, for its
 // kFlatLane entries, the row (-1: the entry is in no row, or past the end) and
-// the entry's value nlist[e0 + k] (0 where the row is -1).  s_mark: this
+// the entry's value nlist[e0 + k] (anything where the row is -1).  s_mark: this
 // warp's kFlatTile words of shared memory.  All lanes call, and all call f.
 // `stop` = min(m, nindex[n]), the end of the last row.
 template <class F>

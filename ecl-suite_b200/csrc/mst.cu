@@ -191,9 +191,10 @@ __global__ void __launch_bounds__(kTPB, kLight ? 5 : 4) mst_scan(FlatCsr g, bool
       unsigned want = 0;  // bit k: entry k may be kept
 #pragma unroll
       for (int k = 0; k < kFlatLane; k++) {
+        if (row[k] < 0) continue;  // before the first row: not an entry of the graph
         if ((unsigned)u[k] >= (unsigned)g.n)
           raise(status, ECL_ERR_BAD_GRAPH, u[k]);
-        else if (row[k] >= 0 && u[k] > row[k])
+        else if (u[k] > row[k])
           want |= 1u << k;
       }
       int a[kFlatLane], b[kFlatLane], w[kFlatLane];

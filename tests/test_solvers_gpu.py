@@ -599,6 +599,24 @@ def test_mst_chain_of_a_short_list_is_climbed_in_steps_that_double(ecl, orc, kin
     assert best_ms(ecl, g.to_device(), "mst") < 3 * best_ms(ecl, plain.to_device(), "mst")
 
 
+@pytest.mark.parametrize("lead", [1, 255, 256, 700])
+@pytest.mark.parametrize("code", ["cc", "gc", "mst"])  # (MIS's priorities go by the entry count, these included)
+def test_entries_outside_all_rows_are_not_looked_at(ecl, orc, code, lead):
+    """A CSR whose first row does not start at 0 (not validated on the host):
+    what stands before it and behind the last row is no part of the graph."""
+    g = ecl.gen_rmat(11, 8, seed=2, weight_seed=3)
+    junk = np.full(lead, 1 << 30, np.int32)
+    h = ecl.Graph(g.nindex + lead, np.concatenate([junk, g.nlist, -junk]),
+                  np.concatenate([-junk, g.eweight, -junk]), True)
+    want, got = getattr(orc, code)(g), getattr(ecl, code)(h.to_device())
+    if code == "mst":
+        assert got[1] == want[1]
+        want, got = want[0], got[0]
+        assert not got[:lead].any() and not got[lead + g.edges:].any()
+        got = got[lead: lead + g.edges]
+    assert np.array_equal(got.cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("n", [1025, 65537, (1 << 20) - 1, (1 << 20) + 1025])
 def test_gc_order_of_equal_degrees(ecl, orc, n):
     """One degree for all vertices: the sort's left-out digits decide between
