@@ -73,6 +73,7 @@ struct SCCCtl {
   int level_chunks[kGiantLevels];  // ... and chunk records of its long rows
   int left[kGiantRounds + 1];  // per backward round: vertices not known to reach the pivot
   int moved[kGiantRounds];     // per backward round: some vertex was found to reach it
+  int back_chunks[kGiantRounds];   // ... and chunk records of its long rows
   int pad[64];
   // %globaltimer at the start and after each grid barrier (the first
   // kStamps - 1): a time profile of sweeps, compactions and retirements that
@@ -230,6 +231,7 @@ constexpr int kGiantPatience = 16;
 constexpr int kGiantEntries = 1 << 20;  // from this many entries on: R-MAT with 0.45 M entries 229 -> 227 us, 1.05 M 266 -> 250,
                                         // 1.8 M 363 -> 261; G(150 k, 600 k) 329 -> 444, G(400 k, 1.6 M) 546 -> 532
 constexpr int kGiantLong = 256;   // longer rows are cut into chunk records of this many entries
+constexpr int kBackLong = 1024;   // ... backward, where most rows are left after a few entries, only rows longer than this
 
 struct Giant {
   unsigned* fwd;  // bit per vertex: reached from the pivot
@@ -440,8 +442,13 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
           for (int k = 0; k < 4; k++) found |= reaches_now(w[k]);
         }
       }
-      unsigned todo = __ballot_sync(kFull, !found && deg > 32);
-      while (todo) {  // the rest of the long rows, by the whole warp
+      // a row that is still not decided: the rest of it by the whole warp, or,
+      // of a long one, as chunk records by all warps (one warp alone with a hub
+      // of 1 M entries that does not reach the pivot: 14 ms, in every round)
+      push_chunks_warp(RowChunks{chunks, &ctl->back_chunks[round], chunk_cap}, kGiantLong, !found && deg > kBackLong, v,
+                       beg, beg + deg, status);
+      unsigned todo = __ballot_sync(kFull, !found && deg > 32 && deg <= kBackLong);
+      while (todo) {
         const int who = __ffs(todo) - 1;
         todo &= todo - 1;
         const int wbeg = __shfl_sync(kFull, beg, who), wdeg = __shfl_sync(kFull, deg, who);
@@ -465,10 +472,33 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
       stg.push(deg > 0 && !found, v, out, &ctl->left[round + 1], n, overflow);
     }
     stg.flush(out, &ctl->left[round + 1], n, overflow);
-    if (moved) s_moved = 1;  // every writer stores the same value
-    __syncthreads();
-    if (threadIdx.x == 0 && s_moved) st(&ctl->moved[round], 1);
+    auto tell = [&]() {  // the block's `moved` to the round's word
+      if (moved) s_moved = 1;  // every writer stores the same value
+      __syncthreads();
+      if (threadIdx.x == 0 && s_moved) st(&ctl->moved[round], 1);
+    };
+    tell();
     if (!grid_sync(&ctl->giant_bar, status)) return;
+    const int nch = chunk_total(RowChunks{chunks, &ctl->back_chunks[round], chunk_cap});
+    for (int c = warp; c < nch; c += nwarps) {
+      const int2 r = chunks[c];  // written before the grid barrier
+      if (reaches_now(r.x)) continue;
+      const int end = min(r.y + kGiantLong, __ldg(&nindex[r.x + 1]));
+      constexpr int K = kGiantLong / 32;
+      int w[K];
+      bool mine = false;
+#pragma unroll
+      for (int k = 0; k < K; k++) w[k] = r.y + 32 * k + lane < end ? __ldg(&nlist[r.y + 32 * k + lane]) : -1;
+#pragma unroll
+      for (int k = 0; k < K; k++) mine = mine || reaches(w[k]) || reaches_now(w[k]);
+      if (!__any_sync(kFull, mine)) continue;
+      if (lane == 0) fetch_or(&next[r.x >> 5], 1u << (r.x & 31));
+      moved = true;
+    }
+    if (nch > 0) {  // the same for every block
+      tell();
+      if (!grid_sync(&ctl->giant_bar, status)) return;
+    }
     if (!ld(&ctl->moved[round])) break;
     cnt = ld(&ctl->left[round + 1]);
     merge_bits(bwd, next, words, tid, nthreads);

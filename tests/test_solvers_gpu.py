@@ -617,6 +617,46 @@ def test_entries_outside_all_rows_are_not_looked_at(ecl, orc, code, lead):
     assert np.array_equal(got.cpu().numpy(), want)
 
 
+def directed(ecl, n, u, v):
+    """CSR of the entries (u, v), each once."""
+    k = np.unique(np.asarray(u, np.int64) * n + np.asarray(v, np.int64))
+    nindex = np.concatenate([[0], np.cumsum(np.bincount(k // n, minlength=n))])
+    return ecl.Graph(nindex, k % n, None)
+
+
+def hub_graph(ecl, hubs, k, back, n=3000000):
+    """A pivot (0) with 2.5 M entries, on a cycle of 32 vertices, and `hubs`
+    vertices below it with k entries each to vertices without any -- but that the
+    last one's last entry is n - 1, which leads to the cycle if `back`."""
+    rng = np.random.default_rng(hubs)
+    ends = lambda size: 100 + rng.permutation(n - 101)[:size]  # noqa: E731
+    u, v = [np.zeros(2500000), np.arange(32)], [ends(2500000), np.arange(1, 33) % 32]
+    u, v = u + [np.full(hubs, 5)], v + [40 + np.arange(hubs)]
+    for h in range(hubs):
+        u.append(np.full(k - 1 if h == hubs - 1 else k, 40 + h))
+        v.append(ends(u[-1].size))
+    u, v = u + [[39 + hubs, n - 1]], v + [[n - 1, 7 if back else 1000]]
+    return directed(ecl, n, np.concatenate(u), np.concatenate(v))
+
+
+@pytest.mark.parametrize("k", [33, 1023, 1024, 1025, 1279, 1280, 1281, 5000])  # rows by lanes, by warps and in records
+@pytest.mark.parametrize("back", [False, True])
+def test_scc_hubs_behind_the_giant_component(ecl, orc, k, back):
+    """What decides whether a hub belongs to the component is the last entry of
+    its row."""
+    g = hub_graph(ecl, 3, k, back)
+    want = orc.scc(g)
+    assert want[0] == (g.nodes - 1 if back else 31) and want[42] == (g.nodes - 1 if back else 42)
+    assert np.array_equal(ecl.scc(g.to_device()).cpu().numpy(), want)
+
+
+def test_scc_hubs_that_do_not_reach_the_pivot_are_shared_by_all_warps(ecl):
+    """Hubs of 0.5 M entries each cost a pass over their entries, not a warp's
+    walk through a row in every round (that: 7 ms a row and round)."""
+    few, many = (hub_graph(ecl, h, k, False).to_device() for h, k in ((1, 33), (4, 500000)))
+    assert best_ms(ecl, many, "scc") < 2.0 + 5 * best_ms(ecl, few, "scc")
+
+
 @pytest.mark.parametrize("n", [1025, 65537, (1 << 20) - 1, (1 << 20) + 1025])
 def test_gc_order_of_equal_degrees(ecl, orc, n):
     """One degree for all vertices: the sort's left-out digits decide between
