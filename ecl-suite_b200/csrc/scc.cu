@@ -218,9 +218,15 @@ __global__ void __launch_bounds__(kTPB) scc_relabel(int n, int* __restrict__ com
 // looks for one out-neighbour known to, and stops at the first: two or three
 // entries a vertex).  What is left for the propagation sweeps -- each of them
 // two random words for every edge -- is the few edges between other vertices
-// on the same side of the search.  The forward search gives up on graphs whose
-// distances are long (kGiantLevels levels, or few vertices reached by level
-// kGiantPatience); the sweeps then run on all edges as before.
+// on the same side of the search.  The search gives up, and the sweeps run on
+// all edges as before, where it would take long or find little: forward after
+// kGiantLevels levels, with few vertices reached by level kGiantPatience, or
+// when two levels in a row neither grow nor shrink much while most vertices are
+// still unreached (meshes and layers; a random graph's levels grow until they
+// hold much of it); backward when most vertices are still candidates and a round
+// after the first finds hardly any, or the candidates looked through add up to
+// twice n and the number found does not grow (a few vertices that reach the
+// pivot one after another, above many that do not: 0.52 -> 0.44 ms of 2.2 lost).
 // Bound by the latency of the two widest levels' look-ups (a third of the time
 // each at R-MAT-22).  Measured, whole solve, sweeps over all edges -> this:
 // directed R-MAT-22 (65 M edges) 2.47 -> 0.83 ms, 500 k vertices (5.7 M) 0.58
@@ -228,8 +234,14 @@ __global__ void __launch_bounds__(kTPB) scc_relabel(int n, int* __restrict__ com
 // it gives up, 17.3 -> 17.4.
 constexpr int kGTPB = 512;
 constexpr int kGiantPatience = 16;
-constexpr int kGiantEntries = 1 << 20;  // from this many entries on: R-MAT with 0.45 M entries 229 -> 227 us, 1.05 M 266 -> 250,
-                                        // 1.8 M 363 -> 261; G(150 k, 600 k) 329 -> 444, G(400 k, 1.6 M) 546 -> 532
+// Entries from which on the search is tried: kGiantEntries where the pivot is a
+// hub (kGiantHub times the average degree), and from kGiantFlat on without one,
+// as a graph without hubs has more levels for its size.  With hubs: R-MAT with
+// 0.45 M entries 229 -> 227 us, 1.05 M 266 -> 250, 1.8 M 363 -> 261.  Without:
+// G(300 k, 1.2 M) 441 -> 528, G(600 k, 2.4 M) 659 -> 595, G(1 M, 4 M) 1078 -> 711.
+constexpr int kGiantEntries = 1 << 20;
+constexpr int kGiantFlat = 1 << 21;
+constexpr int kGiantHub = 32;
 constexpr int kGiantLong = 256;   // longer rows are cut into chunk records of this many entries
 constexpr int kBackLong = 1024;   // ... backward, where most rows are left after a few entries, only rows longer than this
 
@@ -306,6 +318,8 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
     deg = end - beg;
     if (beg < 0 || end < beg || end > m) beg = deg = 0;
   };
+  // no bit set yet (the words of all three arrays lie side by side)
+  for (int i = tid; i < 3 * words; i += nthreads) fwd[i] = 0;  // race-free: thread-owned, barrier next
   // the pivot
   unsigned long long key = 0;
   for (int v = tid; v < n; v += nthreads) {
@@ -318,6 +332,7 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
   if (!grid_sync(&ctl->giant_bar, status)) return;
   key = ld(&ctl->pivot);
   if ((key >> 32) == 0) return;  // no entries at all
+  if (m < kGiantFlat && (long long)(key >> 32) < (long long)kGiantHub * (m / n + 1)) return;
   const int pivot = (int)(0xffffffffu - (unsigned)key);
   if (tid == 0) {
     fetch_or(&fwd[pivot >> 5], 1u << (pivot & 31));
@@ -326,6 +341,7 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
   }
   if (!grid_sync(&ctl->giant_bar, status)) return;
   int qs = 0, qe = 1, level = 0;
+  int flat = 0;  // levels in a row that neither grew nor shrank much
   // chunk records of the frontier's long rows
   auto cut_long_rows = [&]() {
     const RowChunks rc{chunks, &ctl->level_chunks[level], chunk_cap};
@@ -402,15 +418,19 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
     stg.flush(queue + qe, &ctl->level_new[level], n - qe, overflow);
     if (!grid_sync(&ctl->giant_bar, status)) return;
     merge_bits(fwd, next, words, tid, nthreads);
+    const int last = qe - qs, fresh = ld(&ctl->level_new[level]);
     qs = qe;
-    qe += ld(&ctl->level_new[level]);
+    qe += fresh;
+    flat = level >= 4 && qe < n / 8 && 4LL * fresh < 5LL * last && 2LL * fresh >= last ? flat + 1 : 0;
+    if (flat == 2) return;
     level++;
     cut_long_rows();
     level--;
     if (!grid_sync(&ctl->giant_bar, status)) return;
   }
   // backward, inside the vertices reached
-  int cnt = qe;
+  int cnt = qe, cnt1 = 0, found0 = 0;  // candidates, those after the first round, the round before's finds
+  long long looked = 0;
   for (int round = 0;; round++) {
     if (round == kGiantRounds) return;
     const int* in = round == 0 ? queue : ((round & 1) ? candA : candB);
@@ -500,7 +520,13 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
       if (!grid_sync(&ctl->giant_bar, status)) return;
     }
     if (!ld(&ctl->moved[round])) break;
-    cnt = ld(&ctl->left[round + 1]);
+    looked += cnt;
+    const int left = ld(&ctl->left[round + 1]), found_now = cnt - left;
+    if (round == 0) cnt1 = left;
+    if (round > 0 && left > n / 2 && found_now < 3) return;
+    if (looked > 16LL * n || (looked > 2LL * n && cnt1 - left < n / 16 && 2LL * found_now < 3LL * found0)) return;
+    found0 = round == 0 ? 0 : found_now;
+    cnt = left;
     merge_bits(bwd, next, words, tid, nthreads);
     if (!grid_sync(&ctl->giant_bar, status)) return;
   }
@@ -946,7 +972,6 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
     int gocc = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&gocc, scc_giant, kGTPB, 0) != cudaSuccess || gocc < 1)
       return ECL_ERR_CUDA;
-    ECL_CUDA_TRY(cudaMemsetAsync(b.bits, 0, sizeof(unsigned) * 3 * words, stream));
     const int blocks = std::max(1, std::min(dev.sms * gocc, (int)(std::max((long long)g.n, (long long)g.m / 4) / kGTPB)));
     ECL_CUDA_TRY(launch_cooperative(scc_giant, blocks, kGTPB, stream, g.n, g.m, g.nindex, g.nlist, gi.fwd, gi.bwd,
                                     b.bits + 2 * words, b.queue, b.candA, b.candB, b.chunks, (int)row_chunk_capacity(g.m, kMinChunk), b.ctl,

@@ -552,11 +552,12 @@ def path_csr(ecl, n, w, cut=0):
     return ecl.Graph(nindex, col, np.asarray(w)[np.minimum(row, col)], True)
 
 
-def best_ms(ecl, dg, code, **kw):
+def best_ms(ecl, dg, code, max_rounds=0, **kw):
     """Device time of the fastest of five calls, in ms."""
     best = 1e9
     for _ in range(5):
         o = ecl.Opts()
+        o.max_rounds = max_rounds
         getattr(ecl, code)(dg, opts=o, **kw)
         best = min(best, o.elapsed_ms)
     return best
@@ -655,6 +656,35 @@ def test_scc_hubs_that_do_not_reach_the_pivot_are_shared_by_all_warps(ecl):
     walk through a row in every round (that: 7 ms a row and round)."""
     few, many = (hub_graph(ecl, h, k, False).to_device() for h, k in ((1, 33), (4, 500000)))
     assert best_ms(ecl, many, "scc") < 2.0 + 5 * best_ms(ecl, few, "scc")
+
+
+def long_distance_cases(ecl):
+    """Directed graphs of a million entries and more in which the search for a
+    giant component takes long or finds nothing."""
+    rng = np.random.default_rng(2)
+    for layers, wide, deg in ((50, 2000, 20), (300, 5000, 2)):
+        u = np.repeat(np.arange((layers - 1) * wide), deg)
+        yield f"layers{layers}", directed(ecl, layers * wide, u, (u // wide + 1) * wide + rng.integers(0, wide, u.size))
+    g = ecl.gen_grid(1000, 1100, 0.05, seed=1)
+    yield "grid", ecl.Graph(g.nindex, g.nlist, None, False)
+    n = 300000
+    u, v = rng.integers(0, n, (2, 4 * n))
+    yield "random", directed(ecl, n, u, v)
+    # 32 vertices that reach the pivot one after another, above a random graph that does not
+    n = 600000
+    u, v = 100 + rng.integers(0, n - 100, (2, 10 * n))
+    u = np.concatenate([np.zeros(500000), np.arange(32), u])
+    v = np.concatenate([100 + rng.permutation(n - 100)[:500000], np.arange(1, 33) % 32, v])
+    yield "tail", directed(ecl, n, u, v)
+
+
+def test_scc_search_for_a_giant_component_gives_up_in_time(ecl, orc):
+    """A limit on the rounds, which no graph here needs, solves without the
+    search: with it, little time is lost (layers: four times as much)."""
+    for name, g in long_distance_cases(ecl):
+        dg = g.to_device()
+        assert np.array_equal(ecl.scc(dg).cpu().numpy(), orc.scc(g)), name
+        assert best_ms(ecl, dg, "scc") < 1.25 * best_ms(ecl, dg, "scc", max_rounds=g.nodes + 1) + 0.03, name
 
 
 @pytest.mark.parametrize("n", [1025, 65537, (1 << 20) - 1, (1 << 20) + 1025])
