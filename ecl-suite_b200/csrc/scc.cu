@@ -200,9 +200,10 @@ __global__ void __launch_bounds__(kTPB) scc_top(int n, const int* __restrict__ c
 }
 
 __global__ void __launch_bounds__(kTPB) scc_relabel(int n, int* __restrict__ comp, const int* __restrict__ top,
-                                                    const SCCCtl* __restrict__ ctl) {
+                                                    const SCCCtl* __restrict__ ctl, Status* __restrict__ status) {
   dep_wait();
   if (ctl->asym != 0) return;  // as scc_mark
+  if (blockIdx.x == 0 && threadIdx.x == 0) st(&status->rounds, 1);  // no sweep: one pass of hooking
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     const int r = comp[v];
     comp[v] = max(r, __ldg(&top[r]));
@@ -964,7 +965,8 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
     if (st != ECL_OK) return st;
     // (the general path's flags stay zero when the graph is not symmetric)
     ECL_LAUNCH_NEXT(scc_top, dev.sms * 4, kTPB, 0, stream, g.n, label, b.flags, b.ctl);
-    ECL_LAUNCH_NEXT(scc_relabel, dev.grid_blocks(kTPB, g.n, 0), kTPB, 0, stream, g.n, label, b.flags, b.ctl);
+    ECL_LAUNCH_NEXT(scc_relabel, dev.grid_blocks(kTPB, g.n, 0), kTPB, 0, stream, g.n, label, b.flags, b.ctl,
+                    status);
   }
   const size_t words = ((size_t)g.n + 31) / 32;
   const Giant gi{b.bits, b.bits + words};

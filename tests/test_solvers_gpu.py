@@ -658,6 +658,16 @@ def test_scc_hubs_that_do_not_reach_the_pivot_are_shared_by_all_warps(ecl):
     assert best_ms(ecl, many, "scc") < 2.0 + 5 * best_ms(ecl, few, "scc")
 
 
+@pytest.mark.parametrize("flagged", [False, True])
+def test_scc_reports_the_rounds_it_took(ecl, flagged):
+    """opts.rounds of a solve that went through is at least one, whichever way
+    it went."""
+    for g in (ecl.gen_rmat(12, 8, seed=3), ecl.gen_grid(40, 50, 0.1, seed=1), ecl.gen_rmat(17, 16, seed=3)):
+        o = ecl.Opts()
+        ecl.scc(ecl.Graph(g.nindex, g.nlist, None, flagged).to_device(), opts=o)
+        assert o.rounds >= 1
+
+
 def long_distance_cases(ecl):
     """Directed graphs of a million entries and more in which the search for a
     giant component takes long or finds nothing."""
