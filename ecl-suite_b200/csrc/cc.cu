@@ -34,12 +34,18 @@ namespace {
 
 using namespace dev;
 
+typedef unsigned long long u64;
+
 constexpr int kTPB = 256;
 // Default degree bins: lists of <= 16 entries per lane, chunk records of
 // 2048 entries (a launch knob may change both).
 constexpr Bins kCCBins{16, 2048};
 constexpr int kInitScan = 8;   // entries cc_init looks at for a first smaller neighbour
 constexpr int kInitHops = 2;   // hops of cc_init (R-MAT-22, whole solve: 1 hop 0.244 ms, 2 0.227, 4 0.217; G(3 M, 12 M): 0.354, 0.369, 0.396)
+
+// Whether this solve is not wanted after all: an earlier launch has left
+// something other than 0 at `off` (nullptr: it always is).
+__device__ __forceinline__ bool cc_off(const u64* off) { return off && *off != 0; }
 
 // Row [beg, end) of v, or empty when the row is malformed (cc_init reports it).
 __device__ __forceinline__ void cc_row(const int* nindex, int v, int m, int& beg, int& end) {
@@ -150,8 +156,10 @@ __device__ __forceinline__ int cc_first_smaller(int v, int beg, int end, const i
 // [0, m]) raises ECL_ERR_BAD_GRAPH and is treated as empty by every kernel.
 __global__ void __launch_bounds__(kTPB) cc_init(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, int* __restrict__ parent,
-                                                CCCounters* __restrict__ ctr, Status* __restrict__ status) {
+                                                CCCounters* __restrict__ ctr, const u64* off,
+                                                Status* __restrict__ status) {
   dep_wait();
+  if (cc_off(off)) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctr->nchunks = 0;  // race-free: first used by later launches
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     int beg = __ldg(&nindex[v]), end = __ldg(&nindex[v + 1]);
@@ -289,8 +297,9 @@ constexpr int kFlattenBatch = 4;
 enum : int { kPlain = 0, kMark = 1, kMarkUnion = 2 };
 template <int kWhat>
 __global__ void __launch_bounds__(kTPB) cc_flatten(int n, int* __restrict__ parent, Giants gi,
-                                                   unsigned char* __restrict__ ing) {
+                                                   unsigned char* __restrict__ ing, const u64* off) {
   dep_wait();
+  if (cc_off(off)) return;
   const int stride = gridDim.x * kTPB;
   const int giant = kWhat == kMark ? gi.root[0] : -1;
   int known = -1;  // a root of this launch
@@ -383,8 +392,9 @@ int flatten_blocks(const DeviceInfo& dev, int n) {
 template <int kPart>  // 0: one vertex in kFirstOf, 1: the others, 2: all
 __global__ void __launch_bounds__(kTPB) cc_sample(int n, int m, const int* __restrict__ nindex,
                                                   const int* __restrict__ nlist, int* __restrict__ parent,
-                                                  Status* __restrict__ status) {
+                                                  const u64* off, Status* __restrict__ status) {
   dep_wait();
+  if (cc_off(off)) return;
   constexpr int kFirstOf = 8;
   const int count = kPart == 0 ? (n - 1) / kFirstOf + 1 : n;
   for (int i = blockIdx.x * kTPB + threadIdx.x; i < count; i += gridDim.x * kTPB) {
@@ -410,8 +420,9 @@ constexpr int kSplitSample = 1 << 13;
 constexpr int kGiantSlots = 2048;
 
 __global__ void __launch_bounds__(1024) cc_giant(int n, const int* __restrict__ parent, const int* __restrict__ vbase,
-                                                 int* __restrict__ root) {
+                                                 int* __restrict__ root, const u64* off) {
   dep_wait();
+  if (cc_off(off)) return;
   const int base = vbase ? __ldg(&vbase[blockIdx.x]) : 0;
   const int size = vbase ? __ldg(&vbase[blockIdx.x + 1]) - base : n;
   __shared__ int s_root[kGiantSlots], s_count[kGiantSlots];
@@ -456,8 +467,9 @@ __global__ void __launch_bounds__(kTPB) cc_rest(int n, int m, const int* __restr
                                                 const int* __restrict__ nlist, int* __restrict__ parent,
                                                 const unsigned char* __restrict__ ing, int2* __restrict__ chunks,
                                                 int chunk_cap, Bins bins, CCCounters* __restrict__ ctr,
-                                                Status* __restrict__ status) {
+                                                const u64* off, Status* __restrict__ status) {
   dep_wait();
+  if (cc_off(off)) return;
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -507,8 +519,10 @@ __global__ void __launch_bounds__(kTPB) cc_rest_chunks(int n, const int* __restr
                                                        const int* __restrict__ nlist, int* __restrict__ parent,
                                                        const unsigned char* __restrict__ ing,
                                                        const int2* __restrict__ chunks, int chunk_cap, int chunk,
-                                                       const CCCounters* __restrict__ ctr, Status* __restrict__ status) {
+                                                       const CCCounters* __restrict__ ctr, const u64* off,
+                                                       Status* __restrict__ status) {
   dep_wait();
+  if (cc_off(off)) return;
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
@@ -553,7 +567,7 @@ size_t cc_workspace_bytes(int n, int m) {
 namespace ecl {
 
 ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, const DeviceInfo& dev,
-                      cudaStream_t stream, Marker mark, const UnionInfo* uni) {
+                      cudaStream_t stream, Marker mark, const UnionInfo* uni, const u64* off) {
   Carve c{ws};
   CCCounters* ctr;
   int2* chunks;
@@ -563,15 +577,15 @@ ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, 
   const Bins bins = bins_of(dev, kCCBins);
   const int cap = chunk_capacity(g.m, kMinChunk);  // cc_layout sized the records for the smallest chunk
   if (g.flags & ECL_GRAPH_SYMMETRIC) {
-    ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, status);
-    ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, Giants{}, nullptr);
+    ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, off, status);
+    ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, Giants{}, nullptr, off);
     if (g.n >= kSplitSample) {
       ECL_LAUNCH_NEXT(cc_sample<0>, dev.grid_blocks(kTPB, g.n / 8, 0), kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent,
-                 status);
-      ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, Giants{}, nullptr);
-      ECL_LAUNCH_NEXT(cc_sample<1>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
+                 off, status);
+      ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, Giants{}, nullptr, off);
+      ECL_LAUNCH_NEXT(cc_sample<1>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, off, status);
     } else {
-      ECL_LAUNCH_NEXT(cc_sample<2>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, status);
+      ECL_LAUNCH_NEXT(cc_sample<2>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, off, status);
     }
     // A union has a large component in every graph.  With one tree for all of
     // it, cc_rest had the entries of 95 of 96 graphs to look at (28 M in all):
@@ -579,26 +593,26 @@ ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, 
     const bool per_graph = uni && uni->vbase && uni->giants;
     const Giants gi = per_graph ? Giants{uni->giants, uni->vbase, uni->ngraphs} : Giants{&ctr->giant};
     ECL_LAUNCH_NEXT(cc_giant, per_graph ? uni->ngraphs : 1, 1024, 0, stream, g.n, parent, gi.vbase,
-                    per_graph ? uni->giants : &ctr->giant);
-    ECL_LAUNCH_NEXT(per_graph ? cc_flatten<kMarkUnion> : cc_flatten<kMark>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, gi, ing);
+                    per_graph ? uni->giants : &ctr->giant, off);
+    ECL_LAUNCH_NEXT(per_graph ? cc_flatten<kMarkUnion> : cc_flatten<kMark>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, gi, ing, off);
     mark();
     ECL_LAUNCH_NEXT(cc_rest, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ing, chunks, cap, bins, ctr,
-               status);
+               off, status);
     mark();
     ECL_LAUNCH_NEXT(cc_rest_chunks, grid, kTPB, 0, stream, g.n, g.nindex, g.nlist, parent, ing, chunks, cap, bins.chunk,
-               ctr, status);
+               ctr, off, status);
     mark();
-    ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, Giants{}, nullptr);
+    ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, Giants{}, nullptr, off);
     mark();
     return ECL_OK;
   }
-  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, status);
+  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, nullptr, status);
   mark();
   ECL_LAUNCH_NEXT(cc_hook, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, chunks, cap, bins, ctr, status);
   mark();
   ECL_LAUNCH_NEXT(cc_chunks, grid, kTPB, 0, stream, g.n, g.nindex, g.nlist, parent, chunks, cap, bins.chunk, ctr, status);
   mark();
-  ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, Giants{}, nullptr);
+  ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, Giants{}, nullptr, nullptr);
   mark();
   return ECL_OK;
 }
@@ -712,12 +726,12 @@ extern "C" ecl_status ecl_cc_noalloc(int32_t nodes, int32_t edges, const int32_t
   // the counters (adjacent, at the front of the array) before every solve.
   ECL_CUDA_TRY(cudaMemsetAsync(base, 0, kStatusBytes + sizeof(CCCounters), stream));
   const int grid = dev.grid_blocks(kTPB, nodes, edges);
-  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, ctr, status);
+  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, ctr, nullptr, status);
   ECL_LAUNCH_NEXT(cc_hook, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, chunks,
              chunk_capacity(edges, kCCBins.chunk), kCCBins, ctr, status);
   ECL_LAUNCH_NEXT(cc_chunks, grid, kTPB, 0, stream, nodes, nindex, nlist, label, chunks,
              chunk_capacity(edges, kCCBins.chunk), kCCBins.chunk, ctr, status);
-  ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, nodes), kTPB, 0, stream, nodes, label, Giants{}, nullptr);
+  ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, nodes), kTPB, 0, stream, nodes, label, Giants{}, nullptr, nullptr);
   Status hs{};
   ECL_CUDA_TRY(cudaMemcpyAsync(&hs, status, sizeof(hs), cudaMemcpyDeviceToHost, stream));
   ECL_CUDA_TRY(cudaStreamSynchronize(stream));

@@ -121,11 +121,12 @@ __device__ __forceinline__ bool io_raise(unsigned long long* p, unsigned long lo
 // but SCC has never relied on it, so it is checked: the sum over all entries
 // (v, u) of +h(v, u) where v < u and -h(u, v) where v > u, modulo 2^64 with a
 // 64-bit hash h of the pair, is 0 for every symmetric entry list; a list that
-// is not symmetric makes it 0 once in 2^64.  Any other sum, and the general
-// path below runs and overwrites the labels.  Measured, general -> this: 701 x
-// 1031 grid 0.37 -> 0.17 ms, a union of 32 grids of 1.1 M vertices 4.5 ms ->
-// about 0.2; an asymmetric graph that carries the flag pays for the check and
-// the union-find (R-MAT-22: 0.7 ms) and is solved as before.
+// is not symmetric makes it 0 once in 2^64.  Any other sum, and the launches of
+// the union-find leave at once and the general path below runs.  Measured,
+// general -> this: 701 x 1031 grid 0.37 -> 0.17 ms, a union of 32 grids of 1.1 M
+// vertices 4.5 ms -> about 0.2.  A directed graph that carries the flag pays for
+// the check and for launches with nothing to do: R-MAT-20 (16 M edges) 0.35 ->
+// 0.45 ms, R-MAT-16 0.18 -> 0.22.
 
 // Mixing function of splitmix64 (Steele, Lea and Flood, OOPSLA 2014).
 __device__ __forceinline__ unsigned long long scc_mix(unsigned long long x) {
@@ -302,8 +303,9 @@ __device__ __forceinline__ void merge_bits(unsigned* bits, unsigned* next, int w
 __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* __restrict__ nindex,
                                                       const int* __restrict__ nlist, unsigned* fwd, unsigned* bwd,
                                                       unsigned* next, int* queue, int* candA, int* candB, int2* chunks,
-                                                      int chunk_cap, SCCCtl* __restrict__ ctl,
+                                                      int chunk_cap, SCCCtl* __restrict__ ctl, bool checked,
                                                       Status* __restrict__ status) {
+  if (checked && ctl->asym == 0) return;  // as scc_mark
   __shared__ int s_stage[kGTPB / 32][128];
   __shared__ int s_moved;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -595,17 +597,9 @@ __device__ __forceinline__ void scc_mark_batch(const bool (&valid)[kScanBatch], 
 }
 
 template <bool kRest>
-__global__ void __launch_bounds__(kTPB) scc_mark(int n, int m, const int* __restrict__ nindex,
-                                                 const int* __restrict__ nlist, int* __restrict__ flags,
-                                                 int2* __restrict__ wl, RowChunks rc, Bins bins, bool vec,
-                                                 Giant gi, SCCCtl* __restrict__ ctl, bool checked, Status* __restrict__ status) {
-  dep_wait();
-  // nothing to do for a symmetric graph (its labels are written), and one of
-  // the two forms runs, by whether the giant component was found.  Words that
-  // nothing writes in this launch: plain loads, which L1 serves (as relaxed
-  // loads every warp of the grid queues at one L2 word: 6.4 us for 2824 blocks
-  // with nothing to do)
-  if ((checked && ctl->asym == 0) || (ctl->giant_ok != 0) != kRest) return;
+__device__ __forceinline__ void scc_mark_rows(int n, int m, const int* nindex, const int* nlist, int* flags, int2* wl,
+                                              const RowChunks& rc, const Bins& bins, bool vec, const Giant& gi,
+                                              SCCCtl* ctl, Status* status) {
   __shared__ int2 s_stage[kTPB / 32][kRest ? 128 : 1];
   WarpStage<int2, 128, true> stg{s_stage[threadIdx.x >> 5]};
   bool overflow = false;
@@ -654,13 +648,9 @@ __global__ void __launch_bounds__(kTPB) scc_mark(int n, int m, const int* __rest
 }
 
 template <bool kRest>
-__global__ void __launch_bounds__(kTPB) scc_mark_chunks(int n, int m, const int* __restrict__ nindex,
-                                                        const int* __restrict__ nlist, int* __restrict__ flags,
-                                                        int2* __restrict__ wl, RowChunks rc, int chunk, bool vec,
-                                                        Giant gi, SCCCtl* __restrict__ ctl, bool checked,
-                                                        Status* __restrict__ status) {
-  dep_wait();
-  if ((checked && ctl->asym == 0) || (ctl->giant_ok != 0) != kRest) return;  // as scc_mark
+__device__ __forceinline__ void scc_mark_records(int n, int m, const int* nindex, const int* nlist, int* flags, int2* wl,
+                                                 const RowChunks& rc, int chunk, bool vec, const Giant& gi, SCCCtl* ctl,
+                                                 Status* status) {
   __shared__ int2 s_stage[kTPB / 32][kRest ? 128 : 1];
   WarpStage<int2, 128, true> stg{s_stage[threadIdx.x >> 5]};
   bool overflow = false;
@@ -681,6 +671,38 @@ __global__ void __launch_bounds__(kTPB) scc_mark_chunks(int n, int m, const int*
     if (__any_sync(kFull, out) && lane == 0) fetch_or(&flags[r.x], kHasOut);
   }
   if (kRest) stg.flush(wl, &ctl->rest, m, overflow);
+}
+
+// kSearched: scc_giant ran before, and whether it found the component decides
+// between the two forms.  Nothing to do for a symmetric graph (its labels are
+// written).  Both words are plain loads of what nothing writes in these
+// launches, so L1 serves them (as relaxed loads every warp of the grid queues at
+// one L2 word: 6.4 us for 2824 blocks with nothing to do).
+template <bool kSearched>
+__global__ void __launch_bounds__(kTPB) scc_mark(int n, int m, const int* __restrict__ nindex,
+                                                 const int* __restrict__ nlist, int* __restrict__ flags,
+                                                 int2* __restrict__ wl, RowChunks rc, Bins bins, bool vec,
+                                                 Giant gi, SCCCtl* __restrict__ ctl, bool checked, Status* __restrict__ status) {
+  dep_wait();
+  if (checked && ctl->asym == 0) return;
+  if (kSearched && ctl->giant_ok != 0)
+    scc_mark_rows<true>(n, m, nindex, nlist, flags, wl, rc, bins, vec, gi, ctl, status);
+  else
+    scc_mark_rows<false>(n, m, nindex, nlist, flags, wl, rc, bins, vec, gi, ctl, status);
+}
+
+template <bool kSearched>
+__global__ void __launch_bounds__(kTPB) scc_mark_chunks(int n, int m, const int* __restrict__ nindex,
+                                                        const int* __restrict__ nlist, int* __restrict__ flags,
+                                                        int2* __restrict__ wl, RowChunks rc, int chunk, bool vec,
+                                                        Giant gi, SCCCtl* __restrict__ ctl, bool checked,
+                                                        Status* __restrict__ status) {
+  dep_wait();
+  if (checked && ctl->asym == 0) return;
+  if (kSearched && ctl->giant_ok != 0)
+    scc_mark_records<true>(n, m, nindex, nlist, flags, wl, rc, chunk, vec, gi, ctl, status);
+  else
+    scc_mark_records<false>(n, m, nindex, nlist, flags, wl, rc, chunk, vec, gi, ctl, status);
 }
 
 // Word of a trimmed vertex: it is its own SCC, and sweeps skip its edges.
@@ -939,10 +961,8 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
   // a graph flagged symmetric may be solved as connected components (not when
   // the caller limits the rounds: that limit is the general path's)
   const bool check = (g.flags & ECL_GRAPH_SYMMETRIC) != 0 && max_rounds <= 0;
-  // (the same limit; and a flagged graph that is what its flag says needs no
-  // propagation: the search and the second form of the mark passes would be
-  // three launches that leave at once, 8 us on a mesh of 0.7 M vertices)
-  const bool giant = max_rounds <= 0 && !check && g.m >= kGiantEntries;
+  // (the same limit; a flagged graph that is what its flag says leaves the search at once)
+  const bool giant = max_rounds <= 0 && g.m >= kGiantEntries;
   if (max_rounds <= 0 || max_rounds > b.max_rounds) max_rounds = b.max_rounds;
 
   fill_ranges({{b.ctl, sizeof(SCCCtl), 0},
@@ -961,7 +981,7 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
       ECL_LAUNCH_NEXT(scc_symmetry, dev.grid_blocks(kTPB, 0, g.m), kTPB, 0, stream,
                  FlatCsr{g.n, g.m, g.nindex, g.nlist, b.tilerow}, (reinterpret_cast<uintptr_t>(g.nlist) & 15) == 0, b.ctl,
                  status);
-    const ecl_status st = cc_enqueue(g, label, b.cc_ws, status, dev, stream, {}, uni);
+    const ecl_status st = cc_enqueue(g, label, b.cc_ws, status, dev, stream, {}, uni, &b.ctl->asym);
     if (st != ECL_OK) return st;
     // (the general path's flags stay zero when the graph is not symmetric)
     ECL_LAUNCH_NEXT(scc_top, dev.sms * 4, kTPB, 0, stream, g.n, label, b.flags, b.ctl);
@@ -977,18 +997,12 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
     const int blocks = std::max(1, std::min(dev.sms * gocc, (int)(std::max((long long)g.n, (long long)g.m / 4) / kGTPB)));
     ECL_CUDA_TRY(launch_cooperative(scc_giant, blocks, kGTPB, stream, g.n, g.m, g.nindex, g.nlist, gi.fwd, gi.bwd,
                                     b.bits + 2 * words, b.queue, b.candA, b.candB, b.chunks, (int)row_chunk_capacity(g.m, kMinChunk), b.ctl,
-                                    status));
+                                    check, status));
   }
-  ECL_LAUNCH_NEXT(scc_mark<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, gi,
-             b.ctl, check, status);
-  ECL_LAUNCH_NEXT(scc_mark_chunks<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins.chunk,
-             vec, gi, b.ctl, check, status);
-  if (giant) {
-    ECL_LAUNCH_NEXT(scc_mark<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins, vec, gi,
-               b.ctl, false, status);
-    ECL_LAUNCH_NEXT(scc_mark_chunks<true>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags, b.wlA, rc, bins.chunk,
-               vec, gi, b.ctl, false, status);
-  }
+  ECL_LAUNCH_NEXT(giant ? scc_mark<true> : scc_mark<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags,
+                  b.wlA, rc, bins, vec, gi, b.ctl, check, status);
+  ECL_LAUNCH_NEXT(giant ? scc_mark_chunks<true> : scc_mark_chunks<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex,
+                  g.nlist, b.flags, b.wlA, rc, bins.chunk, vec, gi, b.ctl, check, status);
   mark();
   ECL_CUDA_TRY(launch_cooperative(solve, coop_grid, kTPB, stream, g.n, g.m, b.wlA, b.wlB, b.flags, b.io, label, gi,
                                   b.ctl, max_rounds, check, status));

@@ -46,8 +46,11 @@ size_t gc_workspace_bytes(int n, int m);
 size_t mst_workspace_bytes(int n, int m);
 size_t scc_workspace_bytes(int n, int m);
 
+// `off` (symmetric graphs): a device word that launches before these write; not
+// 0: the solve is not wanted, and its launches leave at once.
 ecl_status cc_enqueue(const GraphDev& g, int* label, char* ws, dev::Status* status, const DeviceInfo& dev,
-                      cudaStream_t stream, Marker mark = {}, const UnionInfo* uni = nullptr);
+                      cudaStream_t stream, Marker mark = {}, const UnionInfo* uni = nullptr,
+                      const unsigned long long* off = nullptr);
 ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, dev::Status* status, const DeviceInfo& dev,
                        cudaStream_t stream, int max_sweeps, const UnionInfo* uni = nullptr, Marker mark = {});
 ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, dev::Status* status, const DeviceInfo& dev,

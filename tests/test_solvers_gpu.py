@@ -668,6 +668,16 @@ def test_scc_reports_the_rounds_it_took(ecl, flagged):
         assert o.rounds >= 1
 
 
+@pytest.mark.parametrize("scale", [16, 20])
+def test_scc_of_a_directed_graph_flagged_symmetric_costs_the_check_alone(ecl, orc, scale):
+    """The flag is checked before anything is made of it: a directed graph that
+    carries it is solved as one that does not."""
+    g = ecl.gen_rmat(scale, 16, seed=6, symmetrise=False)
+    plain, flagged = (ecl.Graph(g.nindex, g.nlist, None, f).to_device() for f in (False, True))
+    assert np.array_equal(ecl.scc(flagged).cpu().numpy(), orc.scc(g))
+    assert best_ms(ecl, flagged, "scc") < 1.25 * best_ms(ecl, plain, "scc") + 0.04
+
+
 def long_distance_cases(ecl):
     """Directed graphs of a million entries and more in which the search for a
     giant component takes long or finds nothing."""
