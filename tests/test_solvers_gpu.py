@@ -678,6 +678,17 @@ def test_scc_of_a_directed_graph_flagged_symmetric_costs_the_check_alone(ecl, or
     assert best_ms(ecl, flagged, "scc") < 1.25 * best_ms(ecl, plain, "scc") + 0.04
 
 
+@pytest.mark.parametrize("pairs", [3, 1000, 499, 500, 501])  # (4000 vertices: around a quarter as many entries)
+def test_scc_of_flagged_graphs_with_hardly_any_entries(ecl, orc, pairs):
+    n = 1 << 22 if pairs == 3 else 4000
+    u = 2 * np.arange(pairs) + n // 3
+    g = directed(ecl, n, np.concatenate([u, u + 1]), np.concatenate([u + 1, u]))
+    plain, flagged = (ecl.Graph(g.nindex, g.nlist, None, f).to_device() for f in (False, True))
+    assert np.array_equal(ecl.scc(flagged).cpu().numpy(), orc.scc(g))
+    if n > 4000:
+        assert best_ms(ecl, flagged, "scc") < 1.15 * best_ms(ecl, plain, "scc") + 0.01
+
+
 def long_distance_cases(ecl):
     """Directed graphs of a million entries and more in which the search for a
     giant component takes long or finds nothing."""
