@@ -511,8 +511,9 @@ __device__ int gc_short_row(int beg, int h, const int* nl2, const int* color, St
 // pull achieves it); in shared memory it costs a few hundred cycles.  So the
 // first `core` ranks (core = min(long rows, cap)) are coloured by a cluster
 // of CTAs of 32 warps each (two by default) with the colours in shared
-// memory, indexed by rank -- a copy in every CTA, each colour stored into all
-// copies through distributed shared memory: every higher-priority entry of a
+// memory, indexed by rank -- a copy in every CTA, each colour stored into its own
+// CTA's directly and into the others' through distributed shared memory (its own
+// that way too: 45 ns more a hop): every higher-priority entry of a
 // core row is itself a core vertex (it has a smaller rank), so a core row
 // never waits on global memory.  Two small launches first rewrite
 // the core rows' entries in nl2 from vertex ids to ranks (rank[] is the
@@ -532,19 +533,29 @@ __device__ int gc_short_row(int beg, int h, const int* nl2, const int* color, St
 // test -- undecided and far colours go to a byte that nobody reads -- and keeps
 // the undecided entries in a 32-bit mask.  A byte store needs no atomic: lanes
 // that mark the same colour store the same value.
+//
+// On the chain lies what a warp does between its last neighbour's colour and its
+// own, among 31 other warps' polls.  So all of a row is scanned before any wait
+// (two segments; a longer row's third behind them), the search for the smallest
+// colour starts where it ended before the wait, and the marks are cleared and the
+// next row fetched behind the publication.  Measured, core, a lane polling its
+// lowest entry after each segment, 1016 colours a window and the search from 0 ->
+// this: R-MAT-22 1.35 -> 1.21 ms, R-MAT-16 0.53 -> 0.49, a clique of 1000 vertices
+// 0.91 -> 0.59, of 2000 12.5 -> 1.3, a complete bipartite graph of 2 x 2000 2.6 -> 1.45.
 constexpr int kCoreThreads = 1024;
 constexpr int kCoreWarps = kCoreThreads / 32;
 // Default CTAs of the core's cluster.  A hop between CTAs, through distributed
 // shared memory, costs more than one inside a CTA.  R-MAT-22, core time by
-// CTAs (8192 ranks): 1: 1.59 ms, 2: 1.43, 4: 1.73; core + pull by ranks (2
-// CTAs): 4096: 2.90 ms, 8192: 2.54, 16384: 2.67, 32768: 3.23.
+// CTAs (8192 ranks): 1: 1.50 ms, 2: 1.21, 4: 1.20; core + pull by ranks (2
+// CTAs): 4096: 2.55 ms, 8192: 2.22, 16384: 2.38, 32768: 3.05.
 constexpr int kCoreCtas = 2;
 constexpr int kCoreDefault = 8192;      // default core size (ranks): the measured best at R-MAT-22 with 2 CTAs
 constexpr int kCoreMax = 36864;         // shared memory bound
 constexpr int kSegMax = 1024;           // entries per segment: a bit each of a lane's 32-bit mask
 constexpr unsigned kUncoloured = 0xffffu;
-constexpr int kWin = 1016;              // colours of a mark window; the bytes up to kMarkBytes take what is outside
-constexpr int kMarkBytes = 1024;
+constexpr int kWin = 2032;              // colours of a mark window; a byte behind it takes what is outside
+constexpr int kMarkBytes = 2048;
+constexpr int kFromRow = 512;           // rows from which on the search starts ahead (a shorter row's marks are one load)
 constexpr size_t kCoreSmemLimit = 227 * 1024;
 
 // Dynamic shared memory of a core CTA: colours (16-bit, per rank), then per
@@ -654,11 +665,13 @@ __device__ __forceinline__ unsigned cluster_ctas() {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
-// Stores colour v of the rank at p (a local shared address) into the copy of
-// every CTA of the cluster.
+// Stores colour v of the rank at p (a local shared address) into this CTA's copy
+// and into that of every other CTA of the cluster.
 __device__ __forceinline__ void col_publish(unsigned short* p, unsigned v, int ctas) {
-  const unsigned local = smem_u32(p);
+  col_st(p, v);
+  const unsigned local = smem_u32(p), me = cluster_rank();
   for (int k = 0; k < ctas; k++) {
+    if (k == (int)me) continue;
     unsigned remote;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(k));
     asm volatile("st.relaxed.cluster.shared::cluster.u16 [%0], %1;" ::"r"(remote), "h"((unsigned short)v) : "memory");
@@ -699,39 +712,72 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
 }
 
 // The smallest colour of the window at `off` that the warp's marks leave free,
-// or -1; clears the marks.  All lanes call, behind a __syncwarp.
-__device__ __forceinline__ int gc_core_mex(unsigned char* marks, int off) {
+// or -1, with all below `start` known to be taken; `end` is the last byte that
+// may be set.  128 bytes a ballot, the loads of four of them in flight.  All
+// lanes call, behind a __syncwarp.
+__device__ __forceinline__ int gc_core_mex(const unsigned char* marks, int off, int start, int end) {
   const int lane = threadIdx.x & 31;
-  int c = -1;
-  for (int i = 0; i < kMarkBytes / 128; i++) {
-    const unsigned w = reinterpret_cast<const unsigned*>(marks)[32 * i + lane];
-    unsigned z = (w - 0x01010101u) & ~w & 0x80808080u;  // lowest set bit: the lowest zero byte
-    if (128 * i + 4 * lane >= kWin) z = 0;              // kWin is a multiple of 4
-    const unsigned f = __ballot_sync(kFull, z != 0);
-    if (f) {
-      const int who = __ffs(f) - 1;
-      c = off + 128 * i + 4 * who + ((__ffs(__shfl_sync(kFull, z, who)) - 1) >> 3);
-      break;
+  for (int i0 = start & ~127; i0 <= end; i0 += 512) {
+    unsigned w[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int i = i0 + 128 * k + 4 * lane;
+      w[k] = i < kWin ? *reinterpret_cast<const unsigned*>(marks + i) : ~0u;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const unsigned z = (w[k] - 0x01010101u) & ~w[k] & 0x80808080u;  // lowest set bit: the lowest zero byte
+      const unsigned f = __ballot_sync(kFull, z != 0);
+      if (f) {
+        const int who = __ffs(f) - 1;
+        return off + i0 + 128 * k + 4 * who + ((__ffs(__shfl_sync(kFull, z, who)) - 1) >> 3);
+      }
     }
   }
+  return -1;
+}
+static_assert(kWin % 4 == 0 && kWin < kMarkBytes && kMarkBytes % 512 == 0, "gc_core_mex and gc_core_clear");
+
+// Clears the marks up to byte `end`.  All lanes call.
+__device__ __forceinline__ void gc_core_clear(unsigned char* marks, int end) {
+  for (int i0 = 0; i0 <= end; i0 += 512)
+    reinterpret_cast<uint4*>(marks + i0)[threadIdx.x & 31] = make_uint4(0u, 0u, 0u, 0u);
   __syncwarp();
-  uint4* m4 = reinterpret_cast<uint4*>(marks) + 2 * lane;
-  m4[0] = m4[1] = make_uint4(0u, 0u, 0u, 0u);
-  __syncwarp();
-  return c;
 }
 
-// Colour of a core row of `h` ranks at `row` whose first kWin colours are all
-// taken by its neighbours; every neighbour is coloured by now.
+// Colour of a core row of `h` ranks at `row` (16-byte aligned) whose first kWin
+// colours are all taken by its neighbours; every neighbour is coloured by now.
+// The row is read again for each window, 1024 entries in flight: this lies on
+// the chain of a clique's colours (32 entries at a time, and windows of 1016: a
+// clique of 5000 vertices 166 ms; so: 47).
 __device__ int gc_core_far(const unsigned short* row, int h, const unsigned short* col_s, unsigned char* marks) {
   const int lane = threadIdx.x & 31;
+  const uint4* rv = reinterpret_cast<const uint4*>(row);
+  constexpr int kFlight = 4;
   for (int off = kWin;; off += kWin) {
-    for (int i = lane; i < h; i += 32) {
-      const int d = (int)col_ld(&col_s[__ldg(&row[i])]) - off;
-      if (d >= 0 && d < kWin) marks[d] = 1;
+    gc_core_clear(marks, kWin - 1);
+    for (int i0 = 8 * lane; i0 < h; i0 += 256 * kFlight) {
+      uint4 x[kFlight];
+#pragma unroll
+      for (int s = 0; s < kFlight; s++) {
+        const int e = i0 + 256 * s;
+        x[s] = e < h ? __ldg(&rv[e >> 3]) : make_uint4(0u, 0u, 0u, 0u);  // up to 7 entries of the slot past the row
+      }
+#pragma unroll
+      for (int s = 0; s < kFlight; s++) {
+        const int e = i0 + 256 * s;
+        const unsigned w[4] = {x[s].x, x[s].y, x[s].z, x[s].w};
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          if (e + k >= h) continue;
+          const int d = (int)col_ld(&col_s[(k & 1) ? w[k >> 1] >> 16 : w[k >> 1] & 0xffffu]) - off;
+          if (d >= 0 && d < kWin) marks[d] = 1;
+        }
+      }
     }
     __syncwarp();
-    const int c = gc_core_mex(marks, off);
+    const int c = gc_core_mex(marks, off, 0, kWin - 1);
+    __syncwarp();  // read before they are cleared
     if (c >= 0) return c;
   }
 }
@@ -741,29 +787,33 @@ __device__ int gc_core_far(const unsigned short* row, int h, const unsigned shor
 // packed rows and has at most the buffer's entries; the copy is rounded up to
 // 16 bytes (the row's slot has room).
 struct CoreStage {
-  unsigned short* buf[2];
-  unsigned long long* bar[2];
-  unsigned parity[2] = {0u, 0u};
-  int first[2] = {-1, -1};  // segment in each buffer (-1: none in flight)
+  unsigned short* base;        // the buffers, `seg` entries each
+  unsigned long long* bars;
+  int seg;
+  unsigned parity = 0;         // bit b: of buffer b's next phase
+  int first0 = -1, first1 = -1;  // segment in each buffer (-1: none in flight)
 
+  // (no arrays: indexed by b they would live in local memory, whose loads lay on
+  // the chain)
+  __device__ __forceinline__ unsigned short* buf(int b) const { return base + (b ? seg : 0); }
+  __device__ __forceinline__ int first(int b) const { return b ? first1 : first0; }
+  __device__ __forceinline__ void set_first(int b, int unit) { (b ? first1 : first0) = unit; }
   __device__ __forceinline__ void issue(int b, const int* nl2, int unit, int len) {
-    first[b] = unit;
+    set_first(b, unit);
     if ((threadIdx.x & 31) == 0)
-      bulk_load(buf[b], reinterpret_cast<const char*>(nl2) + (size_t)unit * 16, (2u * (unsigned)len + 15u) & ~15u, bar[b]);
+      bulk_load(buf(b), reinterpret_cast<const char*>(nl2) + (size_t)unit * 16, (2u * (unsigned)len + 15u) & ~15u, bars + b);
   }
   // Waits for buffer b's copy.  False when the wait ran out.
   __device__ __forceinline__ bool wait(int b) {
-    const bool ok = mbar_wait(bar[b], parity[b]);
-    if (ok) parity[b] ^= 1u;  // a copy that did not land stays listed for drain()
+    const bool ok = mbar_wait(bars + b, (parity >> b) & 1u);
+    if (ok) parity ^= 1u << b;  // a copy that did not land stays listed for drain()
     return ok;
   }
   // Bounded wait for every copy still in flight (before leaving on an error).
   __device__ __forceinline__ void drain() {
-    for (int b = 0; b < 2; b++)
-      if (first[b] >= 0) {
-        if (mbar_wait(bar[b], parity[b])) parity[b] ^= 1u;
-        first[b] = -1;
-      }
+    if (first0 >= 0) wait(0);
+    if (first1 >= 0) wait(1);
+    first0 = first1 = -1;
   }
 };
 
@@ -793,16 +843,15 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* __restrict
   const int seg = gc_core_seg(cap);  // row entries staged at a time
   unsigned char* wbase = s_core + gc_core_colour_bytes(cap) + (size_t)(threadIdx.x >> 5) * gc_core_warp_bytes(seg);
   CoreStage stg;
-  stg.bar[0] = reinterpret_cast<unsigned long long*>(wbase);
-  stg.bar[1] = stg.bar[0] + 1;
-  stg.buf[0] = reinterpret_cast<unsigned short*>(wbase + 2 * sizeof(unsigned long long));
-  stg.buf[1] = stg.buf[0] + seg;
-  unsigned char* marks = reinterpret_cast<unsigned char*>(stg.buf[1] + seg);
+  stg.bars = reinterpret_cast<unsigned long long*>(wbase);
+  stg.base = reinterpret_cast<unsigned short*>(wbase + 2 * sizeof(unsigned long long));
+  stg.seg = seg;
+  unsigned char* marks = reinterpret_cast<unsigned char*>(stg.base + 2 * seg);
   for (int r = threadIdx.x; r < core; r += kCoreThreads) col_st(&col_s[r], kUncoloured);
-  reinterpret_cast<uint4*>(marks)[2 * lane] = reinterpret_cast<uint4*>(marks)[2 * lane + 1] = make_uint4(0u, 0u, 0u, 0u);
+  gc_core_clear(marks, kMarkBytes - 1);
   if (lane == 0) {
-    mbar_init(stg.bar[0]);
-    mbar_init(stg.bar[1]);
+    mbar_init(stg.bars);
+    mbar_init(stg.bars + 1);
     mbar_fence_init();
   }
   __syncthreads();
@@ -822,10 +871,13 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* __restrict
     return make_int4(__shfl_sync(kFull, rec.x, src), __shfl_sync(kFull, rec.y, src), __shfl_sync(kFull, rec.z, src),
                      0);
   };
+  // Byte that takes the colours which cannot matter: h entries leave one of the
+  // colours 0 .. h free.  So a row marks, searches and clears h + 2 bytes at most.
+  unsigned beyond = 0;
   // looks entry e of the staged segment up; true when it is undecided
   auto look = [&](unsigned q) -> bool {
     const unsigned c = col_ld(&col_s[q]);
-    marks[min(c, (unsigned)kWin)] = 1;
+    marks[min(c, beyond)] = 1;
     return c == kUncoloured;
   };
   const int nrows = core > warp ? (core - warp + cwarps - 1) / cwarps : 0;
@@ -834,68 +886,90 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* __restrict
     const int r = warp + cwarps * j;
     const int4 row = row_of(j);
     const int unit = row.x, h = row.y, v = row.z;
+    beyond = (unsigned)min(h + 1, kWin);
+    // The first segment of the warp's next row with entries into buffer q (rows
+    // without any are skipped).
+    auto next_row = [&](int q) {
+      for (int jn = j + 1; jn < nrows; jn++) {
+        const int4 nx = row_of(jn);
+        if (nx.y > 0) {
+          stg.issue(q, nl2, nx.x, min(seg, nx.y));
+          return;
+        }
+      }
+    };
     bool stalled = false;
-    for (int off = 0; off < h && !stalled; off += seg) {
-      const int f = unit + off / 8, l = min(seg, h - off);
-      if (stg.first[b] != f) stg.issue(b, nl2, f, l);  // not prefetched
-      // prefetch what comes next: this row's next segment, or the first one
-      // of the warp's next row with entries (rows without any are skipped)
+    int from = 0;  // all colours below are taken
+    // Two segments at a time are scanned before any undecided entry is waited for:
+    // a scan behind the last neighbour's colour would lie on the chain, and costs
+    // microseconds among the other warps' polls.
+    for (int off = 0; off < h && !stalled; off += 2 * seg) {
+      const int f = unit + off / 8, second = h - off - seg;  // entries behind the first of the two
+      if (stg.first(b) != f) stg.issue(b, nl2, f, min(seg, h - off));  // not prefetched
       __syncwarp();  // buffer b ^ 1 was scanned by every lane
-      if (off + seg < h) {
-        stg.issue(b ^ 1, nl2, f + seg / 8, min(seg, h - off - seg));
-      } else {
-        for (int jn = j + 1; jn < nrows; jn++) {
-          const int4 nx = row_of(jn);
-          if (nx.y > 0) {
-            stg.issue(b ^ 1, nl2, nx.x, min(seg, nx.y));
-            break;
-          }
+      if (second > 0)
+        stg.issue(b ^ 1, nl2, f + seg / 8, min(seg, second));
+      else
+        next_row(b ^ 1);
+      unsigned open0 = 0, open1 = 0;
+      for (int part = 0; part <= (second > 0); part++) {
+        const int q = b ^ part, l = min(seg, h - off - part * seg);
+        if (!__all_sync(kFull, stg.wait(q))) {  // every lane polls; the verdict is the warp's
+          raise(status, ECL_ERR_NO_CONVERGENCE, r);
+          stalled = true;
+          break;
         }
-      }
-      if (!__all_sync(kFull, stg.wait(b))) {  // every lane polls; the verdict is the warp's
-        raise(status, ECL_ERR_NO_CONVERGENCE, r);
-        stalled = true;
-        break;
-      }
-      stg.first[b] = -1;
-      const unsigned short* sg = stg.buf[b];
-      // eight entries a lane and step; bit 8 s + k of `wait`: entry k of the
-      // lane's step s is undecided
-      unsigned wait = 0;
-      const uint4* sv = reinterpret_cast<const uint4*>(sg);
-      for (int s = 0; 256 * s < l; s++) {
-        const int e = 256 * s + 8 * lane;
-        unsigned undecided = 0;
-        if (e + 8 <= l) {
-          const uint4 x = sv[32 * s + lane];
-          const unsigned w[4] = {x.x, x.y, x.z, x.w};
-          unsigned c[8];
+        stg.set_first(q, -1);
+        const unsigned short* sg = stg.buf(q);
+        // eight entries a lane and step; bit 8 s + k of `wait`: entry k of the
+        // lane's step s is undecided
+        unsigned wait = 0;
+        const uint4* sv = reinterpret_cast<const uint4*>(sg);
+        for (int s = 0; 256 * s < l; s++) {
+          const int e = 256 * s + 8 * lane;
+          unsigned undecided = 0;
+          if (e + 8 <= l) {
+            const uint4 x = sv[32 * s + lane];
+            const unsigned w[4] = {x.x, x.y, x.z, x.w};
+            unsigned c[8];
 #pragma unroll
-          for (int k = 0; k < 8; k++) c[k] = col_ld(&col_s[(k & 1) ? w[k >> 1] >> 16 : w[k >> 1] & 0xffffu]);
+            for (int k = 0; k < 8; k++) c[k] = col_ld(&col_s[(k & 1) ? w[k >> 1] >> 16 : w[k >> 1] & 0xffffu]);
 #pragma unroll
-          for (int k = 0; k < 8; k++) {
-            marks[min(c[k], (unsigned)kWin)] = 1;
-            undecided |= c[k] == kUncoloured ? 1u << k : 0u;
+            for (int k = 0; k < 8; k++) {
+              marks[min(c[k], beyond)] = 1;
+              undecided |= c[k] == kUncoloured ? 1u << k : 0u;
+            }
+          } else {
+            for (int k = 0; e + k < l; k++) undecided |= look(sg[e + k]) ? 1u << k : 0u;
           }
-        } else {
-          for (int k = 0; e + k < l; k++) undecided |= look(sg[e + k]) ? 1u << k : 0u;
+          wait |= undecided << (8 * s);
         }
-        wait |= undecided << (8 * s);
+        if (part)
+          open1 = wait;
+        else
+          open0 = wait;
       }
-      // Wait for the undecided ones: a lane polls its lowest, on its own and in
-      // as few instructions as can be.  The polls of 32 warps share one
-      // shared-memory pipe, and all the loop does comes on top of every hop of
-      // the chain (R-MAT-22: 1.40 ms; two entries a lane at a time 1.48, four
-      // 1.94, naps of 16 to 100 ns 1.49 to 1.53; scanning the warp's next row
-      // first 1.99, which doubles the undecided entries of that row).
-      unsigned spins = 0;
+      // Wait for the undecided ones: a lane goes round its own and takes whichever
+      // is decided, so that none holds up the others.  (R-MAT-22, core: the ranks
+      // in a list that the lanes share evenly, and the colours handed to registers
+      // by votes and shuffles, 1.39 ms, with naps of 40 to 100 ns 1.47; this 1.21.)
+      unsigned spins = 0, turn = 0;
       unsigned long long t0 = 0;
-      while (wait) {
-        const int k = __ffs(wait) - 1;
-        const unsigned short* p = &col_s[sg[256 * (k >> 3) + 8 * lane + (k & 7)]];
-        unsigned c;
-        while ((c = col_ld(p)) == kUncoloured) {
-          if ((++spins & 1023u) == 0) {
+      __syncwarp();
+      if (h >= kFromRow) from = gc_core_mex(marks, 0, from, (int)beyond);
+      if (from < 0) from = kWin;
+      for (int part = 0; part <= (second > 0) && !stalled; part++) {
+        const unsigned short* sg = stg.buf(b ^ part);
+        unsigned wait = part ? open1 : open0;
+        while (wait) {
+          const unsigned behind = wait & ~((1u << turn) - 1u);
+          const int k = __ffs(behind ? behind : wait) - 1;
+          const unsigned c = col_ld(&col_s[sg[256 * (k >> 3) + 8 * lane + (k & 7)]]);
+          turn = (k + 1) & 31;
+          if (c != kUncoloured) {
+            marks[min(c, beyond)] = 1;
+            wait &= ~(1u << k);
+          } else if ((++spins & 1023u) == 0) {
             if (t0 == 0) t0 = gc_now();
             if (gc_now() - t0 > kStallNs || ld(&status->code) != 0) {
               raise(status, ECL_ERR_NO_CONVERGENCE, r);
@@ -904,25 +978,28 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* __restrict
             }
           }
         }
-        if (stalled) break;
-        marks[min(c, (unsigned)kWin)] = 1;
-        wait &= wait - 1;
       }
       stalled = __any_sync(kFull, stalled);
-      b ^= 1;
+      if (second <= 0)
+        b ^= 1;
+      else if (second > seg && !stalled)
+        stg.issue(b, nl2, f + seg / 4, min(seg, second - seg));
     }
     if (stalled) {
       stg.drain();
       break;
     }
     __syncwarp();
-    int c = gc_core_mex(marks, 0);
+    int c = gc_core_mex(marks, 0, from, (int)beyond);
     if (c < 0) c = gc_core_far(reinterpret_cast<const unsigned short*>(nl2) + (size_t)unit * 8, h, col_s, marks);
     if (lane == 0) {
       col_publish(&col_s[r], (unsigned)c, ctas);
       st(&color[v], c);
     }
     __syncwarp();
+    // behind the publication, off the chain
+    gc_core_clear(marks, (int)beyond);
+    if (h > 0 && (h - 1) / seg % 2 == 1) next_row(b);  // both buffers were the row's own
   }
   // a CTA's shared memory must outlive every store the others make into it:
   // every warp, done or given up (each wait is bounded), meets here

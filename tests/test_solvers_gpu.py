@@ -718,6 +718,29 @@ def test_scc_search_for_a_giant_component_gives_up_in_time(ecl, orc):
         assert best_ms(ecl, dg, "scc") < 1.25 * best_ms(ecl, dg, "scc", max_rounds=g.nodes + 1) + 0.03, name
 
 
+def clique(ecl, n, extra=0):
+    """All pairs of n vertices; vertices n .. n + extra - 1 on a path behind them."""
+    u, v = np.triu_indices(n, 1)
+    w = n - 1 + np.arange(extra)
+    u, v = np.concatenate([u, w]), np.concatenate([v, w + 1])
+    return directed(ecl, n + extra, np.concatenate([u, v]), np.concatenate([v, u]))
+
+
+@pytest.mark.parametrize("n", [33, 511, 513, 1015, 1017, 2030, 2031, 2032, 2033, 2034, 2035, 2049, 4064, 4066, 5000])
+def test_gc_of_cliques_around_the_windows_of_colours(ecl, orc, n):
+    """A clique needs as many colours as it has vertices: rows whose colour lies
+    at the ends of the core's windows (of 2032 colours) and past the second."""
+    g = clique(ecl, n, extra=n % 7)
+    for d in (g, ecl.Graph(g.nindex, g.nlist, None, True)):
+        assert np.array_equal(ecl.gc(d), orc.gc(g))
+
+
+def test_gc_of_cliques_costs_a_hop_for_each_colour(ecl):
+    """Twice the vertices are twice the hops, not eighteen times the time."""
+    small, large = (best_ms(ecl, clique(ecl, n).to_device(), "gc") for n in (1000, 2000))
+    assert large < 4 * small
+
+
 @pytest.mark.parametrize("n", [1025, 65537, (1 << 20) - 1, (1 << 20) + 1025])
 def test_gc_order_of_equal_degrees(ecl, orc, n):
     """One degree for all vertices: the sort's left-out digits decide between
