@@ -22,7 +22,8 @@
 //    the blocker.  No entry is scanned twice: one that was passed is out, or
 //    outranked and cannot join before the vertex is decided.  Lists of <= 16
 //    entries are scanned by their own lane; longer ones, from the second sweep
-//    on, 128 entries per step by the whole warp; a joining vertex claims itself with one CAS, then clears
+//    on, 128 entries per step by the whole warp (up to 32 entries by their lanes
+//    too, where many of the warp have as many); a joining vertex claims itself with one CAS, then clears
 //    its neighbours' bytes (fetch_and);
 //  * a self-loop (the reference spins forever on one: v never outranks
 //    itself) raises ECL_ERR_BAD_GRAPH when it is met; a sweep cap turns any
@@ -41,6 +42,11 @@ constexpr int kTPB = 256;
 // sweep; longer ones wait for the second (a launch knob).  R-MAT-22, mis_run,
 // 32 / 16 / 8: 350 / 297 / 352 us; G(3 M, 24 M): 279 / 287 / 488.
 constexpr int kLaneMax = 16;
+// Lanes of a warp with lists of 17 to 32 entries from which on they scan them
+// themselves.  Never / 4 / 8 / always: 20 k vertices in a row with 20 leaves each
+// 46 / 32 / 33 / 32 us, G(3 M, 36 M) 439 / 371 / 367 / 377, R-MAT-22 320 / 331 /
+// 323 / 341.
+constexpr int kManyMid = 8;
 constexpr int kBatch = 4;  // list entries per lane whose loads are issued together
 constexpr unsigned kIn = 0xfe;
 
@@ -224,7 +230,11 @@ __global__ void __launch_bounds__(kTPB) mis_run(int n, int m, const int* __restr
   // verdicts out and keeps the waiting ones.  All lanes call.
   auto advance = [&](bool go, bool wait, int v, unsigned b, int pos, int end, int blocker) {
     int verdict = kWait;
-    const bool big = go && end - pos > lane_max;
+    // a list of up to twice as many entries by the whole warp, or, where kManyMid
+    // lanes of the warp have one, each by its own lane
+    const bool mid = go && end - pos > lane_max && end - pos <= 2 * lane_max;
+    const bool many = __popc(__ballot_sync(kFull, mid)) >= kManyMid;
+    const bool big = go && end - pos > lane_max && !(mid && many);
     if (go && !big) {
       verdict = mis_scan_lane(v, b, pos, end, n, nlist, st4, &blocker, status);
     }

@@ -718,6 +718,30 @@ def test_scc_search_for_a_giant_component_gives_up_in_time(ecl, orc):
         assert best_ms(ecl, dg, "scc") < 1.25 * best_ms(ecl, dg, "scc", max_rounds=g.nodes + 1) + 0.03, name
 
 
+def caterpillar(ecl, spine, leaves):
+    """A path of `spine` vertices with `leaves` vertices of degree one at each."""
+    s = np.arange(spine)
+    u = np.concatenate([s[:-1], np.repeat(s, leaves)])
+    v = np.concatenate([s[1:], spine + np.arange(spine * leaves)])
+    g = directed(ecl, spine * (leaves + 1), np.concatenate([u, v]), np.concatenate([v, u]))
+    g.symmetric = True
+    return g
+
+
+@pytest.mark.parametrize("leaves", [13, 14, 15, 22, 29, 30, 31])  # lists of up to 16, 17, 32 and 33 entries
+@pytest.mark.parametrize("spine", [7, 8, 39, 40, 1000])  # lanes of a warp that have one, around 8
+def test_mis_lists_of_middle_length(ecl, orc, spine, leaves):
+    g = caterpillar(ecl, spine, leaves)
+    assert np.array_equal(ecl.mis(g), orc.mis(g))
+
+
+def test_mis_lists_of_middle_length_are_scanned_side_by_side(ecl):
+    """Lists of 22 entries in all lanes cost little more than lists of 16 (one
+    after another by the whole warp: 1.8 times as much)."""
+    short, middle = (best_ms(ecl, caterpillar(ecl, 20000, k).to_device(), "mis") for k in (14, 20))
+    assert middle < 1.6 * short
+
+
 def clique(ecl, n, extra=0):
     """All pairs of n vertices; vertices n .. n + extra - 1 on a path behind them."""
     u, v = np.triu_indices(n, 1)
