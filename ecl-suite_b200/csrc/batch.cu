@@ -187,7 +187,7 @@ ecl_status enqueue_run(ecl_batch* b) {
       st = cc_enqueue(g, s.cc, s.ws, stat(0), dev, b->stream, {}, &uni);
       if (st == ECL_OK) local(s.cc);
     }
-    if (st == ECL_OK && (b->codes & ECL_BATCH_MIS)) st = mis_enqueue(g, s.mis, s.ws, stat(1), dev, b->stream, 1 << 22, &uni);
+    if (st == ECL_OK && (b->codes & ECL_BATCH_MIS)) st = mis_enqueue(g, s.mis, s.ws, mis_workspace_bytes(s.n, s.m), stat(1), dev, b->stream, 1 << 22, &uni);
     if (st == ECL_OK && (b->codes & ECL_BATCH_GC)) st = gc_enqueue(g, s.gc, s.ws, stat(2), dev, b->stream, &uni);
     if (st == ECL_OK && (b->codes & ECL_BATCH_MST)) {
       st = mst_enqueue(g, s.mst, s.ws, stat(3), dev, b->stream, nullptr);
@@ -386,7 +386,7 @@ ecl_status ecl_batch_build(ecl_batch* b, uint32_t codes, int64_t max_entries, vo
     size_t wsb = 0;
     if (codes & ECL_BATCH_CC) wsb = std::max(wsb, cc_workspace_bytes(s.n, s.m));
     if (codes & ECL_BATCH_MIS) wsb = std::max(wsb, mis_workspace_bytes(s.n, s.m));
-    if (codes & ECL_BATCH_GC) wsb = std::max(wsb, gc_workspace_bytes(s.n, s.m));
+    if (codes & ECL_BATCH_GC) wsb = std::max(wsb, gc_workspace_bytes(s.n, s.m, true));
     if (codes & ECL_BATCH_MST) wsb = std::max(wsb, mst_workspace_bytes(s.n, s.m));
     if (codes & ECL_BATCH_SCC) wsb = std::max(wsb, scc_workspace_bytes(s.n, s.m));
     s.ws = dalloc<char>(b, wsb, &st);

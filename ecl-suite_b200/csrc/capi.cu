@@ -1,12 +1,7 @@
 // Library-level C ABI entry points that are not tied to one solver.
-#include "runtime.cuh"
+#include "solvers.cuh"
 
 namespace ecl {
-size_t cc_workspace_bytes(int n, int m);
-size_t mis_workspace_bytes(int n, int m);
-size_t gc_workspace_bytes(int n, int m);
-size_t mst_workspace_bytes(int n, int m);
-size_t scc_workspace_bytes(int n, int m);
 size_t apsp_workspace_bytes(int n, int m);
 }  // namespace ecl
 

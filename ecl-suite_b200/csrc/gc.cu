@@ -1099,7 +1099,7 @@ struct GCBufs {
   int4* rowinfo;
 };
 
-void gc_layout(Carve& c, int n, int m, GCBufs* b) {
+void gc_layout(Carve& c, int n, int m, bool uni, GCBufs* b) {
   b->ctl = c.take<GCCtl>(1);
   b->nl2 = c.take<int>((size_t)m + 4);  // 4 spare entries: the core's aligned bulk copies may round up into them
   b->hc = c.take<int>((size_t)n);
@@ -1108,18 +1108,18 @@ void gc_layout(Carve& c, int n, int m, GCBufs* b) {
   b->vals0 = c.take<int>((size_t)n);
   b->vals1 = c.take<int>((size_t)n);
   b->order = c.take<int>((size_t)n);
-  b->sort_temp = c.take<unsigned>(kRadixTempWords);
-  b->vhash = c.take<unsigned>((size_t)n);
+  b->sort_temp = c.take<unsigned>(radix_temp_words(n));
+  b->vhash = c.take<unsigned>(uni ? (size_t)n : 0);
   b->chunks = c.take<int2>(row_chunk_capacity(m, kMinChunk));
   b->rowinfo = c.take<int4>((size_t)std::min(n, kCoreMax));
 }
 
 }  // namespace
 
-size_t gc_workspace_bytes(int n, int m) {
+size_t gc_workspace_bytes(int n, int m, bool uni) {
   Carve c;
   GCBufs b;
-  gc_layout(c, n, m, &b);
+  gc_layout(c, n, m, uni, &b);
   return c.bytes();
 }
 
@@ -1131,7 +1131,7 @@ ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, Status* status, c
                       cudaStream_t stream, const UnionInfo* uni, Marker mark) {
   Carve c{ws};
   GCBufs b;
-  gc_layout(c, g.n, g.m, &b);
+  gc_layout(c, g.n, g.m, uni && uni->vbase, &b);
   // Blocks of the pull per SM: a knob, 2 by default.  Fewer warps poll
   // fewer undecided entries at a time; on R-MAT-22 two blocks per SM colour
   // faster than four (1.81 vs 2.15 ms) -- the polls of four blocks load L2

@@ -210,6 +210,9 @@ __device__ __forceinline__ int mis_scan_warp(int v, unsigned b, int& pos, int en
   return kJoin;
 }
 
+// Without items (kItems false: a workspace of one byte a vertex) every sweep
+// goes through the groups again and scans from the start: R-MAT-22 330 -> 560 us.
+//
 // A warp's g-th group is the vertices 32 (g nwarps + warp) ..+31, and its g-th
 // 32 items lie at the same places, so the warps' lists share one array of n
 // (rounded up) items and need no counters.  Bound by the latency of the chains
@@ -217,6 +220,7 @@ __device__ __forceinline__ int mis_scan_warp(int v, unsigned b, int& pos, int en
 // swept and scanned from the start until decided -> items: R-MAT-22 525 -> 297
 // us, 500 k vertices 169 -> 80, 1000 vertices (fewer blocks) 40 -> 16; with the
 // long lists scanned in the first sweep as well, R-MAT-22 525.
+template <bool kItems>
 __global__ void __launch_bounds__(kTPB) mis_run(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, unsigned* __restrict__ st4,
                                                 int4* __restrict__ items, Status* __restrict__ status, int max_sweeps,
@@ -261,27 +265,36 @@ __global__ void __launch_bounds__(kTPB) mis_run(int n, int m, const int* __restr
     }
     const bool keep = wait || (go && verdict == kWait);
     const unsigned bal = __ballot_sync(kFull, keep);
-    if (keep) items[slot(kept + __popc(bal & ((1u << lane) - 1)))] = make_int4(v, pos, blocker, end);
+    if (kItems && keep) items[slot(kept + __popc(bal & ((1u << lane) - 1)))] = make_int4(v, pos, blocker, end);
     kept += __popc(bal);
   };
-  for (int base = warp * 32; base < n; base += nwarps * 32) {
-    const int v = base + lane;
-    unsigned b = 0;
-    if (v < n) b = byte_of(ld(&st4[v >> 2]), v);
-    const bool und = (b & 1u) != 0;
-    if (!__any_sync(kFull, und)) continue;
-    int beg = 0, end = 0;
-    if (und) {
-      beg = __ldg(&nindex[v]);
-      end = __ldg(&nindex[v + 1]);
-      if (beg < 0 || end < beg || end > m) beg = end = 0;  // reported by mis_init
-    }
-    // long lists first wait for a sweep: their vertices rank low (the priority
-    // falls with the degree), and most are out before they are looked at
-    const bool big = end - beg > lane_max;
-    advance(und && !big, und && big, v, b, beg, end, -1);
-  }
   int sweep = 0;
+  for (bool first = true;; first = false) {  // once; without items, until all are decided
+    for (int base = warp * 32; base < n; base += nwarps * 32) {
+      const int v = base + lane;
+      unsigned b = 0;
+      if (v < n) b = byte_of(ld(&st4[v >> 2]), v);
+      const bool und = (b & 1u) != 0;
+      if (!__any_sync(kFull, und)) continue;
+      int beg = 0, end = 0;
+      if (und) {
+        beg = __ldg(&nindex[v]);
+        end = __ldg(&nindex[v + 1]);
+        if (beg < 0 || end < beg || end > m) beg = end = 0;  // reported by mis_init
+      }
+      // long lists first wait for a sweep: their vertices rank low (the priority
+      // falls with the degree), and most are out before they are looked at
+      const bool big = (kItems || first) && end - beg > lane_max;
+      advance(und && !big, und && big, v, b, beg, end, -1);
+    }
+    if (kItems || kept == 0) break;
+    kept = 0;
+    if (sweep >= max_sweeps) {
+      if (lane == 0) raise(status, ECL_ERR_NO_CONVERGENCE, warp);
+      break;
+    }
+    sweep++;
+  }
   for (; kept > 0; sweep++) {
     if (sweep >= max_sweeps) {
       if (lane == 0) raise(status, ECL_ERR_NO_CONVERGENCE, warp);
@@ -314,7 +327,7 @@ __global__ void __launch_bounds__(kTPB) mis_emit(int n, const unsigned* __restri
 
 void mis_layout(Carve& c, int n, unsigned** st4, int4** items) {
   *st4 = c.take<unsigned>((size_t)(n + 3) / 4);
-  *items = c.take<int4>(((size_t)n + 31) / 32 * 32);
+  if (items) *items = c.take<int4>(((size_t)n + 31) / 32 * 32);
 }
 
 }  // namespace
@@ -328,16 +341,23 @@ size_t mis_workspace_bytes(int n, int m) {
   return c.bytes();
 }
 
+size_t mis_small_workspace_bytes(int n) {
+  Carve c;
+  unsigned* st4;
+  mis_layout(c, n, &st4, nullptr);
+  return c.bytes();
+}
+
 }  // namespace ecl
 
 namespace ecl {
 
-ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, Status* status, const DeviceInfo& dev,
-                       cudaStream_t stream, int max_sweeps, const UnionInfo* uni, Marker mark) {
+ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, size_t ws_bytes, Status* status,
+                       const DeviceInfo& dev, cudaStream_t stream, int max_sweeps, const UnionInfo* uni, Marker mark) {
   Carve c{ws};
   unsigned* st4;
-  int4* items;
-  mis_layout(c, g.n, &st4, &items);
+  int4* items = nullptr;
+  mis_layout(c, g.n, &st4, ws_bytes >= mis_workspace_bytes(g.n, g.m) ? &items : nullptr);
   const int nwords = (g.n + 3) / 4;
   const int grid = dev.grid_blocks(kTPB, g.n, g.m);
   const int* vbase = uni ? uni->vbase : nullptr;
@@ -349,10 +369,11 @@ ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, Status* 
   // so all its blocks must be resident together: a cooperative launch
   // guarantees that even when other solves share the GPU (server slots).
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mis_run, kTPB, 0) != cudaSuccess || occ < 1)
+  auto run = items ? mis_run<true> : mis_run<false>;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, run, kTPB, 0) != cudaSuccess || occ < 1)
     return ECL_ERR_CUDA;
   const int full = dev.sms * std::min(occ, dev.max_threads_per_sm / kTPB);
-  ECL_CUDA_TRY(launch_cooperative(mis_run, std::min(full, (g.n - 1) / kTPB + 1), kTPB, stream, g.n,
+  ECL_CUDA_TRY(launch_cooperative(run, std::min(full, (g.n - 1) / kTPB + 1), kTPB, stream, g.n,
                                   g.m, g.nindex, g.nlist, st4, items, status, max_sweeps,
                                   bins_of(dev, Bins{kLaneMax, kBinChunk}).lane));
   mark();
@@ -372,7 +393,8 @@ extern "C" ecl_status ecl_mis(const ecl_graph_view* g, uint8_t* status_out, ecl_
   GraphNeeds needs;
   needs.symmetric = true;
   needs.no_self_loops = true;
-  ecl_status st = s.begin(needs, g ? mis_workspace_bytes(g->nodes, g->edges) : 0);
+  ecl_status st = s.begin(needs, g ? mis_workspace_bytes(g->nodes, g->edges) : 0,
+                          g ? mis_small_workspace_bytes(g->nodes) : 0);
   if (st != ECL_OK) return s.finish(st);
   unsigned char* out = s.output(status_out, (size_t)s.n);
   if (!out) return s.finish(ECL_ERR_OOM);
@@ -387,7 +409,7 @@ extern "C" ecl_status ecl_mis(const ecl_graph_view* g, uint8_t* status_out, ecl_
   // cannot converge, not a per-graph bound.
   const int max_sweeps = opts->max_rounds > 0 ? opts->max_rounds : (1 << 22);
   s.start_timer();
-  st = mis_enqueue(gd, out, s.ws, s.status, s.dev, s.stream, max_sweeps, nullptr, Marker{&s});
+  st = mis_enqueue(gd, out, s.ws, s.ws_size - kStatusBytes, s.status, s.dev, s.stream, max_sweeps, nullptr, Marker{&s});
   s.stop_timer();
   return s.finish(st);
 }

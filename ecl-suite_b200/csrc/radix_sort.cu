@@ -228,13 +228,12 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
 ecl_status radix_order(unsigned long long* k0, int* v0, unsigned long long* k1, int* v1, int* order, int n,
                        const int* n_dev, const int* max_high, unsigned* temp, bool spread, GridBarrier* bar, int* failed,
                        const DeviceInfo& dev, cudaStream_t stream, Status* status) {
-  // A block per kShare keys: ranking a share is a serial chain of its slices, so
+  // A block per kRadixShare keys: ranking a share is a serial chain of its slices, so
   // blocks are worth their barrier arrivals; a single block needs no barrier at
   // all.  Whole sort with a block per 4096 keys -> this: 5 k keys 36 -> 34 us,
   // 20 k 52 -> 34, 100 k 51 -> 39; the slices spread over the warps, one block of
   // 1000 keys 28 -> 22.
-  constexpr int kShare = 1024;
-  const int blocks = std::max(1, std::min({dev.sms, kRadixMaxBlocks, n / kShare}));
+  const int blocks = std::max(1, std::min({dev.sms, kRadixMaxBlocks, n / kRadixShare}));
   auto kernel = (long long)n <= (long long)blocks * (kRadixTile - 32) ? rs_sort<true> : rs_sort<false>;
   ECL_CUDA_TRY(launch_cooperative(kernel, blocks, kThreads, stream, k0, v0, k1, v1, order, n, n_dev, max_high, temp,
                                   spread, bar, failed, status));

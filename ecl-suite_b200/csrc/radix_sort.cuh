@@ -20,13 +20,18 @@ namespace ecl {
 // Keys a block places per step (1024 threads x 8 keys).
 constexpr int kRadixTile = 8192;
 constexpr int kRadixMaxBlocks = 256;  // blocks the count table holds
-constexpr size_t kRadixTempWords = (size_t)256 * kRadixMaxBlocks;
+constexpr int kRadixShare = 1024;     // a block per this many keys
+// Words of radix_order()'s count table for n keys.
+constexpr size_t radix_temp_words(int n) {
+  return (size_t)256 * (n / kRadixShare < kRadixMaxBlocks ? n / kRadixShare + 1 : kRadixMaxBlocks);
+}
 
 // order[0 .. *n_dev) = the values of the pairs (k0, v0)[0 .. *n_dev) by
 // ascending key, equal keys in their input order.  *n_dev <= n (which sizes
 // the launch), *max_high = the largest d; (k1, v1) is scratch of n pairs, k0
 // and v0 are overwritten; spread: the h of different keys differ, but for a few,
-// and are spread evenly (the time depends on it, the order does not); `temp` holds kRadixTempWords and `bar` is zeroed.
+// and are spread evenly (the time depends on it, the order does not); `temp` holds
+// radix_temp_words(n) and `bar` is zeroed.
 // The order is whole (every value once) whatever status->code says; only when
 // a grid barrier times out it is not: ECL_ERR_NO_CONVERGENCE is raised in
 // `status`, *failed (zeroed before) becomes 1, and readers must check it.

@@ -120,7 +120,7 @@ Solve::~Solve() {
   if (!finished_) finish(ECL_ERR_CUDA);
 }
 
-ecl_status Solve::begin(const GraphNeeds& needs, size_t ws_bytes) {
+ecl_status Solve::begin(const GraphNeeds& needs, size_t ws_bytes, size_t ws_small) {
   if (!g_ || !opts_) return ECL_ERR_INVALID_ARG;
   if (g_->nodes < 1 || g_->edges < 0) return ECL_ERR_BAD_GRAPH;
   if (!g_->nindex || (g_->edges > 0 && !g_->nlist)) return ECL_ERR_INVALID_ARG;
@@ -168,9 +168,10 @@ ecl_status Solve::begin(const GraphNeeds& needs, size_t ws_bytes) {
     eweight = needs.weights ? g_->eweight : nullptr;
   }
 
-  const size_t need = ws_bytes + kStatusBytes;
-  if (opts_->workspace && opts_->workspace_bytes >= need) {
+  size_t need = ws_bytes + kStatusBytes;
+  if (opts_->workspace && opts_->workspace_bytes >= (ws_small ? ws_small : ws_bytes) + kStatusBytes) {
     ws = static_cast<char*>(opts_->workspace);
+    need = std::min(need, opts_->workspace_bytes);
   } else {
     ws = static_cast<char*>(temp(need));
     if (alloc_failed) return ECL_ERR_OOM;

@@ -199,9 +199,10 @@ class Solve {
   ~Solve();
 
   // Checks arguments, validates (if asked), stages the CSR on the device and
-  // provides `ws_bytes` of workspace.  The device Status block is placed at
-  // the start of the workspace and zeroed.
-  ecl_status begin(const GraphNeeds& needs, size_t ws_bytes);
+  // provides `ws_bytes` of workspace, or the caller's if that has `ws_small`
+  // (0: ws_bytes) or more.  The device Status block is placed at the start of
+  // the workspace and zeroed.
+  ecl_status begin(const GraphNeeds& needs, size_t ws_bytes, size_t ws_small = 0);
 
   // Device pointer through which the solver writes an output of `count`
   // elements: the caller's pointer for device-resident graphs, else a
@@ -228,7 +229,7 @@ class Solve {
   const int* eweight = nullptr;
   cudaStream_t stream = nullptr;
   char* ws = nullptr;            // workspace base (Status block first)
-  size_t ws_size = 0;
+  size_t ws_size = 0;            // with the Status block
   dev::Status* status = nullptr;
   DeviceInfo dev;
   bool alloc_failed = false;

@@ -321,8 +321,8 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
     deg = end - beg;
     if (beg < 0 || end < beg || end > m) beg = deg = 0;
   };
-  // no bit set yet (the words of all three arrays lie side by side)
-  for (int i = tid; i < 3 * words; i += nthreads) fwd[i] = 0;  // race-free: thread-owned, barrier next
+  // no bit set yet
+  for (int i = tid; i < words; i += nthreads) fwd[i] = bwd[i] = next[i] = 0;  // race-free: thread-owned, barrier next
   // the pivot
   unsigned long long key = 0;
   for (int v = tid; v < n; v += nthreads) {
@@ -903,13 +903,23 @@ struct SCCBufs {
   int2* wlA;
   int2* wlB;
   int* tilerow;
-  unsigned* bits;  // Giant's two bit arrays and scc_giant's next
+  unsigned* bits;  // Giant's two bit arrays
+  unsigned* next;
   int* queue;
   int* candA;
   int* candB;
   char* cc_ws;
   int max_rounds;
 };
+
+// Sizes at which a graph flagged symmetric is tried as connected components (not
+// with hardly any entries, where the general path trims nearly all vertices at
+// once and CC's passes over them cost more: 4 M vertices with 6 entries 90 us
+// against 136, 1 M with pairs among an eighth of them 71 against 77, among a
+// quarter 79 against 80, among half 93 against 82), and at which the search for
+// the giant component may run (with fewer entries than vertices there is none).
+constexpr bool scc_checked(int n, int m) { return m >= n / 4; }
+constexpr bool scc_searched(int n, int m) { return m >= kGiantEntries && m >= n; }
 
 void scc_layout(Carve& c, int n, int m, SCCBufs* b) {
   b->ctl = c.take<SCCCtl>(1);
@@ -918,17 +928,22 @@ void scc_layout(Carve& c, int n, int m, SCCBufs* b) {
   b->nchunks = c.take<int>(64);
   b->chunks = c.take<int2>(row_chunk_capacity(m, kMinChunk));
   b->io = c.take<unsigned long long>((size_t)n);
-  // The search's lists lie where the second edge list comes later, and the
-  // union-find's scratch where the first one does.
-  b->bits = c.take<unsigned>(3 * (((size_t)n + 31) / 32));
-  b->tilerow = c.take<int>((size_t)flat_tiles(m) + 1);
-  const size_t list = sizeof(int2) * (size_t)(m > 0 ? m : 1), ids = sizeof(int) * (size_t)n;
-  b->cc_ws = c.take<char>(std::max(list, cc_workspace_bytes(n, m)));
+  // The check's and the search's arrays lie where the edge lists come later: the
+  // union-find's scratch, and after it the search's candidates, in the first
+  // one, the check's rows, and after them the search's queue, in the second
+  // (the search is tried with n entries or more, so the lists are long enough),
+  // and its `next` in io.  Only the two bit arrays that the later launches read
+  // are its own.
+  const size_t list = sizeof(int2) * (size_t)(m > 0 ? m : 1);
+  b->cc_ws = c.take<char>(scc_checked(n, m) ? std::max(list, cc_workspace_bytes(n, m)) : list);
   b->wlA = reinterpret_cast<int2*>(b->cc_ws);
-  b->queue = reinterpret_cast<int*>(c.take<char>(std::max(list, 3 * ids)));
-  b->wlB = reinterpret_cast<int2*>(b->queue);
-  b->candA = b->queue + n;
+  b->wlB = c.take<int2>((size_t)(m > 0 ? m : 1));
+  b->tilerow = reinterpret_cast<int*>(b->wlB);
+  b->queue = reinterpret_cast<int*>(b->wlB);
+  b->candA = reinterpret_cast<int*>(b->wlA);
   b->candB = b->candA + n;
+  b->bits = c.take<unsigned>(scc_searched(n, m) ? 2 * (((size_t)n + 31) / 32) : 0);
+  b->next = reinterpret_cast<unsigned*>(b->io);
 }
 
 }  // namespace
@@ -959,14 +974,10 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
   const int coop_grid = dev.sms * occ;
   const int grid = dev.grid_blocks(kTPB, g.n, g.m);
   // a graph flagged symmetric may be solved as connected components (not when
-  // the caller limits the rounds: that limit is the general path's; and not
-  // with hardly any entries, where the general path trims nearly all vertices at
-  // once and CC's passes over them cost more: 4 M vertices with 6 entries 90 us
-  // against 136, 1 M with pairs among an eighth of them 71 against 77, among a
-  // quarter 79 against 80, among half 93 against 82)
-  const bool check = (g.flags & ECL_GRAPH_SYMMETRIC) != 0 && max_rounds <= 0 && g.m >= g.n / 4;
+  // the caller limits the rounds: that limit is the general path's)
+  const bool check = (g.flags & ECL_GRAPH_SYMMETRIC) != 0 && max_rounds <= 0 && scc_checked(g.n, g.m);
   // (the same limit; a flagged graph that is what its flag says leaves the search at once)
-  const bool giant = max_rounds <= 0 && g.m >= kGiantEntries;
+  const bool giant = max_rounds <= 0 && scc_searched(g.n, g.m);
   if (max_rounds <= 0 || max_rounds > b.max_rounds) max_rounds = b.max_rounds;
 
   fill_ranges({{b.ctl, sizeof(SCCCtl), 0},
@@ -1000,7 +1011,7 @@ ecl_status scc_enqueue(const GraphDev& g, int* label, char* ws, Status* status, 
       return ECL_ERR_CUDA;
     const int blocks = std::max(1, std::min(dev.sms * gocc, (int)(std::max((long long)g.n, (long long)g.m / 4) / kGTPB)));
     ECL_CUDA_TRY(launch_cooperative(scc_giant, blocks, kGTPB, stream, g.n, g.m, g.nindex, g.nlist, gi.fwd, gi.bwd,
-                                    b.bits + 2 * words, b.queue, b.candA, b.candB, b.chunks, (int)row_chunk_capacity(g.m, kMinChunk), b.ctl,
+                                    b.next, b.queue, b.candA, b.candB, b.chunks, (int)row_chunk_capacity(g.m, kMinChunk), b.ctl,
                                     check, status));
   }
   ECL_LAUNCH_NEXT(giant ? scc_mark<true> : scc_mark<false>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, b.flags,

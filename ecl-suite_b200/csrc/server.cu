@@ -67,10 +67,10 @@ size_t out_bytes(int code, const GraphDev& g) {
   return 0;
 }
 
-size_t ws_bytes(int code, const GraphDev& g) {
+size_t ws_bytes(int code, const GraphDev& g, bool small) {
   switch (code) {
     case ECL_CC: return cc_workspace_bytes(g.n, g.m);
-    case ECL_MIS: return mis_workspace_bytes(g.n, g.m);
+    case ECL_MIS: return small ? mis_small_workspace_bytes(g.n) : mis_workspace_bytes(g.n, g.m);
     case ECL_GC: return gc_workspace_bytes(g.n, g.m);
     case ECL_MST: return mst_workspace_bytes(g.n, g.m);
     case ECL_SCC: return scc_workspace_bytes(g.n, g.m);
@@ -80,8 +80,18 @@ size_t ws_bytes(int code, const GraphDev& g) {
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-size_t request_bytes(int code, const GraphDev& g) {
-  return align256(kStatusBytes) + align256(ws_bytes(code, g)) + align256(out_bytes(code, g));
+// `small`: with the least workspace that the code can do with.
+size_t request_bytes(int code, const GraphDev& g, bool small = false) {
+  return align256(kStatusBytes) + align256(ws_bytes(code, g, small)) + align256(out_bytes(code, g));
+}
+
+// A request whose full workspace would not fit the budget even alone gets a small one.
+bool small_request(const ecl_server* sv, const ecl_request& r) {
+  return sv->resident + request_bytes(r.code, sv->graphs[(size_t)r.graph].g) > sv->cfg.hbm_budget_bytes;
+}
+
+size_t request_bytes(const ecl_server* sv, const ecl_request& r) {
+  return request_bytes(r.code, sv->graphs[(size_t)r.graph].g, small_request(sv, r));
 }
 
 // Everything request r puts on slot s's stream after its memory is allocated.
@@ -90,13 +100,14 @@ ecl_status enqueue_request(ecl_server* sv, Slot& s, ecl_request& r) {
   char* base = static_cast<char*>(s.mem);
   dev::Status* status = reinterpret_cast<dev::Status*>(base);
   char* ws = base + align256(kStatusBytes);
-  char* out = ws + align256(ws_bytes(r.code, g));
+  const size_t wsb = ws_bytes(r.code, g, small_request(sv, r));
+  char* out = ws + align256(wsb);
   ECL_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(dev::Status), s.stream));
   ecl_status st = ECL_OK;
   unsigned long long* total_dev = nullptr;
   switch (r.code) {
     case ECL_CC: st = cc_enqueue(g, reinterpret_cast<int*>(out), ws, status, sv->dev, s.stream); break;
-    case ECL_MIS: st = mis_enqueue(g, reinterpret_cast<unsigned char*>(out), ws, status, sv->dev, s.stream, 1 << 22); break;
+    case ECL_MIS: st = mis_enqueue(g, reinterpret_cast<unsigned char*>(out), ws, wsb, status, sv->dev, s.stream, 1 << 22); break;
     case ECL_GC: st = gc_enqueue(g, reinterpret_cast<int*>(out), ws, status, sv->dev, s.stream); break;
     case ECL_MST:
       st = mst_enqueue(g, reinterpret_cast<unsigned char*>(out), ws, status, sv->dev, s.stream, &total_dev);
@@ -115,8 +126,7 @@ ecl_status enqueue_request(ecl_server* sv, Slot& s, ecl_request& r) {
 // The request's memory goes back to the pool on the slot's stream whether or
 // not every step was enqueued, so a failed launch leaks nothing.
 ecl_status launch(ecl_server* sv, Slot& s, ecl_request& r) {
-  const GraphDev& g = sv->graphs[(size_t)r.graph].g;
-  const size_t need = request_bytes(r.code, g);
+  const size_t need = request_bytes(sv, r);
   ECL_CUDA_TRY(cudaMallocAsync(&s.mem, need, s.stream));
   s.bytes = need;
   const ecl_status st = enqueue_request(sv, s, r);
@@ -226,7 +236,7 @@ ecl_status ecl_server_run(ecl_server* sv, ecl_request* reqs, int32_t count, ecl_
       r.status = ECL_ERR_INVALID_ARG;
     } else if (r.code == ECL_MST && !sv->graphs[(size_t)r.graph].g.eweight) {
       r.status = ECL_ERR_INVALID_ARG;
-    } else if (sv->resident + request_bytes(r.code, sv->graphs[(size_t)r.graph].g) > sv->cfg.hbm_budget_bytes) {
+    } else if (sv->resident + request_bytes(sv, r) > sv->cfg.hbm_budget_bytes) {
       r.status = ECL_ERR_OOM;  // can never fit, even alone
     }
   }
@@ -284,8 +294,7 @@ ecl_status ecl_server_run(ecl_server* sv, ecl_request* reqs, int32_t count, ecl_
       Slot& s = sv->slots[k];
       if (s.req >= 0) continue;
       auto it = std::find_if(ready.begin(), ready.end(), [&](int i) {
-        return sv->resident + inflight_bytes + request_bytes(reqs[i].code, sv->graphs[(size_t)reqs[i].graph].g) <=
-               sv->cfg.hbm_budget_bytes;
+        return sv->resident + inflight_bytes + request_bytes(sv, reqs[i]) <= sv->cfg.hbm_budget_bytes;
       });
       if (it == ready.end()) break;
       const int i = *it;

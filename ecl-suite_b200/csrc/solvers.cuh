@@ -42,7 +42,10 @@ struct Marker {
 
 size_t cc_workspace_bytes(int n, int m);
 size_t mis_workspace_bytes(int n, int m);
-size_t gc_workspace_bytes(int n, int m);
+// What MIS cannot do without: a workspace from this size on is used, below
+// mis_workspace_bytes() by a slower form.
+size_t mis_small_workspace_bytes(int n);
+size_t gc_workspace_bytes(int n, int m, bool uni = false);  // uni: for a union's hashes too
 size_t mst_workspace_bytes(int n, int m);
 size_t scc_workspace_bytes(int n, int m);
 
@@ -51,8 +54,8 @@ size_t scc_workspace_bytes(int n, int m);
 ecl_status cc_enqueue(const GraphDev& g, int* label, char* ws, dev::Status* status, const DeviceInfo& dev,
                       cudaStream_t stream, Marker mark = {}, const UnionInfo* uni = nullptr,
                       const unsigned long long* off = nullptr);
-ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, dev::Status* status, const DeviceInfo& dev,
-                       cudaStream_t stream, int max_sweeps, const UnionInfo* uni = nullptr, Marker mark = {});
+ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, size_t ws_bytes, dev::Status* status,
+                       const DeviceInfo& dev, cudaStream_t stream, int max_sweeps, const UnionInfo* uni = nullptr, Marker mark = {});
 ecl_status gc_enqueue(const GraphDev& g, int* color, char* ws, dev::Status* status, const DeviceInfo& dev,
                       cudaStream_t stream, const UnionInfo* uni = nullptr, Marker mark = {});
 // *total_dev receives the device address of the forest weight (uint64).

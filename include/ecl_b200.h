@@ -26,7 +26,8 @@
  *    does, library/ECLatomic.h:57-75).
  *  - Scratch memory comes from opts->workspace when it is non-NULL and at
  *    least ecl_workspace_bytes() large; otherwise the call allocates it
- *    stream-ordered and frees it before returning.
+ *    stream-ordered and frees it before returning.  (ecl_mis uses any of 256
+ *    bytes + one a vertex, rounded up to 256, and is slower in a small one.)
  */
 #ifndef ECL_B200_H
 #define ECL_B200_H

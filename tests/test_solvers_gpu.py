@@ -718,6 +718,51 @@ def test_scc_search_for_a_giant_component_gives_up_in_time(ecl, orc):
         assert best_ms(ecl, dg, "scc") < 1.25 * best_ms(ecl, dg, "scc", max_rounds=g.nodes + 1) + 0.03, name
 
 
+# Bytes of scratch that each code has asked for at least since callers could keep
+# one: (nodes, entries) -> bytes.
+FORMER_SCRATCH = {
+    "mis": {(1000, 16000): 1280, (1 << 20, 1 << 22): 1048832, (1 << 24, 1 << 20): 16777472},
+    "gc": {(1000, 16000): 117760, (1 << 20, 1 << 22): 51709952, (1 << 24, 1 << 20): 545982464},
+    "scc": {(1000, 16000): 1321984, (1 << 20, 1 << 22): 81267968, (1 << 24, 1 << 20): 219286784},
+}
+
+
+@pytest.mark.parametrize("code", ["gc", "scc"])
+def test_scratch_stays_within_a_hundredth_of_what_it_was(ecl, code):
+    for (n, m), former in FORMER_SCRATCH[code].items():
+        assert ecl.workspace_bytes(dict(gc=ecl.GC, scc=ecl.SCC)[code], n, m) <= 1.01 * former + 4096, (n, m)
+
+
+@pytest.mark.parametrize("n", [1, 33, 1000, 70001])
+def test_mis_in_a_workspace_of_one_byte_a_vertex(ecl, orc, n):
+    """Workspaces of the size that MIS cannot do without, of one byte less (which
+    the call does not touch), and of both sides of its full size."""
+    import torch
+
+    graphs = [ecl.gen_er(n, min(1.0, 9.0 / n), seed=n, symmetrise=True), undirected(n, [(i, i + 1) for i in range(min(n, 900) - 1)]),
+              undirected(n, [(0, i) for i in range(1, min(n, 700))])]
+    small, full = 256 + ((n + 3) // 4 * 4 + 255) // 256 * 256, ecl.workspace_bytes(ecl.MIS, n, 1)
+    for size in (small - 1, small, full - 1, full):
+        ws = torch.full((size + 64,), 0x5a, dtype=torch.uint8, device="cuda")
+        for g in graphs:
+            got = ecl.mis(g.to_device(), workspace=ws[:size])
+            assert np.array_equal(got.cpu().numpy(), orc.mis(g)), size
+        assert bool((ws[size:] == 0x5a).all()) and bool((ws == 0x5a).all()) == (size < small)
+
+
+def test_server_takes_a_mis_request_that_fits_with_one_byte_a_vertex(ecl, orc):
+    g = ecl.gen_rmat(16, 8, seed=7)
+    resident = 4 * (g.nodes + 1) + 4 * g.edges
+    out = np.zeros(g.nodes, np.uint8)
+    for room, status in ((2 * g.nodes + 512, ecl.OK), (2 * g.nodes, ecl.ERR_OOM), (30 * g.nodes, ecl.OK)):
+        srv = ecl.Server(slots=2, hbm_budget_bytes=resident + room)
+        gid = srv.add_graph(g)
+        out[:] = 7
+        rc, arr, st = srv.run([(ecl.MIS, gid, 0.0, out.ctypes.data)])
+        assert arr[0].status == status
+        assert status != ecl.OK or (np.array_equal(out, orc.mis(g)) and st.peak_bytes <= resident + room)
+
+
 def caterpillar(ecl, spine, leaves):
     """A path of `spine` vertices with `leaves` vertices of degree one at each."""
     s = np.arange(spine)
