@@ -72,7 +72,7 @@ using batchimpl::Super;
 constexpr int kTotalsTile = 4096;
 
 __global__ void __launch_bounds__(256) batch_mst_totals(int ngraphs, int m, const int* __restrict__ ebase,
-                                                        const unsigned* __restrict__ in_mst4,
+                                                        const unsigned* in_mst4,
                                                         const int* __restrict__ eweight,
                                                         unsigned long long* __restrict__ totals) {
   dep_wait();
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(256) batch_mst_totals(int ngraphs, int m, cons
 // vertex's own graph, once a run: on the host, where every result was
 // rewritten after its copy, this was 1.3 ms for the 96 graphs' 2.7 M labels.
 __global__ void __launch_bounds__(256) batch_local(int n, int ngraphs, const int* __restrict__ vbase,
-                                                   int* __restrict__ label) {
+                                                   int* label) {
   dep_wait();
   for (int v = blockIdx.x * 256 + threadIdx.x; v < n; v += gridDim.x * 256)
     label[v] -= __ldg(&vbase[union_graph_of(vbase, ngraphs, v)]);  // race-free: thread-owned, the solve has ended

@@ -156,7 +156,7 @@ __device__ __forceinline__ int cc_first_smaller(int v, int beg, int end, const i
 // [0, m]) raises ECL_ERR_BAD_GRAPH and is treated as empty by every kernel.
 __global__ void __launch_bounds__(kTPB) cc_init(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, int* __restrict__ parent,
-                                                CCCounters* __restrict__ ctr, const u64* off,
+                                                CCCounters* ctr, const u64* off,
                                                 Status* __restrict__ status) {
   dep_wait();
   if (cc_off(off)) return;
@@ -206,7 +206,7 @@ __device__ __forceinline__ int cc_chunk_total(const CCCounters* ctr, int cap) {
 __global__ void __launch_bounds__(kTPB) cc_hook(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, int* __restrict__ parent,
                                                 int2* __restrict__ chunks, int chunk_cap, Bins bins,
-                                                CCCounters* __restrict__ ctr, Status* __restrict__ status) {
+                                                CCCounters* ctr, Status* __restrict__ status) {
   dep_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
@@ -252,8 +252,8 @@ __global__ void __launch_bounds__(kTPB) cc_hook(int n, int m, const int* __restr
 
 __global__ void __launch_bounds__(kTPB) cc_chunks(int n, const int* __restrict__ nindex,
                                                   const int* __restrict__ nlist, int* __restrict__ parent,
-                                                  const int2* __restrict__ chunks, int chunk_cap, int chunk,
-                                                  const CCCounters* __restrict__ ctr, Status* __restrict__ status) {
+                                                  const int2* chunks, int chunk_cap, int chunk,
+                                                  const CCCounters* ctr, Status* __restrict__ status) {
   dep_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
@@ -419,7 +419,7 @@ constexpr int kSplitSample = 1 << 13;
 // links are done when it runs, so the roots it walks to are the final ones.
 constexpr int kGiantSlots = 2048;
 
-__global__ void __launch_bounds__(1024) cc_giant(int n, const int* __restrict__ parent, const int* __restrict__ vbase,
+__global__ void __launch_bounds__(1024) cc_giant(int n, const int* parent, const int* __restrict__ vbase,
                                                  int* __restrict__ root, const u64* off) {
   dep_wait();
   if (cc_off(off)) return;
@@ -460,13 +460,13 @@ __global__ void __launch_bounds__(1024) cc_giant(int n, const int* __restrict__ 
 // linked when u < v (the other direction is handled from u) or when u is in
 // the giant component (u skips its list entirely).
 __device__ __forceinline__ bool cc_rest_wanted(int u, int v, const unsigned char* ing) {
-  return u != v && (u < v || __ldg(&ing[u]));
+  return u != v && (u < v || ing[u]);
 }
 
 __global__ void __launch_bounds__(kTPB) cc_rest(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, int* __restrict__ parent,
-                                                const unsigned char* __restrict__ ing, int2* __restrict__ chunks,
-                                                int chunk_cap, Bins bins, CCCounters* __restrict__ ctr,
+                                                const unsigned char* ing, int2* __restrict__ chunks,
+                                                int chunk_cap, Bins bins, CCCounters* ctr,
                                                 const u64* off, Status* __restrict__ status) {
   dep_wait();
   if (cc_off(off)) return;
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(kTPB) cc_rest(int n, int m, const int* __restr
   for (int base = warp * 32; base < n; base += nwarps * 32) {
     const int v = base + lane;
     int beg = 0, end = 0;
-    if (v < n && !__ldg(&ing[v])) cc_row(nindex, v, m, beg, end);
+    if (v < n && !ing[v]) cc_row(nindex, v, m, beg, end);
     const int deg = end - beg;
     if (deg > bins.chunk) {
       cc_push_chunks(v, beg, deg, bins.chunk, chunks, chunk_cap, ctr, status);
@@ -517,9 +517,9 @@ __global__ void __launch_bounds__(kTPB) cc_rest(int n, int m, const int* __restr
 
 __global__ void __launch_bounds__(kTPB) cc_rest_chunks(int n, const int* __restrict__ nindex,
                                                        const int* __restrict__ nlist, int* __restrict__ parent,
-                                                       const unsigned char* __restrict__ ing,
-                                                       const int2* __restrict__ chunks, int chunk_cap, int chunk,
-                                                       const CCCounters* __restrict__ ctr, const u64* off,
+                                                       const unsigned char* ing,
+                                                       const int2* chunks, int chunk_cap, int chunk,
+                                                       const CCCounters* ctr, const u64* off,
                                                        Status* __restrict__ status) {
   dep_wait();
   if (cc_off(off)) return;

@@ -27,6 +27,13 @@ using aref = cuda::atomic_ref<T, cuda::thread_scope_device>;
 
 // First statement of a kernel that is launched by launch_next(): returns when
 // the kernels before it in the stream have ended and their writes are visible.
+//
+// Loads of what those kernels wrote have to stay behind it.  Atomic ones do, and
+// so do plain ones through ordinary pointers (the statement clobbers memory; L1
+// may serve them).  __ldg, and plain loads through __restrict__ pointers, say that
+// the words do not change while the kernel lives -- and it lives from before the
+// wait, so the compiler might load them there.  In such a kernel they are for
+// the solve's inputs only: nindex, nlist, eweight and a union's tables.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename T>

@@ -64,7 +64,7 @@ __device__ __forceinline__ void flat_rows_range(int n, int m, const int* nindex,
 
 // One tile: f(e0, row, u) with e0 the lane's first entry and, for its
 // kFlatLane entries, the row (-1: the entry is in no row, or past the end) and
-// the entry's value nlist[e0 + k] (anything where the row is -1).  s_mark: this
+// the entry's value nlist[e0 + k] (0 where the row is -1).  s_mark: this
 // warp's kFlatTile words of shared memory.  All lanes call, and all call f.
 // `stop` = min(m, nindex[n]), the end of the last row.
 template <class F>
@@ -81,8 +81,8 @@ __device__ __forceinline__ void flat_tile(const FlatCsr& g, int stop, bool vec, 
 #pragma unroll
     for (int k = 0; k < kFlatLane; k++) u[k] = e0 < g.m - k ? __ldcs(&g.nlist[e0 + k]) : 0;
   }
-  const int v0 = __ldg(&g.tilerow[t]);
-  int v1 = first < g.m - kFlatTile ? __ldg(&g.tilerow[t + 1]) : -1;
+  const int v0 = g.tilerow[t];  // (not by __ldg: an earlier launch wrote it)
+  int v1 = first < g.m - kFlatTile ? g.tilerow[t + 1] : -1;
   if (v1 < 0 || v1 >= g.n) v1 = g.n - 1;
   int row[kFlatLane];
   if (v1 - v0 <= kFlatRowsMax) {
@@ -125,6 +125,11 @@ __device__ __forceinline__ void flat_tile(const FlatCsr& g, int stop, bool vec, 
       }
       row[k] = lo;
     }
+  }
+  if (v0 < 0) {  // entries before the first row are no part of the graph
+#pragma unroll
+    for (int k = 0; k < kFlatLane; k++)
+      if (row[k] < 0) u[k] = 0;
   }
 #pragma unroll
   for (int k = 0; k < kFlatLane; k++)

@@ -68,7 +68,7 @@ struct GCCtl {
 // Priority hash of vertex x: the reference hashes the vertex id; in a union
 // of graphs (vhash != nullptr) it is the hash of x's LOCAL id, precomputed.
 __device__ __forceinline__ unsigned gc_h(const unsigned* vhash, int x) {
-  return vhash ? __ldg(&vhash[x]) : ecl_hash((unsigned)x);
+  return vhash ? vhash[x] : ecl_hash((unsigned)x);
 }
 
 // Entries per lane whose loads are issued together in the init scans.
@@ -87,7 +87,7 @@ __device__ __forceinline__ void gc_class_batch(const int (&u)[kInitBatch], const
 #pragma unroll
   for (int k = 0; k < kInitBatch; k++) {
     const bool ok = valid[k] && (unsigned)u[k] < (unsigned)n && u[k] != v;
-    ku[k] = ok ? __ldg(&keys[n - 1 - u[k]]) : 0ull;
+    ku[k] = ok ? keys[n - 1 - u[k]] : 0ull;
   }
 #pragma unroll
   for (int k = 0; k < kInitBatch; k++) {
@@ -125,7 +125,7 @@ constexpr int kSmallGroup = 4;
 __global__ void __launch_bounds__(kTPB) gc_init(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, int* __restrict__ nl2,
                                                 int* __restrict__ hc, RowChunks rc, Bins bins, int group, bool vec,
-                                                const unsigned long long* __restrict__ keys,
+                                                const unsigned long long* keys,
                                                 Status* __restrict__ status) {
   dep_wait();
   const int lane = threadIdx.x & 31;
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kTPB) gc_init(int n, int m, const int* __restr
     int beg = 0, end = 0;
     if (v < n) csr_row(nindex, v, m, beg, end, status);
     const int dv = end - beg;
-    const unsigned long long kv = (v < n) ? __ldg(&keys[n - 1 - v]) : 0ull;
+    const unsigned long long kv = (v < n) ? keys[n - 1 - v] : 0ull;
     int h = 0;
     push_chunks_warp(rc, bins.chunk, dv > bins.chunk, v, beg, end, status);
     if (v < n && dv <= bins.lane) {
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kTPB) gc_init(int n, int m, const int* __restr
 __global__ void __launch_bounds__(kTPB) gc_init_chunks(int n, int m, const int* __restrict__ nindex,
                                                        const int* __restrict__ nlist, int* __restrict__ nl2,
                                                        int* __restrict__ hc, RowChunks rc, int chunk, bool vec,
-                                                       const unsigned long long* __restrict__ keys,
+                                                       const unsigned long long* keys,
                                                        Status* __restrict__ status) {
   dep_wait();
   const int lane = threadIdx.x & 31;
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kTPB) gc_init_chunks(int n, int m, const int* 
     const int v = r.x;
     const int beg = __ldg(&nindex[v]), end = __ldg(&nindex[v + 1]);
     const int stop = min(r.y + chunk, end);
-    const unsigned long long kv = __ldg(&keys[n - 1 - v]);
+    const unsigned long long kv = keys[n - 1 - v];
     warp_row(r.y, stop, m, vec, nlist, [&](const int(&)[4], const int (&u)[4], const bool (&valid)[4]) {
       int cls[kInitBatch];
       gc_class_batch(u, valid, v, kv, n, keys, status, cls);
@@ -233,7 +233,7 @@ constexpr int kKeyBatch = 4;
 __global__ void __launch_bounds__(kTPB) gc_keys(int n, int m, const int* __restrict__ nindex,
                                                 unsigned long long* __restrict__ keys,
                                                 unsigned long long* __restrict__ skeys, int* __restrict__ svals,
-                                                const unsigned* __restrict__ vhash, int* __restrict__ color,
+                                                const unsigned* vhash, int* __restrict__ color,
                                                 GCCtl* __restrict__ ctl) {
   dep_wait();
   // rows longer than kWarpRow are counted per block and added once per block;
@@ -585,11 +585,11 @@ __device__ __forceinline__ int gc_core_size(const GCCtl* ctl, int cap) {
 }
 
 // rank[order[r]] = r over the core.
-__global__ void __launch_bounds__(kTPB) gc_core_rank(const int* __restrict__ order, int* __restrict__ rank,
-                                                     const GCCtl* __restrict__ ctl, int cap) {
+__global__ void __launch_bounds__(kTPB) gc_core_rank(const int* order, int* __restrict__ rank,
+                                                     const GCCtl* ctl, int cap) {
   dep_wait();
   const int core = gc_core_size(ctl, cap);
-  for (int r = blockIdx.x * kTPB + threadIdx.x; r < core; r += gridDim.x * kTPB) rank[__ldg(&order[r])] = r;
+  for (int r = blockIdx.x * kTPB + threadIdx.x; r < core; r += gridDim.x * kTPB) rank[order[r]] = r;
 }
 
 // Rewrites the higher-priority entries of every core row from vertex ids to
@@ -601,9 +601,9 @@ __global__ void __launch_bounds__(kTPB) gc_core_rank(const int* __restrict__ ord
 // the first entry of step i + 1.  A core row has more than kWarpRow entries,
 // so its 4-byte slot holds the packed ranks and the copies' rounding.
 __global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict__ nindex, int* nl2,
-                                                          const int* __restrict__ hc, const int* __restrict__ order,
-                                                          const int* __restrict__ rank, int4* __restrict__ rowinfo,
-                                                          const GCCtl* __restrict__ ctl, int cap,
+                                                          const int* hc, const int* order,
+                                                          const int* rank, int4* __restrict__ rowinfo,
+                                                          const GCCtl* ctl, int cap,
                                                           Status* __restrict__ status) {
   dep_wait();
   const int lane = threadIdx.x & 31;
@@ -611,15 +611,15 @@ __global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict_
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
   for (int r = warp; r < core; r += nwarps) {
-    const int v = __ldg(&order[r]);
-    const int b = __ldg(&nindex[v]), h = __ldg(&hc[v]);
+    const int v = order[r];
+    const int b = __ldg(&nindex[v]), h = hc[v];  // race-free: not written in this launch
     const int first = (int)(((long long)b + 3) >> 2);  // 16-byte units
     unsigned short* out = reinterpret_cast<unsigned short*>(nl2) + (size_t)first * 8;
     for (int i0 = 0; i0 < h; i0 += 32) {
       const int i = i0 + lane;
       unsigned short q = 0;
       if (i < h) {
-        const int x = __ldg(&rank[nl2[(size_t)b + i]]);
+        const int x = rank[nl2[(size_t)b + i]];
         if ((unsigned)x < (unsigned)r)
           q = (unsigned short)x;
         else  // only where a union's entry leaves its graph for a vertex of the same key
@@ -761,7 +761,7 @@ __device__ int gc_core_far(const unsigned short* row, int h, const unsigned shor
 #pragma unroll
       for (int s = 0; s < kFlight; s++) {
         const int e = i0 + 256 * s;
-        x[s] = e < h ? __ldg(&rv[e >> 3]) : make_uint4(0u, 0u, 0u, 0u);  // up to 7 entries of the slot past the row
+        x[s] = e < h ? rv[e >> 3] : make_uint4(0u, 0u, 0u, 0u);  // up to 7 entries of the slot past the row
       }
 #pragma unroll
       for (int s = 0; s < kFlight; s++) {
@@ -826,8 +826,8 @@ struct CoreStage {
 // any 16-bit value in a row; 2 * 0xffff bytes is inside this CTA's shared
 // memory for every core size, and a wait on what is read there ends on the
 // status word.
-__global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* __restrict__ nl2, const int4* __restrict__ rowinfo,
-                                                           int* __restrict__ color, const GCCtl* __restrict__ ctl,
+__global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const int4* rowinfo,
+                                                           int* __restrict__ color, const GCCtl* ctl,
                                                            int cap, Status* __restrict__ status) {
   dep_wait();
   extern __shared__ __align__(16) unsigned char s_core[];
@@ -865,7 +865,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* __restrict
     if ((j & ~31) != jb) {
       jb = j & ~31;
       const int r = warp + cwarps * (jb + lane);
-      rec = r < core ? __ldg(&rowinfo[r]) : make_int4(0, 0, -1, 0);
+      rec = r < core ? rowinfo[r] : make_int4(0, 0, -1, 0);
     }
     const int src = j & 31;
     return make_int4(__shfl_sync(kFull, rec.x, src), __shfl_sync(kFull, rec.y, src), __shfl_sync(kFull, rec.z, src),

@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kTPB) mis_run(int n, int m, const int* __restr
   if (lane == 0) fetch_max(&status->rounds, sweep + 1);
 }
 
-__global__ void __launch_bounds__(kTPB) mis_emit(int n, const unsigned* __restrict__ st4,
+__global__ void __launch_bounds__(kTPB) mis_emit(int n, const unsigned* st4,
                                                  unsigned char* __restrict__ out) {
   dep_wait();
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {

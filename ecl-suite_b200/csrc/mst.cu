@@ -174,8 +174,8 @@ __device__ __forceinline__ void mst_overflow(bool overflow, Status* status) {
 // now 9 and 13.
 template <bool kLight>
 __global__ void __launch_bounds__(kTPB, kLight ? 5 : 4) mst_scan(FlatCsr g, bool vec, const int* __restrict__ eweight,
-                                                 const int* __restrict__ parent, int4* __restrict__ wl, int cap, bool filter,
-                                                 MSTCtl* __restrict__ ctl, Status* __restrict__ status) {
+                                                 const int* parent, int4* __restrict__ wl, int cap, bool filter,
+                                                 MSTCtl* ctl, Status* __restrict__ status) {
   dep_wait();
   __shared__ int4 stage_buf[kTPB / 32][kStage];
   __shared__ __align__(16) int s_mark[kTPB / 32][kFlatTile];
@@ -191,21 +191,20 @@ __global__ void __launch_bounds__(kTPB, kLight ? 5 : 4) mst_scan(FlatCsr g, bool
       unsigned want = 0;  // bit k: entry k may be kept
 #pragma unroll
       for (int k = 0; k < kFlatLane; k++) {
-        if (row[k] < 0) continue;  // before the first row: not an entry of the graph
         if ((unsigned)u[k] >= (unsigned)g.n)
           raise(status, ECL_ERR_BAD_GRAPH, u[k]);
-        else if (u[k] > row[k])
+        else if (row[k] >= 0 && u[k] > row[k])
           want |= 1u << k;
       }
       int a[kFlatLane], b[kFlatLane], w[kFlatLane];
       if (!kLight) {
 #pragma unroll
-        for (int k = 0; k < kFlatLane; k++) b[k] = (want >> k) & 1u ? __ldg(&parent[u[k]]) : -1;  // race-free: not written in this launch
+        for (int k = 0; k < kFlatLane; k++) b[k] = (want >> k) & 1u ? parent[u[k]] : -1;  // race-free: not written in this launch
 #pragma unroll
         for (int k = 0; k < kFlatLane; k++) {
           a[k] = -1;
           if (!((want >> k) & 1u)) continue;
-          a[k] = k > 0 && row[k] == row[k - 1] && a[k - 1] >= 0 ? a[k - 1] : __ldg(&parent[row[k]]);  // race-free: as above
+          a[k] = k > 0 && row[k] == row[k - 1] && a[k - 1] >= 0 ? a[k - 1] : parent[row[k]];  // race-free: as above
           if (a[k] == b[k]) want &= ~(1u << k);
         }
       }

@@ -44,9 +44,10 @@ void set_last_error_msg(const char* msg);
   } while (0)
 
 // Launch of a kernel that follows another one in its stream and whose first
-// statement is dev::dep_wait(): the programmatic-serialization attribute lets
-// its blocks be placed as the last blocks of the kernel before it leave, and
-// the wait holds them until all that kernel's writes are visible.  A chain of
+// statement is dev::dep_wait() (where it says which loads such a kernel may
+// use): the programmatic-serialization attribute lets its blocks be placed as
+// the last blocks of the kernel before it leave, and the wait holds them until
+// all that kernel's writes are visible.  A chain of
 // twenty small kernels took 55 us so and 70 with plain launches, and twenty
 // passes over 32 MB 203 against 252 (the ends and the starts overlap).  No
 // kernel here signals before its end (that made the large passes slower,

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kTPB) scc_rows(int n, int m, const int* __rest
 }
 
 // Bound by the one read of the entries: the hash is about 20 instructions each.
-__global__ void __launch_bounds__(kTPB) scc_symmetry(FlatCsr g, bool vec, SCCCtl* __restrict__ ctl,
+__global__ void __launch_bounds__(kTPB) scc_symmetry(FlatCsr g, bool vec, SCCCtl* ctl,
                                                      Status* __restrict__ status) {
   dep_wait();
   __shared__ __align__(16) int s_mark[kTPB / 32][kFlatTile];
@@ -180,8 +180,8 @@ __global__ void __launch_bounds__(kTPB) scc_symmetry(FlatCsr g, bool vec, SCCCtl
 // the largest it will meet, and of a warp's lanes in the highest lane's
 // component only that lane counts: the giant component's word then takes one
 // access per warp of the launch, not one per vertex.
-__global__ void __launch_bounds__(kTPB) scc_top(int n, const int* __restrict__ comp, int* __restrict__ top,
-                                                const SCCCtl* __restrict__ ctl) {
+__global__ void __launch_bounds__(kTPB) scc_top(int n, const int* comp, int* __restrict__ top,
+                                                const SCCCtl* ctl) {
   dep_wait();
   if (ctl->asym != 0) return;  // as scc_mark
   const int lane = threadIdx.x & 31;
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kTPB) scc_top(int n, const int* __restrict__ c
   int seen = -1;  // component that this lane or, for it, its warp's highest lane dealt with last
   for (int q = groups - 1 - warp; q >= 0; q -= nwarps) {
     const int v = 32 * q + lane;
-    const int r = v < n ? __ldg(&comp[v]) : -1;
+    const int r = v < n ? comp[v] : -1;
     const unsigned in = __ballot_sync(kFull, r >= 0);
     const int top_lane = 31 - __clz(in);
     const int high = __shfl_sync(kFull, r, top_lane);
@@ -200,14 +200,14 @@ __global__ void __launch_bounds__(kTPB) scc_top(int n, const int* __restrict__ c
   }
 }
 
-__global__ void __launch_bounds__(kTPB) scc_relabel(int n, int* __restrict__ comp, const int* __restrict__ top,
-                                                    const SCCCtl* __restrict__ ctl, Status* __restrict__ status) {
+__global__ void __launch_bounds__(kTPB) scc_relabel(int n, int* comp, const int* top,
+                                                    const SCCCtl* ctl, Status* __restrict__ status) {
   dep_wait();
   if (ctl->asym != 0) return;  // as scc_mark
   if (blockIdx.x == 0 && threadIdx.x == 0) st(&status->rounds, 1);  // no sweep: one pass of hooking
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
     const int r = comp[v];
-    comp[v] = max(r, __ldg(&top[r]));
+    comp[v] = max(r, top[r]);
   }
 }
 
@@ -250,7 +250,7 @@ constexpr int kBackLong = 1024;   // ... backward, where most rows are left afte
 struct Giant {
   unsigned* fwd;  // bit per vertex: reached from the pivot
   unsigned* bwd;  // bit per vertex: reaches the pivot (complete inside fwd)
-  __device__ __forceinline__ bool has(const unsigned* bits, int v) const { return (__ldg(&bits[v >> 5]) >> (v & 31)) & 1u; }
+  __device__ __forceinline__ bool has(const unsigned* bits, int v) const { return (bits[v >> 5] >> (v & 31)) & 1u; }
   // After scc_giant's launch.
   __device__ __forceinline__ bool in(int v) const { return has(fwd, v) && has(bwd, v); }
 };
@@ -303,7 +303,7 @@ __device__ __forceinline__ void merge_bits(unsigned* bits, unsigned* next, int w
 __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* __restrict__ nindex,
                                                       const int* __restrict__ nlist, unsigned* fwd, unsigned* bwd,
                                                       unsigned* next, int* queue, int* candA, int* candB, int2* chunks,
-                                                      int chunk_cap, SCCCtl* __restrict__ ctl, bool checked,
+                                                      int chunk_cap, SCCCtl* ctl, bool checked,
                                                       Status* __restrict__ status) {
   if (checked && ctl->asym == 0) return;  // as scc_mark
   __shared__ int s_stage[kGTPB / 32][128];
@@ -682,7 +682,7 @@ template <bool kSearched>
 __global__ void __launch_bounds__(kTPB) scc_mark(int n, int m, const int* __restrict__ nindex,
                                                  const int* __restrict__ nlist, int* __restrict__ flags,
                                                  int2* __restrict__ wl, RowChunks rc, Bins bins, bool vec,
-                                                 Giant gi, SCCCtl* __restrict__ ctl, bool checked, Status* __restrict__ status) {
+                                                 Giant gi, SCCCtl* ctl, bool checked, Status* __restrict__ status) {
   dep_wait();
   if (checked && ctl->asym == 0) return;
   if (kSearched && ctl->giant_ok != 0)
@@ -695,7 +695,7 @@ template <bool kSearched>
 __global__ void __launch_bounds__(kTPB) scc_mark_chunks(int n, int m, const int* __restrict__ nindex,
                                                         const int* __restrict__ nlist, int* __restrict__ flags,
                                                         int2* __restrict__ wl, RowChunks rc, int chunk, bool vec,
-                                                        Giant gi, SCCCtl* __restrict__ ctl, bool checked,
+                                                        Giant gi, SCCCtl* ctl, bool checked,
                                                         Status* __restrict__ status) {
   dep_wait();
   if (checked && ctl->asym == 0) return;
@@ -721,7 +721,7 @@ struct SweepOcc {
 template <int kSweepBatch>
 __global__ void __launch_bounds__(kTPB, SweepOcc<kSweepBatch>::blocks) scc_solve(int n, int m0, int2* __restrict__ wlA, int2* __restrict__ wlB,
                                                   const int* __restrict__ flags, unsigned long long* __restrict__ io,
-                                                  int* __restrict__ label, Giant gi, SCCCtl* __restrict__ ctl,
+                                                  int* __restrict__ label, Giant gi, SCCCtl* ctl,
                                                   int max_rounds, bool checked,
                                                   Status* __restrict__ status) {
   if (checked && ld(&ctl->asym) == 0) return;  // as scc_mark
