@@ -635,7 +635,7 @@ __global__ void apsp_edges(int* __restrict__ A, long ld, int n, int m, const int
         raise(status, ECL_ERR_BAD_GRAPH, j);
         continue;
       }
-      A[(long)i * ld + u] = w;
+      A[(long)i * ld + u] = w;  // race-free: one thread writes a row, no reader in this launch
     }
   }
 }

@@ -191,7 +191,7 @@ __device__ __forceinline__ void cc_push_chunks(int v, int beg, int deg, int chun
   const int at = fetch_add(&ctr->nchunks, nc);
   for (int c = 0; c < nc; c++) {
     if ((unsigned)(at + c) < (unsigned)cap)
-      chunks[at + c] = make_int2(v, beg + c * chunk);
+      chunks[at + c] = make_int2(v, beg + c * chunk);  // race-free: the slot is this reservation's, no reader in this launch
     else
       raise(status, ECL_ERR_BAD_GRAPH, v);
   }
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kTPB) cc_chunks(int n, const int* __restrict__
   const int nwarps = (gridDim.x * kTPB) >> 5;
   const int total = cc_chunk_total(ctr, chunk_cap);
   for (int c = warp; c < total; c += nwarps) {
-    const int2 rec = chunks[c];
+    const int2 rec = chunks[c];  // race-free: not written in this launch
     const int v = rec.x;
     const int end = min(rec.y + chunk, __ldg(&nindex[v + 1]));
     int rv = -1;
@@ -354,6 +354,7 @@ __global__ void __launch_bounds__(kTPB) cc_flatten(int n, int* __restrict__ pare
       for (int k = 0; k < kFlattenBatch; k++)
         if (q[k] >= 0) {
           const long long v = v0 + (long long)k * stride;
+          // race-free: thread-owned, no reader in this launch
           ing[v] = q[k] == (kWhat == kMarkUnion ? gi.root[union_graph_of(gi.vbase, gi.ngraphs, (int)v)] : giant);
         }
     }
@@ -460,7 +461,7 @@ __global__ void __launch_bounds__(1024) cc_giant(int n, const int* parent, const
 // linked when u < v (the other direction is handled from u) or when u is in
 // the giant component (u skips its list entirely).
 __device__ __forceinline__ bool cc_rest_wanted(int u, int v, const unsigned char* ing) {
-  return u != v && (u < v || ing[u]);
+  return u != v && (u < v || ing[u]);  // race-free: not written in this launch
 }
 
 __global__ void __launch_bounds__(kTPB) cc_rest(int n, int m, const int* __restrict__ nindex,
@@ -476,7 +477,7 @@ __global__ void __launch_bounds__(kTPB) cc_rest(int n, int m, const int* __restr
   for (int base = warp * 32; base < n; base += nwarps * 32) {
     const int v = base + lane;
     int beg = 0, end = 0;
-    if (v < n && !ing[v]) cc_row(nindex, v, m, beg, end);
+    if (v < n && !ing[v]) cc_row(nindex, v, m, beg, end);  // race-free: not written in this launch
     const int deg = end - beg;
     if (deg > bins.chunk) {
       cc_push_chunks(v, beg, deg, bins.chunk, chunks, chunk_cap, ctr, status);
@@ -528,7 +529,7 @@ __global__ void __launch_bounds__(kTPB) cc_rest_chunks(int n, const int* __restr
   const int nwarps = (gridDim.x * kTPB) >> 5;
   const int total = cc_chunk_total(ctr, chunk_cap);
   for (int c = warp; c < total; c += nwarps) {
-    const int2 rec = chunks[c];
+    const int2 rec = chunks[c];  // race-free: not written in this launch
     const int v = rec.x;
     const int end = min(rec.y + chunk, __ldg(&nindex[v + 1]));
     int rv = -1;

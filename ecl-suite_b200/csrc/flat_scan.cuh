@@ -51,13 +51,13 @@ __device__ __forceinline__ void flat_rows_range(int n, int m, const int* nindex,
     }
     const bool many = t1 - t0 > 32;
     if (!many)
-      for (int t = t0; t < t1; t++) tilerow[t] = v;
+      for (int t = t0; t < t1; t++) tilerow[t] = v;  // race-free: a tile has one row, no reader in this launch
     unsigned todo = __ballot_sync(kFull, many);
     while (todo) {
       const int who = __ffs(todo) - 1;
       todo &= todo - 1;
       const int wv = __shfl_sync(kFull, v, who), w0 = __shfl_sync(kFull, t0, who), w1 = __shfl_sync(kFull, t1, who);
-      for (int t = w0 + lane; t < w1; t += 32) tilerow[t] = wv;
+      for (int t = w0 + lane; t < w1; t += 32) tilerow[t] = wv;  // race-free: as above
     }
   }
 }

@@ -68,7 +68,7 @@ struct GCCtl {
 // Priority hash of vertex x: the reference hashes the vertex id; in a union
 // of graphs (vhash != nullptr) it is the hash of x's LOCAL id, precomputed.
 __device__ __forceinline__ unsigned gc_h(const unsigned* vhash, int x) {
-  return vhash ? vhash[x] : ecl_hash((unsigned)x);
+  return vhash ? vhash[x] : ecl_hash((unsigned)x);  // race-free: not written in the launches that call this
 }
 
 // Entries per lane whose loads are issued together in the init scans.
@@ -87,7 +87,7 @@ __device__ __forceinline__ void gc_class_batch(const int (&u)[kInitBatch], const
 #pragma unroll
   for (int k = 0; k < kInitBatch; k++) {
     const bool ok = valid[k] && (unsigned)u[k] < (unsigned)n && u[k] != v;
-    ku[k] = ok ? keys[n - 1 - u[k]] : 0ull;
+    ku[k] = ok ? keys[n - 1 - u[k]] : 0ull;  // race-free: not written in this launch
   }
 #pragma unroll
   for (int k = 0; k < kInitBatch; k++) {
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kTPB) gc_union_hash(int n, const int* __restri
       if (__ldg(&vbase[mid]) <= v) lo = mid;
       else hi = mid - 1;
     }
-    vhash[v] = ecl_hash((unsigned)(v - __ldg(&vbase[lo])));
+    vhash[v] = ecl_hash((unsigned)(v - __ldg(&vbase[lo])));  // race-free: thread-owned, no reader in this launch
   }
 }
 
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kTPB) gc_init(int n, int m, const int* __restr
     int beg = 0, end = 0;
     if (v < n) csr_row(nindex, v, m, beg, end, status);
     const int dv = end - beg;
-    const unsigned long long kv = (v < n) ? keys[n - 1 - v] : 0ull;
+    const unsigned long long kv = (v < n) ? keys[n - 1 - v] : 0ull;  // race-free: not written in this launch
     int h = 0;
     push_chunks_warp(rc, bins.chunk, dv > bins.chunk, v, beg, end, status);
     if (v < n && dv <= bins.lane) {
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kTPB) gc_init(int n, int m, const int* __restr
         gc_class_batch(u, valid, v, kv, n, keys, status, cls);
 #pragma unroll
         for (int k = 0; k < kInitBatch; k++)
-          if (cls[k] == 1) nl2[beg + h++] = u[k];
+          if (cls[k] == 1) nl2[beg + h++] = u[k];  // race-free: v's own slot, no reader in this launch
       }
     }
     unsigned todo = __ballot_sync(kFull, dv > bins.lane && dv <= bins.chunk);
@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(kTPB) gc_init(int n, int m, const int* __restr
 #pragma unroll
         for (int k = 0; k < kInitBatch; k++) {
           const unsigned bh = __ballot_sync(kFull, cls[k] == 1);
+          // race-free: wv's own slot, no reader in this launch
           if (cls[k] == 1) nl2[wbeg + wh + __popc(bh & ((1u << lane) - 1))] = u[k];
           wh += __popc(bh);
         }
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(kTPB) gc_init_chunks(int n, int m, const int* 
     const int v = r.x;
     const int beg = __ldg(&nindex[v]), end = __ldg(&nindex[v + 1]);
     const int stop = min(r.y + chunk, end);
-    const unsigned long long kv = keys[n - 1 - v];
+    const unsigned long long kv = keys[n - 1 - v];  // race-free: not written in this launch
     warp_row(r.y, stop, m, vec, nlist, [&](const int(&)[4], const int (&u)[4], const bool (&valid)[4]) {
       int cls[kInitBatch];
       gc_class_batch(u, valid, v, kv, n, keys, status, cls);
@@ -211,6 +212,7 @@ __global__ void __launch_bounds__(kTPB) gc_init_chunks(int n, int m, const int* 
       hbase = __shfl_sync(kFull, hbase, 0);
 #pragma unroll
       for (int k = 0; k < kInitBatch; k++) {
+        // race-free: the places are this reservation's
         if (cls[k] == 1) nl2[beg + hbase + __popc(bh[k] & ((1u << lane) - 1))] = u[k];
         hbase += __popc(bh[k]);
       }
@@ -269,7 +271,7 @@ __global__ void __launch_bounds__(kTPB) gc_keys(int n, int m, const int* __restr
       key[k] = 0;
       if (i < n) {
         key[k] = ~(((unsigned long long)deg[k] << 32) | gc_h(vhash, v));
-        keys[i] = key[k];
+        keys[i] = key[k];  // race-free: thread-owned, no reader in this launch
         dmax = max(dmax, (int)min(deg[k], 0x7fffffffu));
         if (deg[k] == 0) color[v] = 0;  // race-free: the output, thread-owned; nothing reads it in this launch
       }
@@ -294,8 +296,8 @@ __global__ void __launch_bounds__(kTPB) gc_keys(int n, int m, const int* __restr
     for (int k = 0; k < kKeyBatch; k++) {
       if (deg[k] == 0) continue;
       const int at = s_base + s_woff[k * (kTPB / 32) + wid] + __popc(bal[k] & ((1u << lane) - 1));
-      skeys[at] = key[k];
-      svals[at] = n - 1 - (int)(bbase + k * kTPB + threadIdx.x);
+      skeys[at] = key[k];  // race-free: the place is this reservation's
+      svals[at] = n - 1 - (int)(bbase + k * kTPB + threadIdx.x);  // race-free: as above
     }
     __syncthreads();  // s_woff and s_base are rewritten next step
   }
@@ -589,6 +591,7 @@ __global__ void __launch_bounds__(kTPB) gc_core_rank(const int* order, int* __re
                                                      const GCCtl* ctl, int cap) {
   dep_wait();
   const int core = gc_core_size(ctl, cap);
+  // race-free: order is whole and has each vertex once
   for (int r = blockIdx.x * kTPB + threadIdx.x; r < core; r += gridDim.x * kTPB) rank[order[r]] = r;
 }
 
@@ -611,7 +614,7 @@ __global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict_
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
   for (int r = warp; r < core; r += nwarps) {
-    const int v = order[r];
+    const int v = order[r];  // race-free: not written in this launch
     const int b = __ldg(&nindex[v]), h = hc[v];  // race-free: not written in this launch
     const int first = (int)(((long long)b + 3) >> 2);  // 16-byte units
     unsigned short* out = reinterpret_cast<unsigned short*>(nl2) + (size_t)first * 8;
@@ -619,7 +622,7 @@ __global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict_
       const int i = i0 + lane;
       unsigned short q = 0;
       if (i < h) {
-        const int x = rank[nl2[(size_t)b + i]];
+        const int x = rank[nl2[(size_t)b + i]];  // race-free: rank is not written, nl2 by this warp in its own row
         if ((unsigned)x < (unsigned)r)
           q = (unsigned short)x;
         else  // only where a union's entry leaves its graph for a vertex of the same key
@@ -629,7 +632,7 @@ __global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict_
       if (i < h) out[i] = q;
       __syncwarp();
     }
-    if (lane == 0) rowinfo[r] = make_int4(first, h, v, 0);
+    if (lane == 0) rowinfo[r] = make_int4(first, h, v, 0);  // race-free: the warp's own, no reader in this launch
   }
 }
 
@@ -865,7 +868,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const
     if ((j & ~31) != jb) {
       jb = j & ~31;
       const int r = warp + cwarps * (jb + lane);
-      rec = r < core ? rowinfo[r] : make_int4(0, 0, -1, 0);
+      rec = r < core ? rowinfo[r] : make_int4(0, 0, -1, 0);  // race-free: not written in this launch
     }
     const int src = j & 31;
     return make_int4(__shfl_sync(kFull, rec.x, src), __shfl_sync(kFull, rec.y, src), __shfl_sync(kFull, rec.z, src),
@@ -1279,26 +1282,26 @@ extern "C" ecl_status ecl_gc_critical_path(const ecl_graph_view* g, int32_t core
     key[(size_t)v] = ((unsigned long long)deg << 32) | dev::ecl_hash((unsigned)v);
     nbig += deg > (unsigned)kWarpRow;
   }
-  std::vector<int> order((size_t)n);
-  for (int v = 0; v < n; v++) order[(size_t)v] = v;
-  std::sort(order.begin(), order.end(), [&](int a, int b) {
+  std::vector<int> by_rank((size_t)n);
+  for (int v = 0; v < n; v++) by_rank[(size_t)v] = v;
+  std::sort(by_rank.begin(), by_rank.end(), [&](int a, int b) {
     return key[(size_t)a] != key[(size_t)b] ? key[(size_t)a] > key[(size_t)b] : a > b;
   });
-  std::vector<int> rank((size_t)n);
-  for (int r = 0; r < n; r++) rank[(size_t)order[(size_t)r]] = r;
+  std::vector<int> place((size_t)n);
+  for (int r = 0; r < n; r++) place[(size_t)by_rank[(size_t)r]] = r;
   const int core = std::min(nbig, core_ranks > 0 ? core_ranks : kCoreDefault);
   std::vector<int> hop((size_t)n, 0);
   std::vector<double> path((size_t)n, 0.0);
   int best = 0, best_core = 0;
   double best_path = 0.0;
   for (int r = 0; r < n; r++) {
-    const int v = order[(size_t)r];
+    const int v = by_rank[(size_t)r];
     int h = -1;
     double t = -1.0;
     for (int i = nindex[v]; i < nindex[v + 1]; i++) {
       const int u = nlist[i];
       if (u < 0 || u >= n) return ECL_ERR_BAD_GRAPH;
-      if (u == v || rank[(size_t)u] > r) continue;
+      if (u == v || place[(size_t)u] > r) continue;
       h = std::max(h, hop[(size_t)u]);
       t = std::max(t, path[(size_t)u]);
     }

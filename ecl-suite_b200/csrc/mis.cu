@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(kTPB) mis_run(int n, int m, const int* __restr
     }
     const bool keep = wait || (go && verdict == kWait);
     const unsigned bal = __ballot_sync(kFull, keep);
+    // race-free: the warp's own
     if (kItems && keep) items[slot(kept + __popc(bal & ((1u << lane) - 1)))] = make_int4(v, pos, blocker, end);
     kept += __popc(bal);
   };

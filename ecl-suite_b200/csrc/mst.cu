@@ -372,7 +372,7 @@ __device__ __noinline__ void mst_solo(int4* list, int sz, int& r, int* parent, u
     }
     if (!__syncthreads_or(live)) break;
     for (int i = threadIdx.x; i < sz; i += kBorTPB) {
-      const int4 e = list[i];
+      const int4 e = list[i];  // race-free: this thread's own, relabelled before the block barrier
       if (e.x < 0) continue;
       const u64 key = ((u64)(unsigned)e.z << 32) | (unsigned)e.w;
       bool had;
@@ -391,7 +391,7 @@ __device__ __noinline__ void mst_solo(int4* list, int sz, int& r, int* parent, u
 #pragma unroll
       for (int k = 0; k < kSoloBatch; k++) {
         const int i = i0 + k * kBorTPB;
-        e[k] = i < sz ? list[i] : make_int4(-1, -1, 0, 0);
+        e[k] = i < sz ? list[i] : make_int4(-1, -1, 0, 0);  // race-free: not written in this phase
       }
 #pragma unroll
       for (int k = 0; k < kSoloBatch; k++) {
@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(kBorTPB, 1) mst_boruvka(int n, int pass, int4*
     for (long long i0 = tid - lane; i0 < nr; i0 += nthreads) {  // whole warps: they append together
       const long long i = i0 + lane;
       int v = -1;
-      if (i < nr) v = r == 0 ? (int)i : rin[i];
+      if (i < nr) v = r == 0 ? (int)i : rin[i];  // race-free: written before the grid barrier
       bool root = false;
       if (v >= 0 && ld(&minv[v]) != ~0ull) {  // took part in this round
         st(&minv[v], ~0ull);
@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(kBorTPB, 1) mst_boruvka(int n, int pass, int4*
     while (left) {
       left = false;
       for (long long i = tid; i < nr; i += nthreads) {
-        const int v = r == 0 ? (int)i : rin[i];
+        const int v = r == 0 ? (int)i : rin[i];  // race-free: as above
         const int p = ld(&parent[v]);
         left |= p != v && !mst_jump(v, p, parent);
       }

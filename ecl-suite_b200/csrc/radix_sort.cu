@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
 #pragma unroll
       for (int j = 0; j < kItems; j++) {
         const int i = j < per ? i0 + 32 * j : end;
-        k[j] = i < end ? kin[i] : 0ull;  // written before the last grid barrier
-        if (values) v[j] = i < end ? vin[i] : 0;
+        k[j] = i < end ? kin[i] : 0ull;  // race-free: written before the last grid barrier
+        if (values) v[j] = i < end ? vin[i] : 0;  // race-free: as above
       }
       for (int d = lane; d < kDigits / 2; d += 32) reinterpret_cast<unsigned*>(s_warp[warp])[d] = 0;
       __syncwarp();
@@ -190,8 +190,8 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
         if (j >= per || i0 + 32 * j >= end) continue;
         const int d = digit_of(k[j], shift);
         const unsigned pos = s_base[d] + s_warp[warp][d] + rank[j];
-        if (!last || skip > 0) kout[pos] = k[j];
-        vout[pos] = v[j];
+        if (!last || skip > 0) kout[pos] = k[j];  // race-free: a place has one key, read behind the next grid barrier
+        vout[pos] = v[j];  // race-free: as above
       }
       __syncthreads();
       if (!one && quarter == 0) s_base[dig] += tile;
@@ -207,19 +207,19 @@ __global__ void __launch_bounds__(kThreads, 1) rs_sort(unsigned long long* k0, i
   const unsigned long long* kin = (passes & 1) ? k1 : k0;
   const int* vin = (passes & 1) ? v1 : v0;
   for (int i = blockIdx.x * kThreads + threadIdx.x; i < n; i += blocks * kThreads) {
-    const unsigned long long key = kin[i];  // written before the last grid barrier
+    const unsigned long long key = kin[i];  // race-free: written before the last grid barrier
     int pos = i;
     for (int j = i - 1; j >= 0; j--) {
-      const unsigned long long x = kin[j];
+      const unsigned long long x = kin[j];  // race-free: as above
       if ((x ^ key) >> (8 * skip)) break;
       pos -= x > key;
     }
     for (int j = i + 1; j < n; j++) {
-      const unsigned long long x = kin[j];
+      const unsigned long long x = kin[j];  // race-free: as above
       if ((x ^ key) >> (8 * skip)) break;
       pos += x < key;
     }
-    order[pos] = vin[i];
+    order[pos] = vin[i];  // race-free: a place has one key; vin as above
   }
 }
 

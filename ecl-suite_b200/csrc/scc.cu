@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kTPB) scc_top(int n, const int* comp, int* __r
   int seen = -1;  // component that this lane or, for it, its warp's highest lane dealt with last
   for (int q = groups - 1 - warp; q >= 0; q -= nwarps) {
     const int v = 32 * q + lane;
-    const int r = v < n ? comp[v] : -1;
+    const int r = v < n ? comp[v] : -1;  // race-free: not written in this launch
     const unsigned in = __ballot_sync(kFull, r >= 0);
     const int top_lane = 31 - __clz(in);
     const int high = __shfl_sync(kFull, r, top_lane);
@@ -206,8 +206,8 @@ __global__ void __launch_bounds__(kTPB) scc_relabel(int n, int* comp, const int*
   if (ctl->asym != 0) return;  // as scc_mark
   if (blockIdx.x == 0 && threadIdx.x == 0) st(&status->rounds, 1);  // no sweep: one pass of hooking
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
-    const int r = comp[v];
-    comp[v] = max(r, top[r]);
+    const int r = comp[v];  // race-free: thread-owned
+    comp[v] = max(r, top[r]);  // race-free: thread-owned; top is not written in this launch
   }
 }
 
@@ -250,6 +250,7 @@ constexpr int kBackLong = 1024;   // ... backward, where most rows are left afte
 struct Giant {
   unsigned* fwd;  // bit per vertex: reached from the pivot
   unsigned* bwd;  // bit per vertex: reaches the pivot (complete inside fwd)
+  // race-free: not written where this is called
   __device__ __forceinline__ bool has(const unsigned* bits, int v) const { return (bits[v >> 5] >> (v & 31)) & 1u; }
   // After scc_giant's launch.
   __device__ __forceinline__ bool in(int v) const { return has(fwd, v) && has(bwd, v); }
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
   if (tid == 0) {
     fetch_or(&fwd[pivot >> 5], 1u << (pivot & 31));
     fetch_or(&bwd[pivot >> 5], 1u << (pivot & 31));
-    queue[0] = pivot;
+    queue[0] = pivot;  // race-free: one thread, read behind the next grid barrier
   }
   if (!grid_sync(&ctl->giant_bar, status)) return;
   int qs = 0, qe = 1, level = 0;
@@ -350,7 +351,7 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
     const RowChunks rc{chunks, &ctl->level_chunks[level], chunk_cap};
     for (int i0 = qs + warp * 32; i0 < qe; i0 += nwarps * 32) {
       const int i = i0 + lane;
-      const int v = i < qe ? queue[i] : 0;  // written before the last grid barrier
+      const int v = i < qe ? queue[i] : 0;  // race-free: written before the last grid barrier
       int beg = 0, deg = 0;
       if (i < qe) row_of(v, beg, deg);
       push_chunks_warp(rc, kGiantLong, deg > kGiantLong, v, beg, beg + deg, status);
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
     if (level + 1 == kGiantLevels || (level == kGiantPatience && qe < n / 64)) return;  // long distances: not this way
     const int nch = chunk_total(RowChunks{chunks, &ctl->level_chunks[level], chunk_cap});
     for (int c = warp; c < nch; c += nwarps) {
-      const int2 r = chunks[c];
+      const int2 r = chunks[c];  // race-free: written before the last grid barrier
       const int end = min(r.y + kGiantLong, __ldg(&nindex[r.x + 1]));
       constexpr int K = kGiantLong / 32;
       int vv[K], j[K];
@@ -407,7 +408,7 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
     const int per = min(32, (qe - qs - 1) / nwarps + 1);
     for (int i0 = qs + warp * per; i0 < qe; i0 += nwarps * per) {
       const int i = lane < per ? i0 + lane : qe;
-      const int v = i < qe ? queue[i] : 0;  // written before the last grid barrier
+      const int v = i < qe ? queue[i] : 0;  // race-free: written before the last grid barrier
       int beg = 0, deg = 0;
       if (i < qe) row_of(v, beg, deg);
       if (deg > kGiantLong) deg = 0;  // in chunk records
@@ -450,7 +451,7 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
     const int per = min(32, (cnt - 1) / nwarps + 1);
     for (int i0 = warp * per; i0 < cnt; i0 += nwarps * per) {
       const int i = lane < per ? i0 + lane : cnt;
-      const int v = i < cnt ? in[i] : 0;  // written before the last grid barrier
+      const int v = i < cnt ? in[i] : 0;  // race-free: written before the last grid barrier
       int beg = 0, deg = 0;
       if (i < cnt && !reaches(v)) row_of(v, beg, deg);
       bool found = false;
@@ -504,7 +505,7 @@ __global__ void __launch_bounds__(kGTPB, 3) scc_giant(int n, int m, const int* _
     if (!grid_sync(&ctl->giant_bar, status)) return;
     const int nch = chunk_total(RowChunks{chunks, &ctl->back_chunks[round], chunk_cap});
     for (int c = warp; c < nch; c += nwarps) {
-      const int2 r = chunks[c];  // written before the grid barrier
+      const int2 r = chunks[c];  // race-free: written before the last grid barrier
       if (reaches_now(r.x)) continue;
       const int end = min(r.y + kGiantLong, __ldg(&nindex[r.x + 1]));
       constexpr int K = kGiantLong / 32;
@@ -828,7 +829,7 @@ __global__ void __launch_bounds__(kTPB, SweepOcc<kSweepBatch>::blocks) scc_solve
           for (int k = 0; k < kSweepBatch; k++) {
             const bool keep = A[k] != kDead && io_in(A[k]) != io_out(A[k]) && A[k] == B[k];
             const int at = warp_append(&ctl->kept[sweep], keep);
-            if (keep && at < m0) nxt[at] = e[k];
+            if (keep && at < m0) nxt[at] = e[k];  // race-free: the place is this reservation's, read behind a grid barrier
           }
         }
       }
@@ -856,14 +857,14 @@ __global__ void __launch_bounds__(kTPB, SweepOcc<kSweepBatch>::blocks) scc_solve
           bool keep = false;
           int2 e = make_int2(0, 0);
           if (i < size) {
-            e = cur[i];
+            e = cur[i];  // race-free: not written in this round
             if ((unsigned)e.x < (unsigned)n && (unsigned)e.y < (unsigned)n) {
               const unsigned long long A = ld(&io[e.x]);
               keep = A != kDead && io_in(A) != io_out(A) && A == ld(&io[e.y]);
             }
           }
           const int at = warp_append(&ctl->kept[sweep - 1], keep);
-          if (keep && at < m0) nxt[at] = e;
+          if (keep && at < m0) nxt[at] = e;  // race-free: the place is this reservation's, read behind a grid barrier
         }
         if (!grid_sync(&ctl->bar, status)) return;
         break;
