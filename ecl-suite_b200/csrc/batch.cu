@@ -500,9 +500,16 @@ ecl_status ecl_batch_tune(ecl_batch* b, int32_t trials, ecl_tune* best) {
     std::vector<float> values;
     void (*set)(ecl_tune&, float);
   };
+  // MST's split starts from the default for the batch's average degree.
+  int64_t n = 0, m = 0;
+  for (const Super& s : b->sup) n += s.n, m += s.m;
+  const int avg = (int)std::min<int64_t>(m / std::max<int64_t>(n, 1), INT32_MAX);
+  std::vector<float> light = {mst_default_light(1, avg)};
+  for (float f : {0.75f, 1.5f, 3.f, 0.4f})
+    if (f != light[0]) light.push_back(f);
   const std::vector<Knob> knobs = {
       {true, {64.f, 32.f, 16.f, 8.f}, [](ecl_tune& t, float v) { t.blocks_per_sm = (int32_t)v; }},
-      {(b->codes & ECL_BATCH_MST) != 0, {0.75f, 1.5f, 3.f}, [](ecl_tune& t, float v) { t.mst_light_factor = v; }},
+      {(b->codes & ECL_BATCH_MST) != 0, light, [](ecl_tune& t, float v) { t.mst_light_factor = v; }},
       {true, {32.f, 16.f, 8.f}, [](ecl_tune& t, float v) { t.row_lane_max = (int32_t)v; }},
       {true, {256.f, 128.f, 512.f, 2048.f}, [](ecl_tune& t, float v) { t.row_chunk = (int32_t)v; }},
       {(b->codes & ECL_BATCH_GC) != 0, {8192.f, 4096.f, 16384.f}, [](ecl_tune& t, float v) { t.gc_core_ranks = (int32_t)v; }},

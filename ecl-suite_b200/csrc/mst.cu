@@ -10,7 +10,7 @@
 //
 // B200 design:
 //  * mst_threshold: one block of mst_init samples 1024 weights and picks
-//    the quantile that leaves ~0.75 n (2 n in a sparse graph) light CSR
+//    the quantile that leaves ~0.75 n (1.5 n in a sparse graph) light CSR
 //    entries, with no host round trip; below 4 entries a vertex there is one
 //    pass over all entries instead of a light and a heavy one;
 //  * mst_scan: builds a worklist of int4 {a, b, weight, j} from the CSR in
@@ -45,12 +45,13 @@ typedef unsigned long long u64;
 constexpr int kTPB = 256;
 constexpr int kMaxRounds = 64;
 // Light entries aimed at, in multiples of n: 0.75 from this average degree on,
-// 2 below.  Rounds whose list does not shrink cost most; in a sparse random
+// 1.5 below.  Rounds whose list does not shrink cost most; in a sparse random
 // graph the light edges have to join most vertices (about n of them) before
-// the heavy pass drops the bulk of its entries in the scan, while a dense
-// power-law graph's hubs do that with few.  Measured, 0.75 / 1.5 / 2.5: G(3 M,
-// 12 M) 2.06 / 1.12 / 1.09 ms, G(150 k, 600 k) 0.314 / 0.302 / 0.299, R-MAT-22
-// (degree 30) 1.67 / 1.69 / 1.78.
+// the heavy pass drops the bulk of its entries in the scan, while a power-law
+// graph's hubs do that with few.  Measured, 0.75 / 1.5 / 2: G(3 M, 12 M) 1.94 /
+// 1.02 / 0.95 ms, G(1 M, 3 M) 0.65 / 0.50 / 0.45, G(150 k, 600 k) 0.274 / 0.272 /
+// 0.269, R-MAT-22 of degree 7 0.83 / 0.89 / 0.98, of degree 15 (scale 20) 0.455 /
+// 0.443 / 0.472, of degree 30 1.67 / 1.69 / 1.78.
 constexpr int kDenseDegree = 16;
 constexpr int kSamples = 1024;
 
@@ -634,6 +635,8 @@ void mst_layout(Carve& c, int n, int m, bool symmetric, MSTBufs* b) {
 
 }  // namespace
 
+float mst_default_light(int n, int m) { return m / n >= kDenseDegree ? 0.75f : 1.5f; }
+
 size_t mst_workspace_bytes(int n, int m) {
   Carve c;
   MSTBufs b;
@@ -665,7 +668,7 @@ ecl_status mst_enqueue(const GraphDev& g, unsigned char* in_mst, char* ws, Statu
   // No light pass below 4 entries a vertex: all weights pass the first scan,
   // and the second would find nothing.
   const bool filter = g.m / g.n >= 4;
-  const float light = dev.mst_light_factor > 0.f ? dev.mst_light_factor : (g.m / g.n >= kDenseDegree ? 0.75f : 2.f);
+  const float light = dev.mst_light_factor > 0.f ? dev.mst_light_factor : mst_default_light(g.n, g.m);
   ECL_LAUNCH_NEXT(mst_init, grid + filter, kTPB, 0, stream, g.n, g.m, g.nindex, b.parent, b.minv, b.tilerow, g.eweight,
                   b.ctl, light, filter, status);
   if (g.m > 0) {

@@ -47,6 +47,7 @@ size_t mis_workspace_bytes(int n, int m);
 size_t mis_small_workspace_bytes(int n);
 size_t gc_workspace_bytes(int n, int m, bool uni = false);  // uni: for a union's hashes too
 size_t mst_workspace_bytes(int n, int m);
+float mst_default_light(int n, int m);  // the light factor where no knob sets one
 size_t scc_workspace_bytes(int n, int m);
 
 // `off` (symmetric graphs): a device word that launches before these write; not

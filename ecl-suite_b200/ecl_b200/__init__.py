@@ -416,13 +416,22 @@ BATCH_CC, BATCH_MIS, BATCH_GC, BATCH_MST, BATCH_SCC = 0x1, 0x2, 0x4, 0x8, 0x10
 class Tune(C.Structure):
     """ecl_tune: launch knobs (0 = built-in default); they never change results."""
 
-    _fields_ = [("blocks_per_sm", C.c_int32), ("mst_light_factor", C.c_float), ("gc_core_ranks", C.c_int32),
+    _fields_ = [("blocks_per_sm", C.c_int32), ("mst_light_factor_f32", C.c_float), ("gc_core_ranks", C.c_int32),
                 ("row_lane_max", C.c_int32), ("row_chunk", C.c_int32), ("scc_sweep_batch", C.c_int32),
                 ("gc_poll_ns", C.c_int32), ("row_vec", C.c_int32),
                 ("gc_pull_blocks", C.c_int32), ("gc_core_ctas", C.c_int32)]
 
+    @property
+    def mst_light_factor(self) -> float:
+        """As it was set: the shortest decimal that is this C float (0.4, not 0.4000000059604645)."""
+        return float(str(np.float32(self.mst_light_factor_f32)))
+
+    @mst_light_factor.setter
+    def mst_light_factor(self, value: float) -> None:
+        self.mst_light_factor_f32 = value
+
     def as_dict(self):
-        return {name: getattr(self, name) for name, _ in self._fields_}
+        return {name: getattr(self, name) for name in (f.removesuffix("_f32") for f, _ in self._fields_)}
 
 
 _sig("ecl_set_tune", C.c_int, [C.POINTER(Tune)])

@@ -90,7 +90,7 @@ typedef struct ecl_opts {
 typedef struct ecl_tune {
   int32_t blocks_per_sm;  /* blocks of 256 threads per SM in the grid-stride kernels' grids, 1..128; 0 = 64 */
   float mst_light_factor; /* MST light-edge target, in multiples of n; 0 = 0.75 from 16 entries a vertex
-                             on, else 2 */
+                             on, else 1.5 */
   int32_t gc_core_ranks;  /* GC: leading ranks coloured in shared memory (the core), 0..36864; 0 = 8192 */
   int32_t row_lane_max;   /* row scans (not MST's, which go by entries): rows of at most this many entries go
                              to one lane, 0..32; 0 = per code */
