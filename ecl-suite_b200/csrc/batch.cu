@@ -82,14 +82,7 @@ __global__ void __launch_bounds__(256) batch_mst_totals(int ngraphs, int m, cons
   const int tiles = m / kTotalsTile + (m % kTotalsTile != 0);
   for (int t = warp; t < tiles; t += nwarps) {
     const int e0 = t * kTotalsTile, e1 = min(m - e0, kTotalsTile) + e0;
-    int g = 0, hi = ngraphs - 1;  // the last graph that starts at or before e0
-    while (g < hi) {
-      const int mid = (g + hi + 1) >> 1;
-      if (__ldg(&ebase[mid]) <= e0)
-        g = mid;
-      else
-        hi = mid - 1;
-    }
+    int g = union_graph_of(ebase, ngraphs, e0);
     for (int b = e0; b < e1; g++) {
       const int e = min(e1, __ldg(&ebase[g + 1]));
       unsigned long long s = 0;

@@ -82,7 +82,8 @@ __device__ __forceinline__ T fetch_and(T* p, T v) {
 // Read-only input loads (never written during a solve).
 __device__ __forceinline__ int ldg(const int* p) { return __ldg(p); }
 
-// Graph of union vertex v: the last g with vbase[g] <= v (binary search).
+// Graph of union vertex v: the last g with vbase[g] <= v (binary search); of
+// union entry v with the graphs' entry bases.
 __device__ __forceinline__ int union_graph_of(const int* vbase, int ngraphs, int v) {
   int lo = 0, hi = ngraphs - 1;
   while (lo < hi) {

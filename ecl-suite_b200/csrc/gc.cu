@@ -106,13 +106,8 @@ __global__ void __launch_bounds__(kTPB) gc_union_hash(int n, const int* __restri
                                                       unsigned* __restrict__ vhash) {
   dep_wait();
   for (int v = blockIdx.x * kTPB + threadIdx.x; v < n; v += gridDim.x * kTPB) {
-    int lo = 0, hi = ngraphs - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(&vbase[mid]) <= v) lo = mid;
-      else hi = mid - 1;
-    }
-    vhash[v] = ecl_hash((unsigned)(v - __ldg(&vbase[lo])));  // race-free: thread-owned, no reader in this launch
+    const int base = __ldg(&vbase[union_graph_of(vbase, ngraphs, v)]);
+    vhash[v] = ecl_hash((unsigned)(v - base));  // race-free: thread-owned, no reader in this launch
   }
 }
 
