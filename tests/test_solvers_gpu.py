@@ -651,6 +651,30 @@ def test_scc_hubs_behind_the_giant_component(ecl, orc, k, back):
     assert np.array_equal(ecl.scc(g.to_device()).cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("reached", [False, True])
+@pytest.mark.parametrize("back", [False, True])
+def test_scc_rows_at_the_ends_of_chunk_records(ecl, orc, reached, back):
+    """Rows of exactly one and two records of the search (256 entries) and of the
+    mark pass (128), and one entry less and more, whose last entry decides: it
+    closes a cycle of the row's vertex and, with `back`, leads to the pivot."""
+    rng = np.random.default_rng(5)
+    n, sizes = 1500000, [127, 128, 129, 255, 256, 257, 383, 384, 385, 511, 512, 513]
+    ends = lambda size: 100 + rng.permutation(n - 200)[:size]  # noqa: E731
+    u, v = [np.zeros(1200000), np.arange(32)], [ends(1200000), np.arange(1, 33) % 32]
+    for i, k in enumerate(sizes):
+        u += [np.full(k, 40 + i), [n - 1 - i]]
+        v += [np.append(ends(k - 1), n - 1 - i), [40 + i]]
+        if reached:
+            u, v = u + [[3]], v + [[40 + i]]
+        if back:
+            u, v = u + [[n - 1 - i]], v + [[9]]
+    g = directed(ecl, n, np.concatenate(u), np.concatenate(v))
+    assert [int(g.nindex[40 + i + 1] - g.nindex[40 + i]) for i in range(len(sizes))] == sizes
+    want = orc.scc(g)
+    assert want[40] == n - 1 and (want[0] == n - 1) == (reached and back)
+    assert np.array_equal(ecl.scc(g.to_device()).cpu().numpy(), want)
+
+
 def test_scc_hubs_that_do_not_reach_the_pivot_are_shared_by_all_warps(ecl):
     """Hubs of 0.5 M entries each cost a pass over their entries, not a warp's
     walk through a row in every round (that: 7 ms a row and round)."""

@@ -92,3 +92,46 @@ for k in range(3):
     assert rt.cudaDeviceReset() == 0
 print("done")
 """)
+
+
+@pytest.mark.parametrize("threads", ["1", "3", "4", "8"])
+def test_copies_with_any_number_of_host_threads(threads):
+    """Below four host threads every copy is plain, from four on they fill the
+    blocks; the results are the same."""
+    run("""
+for n in (65537, 262145, 1350001):
+    check(*graph(n))
+print("done")
+""", OMP_NUM_THREADS=threads)
+
+
+@pytest.mark.parametrize("users", [1, 4, 5, 9])  # as many as there are blocks, and more
+def test_blocks_shared_by_threads(users):
+    """Every call of every thread goes through and is right; an exception in a
+    thread ends the test."""
+    run(f"""
+from concurrent.futures import ThreadPoolExecutor
+
+graphs = [graph(n) for n in (65537, 262145, 300001, 1048577)]
+with ThreadPoolExecutor({users}) as pool:
+    jobs = [pool.submit(check, *graphs[(k + i) % len(graphs)]) for k in range({users}) for i in range(2 * len(graphs))]
+    assert sum(j.result() for j in jobs) == {users} * 2 * len(graphs)
+print("done")
+""", OMP_NUM_THREADS="4")
+
+
+def test_page_locked_arrays_are_copied_as_they_are():
+    run("""
+import torch
+
+g, want, total = graph(300001)
+pin = lambda a: torch.from_numpy(a).pin_memory().numpy()
+locked = ecl.Graph(pin(g.nindex), pin(g.nlist), pin(g.eweight), True)
+out = torch.empty(g.nodes, dtype=torch.int32).pin_memory().numpy()
+ecl.cc(locked, out=out)
+assert np.array_equal(out, want)
+for _ in range(2):
+    check(locked, want, total)
+    check(g, want, total)
+print("done")
+""", OMP_NUM_THREADS="4")
