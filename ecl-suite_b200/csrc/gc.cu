@@ -61,7 +61,8 @@ struct GCCtl {
   int maxdeg;      // largest degree: how many digits of it the sort looks at
   int sort_failed;  // the sort gave up: the order is not whole, and nothing is indexed by it
   int bad_rows;  // some row is malformed, so rows may overlap
-  int pad2[26];
+  int nwide;     // core rows of more than two segments
+  int pad2[25];
   GridBarrier sort_bar;
 };
 
@@ -532,8 +533,8 @@ __device__ int gc_short_row(int beg, int h, const int* nl2, const int* color, St
 // that mark the same colour store the same value.
 //
 // On the chain lies what a warp does between its last neighbour's colour and its
-// own, among 31 other warps' polls.  So all of a row is scanned before any wait
-// (two segments; a longer row's third behind them), the search for the smallest
+// own, among 31 other warps' polls.  So all of a row is scanned before any wait,
+// the search for the smallest
 // colour starts where it ended before the wait, and the marks are cleared and the
 // next row fetched behind the publication.  Measured, core, a lane polling its
 // lowest entry after each segment, 1016 colours a window and the search from 0 ->
@@ -552,15 +553,17 @@ constexpr int kSegMax = 1024;           // entries per segment: a bit each of a 
 constexpr unsigned kUncoloured = 0xffffu;
 constexpr int kWin = 2032;              // colours of a mark window; a byte behind it takes what is outside
 constexpr int kMarkBytes = 2048;
+constexpr int kCorePend = 256;          // undecided entries that a warp's list holds (rows of more than two segments)
 constexpr int kFromRow = 512;           // rows from which on the search starts ahead (a shorter row's marks are one load)
 constexpr size_t kCoreSmemLimit = 227 * 1024;
 
 // Dynamic shared memory of a core CTA: colours (16-bit, per rank), then per
-// warp two mbarriers, two staging buffers of `seg` entries and the mark bytes.
+// warp two mbarriers, two staging buffers of `seg` entries, the mark bytes and
+// the list of undecided entries.
 // The buffers take what the colours leave, up to kSegMax entries.
 __host__ __device__ constexpr size_t gc_core_colour_bytes(int cap) { return ((size_t)cap * 2 + 15) & ~size_t(15); }
 __host__ __device__ constexpr size_t gc_core_warp_bytes(int seg) {
-  return 2 * sizeof(unsigned long long) + (size_t)seg * 2 * sizeof(unsigned short) + kMarkBytes;
+  return 2 * sizeof(unsigned long long) + ((size_t)seg * 2 + kCorePend) * sizeof(unsigned short) + kMarkBytes;
 }
 __host__ __device__ constexpr int gc_core_seg(int cap) {
   const size_t fixed = gc_core_colour_bytes(cap) + kCoreWarps * gc_core_warp_bytes(0);
@@ -601,7 +604,7 @@ __global__ void __launch_bounds__(kTPB) gc_core_rank(const int* order, int* __re
 __global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict__ nindex, int* nl2,
                                                           const int* hc, const int* order,
                                                           const int* rank, int4* __restrict__ rowinfo,
-                                                          const GCCtl* ctl, int cap,
+                                                          GCCtl* ctl, int cap,
                                                           Status* __restrict__ status) {
   dep_wait();
   const int lane = threadIdx.x & 31;
@@ -628,6 +631,7 @@ __global__ void __launch_bounds__(kTPB) gc_core_translate(const int* __restrict_
       __syncwarp();
     }
     if (lane == 0) rowinfo[r] = make_int4(first, h, v, 0);  // race-free: the warp's own, no reader in this launch
+    if (lane == 0 && h > 2 * gc_core_seg(cap)) fetch_add(&ctl->nwide, 1);
   }
 }
 
@@ -780,38 +784,87 @@ __device__ int gc_core_far(const unsigned short* row, int h, const unsigned shor
   }
 }
 
+// The undecided entries of two segments (masks open0, open1 of those at sg0, sg1)
+// behind the `np` ranks of the warp's list: its new length, or -1 when they do not
+// fit.
+__device__ __forceinline__ int gc_core_keep(unsigned open0, unsigned open1, const unsigned short* sg0,
+                                         const unsigned short* sg1, unsigned short* pend, int np) {
+  const int lane = threadIdx.x & 31;
+  const int mine = __popc(open0) + __popc(open1);
+  int at = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(kFull, at, o);
+    if (lane >= o) at += x;
+  }
+  const int total = __shfl_sync(kFull, at, 31);
+  if (np + total > kCorePend) return -1;
+  at += np - mine;
+  for (int part = 0; part < 2; part++) {
+    const unsigned short* sg = part ? sg1 : sg0;
+    for (unsigned open = part ? open1 : open0; open; open &= open - 1) {
+      const int k = __ffs(open) - 1;
+      pend[at++] = sg[256 * (k >> 3) + 8 * lane + (k & 7)];
+    }
+  }
+  __syncwarp();
+  return np + total;
+}
+
+// Waits for the ranks in the warp's list and marks their colours; true on a stall.
+__device__ __forceinline__ bool gc_core_settle(const unsigned short* pend, int np, const unsigned short* col_s,
+                                            unsigned char* marks, unsigned beyond, int r, Status* status) {
+  bool lost = false;
+  unsigned spins = 0;
+  unsigned long long t0 = 0;
+  for (int j = threadIdx.x & 31; j < np && !lost; j += 32) {
+    const unsigned short* p = &col_s[pend[j]];
+    unsigned c;
+    while ((c = col_ld(p)) == kUncoloured) {
+      if ((++spins & 1023u) != 0) continue;
+      if (t0 == 0) t0 = gc_now();
+      if (gc_now() - t0 > kStallNs || ld(&status->code) != 0) {
+        raise(status, ECL_ERR_NO_CONVERGENCE, r);
+        lost = true;
+        break;
+      }
+    }
+    if (!lost) marks[min(c, beyond)] = 1;
+  }
+  return __any_sync(kFull, lost);
+}
+
 // Per-warp staging of row segments: two buffers, each with its mbarrier and
 // the parity of its next phase.  A segment starts at a 16-byte unit of the
 // packed rows and has at most the buffer's entries; the copy is rounded up to
 // 16 bytes (the row's slot has room).
 struct CoreStage {
-  unsigned short* base;        // the buffers, `seg` entries each
-  unsigned long long* bars;
+  unsigned short* base;  // the buffers, `seg` entries each; the mbarriers lie before them, the marks behind
   int seg;
-  unsigned parity = 0;         // bit b: of buffer b's next phase
-  int first0 = -1, first1 = -1;  // segment in each buffer (-1: none in flight)
+  unsigned state = 0;  // bit b: parity of buffer b's next phase; bit 2 + b: a copy into it is in flight
 
-  // (no arrays: indexed by b they would live in local memory, whose loads lay on
-  // the chain)
+  // (as few registers as can be, and no arrays, which would lie in local memory:
+  // both cost on the chain)
   __device__ __forceinline__ unsigned short* buf(int b) const { return base + (b ? seg : 0); }
-  __device__ __forceinline__ int first(int b) const { return b ? first1 : first0; }
-  __device__ __forceinline__ void set_first(int b, int unit) { (b ? first1 : first0) = unit; }
+  __device__ __forceinline__ unsigned long long* bar(int b) const {
+    return reinterpret_cast<unsigned long long*>(base) - 2 + b;
+  }
+  __device__ __forceinline__ unsigned char* marks() const { return reinterpret_cast<unsigned char*>(base + 2 * seg); }
   __device__ __forceinline__ void issue(int b, const int* nl2, int unit, int len) {
-    set_first(b, unit);
+    state |= 4u << b;
     if ((threadIdx.x & 31) == 0)
-      bulk_load(buf(b), reinterpret_cast<const char*>(nl2) + (size_t)unit * 16, (2u * (unsigned)len + 15u) & ~15u, bars + b);
+      bulk_load(buf(b), reinterpret_cast<const char*>(nl2) + (size_t)unit * 16, (2u * (unsigned)len + 15u) & ~15u, bar(b));
   }
   // Waits for buffer b's copy.  False when the wait ran out.
   __device__ __forceinline__ bool wait(int b) {
-    const bool ok = mbar_wait(bars + b, (parity >> b) & 1u);
-    if (ok) parity ^= 1u << b;  // a copy that did not land stays listed for drain()
+    const bool ok = mbar_wait(bar(b), (state >> b) & 1u);
+    if (ok) state ^= 5u << b;  // a copy that did not land stays listed for drain()
     return ok;
   }
   // Bounded wait for every copy still in flight (before leaving on an error).
   __device__ __forceinline__ void drain() {
-    if (first0 >= 0) wait(0);
-    if (first1 >= 0) wait(1);
-    first0 = first1 = -1;
+    if (state & 4u) wait(0);
+    if (state & 8u) wait(1);
   }
 };
 
@@ -824,10 +877,14 @@ struct CoreStage {
 // any 16-bit value in a row; 2 * 0xffff bytes is inside this CTA's shared
 // memory for every core size, and a wait on what is read there ends on the
 // status word.
-__global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const int4* rowinfo,
-                                                           int* __restrict__ color, const GCCtl* ctl,
-                                                           int cap, Status* __restrict__ status) {
-  dep_wait();
+// kWide: for cores with many rows of more than two segments, whose undecided
+// entries go to a list.  A form of its own, as it costs each hop of any row: a
+// sixteenth of the rows have to be such.  Measured, core, without / with the list:
+// R-MAT-22 1.22 / 1.59 ms, a clique of 500 vertices 0.30 / 0.39, of 5000 47 / 40, a
+// complete 40-partite graph of 4000 5.7 / 3.4.
+template <bool kWide>
+__device__ __forceinline__ void gc_core_run(const int* nl2, const int4* rowinfo, int* color, const GCCtl* ctl, int cap,
+                                            Status* status) {
   extern __shared__ __align__(16) unsigned char s_core[];
   const int lane = threadIdx.x & 31;
   const int core = gc_core_size(ctl, cap);
@@ -841,15 +898,15 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const
   const int seg = gc_core_seg(cap);  // row entries staged at a time
   unsigned char* wbase = s_core + gc_core_colour_bytes(cap) + (size_t)(threadIdx.x >> 5) * gc_core_warp_bytes(seg);
   CoreStage stg;
-  stg.bars = reinterpret_cast<unsigned long long*>(wbase);
   stg.base = reinterpret_cast<unsigned short*>(wbase + 2 * sizeof(unsigned long long));
   stg.seg = seg;
-  unsigned char* marks = reinterpret_cast<unsigned char*>(stg.base + 2 * seg);
+  unsigned char* const marks = stg.marks();
+  unsigned short* pend = reinterpret_cast<unsigned short*>(marks + kMarkBytes);
   for (int r = threadIdx.x; r < core; r += kCoreThreads) col_st(&col_s[r], kUncoloured);
   gc_core_clear(marks, kMarkBytes - 1);
   if (lane == 0) {
-    mbar_init(stg.bars);
-    mbar_init(stg.bars + 1);
+    mbar_init(stg.bar(0));
+    mbar_init(stg.bar(1));
     mbar_fence_init();
   }
   __syncthreads();
@@ -858,16 +915,16 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const
   // Row j of this warp is rank warp + cwarps j; lane L holds the row record
   // of row jb + L (records are fetched 32 rows at a time).
   int jb = -32;
-  int4 rec = make_int4(0, 0, -1, 0);
-  auto row_of = [&](int j) -> int4 {  // all lanes call
+  int3 rec = make_int3(0, 0, -1);
+  auto row_of = [&](int j) -> int3 {  // all lanes call
     if ((j & ~31) != jb) {
       jb = j & ~31;
       const int r = warp + cwarps * (jb + lane);
-      rec = r < core ? rowinfo[r] : make_int4(0, 0, -1, 0);  // race-free: not written in this launch
+      const int4 x = r < core ? rowinfo[r] : make_int4(0, 0, -1, 0);  // race-free: not written in this launch
+      rec = make_int3(x.x, x.y, x.z);
     }
     const int src = j & 31;
-    return make_int4(__shfl_sync(kFull, rec.x, src), __shfl_sync(kFull, rec.y, src), __shfl_sync(kFull, rec.z, src),
-                     0);
+    return make_int3(__shfl_sync(kFull, rec.x, src), __shfl_sync(kFull, rec.y, src), __shfl_sync(kFull, rec.z, src));
   };
   // Byte that takes the colours which cannot matter: h entries leave one of the
   // colours 0 .. h free.  So a row marks, searches and clears h + 2 bytes at most.
@@ -879,36 +936,38 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const
     return c == kUncoloured;
   };
   const int nrows = core > warp ? (core - warp + cwarps - 1) / cwarps : 0;
-  int b = 0;  // buffer holding (or about to hold) the segment to scan next
+  // The first segment of the warp's next row with entries behind row j, into buffer
+  // q (rows without any are skipped).
+  auto next_row = [&](int j, int q) {
+    for (int jn = j + 1; jn < nrows; jn++) {
+      const int3 nx = row_of(jn);
+      if (nx.y > 0) {
+        stg.issue(q, nl2, nx.x, min(seg, nx.y));
+        return;
+      }
+    }
+  };
+  int b = 0;  // buffer of the next row's first segment
+  next_row(-1, b);
   for (int j = 0; j < nrows; j++) {
     const int r = warp + cwarps * j;
-    const int4 row = row_of(j);
+    const int3 row = row_of(j);
     const int unit = row.x, h = row.y, v = row.z;
     beyond = (unsigned)min(h + 1, kWin);
-    // The first segment of the warp's next row with entries into buffer q (rows
-    // without any are skipped).
-    auto next_row = [&](int q) {
-      for (int jn = j + 1; jn < nrows; jn++) {
-        const int4 nx = row_of(jn);
-        if (nx.y > 0) {
-          stg.issue(q, nl2, nx.x, min(seg, nx.y));
-          return;
-        }
-      }
-    };
     bool stalled = false;
     int from = 0;  // all colours below are taken
-    // Two segments at a time are scanned before any undecided entry is waited for:
-    // a scan behind the last neighbour's colour would lie on the chain, and costs
-    // microseconds among the other warps' polls.
+    int np = 0;    // entries in `pend`
+    // All of a row is scanned before any undecided entry is waited for: a scan
+    // behind the last neighbour's colour would lie on the chain, and costs
+    // microseconds among the other warps' polls.  Two segments at a time; of a
+    // longer row the undecided ones so far go to a list (kWide), if it holds them.
     for (int off = 0; off < h && !stalled; off += 2 * seg) {
       const int f = unit + off / 8, second = h - off - seg;  // entries behind the first of the two
-      if (stg.first(b) != f) stg.issue(b, nl2, f, min(seg, h - off));  // not prefetched
       __syncwarp();  // buffer b ^ 1 was scanned by every lane
       if (second > 0)
         stg.issue(b ^ 1, nl2, f + seg / 8, min(seg, second));
       else
-        next_row(b ^ 1);
+        next_row(j, b ^ 1);
       unsigned open0 = 0, open1 = 0;
       for (int part = 0; part <= (second > 0); part++) {
         const int q = b ^ part, l = min(seg, h - off - part * seg);
@@ -917,7 +976,6 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const
           stalled = true;
           break;
         }
-        stg.set_first(q, -1);
         const unsigned short* sg = stg.buf(q);
         // eight entries a lane and step; bit 8 s + k of `wait`: entry k of the
         // lane's step s is undecided
@@ -947,6 +1005,10 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const
         else
           open0 = wait;
       }
+      if (kWide && second > seg) {
+        const int kept = gc_core_keep(open0, open1, stg.buf(b), stg.buf(b ^ 1), pend, np);
+        if (kept >= 0) np = kept, open0 = open1 = 0;
+      }
       // Wait for the undecided ones: a lane goes round its own and takes whichever
       // is decided, so that none holds up the others.  (R-MAT-22, core: the ranks
       // in a list that the lanes share evenly, and the colours handed to registers
@@ -954,7 +1016,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const
       unsigned spins = 0, turn = 0;
       unsigned long long t0 = 0;
       __syncwarp();
-      if (h >= kFromRow) from = gc_core_mex(marks, 0, from, (int)beyond);
+      if (h >= kFromRow && (!kWide || second <= seg)) from = gc_core_mex(marks, 0, from, (int)beyond);
       if (from < 0) from = kWin;
       for (int part = 0; part <= (second > 0) && !stalled; part++) {
         const unsigned short* sg = stg.buf(b ^ part);
@@ -983,6 +1045,7 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const
       else if (second > seg && !stalled)
         stg.issue(b, nl2, f + seg / 4, min(seg, second - seg));
     }
+    if (kWide && np > 0 && !stalled) stalled = gc_core_settle(pend, np, col_s, marks, beyond, r, status);
     if (stalled) {
       stg.drain();
       break;
@@ -997,11 +1060,21 @@ __global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const
     __syncwarp();
     // behind the publication, off the chain
     gc_core_clear(marks, (int)beyond);
-    if (h > 0 && (h - 1) / seg % 2 == 1) next_row(b);  // both buffers were the row's own
+    if (h > 0 && (h - 1) / seg % 2 == 1) next_row(j, b);  // both buffers were the row's own
   }
   // a CTA's shared memory must outlive every store the others make into it:
   // every warp, done or given up (each wait is bounded), meets here
   if (ctas > 1) cluster_sync();
+}
+
+__global__ void __launch_bounds__(kCoreThreads, 1) gc_core(const int* nl2, const int4* rowinfo,
+                                                           int* __restrict__ color, const GCCtl* ctl,
+                                                           int cap, Status* __restrict__ status) {
+  dep_wait();
+  if (16LL * ld(&ctl->nwide) > gc_core_size(ctl, cap))  // the same for all CTAs
+    gc_core_run<true>(nl2, rowinfo, color, ctl, cap, status);
+  else
+    gc_core_run<false>(nl2, rowinfo, color, ctl, cap, status);
 }
 
 __global__ void __launch_bounds__(kTPB) gc_pull(int n, const int* __restrict__ nindex, const int* __restrict__ nl2,

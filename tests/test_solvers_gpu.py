@@ -830,6 +830,33 @@ def test_gc_of_cliques_around_the_windows_of_colours(ecl, orc, n):
         assert np.array_equal(ecl.gc(d), orc.gc(g))
 
 
+def multipartite(ecl, n, parts):
+    """All pairs of n vertices in different parts."""
+    u, v = np.triu_indices(n, 1)
+    q = u % parts != v % parts
+    return directed(ecl, n, np.concatenate([u[q], v[q]]), np.concatenate([v[q], u[q]]))
+
+
+@pytest.mark.parametrize("n,parts", [(2300, 1150), (3000, 40), (4200, 2), (4500, 700), (6200, 31)])
+def test_gc_of_rows_of_more_than_two_segments(ecl, orc, n, parts):
+    """Core rows of up to six segments of 1024 entries, in cores on both sides of
+    the rule that keeps a list of their undecided entries."""
+    g = multipartite(ecl, n, parts)
+    assert np.array_equal(ecl.gc(g), orc.gc(g))
+    old = ecl.set_tune(gc_core_ranks=36864)  # shorter segments
+    try:
+        assert np.array_equal(ecl.gc(g), orc.gc(g))
+    finally:
+        ecl.set_tune(old)
+
+
+def test_gc_of_long_rows_is_not_scanned_on_the_chain(ecl):
+    """Rows of up to four segments cost what shorter ones do for each entry (a
+    segment scanned behind the last neighbour's colour: four times and more)."""
+    short, long_ = (best_ms(ecl, multipartite(ecl, n, 1000).to_device(), "gc") for n in (2000, 4000))
+    assert long_ < 3.3 * short
+
+
 def test_gc_of_cliques_costs_a_hop_for_each_colour(ecl):
     """Twice the vertices are twice the hops, not eighteen times the time."""
     small, large = (best_ms(ecl, clique(ecl, n).to_device(), "gc") for n in (1000, 2000))
