@@ -47,6 +47,14 @@ constexpr int kLaneMax = 16;
 // 46 / 32 / 33 / 32 us, G(3 M, 36 M) 439 / 371 / 367 / 377, R-MAT-22 320 / 331 /
 // 323 / 341.
 constexpr int kManyMid = 8;
+// Vertices of a warp's group: 32, and down to kSmallGroup where the lists have
+// more than kDenseRow entries on average and groups of 32 would leave warps of
+// the device without any, as a group's lists, a dozen steps of the whole warp
+// each, run one after another.  32 -> this: a complete bipartite graph of 2 x 1500
+// vertices 575 -> 119 us (whole solve), a clique of 1200 326 -> 93, 30 cliques of
+// 300 135 -> 69; with lists of 100 entries, 100 k of them, 156 -> 167.
+constexpr int kSmallGroup = 4;
+constexpr int kDenseRow = 128;
 constexpr int kBatch = 4;  // list entries per lane whose loads are issued together
 constexpr unsigned kIn = 0xfe;
 
@@ -213,23 +221,25 @@ __device__ __forceinline__ int mis_scan_warp(int v, unsigned b, int& pos, int en
 // Without items (kItems false: a workspace of one byte a vertex) every sweep
 // goes through the groups again and scans from the start: R-MAT-22 330 -> 560 us.
 //
-// A warp's g-th group is the vertices 32 (g nwarps + warp) ..+31, and its g-th
-// 32 items lie at the same places, so the warps' lists share one array of n
-// (rounded up) items and need no counters.  Bound by the latency of the chains
-// of decisions: DRAM and L2 are far from busy.  Measured, groups of 32 vertices
-// swept and scanned from the start until decided -> items: R-MAT-22 525 -> 297
-// us, 500 k vertices 169 -> 80, 1000 vertices (fewer blocks) 40 -> 16; with the
-// long lists scanned in the first sweep as well, R-MAT-22 525.
+// A warp's g-th group is the vertices group (g nwarps + warp) .. + group - 1 (group:
+// a power of two, at most 32), and its g-th `group` items lie at the same places,
+// so the warps' lists share one array of n (rounded up) items and need no
+// counters.  Bound by the latency of the chains of decisions: DRAM and L2 are far
+// from busy.  Measured, groups of 32 vertices swept and scanned from the start
+// until decided -> items: R-MAT-22 525 -> 297 us, 500 k vertices 169 -> 80, 1000
+// vertices (fewer blocks) 40 -> 16; with the long lists scanned in the first sweep
+// as well, R-MAT-22 525.
 template <bool kItems>
 __global__ void __launch_bounds__(kTPB) mis_run(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, unsigned* __restrict__ st4,
                                                 int4* __restrict__ items, Status* __restrict__ status, int max_sweeps,
-                                                int lane_max) {
+                                                int lane_max, int group) {
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
+  const int gshift = __ffs(group) - 1;
   int kept = 0;  // items of this warp's list
-  auto slot = [&](int k) -> long long { return ((long long)(k >> 5) * nwarps + warp) * 32 + (k & 31); };
+  auto slot = [&](int k) -> long long { return (((long long)(k >> gshift) * nwarps + warp) << gshift) + (k & (group - 1)); };
   // Scans on for the lanes with `go` (entries [pos, end) of v), carries the
   // verdicts out and keeps the waiting ones.  All lanes call.
   auto advance = [&](bool go, bool wait, int v, unsigned b, int pos, int end, int blocker) {
@@ -271,8 +281,8 @@ __global__ void __launch_bounds__(kTPB) mis_run(int n, int m, const int* __restr
   };
   int sweep = 0;
   for (bool first = true;; first = false) {  // once; without items, until all are decided
-    for (int base = warp * 32; base < n; base += nwarps * 32) {
-      const int v = base + lane;
+    for (long long base = (long long)warp * group; base < n; base += (long long)nwarps * group) {
+      const int v = lane < group && base + lane < n ? (int)(base + lane) : n;
       unsigned b = 0;
       if (v < n) b = byte_of(ld(&st4[v >> 2]), v);
       const bool und = (b & 1u) != 0;
@@ -374,9 +384,12 @@ ecl_status mis_enqueue(const GraphDev& g, unsigned char* out, char* ws, size_t w
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, run, kTPB, 0) != cudaSuccess || occ < 1)
     return ECL_ERR_CUDA;
   const int full = dev.sms * std::min(occ, dev.max_threads_per_sm / kTPB);
-  ECL_CUDA_TRY(launch_cooperative(run, std::min(full, (g.n - 1) / kTPB + 1), kTPB, stream, g.n,
+  int group = 32;
+  if (g.m / g.n > kDenseRow)  // kSmallGroup says why
+    while (group > kSmallGroup && g.n / group < full * (kTPB / 32)) group /= 2;
+  ECL_CUDA_TRY(launch_cooperative(run, std::min(full, (g.n - 1) / (group * (kTPB / 32)) + 1), kTPB, stream, g.n,
                                   g.m, g.nindex, g.nlist, st4, items, status, max_sweeps,
-                                  bins_of(dev, Bins{kLaneMax, kBinChunk}).lane));
+                                  bins_of(dev, Bins{kLaneMax, kBinChunk}).lane, group));
   mark();
   ECL_LAUNCH_NEXT(mis_emit, grid, kTPB, 0, stream, g.n, st4, out);
   mark();

@@ -872,3 +872,32 @@ def test_gc_order_of_equal_degrees(ecl, orc, n):
     ring.sort(axis=1)
     g = ecl.Graph((2 * np.arange(n + 1)).astype(np.int32), ring.ravel().astype(np.int32), None, True)
     assert np.array_equal(ecl.gc(g), orc.gc(g))
+
+
+def cliques(ecl, count, size, tail=0):
+    """`count` cliques of `size` vertices, and `tail` vertices without entries."""
+    u, v = np.triu_indices(size, 1)
+    base = np.repeat(np.arange(count) * size, u.size)
+    u, v = np.tile(u, count) + base, np.tile(v, count) + base
+    g = directed(ecl, count * size + tail, np.concatenate([u, v]), np.concatenate([v, u]))
+    g.symmetric = True
+    return g
+
+
+# average degrees on both sides of a lane's list (16) and of 128; groups of 4, 8, 16 and 32 vertices a warp,
+# the last one whole and not
+@pytest.mark.parametrize("count,size,tail", [
+    (1, 18, 0), (3, 17, 1), (3, 18, 1), (4300, 18, 2), (4300, 18, 3), (8500, 18, 5), (17000, 18, 11), (1, 129, 0),
+    (1, 130, 0), (3, 131, 0), (3, 131, 2), (250, 140, 5), (500, 140, 9), (900, 133, 3)])
+@pytest.mark.parametrize("code", ["cc", "mis", "scc"])
+def test_small_groups_of_vertices(ecl, orc, code, count, size, tail):
+    g = cliques(ecl, count, size, tail)
+    assert np.array_equal(getattr(ecl, code)(g), getattr(orc, code)(g))
+
+
+def test_mis_of_small_dense_graphs_uses_the_whole_device(ecl):
+    """With 32 vertices to a warp, 94 warps scanned the 3000 lists: five times as long."""
+    u, v = np.repeat(np.arange(1500), 1500), 1500 + np.tile(np.arange(1500), 1500)
+    g = directed(ecl, 3000, np.concatenate([u, v]), np.concatenate([v, u]))
+    g.symmetric = True
+    assert best_ms(ecl, g.to_device(), "mis") < 8 * best_ms(ecl, cliques(ecl, 40, 40).to_device(), "mis")
