@@ -12,7 +12,8 @@
 // further down: link two entries of every list, find the giant component,
 // then skip every list inside it):
 //  * cc_init   - parent[v] = first smaller neighbour among the first
-//                kInitScan entries, kInitHops times over (free hooks).
+//                kInitScan entries (free hooks; the sampling path goes two
+//                such steps).
 //  * cc_hook   - one pass over the vertices, 32 per warp.  Lists of <= 16
 //                entries are walked by their own lane; lists of up to
 //                2048 entries are walked by the whole warp (ballot loop,
@@ -42,6 +43,12 @@ constexpr int kTPB = 256;
 constexpr Bins kCCBins{16, 2048};
 constexpr int kInitScan = 8;   // entries cc_init looks at for a first smaller neighbour
 constexpr int kInitHops = 2;   // hops of cc_init (R-MAT-22, whole solve: 1 hop 0.244 ms, 2 0.227, 4 0.217; G(3 M, 12 M): 0.354, 0.369, 0.396)
+// ... and where every entry is linked afterwards, with nothing sampled first: two
+// hops leave a vertex and the one between in two trees, whose link is one more
+// that climbs through the hubs' words.  1 hop / 2 (median): 300 k vertices, 3 M
+// entries to power-law ends 0.69 / 0.94 ms, from such 0.56 / 0.69; 10 M entries of
+// 1 M vertices 0.87 / 0.81 and 0.71 / 0.68; uniform ends, 3 M entries 0.89 / 0.65, 8 M 0.36 / 0.37.
+constexpr int kInitHopsAll = 1;
 
 // Whether this solve is not wanted after all: an earlier launch has left
 // something other than 0 at `off` (nullptr: it always is).
@@ -148,7 +155,7 @@ __device__ __forceinline__ int cc_first_smaller(int v, int beg, int end, const i
   return v;
 }
 
-// parent[v] = the vertex kInitHops first-smaller-neighbour hops from v.  The
+// parent[v] = the vertex `hops` first-smaller-neighbour hops from v.  The
 // hops go through the CSR, which nothing writes, so L1 serves the rows of the
 // hubs that most vertices of a power-law graph hop to; the same steps through
 // parent[] afterwards queue at the hubs' words.
@@ -156,7 +163,7 @@ __device__ __forceinline__ int cc_first_smaller(int v, int beg, int end, const i
 // [0, m]) raises ECL_ERR_BAD_GRAPH and is treated as empty by every kernel.
 __global__ void __launch_bounds__(kTPB) cc_init(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, int* __restrict__ parent,
-                                                CCCounters* ctr, const u64* off,
+                                                CCCounters* ctr, int hops, const u64* off,
                                                 Status* __restrict__ status) {
   dep_wait();
   if (cc_off(off)) return;
@@ -168,7 +175,7 @@ __global__ void __launch_bounds__(kTPB) cc_init(int n, int m, const int* __restr
       beg = end = 0;
     }
     int p = cc_first_smaller(v, beg, end, nlist);
-    for (int h = 1; h < kInitHops && p != v; h++) {
+    for (int h = 1; h < hops && p != v; h++) {
       cc_row(nindex, p, m, beg, end);
       const int q = cc_first_smaller(p, beg, end, nlist);
       if (q == p) break;
@@ -578,7 +585,7 @@ ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, 
   const Bins bins = bins_of(dev, kCCBins);
   const int cap = chunk_capacity(g.m, kMinChunk);  // cc_layout sized the records for the smallest chunk
   if (g.flags & ECL_GRAPH_SYMMETRIC) {
-    ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, off, status);
+    ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, kInitHops, off, status);
     ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, Giants{}, nullptr, off);
     if (g.n >= kSplitSample) {
       ECL_LAUNCH_NEXT(cc_sample<0>, dev.grid_blocks(kTPB, g.n / 8, 0), kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent,
@@ -607,7 +614,7 @@ ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, 
     mark();
     return ECL_OK;
   }
-  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, nullptr, status);
+  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, kInitHopsAll, nullptr, status);
   mark();
   ECL_LAUNCH_NEXT(cc_hook, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, chunks, cap, bins, ctr, status);
   mark();
@@ -727,7 +734,7 @@ extern "C" ecl_status ecl_cc_noalloc(int32_t nodes, int32_t edges, const int32_t
   // the counters (adjacent, at the front of the array) before every solve.
   ECL_CUDA_TRY(cudaMemsetAsync(base, 0, kStatusBytes + sizeof(CCCounters), stream));
   const int grid = dev.grid_blocks(kTPB, nodes, edges);
-  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, ctr, nullptr, status);
+  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, ctr, kInitHopsAll, nullptr, status);
   ECL_LAUNCH_NEXT(cc_hook, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, chunks,
              chunk_capacity(edges, kCCBins.chunk), kCCBins, ctr, status);
   ECL_LAUNCH_NEXT(cc_chunks, grid, kTPB, 0, stream, nodes, nindex, nlist, label, chunks,
