@@ -901,3 +901,9 @@ def test_mis_of_small_dense_graphs_uses_the_whole_device(ecl):
     g = directed(ecl, 3000, np.concatenate([u, v]), np.concatenate([v, u]))
     g.symmetric = True
     assert best_ms(ecl, g.to_device(), "mis") < 8 * best_ms(ecl, cliques(ecl, 40, 40).to_device(), "mis")
+
+
+def test_cc_of_small_dense_graphs_uses_the_whole_device(ecl):
+    """As many entries in long lists as in short ones; the long ones took twice as long."""
+    few, many = (best_ms(ecl, cliques(ecl, c, k).to_device(), "cc") for c, k in ((30, 300), (2000, 40)))
+    assert few < 1.5 * many
