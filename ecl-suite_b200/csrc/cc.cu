@@ -155,15 +155,16 @@ __device__ __forceinline__ int cc_first_smaller(int v, int beg, int end, const i
   return v;
 }
 
-// parent[v] = the vertex `hops` first-smaller-neighbour hops from v.  The
+// parent[v] = the vertex kHops first-smaller-neighbour hops from v.  The
 // hops go through the CSR, which nothing writes, so L1 serves the rows of the
 // hubs that most vertices of a power-law graph hop to; the same steps through
 // parent[] afterwards queue at the hubs' words.
 // Also checks the CSR rows once: a malformed row (end < beg, or outside
 // [0, m]) raises ECL_ERR_BAD_GRAPH and is treated as empty by every kernel.
+template <int kHops>
 __global__ void __launch_bounds__(kTPB) cc_init(int n, int m, const int* __restrict__ nindex,
                                                 const int* __restrict__ nlist, int* __restrict__ parent,
-                                                CCCounters* ctr, int hops, const u64* off,
+                                                CCCounters* ctr, const u64* off,
                                                 Status* __restrict__ status) {
   dep_wait();
   if (cc_off(off)) return;
@@ -175,7 +176,7 @@ __global__ void __launch_bounds__(kTPB) cc_init(int n, int m, const int* __restr
       beg = end = 0;
     }
     int p = cc_first_smaller(v, beg, end, nlist);
-    for (int h = 1; h < hops && p != v; h++) {
+    for (int h = 1; h < kHops && p != v; h++) {
       cc_row(nindex, p, m, beg, end);
       const int q = cc_first_smaller(p, beg, end, nlist);
       if (q == p) break;
@@ -488,8 +489,8 @@ __global__ void __launch_bounds__(kTPB) cc_rest(int n, int m, const int* __restr
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * kTPB + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * kTPB) >> 5;
-  for (long long base = (long long)warp * group; base < n; base += (long long)nwarps * group) {
-    const int v = lane < group && base + lane < n ? (int)(base + lane) : n;
+  for (unsigned base = warp * group; base < (unsigned)n; base += nwarps * group) {
+    const int v = lane < group ? (int)min(base + lane, (unsigned)n) : n;
     int beg = 0, end = 0;
     if (v < n && !ing[v]) cc_row(nindex, v, m, beg, end);  // race-free: not written in this launch
     const int deg = end - beg;
@@ -592,7 +593,7 @@ ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, 
   const Bins bins = bins_of(dev, kCCBins);
   const int cap = chunk_capacity(g.m, kMinChunk);  // cc_layout sized the records for the smallest chunk
   if (g.flags & ECL_GRAPH_SYMMETRIC) {
-    ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, kInitHops, off, status);
+    ECL_LAUNCH_NEXT(cc_init<kInitHops>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, off, status);
     ECL_LAUNCH_NEXT(cc_flatten<kPlain>, flatten_blocks(dev, g.n), kTPB, 0, stream, g.n, parent, Giants{}, nullptr, off);
     if (g.n >= kSplitSample) {
       ECL_LAUNCH_NEXT(cc_sample<0>, dev.grid_blocks(kTPB, g.n / 8, 0), kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent,
@@ -624,7 +625,7 @@ ecl_status cc_enqueue(const GraphDev& g, int* parent, char* ws, Status* status, 
     mark();
     return ECL_OK;
   }
-  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, kInitHopsAll, nullptr, status);
+  ECL_LAUNCH_NEXT(cc_init<kInitHopsAll>, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, ctr, nullptr, status);
   mark();
   ECL_LAUNCH_NEXT(cc_hook, grid, kTPB, 0, stream, g.n, g.m, g.nindex, g.nlist, parent, chunks, cap, bins, ctr, status);
   mark();
@@ -744,7 +745,7 @@ extern "C" ecl_status ecl_cc_noalloc(int32_t nodes, int32_t edges, const int32_t
   // the counters (adjacent, at the front of the array) before every solve.
   ECL_CUDA_TRY(cudaMemsetAsync(base, 0, kStatusBytes + sizeof(CCCounters), stream));
   const int grid = dev.grid_blocks(kTPB, nodes, edges);
-  ECL_LAUNCH_NEXT(cc_init, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, ctr, kInitHopsAll, nullptr, status);
+  ECL_LAUNCH_NEXT(cc_init<kInitHopsAll>, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, ctr, nullptr, status);
   ECL_LAUNCH_NEXT(cc_hook, grid, kTPB, 0, stream, nodes, edges, nindex, nlist, label, chunks,
              chunk_capacity(edges, kCCBins.chunk), kCCBins, ctr, status);
   ECL_LAUNCH_NEXT(cc_chunks, grid, kTPB, 0, stream, nodes, nindex, nlist, label, chunks,

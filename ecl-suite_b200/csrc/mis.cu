@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(kTPB) mis_run(int n, int m, const int* __restr
   };
   int sweep = 0;
   for (bool first = true;; first = false) {  // once; without items, until all are decided
-    for (long long base = (long long)warp * group; base < n; base += (long long)nwarps * group) {
-      const int v = lane < group && base + lane < n ? (int)(base + lane) : n;
+    for (unsigned base = warp * group; base < (unsigned)n; base += nwarps * group) {
+      const int v = lane < group ? (int)min(base + lane, (unsigned)n) : n;
       unsigned b = 0;
       if (v < n) b = byte_of(ld(&st4[v >> 2]), v);
       const bool und = (b & 1u) != 0;

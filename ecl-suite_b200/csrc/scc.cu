@@ -241,6 +241,9 @@ constexpr int kGiantPatience = 16;
 // as a graph without hubs has more levels for its size.  With hubs: R-MAT with
 // 0.45 M entries 229 -> 227 us, 1.05 M 266 -> 250, 1.8 M 363 -> 261.  Without:
 // G(300 k, 1.2 M) 441 -> 528, G(600 k, 2.4 M) 659 -> 595, G(1 M, 4 M) 1078 -> 711.
+// What is lost where it finds nothing, or half of what there is: an acyclic graph
+// of 300 k vertices and 3 M random edges 907 -> 1002, two random graphs of 300 k
+// vertices side by side 655 -> 849, 3 M edges from power-law ends 562 -> 643.
 constexpr int kGiantEntries = 1 << 20;
 constexpr int kGiantFlat = 1 << 21;
 constexpr int kGiantHub = 32;
